@@ -1,4 +1,5 @@
-/* batch.cu -- many biome-map requests of uneven size in one persistent launch.
+/* batch.cu -- many biome-map requests of uneven size in a few persistent launches: Overworld requests under the ENGINE
+ * rule go to the tile kernels of owtile.cu, one per branch, everything else to k_batch here.
  *
  * A request is (world: version + dimension + preset, seed, quart region qx0..qx0+nx-1 x qz0..qz0+nz-1 at
  * quart y, tie rule).  The host splits every request into tiles -- 128 quart cells (8 x 16; the autotuner
@@ -6,8 +7,7 @@
  * and numbers them.  k_batch runs one CTA per SM slot for the whole batch; each CTA takes the next tile
  * from a device counter (the work queue), finds its request among the requests' first-tile numbers, stages
  * that request's seed lattices in shared memory when they differ from the previous tile's, and computes the
- * tile (for a double-branch Overworld tile, first the shift noises' per-column and per-row splits).  Uneven
- * requests therefore cost no idle SMs and no per-request launches.
+ * tile.  Uneven requests therefore cost no idle SMs and no per-request launches.
  *
  * The seed lattices of every (world, seed) of the batch are built beforehand by k_setup_list_* into a
  * state pool (the served form keeps that pool across batches as a device cache).
@@ -21,6 +21,7 @@
 #include <stdint.h>
 
 #include "batch.h"
+#include "batchdev.cuh"
 #include "climate.cuh"
 #include "endtile.cuh"
 #include "launch.h"
@@ -129,75 +130,40 @@ __global__ void __launch_bounds__(LNT) k_setup_list_end(const MgSetupEntry *__re
 }
 
 /* ---------------------------------------------------------------- the persistent batch kernel */
-/* The lattices of an Overworld/Nether request (with an Overworld tile's shift table) and the
- * End's scratch are never live in the same tile, so they share storage: 21 KB per CTA, which leaves the
- * register budget as the occupancy limit (up to 9 CTAs per SM). */
+/* The lattices of an Overworld/Nether request and the End's scratch are never live in the same tile, so they share
+ * storage: 17 KB per CTA, which leaves the register budget as the occupancy limit (up to 9 CTAs per SM). */
 struct BatchEnd {
     uint8_t endp[256];
     EndTile tile;
 };
-/* the lattices of an Overworld/Nether request, and the shift table of an Overworld tile (double or float
- * branch) */
-struct BatchLat {
-    MgLattice lat[MG_MAX_TABLES];
-    union {
-        ShiftTable<8, BNT / 8> shift;   /* double-branch Overworld tile */
-        ShiftTableF<8, BNT / 8> shiftf; /* float-branch Overworld tile */
-    };
-};
 struct BatchSmem {
     union {
-        BatchLat o;
+        MgLattice lat[MG_MAX_TABLES];
         BatchEnd end;
     };
-    WarpTreeScratch wt[BNT / 32]; /* each warp's R-tree candidate list (Overworld, ENGINE rule) */
-    PendSink sink;  /* where double-branch Overworld cells left to the exact evaluation are recorded */
-    double depth_g; /* the double-branch Overworld tile's depth gradient (depth_grad_d) */
     int tile, req, state;
 };
 
-/* a biome id to the output: written once and never read back by the kernel, so stored with the streaming
- * (evict-first) policy, which keeps the streamed output from evicting the threads' local memory from L2 */
-__device__ __forceinline__ void put_id(uint8_t *p, int v) { __stcs(p, (unsigned char)v); }
-
-/* tab, tabf: the tile's shift table (double- or float-branch Overworld, ENGINE rule) or null; g: with the
- * double branch's table, the tile's depth gradient.  Each code path's cells (and the End's tiles, batch_end) are a function of their own, out of
- * line: the persistent kernel is then a dispatcher, and each path's registers are allocated for that path
- * alone (measured 0.3 % faster on the mixed batch than all paths inlined into the kernel). */
+/* The cells of an Overworld or Nether tile.  Each code path's cells (and the End's tiles, batch_end) are a function of their
+ * own, out of line: the persistent kernel is then a dispatcher, and each path's registers are allocated for that path
+ * alone. */
 template <bool FM, int DIM, int TILE_W>
-__device__ __noinline__ void batch_cells(const MgWorldDesc &W, const MgSpline &S, const MgLattice *T,
-                                            const MgTreeNode *tree, const MgBatchReq &R, int tx0, int tz0,
-                                            const ShiftTable<8, BNT / 8> *tab, const ShiftTableF<8, BNT / 8> *tabf,
-                                            double g, WarpTreeScratch *wt, const PendSink *sink, uint8_t *out) {
+__device__ __noinline__ void batch_cells(const MgWorldDesc &W, const MgSpline &S, const MgLattice *T, const MgTreeNode *tree,
+                                         const MgBatchReq &R, int tx0, int tz0, uint8_t *out) {
     const int col = threadIdx.x % TILE_W, row = threadIdx.x / TILE_W;
     const int ix = tx0 + col, iz = tz0 + row;
-    const bool in = ix < R.nx && iz < R.nz;
+    if (ix >= R.nx || iz >= R.nz) return;
     const int qx = R.qx0 + ix, qz = R.qz0 + iz;
+    int b;
     if (R.tie == MG_TIE_CHUNK_CELL) { /* the request's rule: the same for the whole CTA */
-        if (in) put_id(out + R.out_off + (size_t)iz * R.nx + ix, cell_chunk<FM, DIM>(W, S, T, tree, qx, R.qy, qz));
-        return;
-    }
-    int32_t tg[6] = {0, 0, 0, 0, 0, 0};
-    const int64_t o = R.out_off + (int64_t)iz * R.nx + ix;
-    if (!FM && DIM == MG_OVERWORLD && TILE_W == 8 && tab) {
-        /* a cell whose screen left a value to the exact evaluation is recorded for the second launch (the
-         * double branch's tree search is per lane, so the lane may leave here) */
-        if (in && !climate_ow_d_tab_defer(W, S, T, *tab, col, row, qx, R.qy, qz, g, tg, sink, o)) return;
-    } else if (FM && DIM == MG_OVERWORLD && TILE_W == 8 && tabf) {
-        if (in) climate_ow_f_tab(W, S, T, *tabf, col, row, qx, R.qy, qz, tg);
-    } else if (in) {
-        cell_target<FM, DIM>(W, S, T, qx, R.qy, qz, tg);
-    }
-    int leaf;
-    /* one pruned walk of the tree per warp of 8 x 4 cells for wide trees (built only into the float branch's
-     * code: the double branch's versions, 26.1 and 26.2, have 6 children per node) */
-    if (FM && DIM == MG_OVERWORLD && W.tree_fanout >= MG_WARP_TREE_FANOUT) {
-        leaf = tree_search_warp(tree, tg, in, wt[threadIdx.x >> 5]);
+        b = cell_chunk<FM, DIM>(W, S, T, tree, qx, R.qy, qz);
     } else {
+        int32_t tg[6];
+        cell_target<FM, DIM>(W, S, T, qx, R.qy, qz, tg);
         uint64_t d;
-        leaf = in ? tree_search(tree, tg, -1, d) : -1;
+        b = tree[tree_search(tree, tg, -1, d)].biome;
     }
-    if (in) put_id(out + o, tree[leaf].biome);
+    put_id(out + R.out_off + (size_t)iz * R.nx + ix, b);
 }
 
 /* End tile: chunks [cx0, cx0 + END_TC) x [cz0, cz0 + END_TC) counted from the chunk of the request's
@@ -216,39 +182,16 @@ __device__ __noinline__ void batch_end(const MgWorldDesc &W, BatchSmem &sm, cons
     }
 }
 
-/* The request holding tile `tile`: the last r with reqs[r].tile0 <= tile (tile0 is non-decreasing and
- * reqs[0].tile0 == 0), found by the 32 lanes of a warp in rounds of 32 probes -- the probes that are <= tile
- * form a prefix, whose length narrows the range 32-fold -- so 3 rounds of loads for 10,000 requests where a
- * binary search by one thread made 14 dependent ones while the CTA waited. */
-__device__ __forceinline__ int find_req(const MgBatchReq *__restrict__ reqs, int nreq, long long tile) {
-    const int lane = threadIdx.x & 31;
-    int lo = 0, hi = nreq - 1;
-    while (hi > lo) {
-        const int step = (hi - lo + 31) / 32;
-        const int p = lo + (lane + 1) * step;
-        const unsigned m = __ballot_sync(0xFFFFFFFFu, p <= hi && reqs[p].tile0 <= tile);
-        lo += __popc(m) * step;
-        hi = min(hi, lo + step - 1);
-    }
-    return lo;
-}
-
 /* TILE_W: tile width in cells (tiles are 128 cells); MINB: resident CTAs per SM the register allocation
  * is sized for (6: 80 registers, 7: 72, 8: 64, 9: 56) */
 template <int TILE_W, int MINB>
 __global__ void __launch_bounds__(BNT, MINB) k_batch(const MgWorldDesc *__restrict__ worlds, const MgTreeNode *const *__restrict__ trees,
                                                const MgBatchReq *__restrict__ reqs, int nreq, long long ntiles,
                                                const MgLattice *__restrict__ pool, unsigned long long *__restrict__ counter,
-                                               MgPending *__restrict__ pend, long long pend_cap,
                                                uint8_t *__restrict__ out) {
     extern __shared__ uint4 smem_raw[];
     BatchSmem &sm = *reinterpret_cast<BatchSmem *>(smem_raw);
-    if (threadIdx.x == 0) {
-        sm.state = -1;
-        sm.sink.rec = pend;
-        sm.sink.count = counter + 1;
-        sm.sink.cap = pend ? pend_cap : 0;
-    }
+    if (threadIdx.x == 0) sm.state = -1;
     for (;;) {
         __syncthreads();
         if (threadIdx.x < 32) { /* warp 0 takes the next tile and finds its request */
@@ -259,10 +202,6 @@ __global__ void __launch_bounds__(BNT, MINB) k_batch(const MgWorldDesc *__restri
             if (threadIdx.x == 0) {
                 sm.tile = (int)(r >= 0 ? tile - reqs[r].tile0 : -1);
                 sm.req = r;
-                if (r >= 0) {
-                    sm.sink.world = reqs[r].world;
-                    sm.sink.state = reqs[r].state;
-                }
             }
         }
         __syncthreads();
@@ -278,7 +217,7 @@ __global__ void __launch_bounds__(BNT, MINB) k_batch(const MgWorldDesc *__restri
                 for (int i = threadIdx.x; i < 256; i += BNT) sm.end.endp[i] = pool[R.state].p[i];
             } else {
                 const uint4 *a = reinterpret_cast<const uint4 *>(pool + R.state);
-                uint4 *b = reinterpret_cast<uint4 *>(sm.o.lat);
+                uint4 *b = reinterpret_cast<uint4 *>(sm.lat);
                 for (int i = threadIdx.x; i < W.ntables * (int)(sizeof(MgLattice) / 16); i += BNT) b[i] = a[i];
             }
         }
@@ -297,65 +236,29 @@ __global__ void __launch_bounds__(BNT, MINB) k_batch(const MgWorldDesc *__restri
         const int tx0 = (tile % tw) * TILE_W, tz0 = (tile / tw) * TILE_H;
         const MgTreeNode *tree = trees[R.world];
         if (W.fmode) {
-            if (W.dim == MG_OVERWORLD) {
-                /* the tile's shift splits, computed once per column and row (ENGINE rule) */
-                const bool tab = TILE_W == 8 && R.tie != MG_TIE_CHUNK_CELL && shift_table_ok(W);
-                if (tab) {
-                    shift_table_fill_f<8, BNT / 8, BNT>(W.noise[0], sm.o.lat, R.qx0 + tx0, R.qz0 + tz0, sm.o.shiftf);
-                    __syncthreads();
-                }
-                batch_cells<true, MG_OVERWORLD, TILE_W>(W, W.spline, sm.o.lat, tree, R, tx0, tz0, nullptr,
-                                                        tab ? &sm.o.shiftf : nullptr, 0.0, sm.wt, &sm.sink, out);
-            } else {
-                batch_cells<true, MG_NETHER, TILE_W>(W, W.spline, sm.o.lat, tree, R, tx0, tz0, nullptr, nullptr, 0.0, sm.wt,
-                                                     &sm.sink, out);
-            }
+            if (W.dim == MG_OVERWORLD) batch_cells<true, MG_OVERWORLD, TILE_W>(W, W.spline, sm.lat, tree, R, tx0, tz0, out);
+            else batch_cells<true, MG_NETHER, TILE_W>(W, W.spline, sm.lat, tree, R, tx0, tz0, out);
         } else if (W.dim == MG_OVERWORLD) {
-            /* the tile's shift splits, computed once per column and row (ENGINE rule) */
-            const bool tab = TILE_W == 8 && R.tie != MG_TIE_CHUNK_CELL && shift_table_ok(W);
-            if (tab) {
-                shift_table_fill<8, BNT / 8, BNT>(W.noise[0], sm.o.lat, R.qx0 + tx0, R.qz0 + tz0, sm.o.shift);
-                if (threadIdx.x == BNT - 1) sm.depth_g = depth_grad_d(W, R.qy * 4); /* a thread with fewer entries */
-                __syncthreads();
-            }
-            batch_cells<false, MG_OVERWORLD, TILE_W>(W, W.spline, sm.o.lat, tree, R, tx0, tz0, tab ? &sm.o.shift : nullptr,
-                                                     nullptr, tab ? sm.depth_g : 0.0, sm.wt, &sm.sink, out);
+            batch_cells<false, MG_OVERWORLD, TILE_W>(W, W.spline, sm.lat, tree, R, tx0, tz0, out);
         } else {
-            batch_cells<false, MG_NETHER, TILE_W>(W, W.spline, sm.o.lat, tree, R, tx0, tz0, nullptr, nullptr, 0.0, sm.wt,
-                                                  &sm.sink, out);
+            batch_cells<false, MG_NETHER, TILE_W>(W, W.spline, sm.lat, tree, R, tx0, tz0, out);
         }
     }
 }
 
-/* The recorded cells (MgPending): one thread each, the exact evaluation of the values the screen left, the
- * climate finish and the R-tree search (the lanes' targets are unrelated), then the cell's output byte. */
-__global__ void __launch_bounds__(128) k_batch_exact(const MgWorldDesc *__restrict__ worlds,
-                                                     const MgTreeNode *const *__restrict__ trees,
-                                                     const MgLattice *__restrict__ pool,
-                                                     const MgPending *__restrict__ pend,
-                                                     const unsigned long long *__restrict__ npend, long long cap,
-                                                     uint8_t *__restrict__ out) {
-    const long long n = min((long long)*npend, cap);
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const MgPending P = pend[i];
-        const MgWorldDesc &W = worlds[P.world];
-        int32_t tg[6];
-        pending_targets(W, pool + P.state, P, tg);
-        const MgTreeNode *tree = trees[P.world];
-        uint64_t d;
-        put_id(out + P.out, tree[tree_search_scattered(tree, tg, -1, d)].biome);
-    }
-}
-
 /* ---------------------------------------------------------------- host side */
-long long batch_pending_cap(long long cells) { return cells > 0 ? cells / 256 + 1024 : 0; }
-
 /* tile shapes the autotuner chooses from: tile width, and the register budget (resident CTAs per SM: 9, 7,
  * 6, 8) in k_batch's second template argument */
 const int kBatchTileWidths[BATCH_SHAPES] = {8, 8, 8, 8};
 static int g_resident[BATCH_SHAPES] = {0, 0, 0, 0}; /* CTAs per SM x SMs, per shape (batch_prepare) */
 
-long long batch_tiles(int dim, int qx0, int qz0, int nx, int nz, int shape) {
+int batch_group(const MgWorldDesc &W, int tie) {
+    if (tie != MG_TIE_ENGINE || !ow_tile_supported(W)) return BATCH_REST;
+    return W.fmode ? BATCH_OW_F : BATCH_OW_D;
+}
+
+long long batch_tiles(int group, int dim, int qx0, int qz0, int nx, int nz, int shape) {
+    if (group != BATCH_REST) return ow_tiles(nx, nz);
     if (dim == MG_END) {
         const long long ncx = ((qx0 + nx - 1) >> 2) - (qx0 >> 2) + 1, ncz = ((qz0 + nz - 1) >> 2) - (qz0 >> 2) + 1;
         return ((ncx + END_TC - 1) / END_TC) * ((ncz + END_TC - 1) / END_TC);
@@ -403,41 +306,47 @@ int batch_prepare(int *ctas_per_sm) {
     if (!rc) rc = prepare_t<8, 7>(1, sms);
     if (!rc) rc = prepare_t<8, 6>(2, sms);
     if (!rc) rc = prepare_t<8, 8>(3, sms);
+    if (!rc) rc = ow_prepare(sms);
     if (!rc) prepared_dev = dev;
     if (ctas_per_sm) *ctas_per_sm = g_resident[0] / (sms > 0 ? sms : 1);
     return rc;
 }
 
-/* ctas: upper bound on the persistent grid (0: every resident CTA of the shape) */
-int launch_batch(const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees, const MgBatchReq *d_reqs, int nreq,
-                 long long ntiles, const MgLattice *d_pool, unsigned long long *d_counter, MgPending *d_pend,
-                 long long pend_cap, uint8_t *d_out, int ctas, int shape, cudaStream_t st) {
-    if (ntiles <= 0) return 0;
+int launch_batch(const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees, const MgBatchReq *d_reqs,
+                 const BatchGroups &g, const MgLattice *d_pool, unsigned long long *d_counter, MgOpenCell *d_open,
+                 long long open_cap, uint8_t *d_out, int ctas, int shape, cudaStream_t st) {
+    if (g.tiles[0] + g.tiles[1] + g.tiles[2] <= 0) return 0;
     if (shape < 0 || shape >= BATCH_SHAPES || g_resident[shape] <= 0) return (int)cudaErrorInvalidValue;
-    if (!d_pend) pend_cap = 0;
-    cudaError_t e = cudaMemsetAsync(d_counter, 0, 2 * sizeof(unsigned long long), st);
+    cudaError_t e = cudaMemsetAsync(d_counter, 0, BATCH_COUNTERS * sizeof(unsigned long long), st);
     if (e) return (int)e;
-    int grid = g_resident[shape];
-    if (ctas > 0 && ctas < grid) grid = ctas;
-    if ((long long)grid > ntiles) grid = (int)ntiles;
-    const size_t sm = sizeof(BatchSmem);
-    {
-        ProfScope ps_(K_BATCH, st);
-        switch (shape) {
-        case 1: k_batch<8, 7><<<grid, BNT, sm, st>>>(d_worlds, d_trees, d_reqs, nreq, ntiles, d_pool, d_counter, d_pend, pend_cap, d_out); break;
-        case 2: k_batch<8, 6><<<grid, BNT, sm, st>>>(d_worlds, d_trees, d_reqs, nreq, ntiles, d_pool, d_counter, d_pend, pend_cap, d_out); break;
-        case 3: k_batch<8, 8><<<grid, BNT, sm, st>>>(d_worlds, d_trees, d_reqs, nreq, ntiles, d_pool, d_counter, d_pend, pend_cap, d_out); break;
-        default: k_batch<8, 9><<<grid, BNT, sm, st>>>(d_worlds, d_trees, d_reqs, nreq, ntiles, d_pool, d_counter, d_pend, pend_cap, d_out); break;
+    unsigned long long *nopen = d_counter + BATCH_GROUPS;
+    int rc = launch_ow_tiles(false, d_worlds, d_trees, d_reqs, g.n[0], g.tiles[0], d_pool, d_counter, d_open, nopen, open_cap, d_out, st);
+    if (!rc) rc = launch_ow_tiles(true, d_worlds, d_trees, d_reqs + g.n[0], g.n[1], g.tiles[1], d_pool, d_counter + 1, nullptr,
+                                  nullptr, 0, d_out, st);
+    if (rc) return rc;
+    if (g.tiles[BATCH_REST] > 0) {
+        const MgBatchReq *rq = d_reqs + g.n[0] + g.n[1];
+        const int nreq = g.n[BATCH_REST];
+        const long long ntiles = g.tiles[BATCH_REST];
+        unsigned long long *cnt = d_counter + BATCH_REST;
+        int grid = g_resident[shape];
+        if (ctas > 0 && ctas < grid) grid = ctas;
+        if ((long long)grid > ntiles) grid = (int)ntiles;
+        const size_t sm = sizeof(BatchSmem);
+        {
+            ProfScope ps_(K_BATCH, st);
+            switch (shape) {
+            case 1: k_batch<8, 7><<<grid, BNT, sm, st>>>(d_worlds, d_trees, rq, nreq, ntiles, d_pool, cnt, d_out); break;
+            case 2: k_batch<8, 6><<<grid, BNT, sm, st>>>(d_worlds, d_trees, rq, nreq, ntiles, d_pool, cnt, d_out); break;
+            case 3: k_batch<8, 8><<<grid, BNT, sm, st>>>(d_worlds, d_trees, rq, nreq, ntiles, d_pool, cnt, d_out); break;
+            default: k_batch<8, 9><<<grid, BNT, sm, st>>>(d_worlds, d_trees, rq, nreq, ntiles, d_pool, cnt, d_out); break;
+            }
         }
-    }
-    count_launch_external();
-    if ((e = cudaGetLastError())) return (int)e;
-    if (pend_cap > 0) { /* the recorded cells; the grid covers the usual count, larger counts loop */
-        ProfScope ps_(K_BATCH_EXACT, st);
-        k_batch_exact<<<2 * 152, 128, 0, st>>>(d_worlds, d_trees, d_pool, d_pend, d_counter + 1, pend_cap, d_out);
         count_launch_external();
+        if ((e = cudaGetLastError())) return (int)e;
     }
-    return (int)cudaGetLastError();
+    if (g.tiles[0] > 0 && d_open && open_cap > 0) rc = launch_ow_open(d_worlds, d_trees, d_reqs, d_pool, d_open, nopen, open_cap, d_out, st);
+    return rc;
 }
 
 }  // namespace mg

@@ -24,25 +24,47 @@ typedef struct {
 } MgSetupEntry;
 
 #define BATCH_SHAPES 4
+/* The requests of a batch come in three groups, each contiguous and with a tile numbering of its own: Overworld
+ * requests under the ENGINE rule by branch (owtile.cu: 16 x 16-cell tiles), then everything else (batch.cu). */
+enum { BATCH_OW_D = 0, BATCH_OW_F = 1, BATCH_REST = 2, BATCH_GROUPS = 3 };
 namespace mg {
-/* records to provide for a batch with `cells` double-branch Overworld cells (a bound far above the
- * measured 1.5-3.5e-4 share of unsettled values; cells beyond it take the exact path in place) */
-long long batch_pending_cap(long long cells);
+struct BatchGroups {
+    int n[BATCH_GROUPS];
+    long long tiles[BATCH_GROUPS];
+};
+/* device counters of a batch: tiles taken per group, cells recorded as open */
+#define BATCH_COUNTERS (BATCH_GROUPS + 1)
+int batch_group(const MgWorldDesc &W, int tie);
+/* owtile.cu: tiles of a request, the worlds it takes, attributes, launch */
+bool ow_tile_supported(const MgWorldDesc &W);
+long long ow_tiles(int nx, int nz);
+int ow_prepare(int sms);
+/* records to provide for a batch with `cells` double-branch Overworld cells (about 2 % keep a target open; cells beyond the
+ * record are evaluated in place) */
+long long ow_open_cap(long long cells);
+/* fm: the float branch's kernel; the double branch's records the cells it leaves open */
+int launch_ow_tiles(bool fm, const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees, const MgBatchReq *d_reqs, int nreq,
+                    long long ntiles, const MgLattice *d_pool, unsigned long long *d_counter, MgOpenCell *d_open,
+                    unsigned long long *d_nopen, long long open_cap, uint8_t *d_out, cudaStream_t st);
+/* the exact evaluation of the recorded cells */
+int launch_ow_open(const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees, const MgBatchReq *d_reqs, const MgLattice *d_pool,
+                   const MgOpenCell *d_open, const unsigned long long *d_nopen, long long open_cap, uint8_t *d_out, cudaStream_t st);
 /* tile widths of the four Overworld/Nether tile shapes (128 cells each; the shapes also differ in the
  * register budget: 9, 7, 6 and 8 resident CTAs per SM) */
 extern const int kBatchTileWidths[BATCH_SHAPES];
-/* tiles of a request: 128 quart cells of shape `shape` (Overworld, Nether) or 8 x 8 chunks (End) */
-long long batch_tiles(int dim, int qx0, int qz0, int nx, int nz, int shape);
+/* tiles of a request of group `group`: 16 x 16 cells (owtile.cu); in the rest, 128 quart cells of shape `shape`
+ * (Overworld, Nether) or 8 x 8 chunks (End) */
+long long batch_tiles(int group, int dim, int qx0, int qz0, int nx, int nz, int shape);
 /* lattices of a list of entries of one dimension; Overworld needs the prefix sums of lattices per entry */
 int launch_setup_list(const MgWorldDesc *d_worlds, int dim, const MgSetupEntry *d_ent, int n, const int *d_first,
                       long long total_lattices, MgLattice *d_pool, cudaStream_t st);
 /* kernel attributes and resident grid sizes; call before any stream capture */
 int batch_prepare(int *ctas_per_sm);
-/* ctas: upper bound on the persistent grid, 0 = every resident CTA of the shape.  d_counter holds two
- * counters (tiles taken, cells recorded); with d_pend (pend_cap records) the double-branch Overworld cells
- * left to the exact evaluation are recorded and finished by a second launch, without it in place. */
-int launch_batch(const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees, const MgBatchReq *d_reqs, int nreq,
-                 long long ntiles, const MgLattice *d_pool, unsigned long long *d_counter, MgPending *d_pend,
-                 long long pend_cap, uint8_t *d_out, int ctas, int shape, cudaStream_t st);
+/* d_reqs: the requests in group order.  ctas: upper bound on the rest's persistent grid, 0 = every resident CTA of
+ * the shape.  d_counter: BATCH_COUNTERS counters; with d_open (open_cap records) the double-branch Overworld cells the tile
+ * kernel leaves open are recorded and finished by a last launch, without it in place. */
+int launch_batch(const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees, const MgBatchReq *d_reqs,
+                 const BatchGroups &g, const MgLattice *d_pool, unsigned long long *d_counter, MgOpenCell *d_open,
+                 long long open_cap, uint8_t *d_out, int ctas, int shape, cudaStream_t st);
 }  // namespace mg
 #endif

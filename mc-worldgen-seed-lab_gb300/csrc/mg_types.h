@@ -48,6 +48,11 @@ typedef struct {
      * reference's double value in units of 2^-59 (rounded up; < 0: not screened this way) */
     int64_t c31[MG_MAX_OCT];
     int64_t fix_eq32;
+    /* double branch, the tile kernels' table form: amp_d[k] * vf_d[k] * vfac times 2^29 rounded, and the bound on the
+     * difference between its value and the reference's double value in units of 2^-29 (rounded up; < 0: not available) */
+    int32_t c29[MG_MAX_OCT];
+    int32_t tile_eq;
+    int32_t tile_pad;
 } MgNoise;
 
 /* Offset spline (CubicSpline over continents, erosion, ridges, ridges_folded), float.
@@ -102,6 +107,10 @@ typedef struct {
     double end_f2, end_g2;         /* 2-D simplex skew 0.5*(sqrt(3)-1) and unskew (3-sqrt(3))/6 */
     int32_t tree_root, tree_nodes, tree_leaves;
     int32_t tree_fanout;           /* most children of a node (the build's children per node: 6 or 19) */
+    /* the leaves again, clustered, for a search that shares its pruning among a tile's cells: groups of up to 32 leaves with
+     * their box (count, first: the group's leaves counted from node leaf_off) at nodes [group_off, group_off + groups) of the
+     * same array, and the leaves from node leaf_off on, whose `first` is their rank in the tree's depth-first order */
+    int32_t group_off, groups, leaf_off, group_pad;
     MgSpline spline;
 } MgWorldDesc;
 
@@ -130,21 +139,12 @@ typedef struct __attribute__((aligned(16))) {
     uint8_t p[256];
 } MgLattice;
 
-/* A double-branch Overworld cell whose screened climate left a value to the exact double evaluation
- * (about one cell in a thousand): the batch kernel records it here instead of running that evaluation inside
- * a warp whose other lanes would wait for it, and a second kernel finishes the recorded cells densely, one per
- * thread.  72 bytes. */
+/* A double-branch Overworld cell of the tile kernel with a quantised target its bounds left open: finished by the exact
+ * evaluation of a later launch. */
 typedef struct {
-    double x, z;      /* the climate noises' input: the cell's shifted coordinates */
-    double g;         /* depth gradient at the cell's y */
-    int64_t out;      /* output byte of the cell */
-    float f[4];       /* temperature, vegetation (a float with the settled target), continentalness, erosion */
-    float rv, rf;     /* ridge and ridges_folded floats, when settled */
-    int32_t world;    /* index into the batch's world table */
-    int32_t state;    /* first lattice of its seed in the state pool */
-    uint32_t pend;    /* bit k < 4: climate noise k + 1 unsettled; bit 4: the ridge (with ridges_folded) */
-    int32_t pad;
-} MgPending;
+    int32_t req;  /* request, counted from the batch's first */
+    int32_t cell; /* row-major cell of the request */
+} MgOpenCell;
 
 /* One seed-search observation (the reference's McgObs, engine/cuda/mc_gpu.cuh:47-54): a quart cell, or a
  * block resolved through BiomeManager's zoom when flags has MG_OBS_BLOCK; flags' low byte is the End window

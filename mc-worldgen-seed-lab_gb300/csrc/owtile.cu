@@ -1,0 +1,700 @@
+/* owtile.cu -- the batched form's Overworld requests (ENGINE rule): persistent kernels over 16 x 16-cell tiles whose
+ * octaves read tables of lattice nodes (owtile.cuh). */
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "batch.h"
+#include "batchdev.cuh"
+#include "launch.h"
+#include "owtile.cuh"
+#include "prof.h"
+
+namespace mg {
+
+/* nodes a tile's table holds: the shift noises' (about 610) or the climate octaves' (about 680 on average) */
+#define OT_CAP_F 1024
+
+struct OtSmemF {
+    MgLattice lat[MG_MAX_TABLES];
+    float4 np[OT_CAP_F];
+    float2 nq[OT_CAP_F];
+    OtShiftF sh[2 * OT_MAXLEV][4 * OT_W]; /* per lattice: X + ox, X + oy, Z + oz, Z + ox (16 entries each) */
+    OtOctF oct[MG_MAX_TABLES];            /* the climate octaves in evaluation order */
+    OtBuild build, sbuild;                /* climate and shift tables */
+    OtSearch rt;
+    int lo[2], hi[2];                     /* range of the shifted x and z over the tile, in 1/16 of a quart from its corner */
+    int tile, req, state, over;
+};
+
+/* the old per-cell form, for a tile whose nodes do not fit (out of line: rare) */
+static __device__ __noinline__ void ot_cell_f(const MgWorldDesc &W, const MgLattice *T, int qx, int qy, int qz, int32_t *tg) {
+    int32_t t[6];
+    climate_ow<true>(W, W.spline, T, qx, qy, qz, t);
+    for (int k = 0; k < 6; k++) tg[k] = t[k];
+}
+
+/* next tile and its request (one whole warp calls it) */
+template <typename SM>
+__device__ __forceinline__ void ot_next(SM &sm, const MgBatchReq *__restrict__ reqs, int nreq, long long ntiles,
+                                        unsigned long long *__restrict__ counter) {
+    long long tile = 0;
+    if ((threadIdx.x & 31) == 0) tile = (long long)atomicAdd(counter, 1ULL);
+    tile = __shfl_sync(0xFFFFFFFFu, tile, 0);
+    const int r = tile < ntiles ? find_req(reqs, nreq, tile) : -1;
+    if ((threadIdx.x & 31) == 0) {
+        sm.tile = r >= 0 ? (int)(tile - reqs[r].tile0) : 0;
+        sm.req = r;
+    }
+}
+
+/* Float branch (26.3 on), bit for bit the per-cell form's operations.  Bound by instruction issue (66 % of peak; the octaves'
+ * separately rounded lerps, the splits' mantissa shifts, the tree scan).  64 registers and 55 KB of shared memory: 4 CTAs,
+ * 32 warps per SM.  The uneven batch's 70.8 M float-branch cells: 47.6 ms in the per-cell form, 37.9 ms here. */
+__global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const MgWorldDesc *__restrict__ worlds, const MgTreeNode *const *__restrict__ trees,
+                                                   const MgBatchReq *__restrict__ reqs, int nreq, long long ntiles,
+                                                   const MgLattice *__restrict__ pool, unsigned long long *__restrict__ counter,
+                                                   uint8_t *__restrict__ out) {
+    extern __shared__ uint4 smem_raw[];
+    OtSmemF &sm = *reinterpret_cast<OtSmemF *>(smem_raw);
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int col = ot_col(), row = ot_row();
+    if (t == 0) sm.state = -1;
+    if (warp == 0) ot_next(sm, reqs, nreq, ntiles, counter);
+    __syncthreads();
+    for (;;) {
+        const int r = sm.req;
+        if (r < 0) return;
+        const int tile = sm.tile;
+        const MgBatchReq R = reqs[r];
+        const MgWorldDesc &W = worlds[R.world];
+        const MgNoise &O = W.noise[0];
+        const int nlev = O.nlev, nsh = 2 * nlev, nclim = W.ntables - nsh;
+        const int tw = (R.nx + OT_W - 1) / OT_W;
+        const int tx0 = (tile % tw) * OT_W, tz0 = (tile / tw) * OT_W;
+        const int qx0 = R.qx0 + tx0, qz0 = R.qz0 + tz0;
+        /* beyond the world border the wrap may move a cell: the per-cell form takes the tile */
+        const bool far = qx0 <= -OT_COORD_LIM || qz0 <= -OT_COORD_LIM || qx0 >= OT_COORD_LIM || qz0 >= OT_COORD_LIM;
+        if (R.state != sm.state) { /* the request's lattices, octave constants and shift table layout */
+            const uint4 *a = reinterpret_cast<const uint4 *>(pool + R.state);
+            uint4 *b = reinterpret_cast<uint4 *>(sm.lat);
+            for (int i = t; i < W.ntables * (int)(sizeof(MgLattice) / 16); i += OT_NT) b[i] = a[i];
+            __syncthreads();
+            if (t == 0) sm.state = R.state;
+            if (t < nclim) { /* octave t in evaluation order */
+                int n = 1;
+                while (n < MG_OW_NOISES - 1 && t + nsh >= W.noise[n + 1].base) n++;
+                const MgNoise &N = W.noise[n];
+                const int e = t + nsh - N.base, k = e >> 1;
+                const int l = N.base + (e & 1) * N.nlev + k;
+                const MgLattice &L = sm.lat[l];
+                sm.build.nx[t] = (int16_t)l; /* the climate tables' lattice (their row length is the range's) */
+                OtOctF &o = sm.oct[t];
+                o.ox = L.ox;
+                o.oz = L.oz;
+                o.f = N.freq[k];
+                o.amp = N.amp_f[k];
+                o.uy = L.z0.f.uy;
+            }
+            if (warp == 7) { /* shift tables: lattice j's (x, 0, z) form is table 2 j, its (x, y, 0) form 2 j + 1 */
+                const int m = lane < 2 * nsh ? ot_shift_nodes(O.freq[(lane >> 1) % nlev]) : 0;
+                int off = (m * m + 31) / 32, n = off;
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int v = __shfl_up_sync(0xFFFFFFFFu, off, d);
+                    if (lane >= d) off += v;
+                }
+                sm.sbuild.unit0[lane] = lane < 2 * nsh ? off - n : 0x7FFFFFFF;
+                sm.sbuild.unit0[lane + 32] = 0x7FFFFFFF;
+                sm.sbuild.n[lane] = (int16_t)(m * m);
+                sm.sbuild.nx[lane] = (int16_t)m;
+                sm.sbuild.inv[lane] = (m ? (65536 + m - 1) / m : 0);
+                if (lane == 31) sm.sbuild.units = off;
+            }
+            __syncthreads();
+        }
+        /* ---- 1: the shift noises' splits per column and row, and their nodes */
+        for (int e = far ? nsh * 4 * OT_W : t; e < nsh * 4 * OT_W; e += OT_NT) {
+            const int j = e / (4 * OT_W), q = e % (4 * OT_W), fam = q / OT_W, idx = q % OT_W;
+            const MgLattice &L = sm.lat[j];
+            const double f = O.freq[j % nlev];
+            const double off = fam == 0 || fam == 3 ? L.ox : (fam == 1 ? L.oy : L.oz);
+            double c = fam < 2 ? (double)(qx0 + idx) : (double)(qz0 + idx), c0 = fam < 2 ? (double)qx0 : (double)qz0;
+            if (j >= nlev) { c = c * MG_SECOND_STACK; c0 = c0 * MG_SECOND_STACK; }
+            OtShiftF s;
+            int i;
+            ot_split_f(c, f, off, i, s.f);
+            s.g = s.f - 1.0f;
+            s.u = fade<float>(s.f);
+            const int tab = 2 * j + (fam & 1), rel = i - ifloor(__fma_rn(c0, f, off));
+            /* x-like coordinates (families 0 and 3) step one node, the others a row; the table's place with the first */
+            s.node = fam == 0 || fam == 3 ? rel + 32 * sm.sbuild.unit0[tab] : rel * sm.sbuild.nx[tab];
+            sm.sh[j][q] = s;
+        }
+        for (int u = far ? sm.sbuild.units : warp; u < sm.sbuild.units; u += OT_NT / 32) {
+            const int tab = ot_find_unit(sm.sbuild, u);
+            const int n = (u - sm.sbuild.unit0[tab]) * 32 + lane;
+            if (n >= sm.sbuild.n[tab]) continue;
+            const int j = tab >> 1, z0 = tab & 1, nx = sm.sbuild.nx[tab];
+            const int k = n * sm.sbuild.inv[tab] >> 16, i = n - k * nx;
+            const MgLattice &L = sm.lat[j];
+            const double f = O.freq[j % nlev];
+            double X = (double)qx0, Z = (double)qz0;
+            if (j >= nlev) { X = X * MG_SECOND_STACK; Z = Z * MG_SECOND_STACK; }
+            const int ib = ifloor(__fma_rn(z0 ? Z : X, f, L.ox)), kb = ifloor(__fma_rn(z0 ? X : Z, f, z0 ? L.oy : L.oz));
+            const int at = 32 * sm.sbuild.unit0[tab] + n;
+            ot_node_f(L, z0, ib + i, kb + k, sm.np[at], sm.nq[at]);
+        }
+        if (t == 0) {
+            sm.lo[0] = sm.lo[1] = 0x7FFFFFFF;
+            sm.hi[0] = sm.hi[1] = -0x7FFFFFFF;
+            sm.over = far;
+        }
+        __syncthreads();
+        /* ---- 2: the shift noises and the shifted coordinates of the cell */
+        const int ix = tx0 + col, iz = tz0 + row;
+        const bool in = ix < R.nx && iz < R.nz;
+        double x = 0.0, z = 0.0;
+        if (!far) {
+            float sa = 0.0f, sb = 0.0f;
+#pragma unroll 1
+            for (int q = 0; q < nsh; q++) { /* level by level, first stack then second: each sum in its order */
+                const int k = q >> 1, j = (q & 1) * nlev + k;
+                const OtShiftF ax = sm.sh[j][col], by = sm.sh[j][OT_W + col], az = sm.sh[j][2 * OT_W + row],
+                               bx = sm.sh[j][3 * OT_W + row];
+                const float amp = O.amp_f[k];
+                sa += amp * ot_octave_f<false>(sm.np, sm.nq, ax.node + az.node, sm.sbuild.nx[2 * j], ax.f, ax.g, ax.u, az.f,
+                                               az.g, az.u, sm.lat[j].z0.f.uy);
+                sb += amp * ot_octave_f<true>(sm.np, sm.nq, bx.node + by.node, sm.sbuild.nx[2 * j + 1], bx.f, bx.g, bx.u, by.f,
+                                              by.g, by.u, sm.lat[j].z0.f.uz);
+            }
+            const float sx = sa * 4.0f, sz = sb * 4.0f;
+            x = (double)(qx0 + col) + (double)sx;
+            z = (double)(qz0 + row) + (double)sz;
+            const int rx = __float2int_rd(((float)col + sx) * 16.0f), rz = __float2int_rd(((float)row + sz) * 16.0f);
+            const int x0 = __reduce_min_sync(0xFFFFFFFFu, in ? rx : 0x7FFFFFFF), x1 = __reduce_max_sync(0xFFFFFFFFu, in ? rx : -0x7FFFFFFF);
+            const int z0 = __reduce_min_sync(0xFFFFFFFFu, in ? rz : 0x7FFFFFFF), z1 = __reduce_max_sync(0xFFFFFFFFu, in ? rz : -0x7FFFFFFF);
+            if (lane == 0 && x0 <= x1) {
+                atomicMin(&sm.lo[0], x0);
+                atomicMax(&sm.hi[0], x1);
+                atomicMin(&sm.lo[1], z0);
+                atomicMax(&sm.hi[1], z1);
+            }
+        }
+        __syncthreads();
+        /* ---- 3: the climate octaves' node ranges (warp 0), the next tile (warp 1) */
+        if (warp == 0 && !far) {
+            /* one sixteenth more on either side covers the float sum's rounding */
+            const double xl = (double)qx0 + (double)(sm.lo[0] - 1) * 0.0625, xh = (double)qx0 + (double)(sm.hi[0] + 2) * 0.0625;
+            const double zl = (double)qz0 + (double)(sm.lo[1] - 1) * 0.0625, zh = (double)qz0 + (double)(sm.hi[1] + 2) * 0.0625;
+            int nodes = 0, units = 0, bad = 0;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int e = lane + 32 * h;
+                OtRange g{0, 0, 0, 0};
+                int n = 0;
+                if (e < nclim) {
+                    OtOctF &o = sm.oct[e];
+                    const double c = (e & 1) ? MG_SECOND_STACK : 1.0; /* every noise starts at an even octave */
+                    g.ib = ifloor(__fma_rn(xl * c, o.f, o.ox));
+                    g.kb = ifloor(__fma_rn(zl * c, o.f, o.oz));
+                    const int nx = ifloor(__fma_rn(xh * c, o.f, o.ox)) - g.ib + 2, nz = ifloor(__fma_rn(zh * c, o.f, o.oz)) - g.kb + 2;
+                    bad |= nx > 32 || nz > 32;
+                    g.nx = nx;
+                    n = nx * nz;
+                }
+                int a = n, b = (n + 31) / 32;
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int va = __shfl_up_sync(0xFFFFFFFFu, a, d), vb = __shfl_up_sync(0xFFFFFFFFu, b, d);
+                    if (lane >= d) { a += va; b += vb; }
+                }
+                g.off = nodes + a - n;
+                if (e < nclim) sm.oct[e].r = g;
+                sm.build.unit0[e] = e < nclim ? units + b - (n + 31) / 32 : 0x7FFFFFFF;
+                sm.build.n[e] = (int16_t)n;
+                sm.build.inv[e] = (g.nx ? (65536 + g.nx - 1) / g.nx : 0);
+                nodes += __shfl_sync(0xFFFFFFFFu, a, 31);
+                units += __shfl_sync(0xFFFFFFFFu, b, 31);
+            }
+            if (__any_sync(0xFFFFFFFFu, bad) || nodes > OT_CAP_F) {
+                if (lane == 0) sm.over = 1;
+            } else if (lane == 0) {
+                sm.build.units = units;
+            }
+        } else if (warp == 1) {
+            ot_next(sm, reqs, nreq, ntiles, counter);
+        } else if (warp == 2) {
+            ot_search_init(sm.rt, lane);
+        }
+        __syncthreads();
+        const bool over = sm.over != 0;
+        /* ---- 4: the climate octaves' nodes */
+        if (!over) {
+            for (int u = warp; u < sm.build.units; u += OT_NT / 32) {
+                const int e = ot_find_unit(sm.build, u);
+                const int n = (u - sm.build.unit0[e]) * 32 + lane;
+                if (n >= sm.build.n[e]) continue;
+                const OtRange g = sm.oct[e].r;
+                const int k = n * sm.build.inv[e] >> 16, i = n - k * g.nx;
+                ot_node_f(sm.lat[sm.build.nx[e]], false, g.ib + i, g.kb + k, sm.np[g.off + n], sm.nq[g.off + n]);
+            }
+        }
+        __syncthreads();
+        /* ---- 5: the climate noises, the targets, the R-tree */
+        int32_t tg[6] = {0, 0, 0, 0, 0, 0};
+        if (in) {
+            if (!over) {
+                double xc = x * MG_SECOND_STACK, zc = z * MG_SECOND_STACK;
+                /* kept in registers: the compiler would form the products again in every octave (FP64 pipe) */
+                asm volatile("" : "+d"(xc), "+d"(zc));
+                float v[MG_OW_NOISES - 1];
+                int e = 0;
+#pragma unroll
+                for (int n = 0; n < MG_OW_NOISES - 1; n++) {
+                    const int end = e + 2 * W.noise[n + 1].nlev;
+                    float acc = 0.0f;
+#pragma unroll 1
+                    for (; e < end; e++) {
+                        const OtOctF o = sm.oct[e];
+                        int ia, ib;
+                        float fa, fb;
+                        ot_split_f((e & 1) ? xc : x, o.f, o.ox, ia, fa);
+                        ot_split_f((e & 1) ? zc : z, o.f, o.oz, ib, fb);
+                        const int at = o.r.off + (ib - o.r.kb) * o.r.nx + (ia - o.r.ib);
+                        acc += o.amp * ot_octave_f<false>(sm.np, sm.nq, at, o.r.nx, fa, fa - 1.0f, fade<float>(fa), fb, fb - 1.0f,
+                                                          fade<float>(fb), o.uy);
+                    }
+                    v[n] = acc;
+                }
+                climate_finish_f(W, W.spline, v[0], v[1], v[2], v[3], v[4], R.qy * 4, tg);
+            } else {
+                ot_cell_f(W, sm.lat, qx0 + col, R.qy, qz0 + row, tg);
+            }
+        }
+        const MgTreeNode *tree = trees[R.world], *leaves = tree + W.leaf_off;
+        const OtWarpBox box = ot_search_box(sm.rt, tg, tg, in);
+        __syncthreads();
+        ot_search_list(sm.rt, W, tree);
+        __syncthreads();
+        if (box.any) {
+            const int n = ot_search_warp(sm.rt, box, tree, leaves, sm.rt.wl[warp]);
+            if (in) put_id(out + R.out_off + (int64_t)iz * R.nx + ix, ot_biome(tree, leaves, sm.rt.wl[warp], n, tg));
+        }
+        __syncthreads(); /* the tables are free for the next tile */
+    }
+}
+
+/* ============================================================================ double branch */
+#define OT_CAP_D 896 /* edges a tile's table holds */
+#define OT_STACK_C ((int64_t)((MG_SECOND_STACK - 1.0) * 0x1.0p64)) /* exact */
+
+/* entry of the shift tables: fraction and smoothstep (units of 2^-31), edge index part */
+struct __align__(16) OtShiftD {
+    int32_t f, u, edge, pad;
+};
+struct OtSmemD {
+    MgLattice lat[MG_MAX_TABLES];
+    int4 ep[OT_CAP_D];
+    int2 eq[OT_CAP_D];
+    OtShiftD sh[2 * OT_MAXLEV][4 * OT_W];
+    OtOctD oct[MG_MAX_TABLES];
+    int64_t oct_o[MG_MAX_TABLES][2]; /* the climate octaves' offsets in units of 2^-32 */
+    int2 oct_b[MG_MAX_TABLES];       /* their first cells */
+    OtFix fix[MG_MAX_TABLES], sfix[OT_SHIFT_TABS]; /* climate octaves; shift tables */
+    OtBuild build, sbuild;
+    OtSearch rt;
+    int lo[2], hi[2];
+    int tile, req, state, over;
+    int32_t depth; /* depth gradient and offset constant at the request's y, units of 2^-28 */
+};
+
+/* a cell left open: recorded for the later launch, or evaluated here when the record is full */
+static __device__ __noinline__ int ot_open_d(const MgWorldDesc &W, const MgLattice *T, const MgTreeNode *tree, int qx, int qy, int qz) {
+    int32_t tg[6];
+    climate_ow<false>(W, W.spline, T, qx, qy, qz, tg);
+    uint64_t d;
+    return tree[tree_search_scattered(tree, tg, -1, d)].biome;
+}
+
+/* Double branch (26.1, 26.2).  The per-cell form was bound by the FP64 pipe (12 exact shift octaves, 348 operations of 446 a
+ * cell at two lanes per SM and clock) beside 40 octaves of 64 x 64-bit products; here nothing per cell uses FP64 and an octave
+ * is 11 32 x 32-bit products.  Bound by instruction issue and the wide multiplies.  The uneven batch's 151.6 M double-branch
+ * cells: 222.5 ms in the per-cell form, 79.2 ms here (k_ow_open 0.6 ms of it). */
+__global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict__ worlds, const MgTreeNode *const *__restrict__ trees,
+                                                   const MgBatchReq *__restrict__ reqs, int nreq, long long ntiles,
+                                                   const MgLattice *__restrict__ pool, unsigned long long *__restrict__ counter,
+                                                   MgOpenCell *__restrict__ open, unsigned long long *__restrict__ nopen,
+                                                   long long open_cap, uint8_t *__restrict__ out) {
+    extern __shared__ uint4 smem_raw[];
+    OtSmemD &sm = *reinterpret_cast<OtSmemD *>(smem_raw);
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int col = ot_col(), row = ot_row();
+    if (t == 0) sm.state = -1;
+    if (warp == 0) ot_next(sm, reqs, nreq, ntiles, counter);
+    __syncthreads();
+    for (;;) {
+        const int r = sm.req;
+        if (r < 0) return;
+        const int tile = sm.tile;
+        const MgBatchReq R = reqs[r];
+        const MgWorldDesc &W = worlds[R.world];
+        const MgNoise &O = W.noise[0];
+        const int nlev = O.nlev, nsh = 2 * nlev, nclim = W.ntables - nsh;
+        const int tw = (R.nx + OT_W - 1) / OT_W;
+        const int tx0 = (tile % tw) * OT_W, tz0 = (tile / tw) * OT_W;
+        const int qx0 = R.qx0 + tx0, qz0 = R.qz0 + tz0;
+        const bool far = qx0 <= -OT_COORD_LIM || qz0 <= -OT_COORD_LIM || qx0 >= OT_COORD_LIM || qz0 >= OT_COORD_LIM;
+        if (R.state != sm.state) { /* the request's lattices, octave constants and shift table layout */
+            const uint4 *a = reinterpret_cast<const uint4 *>(pool + R.state);
+            uint4 *b = reinterpret_cast<uint4 *>(sm.lat);
+            for (int i = t; i < W.ntables * (int)(sizeof(MgLattice) / 16); i += OT_NT) b[i] = a[i];
+            __syncthreads();
+            if (t == 0) sm.state = R.state;
+            if (t < nclim) { /* octave t in evaluation order */
+                int n = 1;
+                while (n < MG_OW_NOISES - 1 && t + nsh >= W.noise[n + 1].base) n++;
+                const MgNoise &N = W.noise[n];
+                const int e = t + nsh - N.base, k = e >> 1;
+                const int l = N.base + (e & 1) * N.nlev + k;
+                const MgLattice &L = sm.lat[l];
+                sm.build.nx[t] = (int16_t)l; /* the climate tables' lattice */
+                sm.oct_o[t][0] = __double2ll_rn(L.ox * 0x1.0p32);
+                sm.oct_o[t][1] = __double2ll_rn(L.oz * 0x1.0p32);
+                sm.oct[t].k = -N.fexp[k];
+                sm.oct[t].c29 = N.c29[k];
+                sm.fix[t] = ot_fix(L.fyd, L.uyd);
+            } else if (t >= 64 && t < 64 + 2 * nsh) { /* shift tables: lattice j's (x, 0, z) form is 2 j, its (x, y, 0) form 2 j + 1 */
+                const MgLattice &L = sm.lat[(t - 64) >> 1];
+                sm.sfix[t - 64] = (t & 1) ? ot_fix(L.fzd, L.uzd) : ot_fix(L.fyd, L.uyd);
+            }
+            if (warp == 7) {
+                const int m = lane < 2 * nsh ? ot_shift_nodes(O.freq[(lane >> 1) % nlev]) : 0;
+                int off = (m * m + 31) / 32, n = off;
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int v = __shfl_up_sync(0xFFFFFFFFu, off, d);
+                    if (lane >= d) off += v;
+                }
+                sm.sbuild.unit0[lane] = lane < 2 * nsh ? off - n : 0x7FFFFFFF;
+                sm.sbuild.unit0[lane + 32] = 0x7FFFFFFF;
+                sm.sbuild.n[lane] = (int16_t)(m * m);
+                sm.sbuild.nx[lane] = (int16_t)m;
+                sm.sbuild.inv[lane] = (m ? (65536 + m - 1) / m : 0);
+                if (lane == 31) sm.sbuild.units = off;
+            }
+            __syncthreads();
+        }
+        /* ---- 1: the shift noises' splits per column and row, and their edges */
+        for (int e = far ? nsh * 4 * OT_W : t; e < nsh * 4 * OT_W; e += OT_NT) {
+            const int j = e / (4 * OT_W), q = e % (4 * OT_W), fam = q / OT_W, idx = q % OT_W;
+            const MgLattice &L = sm.lat[j];
+            const double f = O.freq[j % nlev];
+            const double off = fam == 0 || fam == 3 ? L.ox : (fam == 1 ? L.oy : L.oz);
+            double c = fam < 2 ? (double)(qx0 + idx) : (double)(qz0 + idx), c0 = fam < 2 ? (double)qx0 : (double)qz0;
+            if (j >= nlev) { c = c * MG_SECOND_STACK; c0 = c0 * MG_SECOND_STACK; }
+            int i;
+            uint64_t F;
+            if (!ot_split(c, f, off, i, F)) { /* rare: the sum near zero or beyond 2^20 */
+                const double s = __fma_rn(c, f, off);
+                i = ifloor(s);
+                F = (uint64_t)__double2ll_rn((s - (double)i) * 0x1.0p63) << 1;
+            }
+            OtShiftD s;
+            s.f = (int32_t)min((uint32_t)(((F >> 32) + 1) >> 1), 0x7FFFFFFFu);
+            s.u = (int32_t)min((uint32_t)((fadeq((int64_t)(F >> (64 - MG_Q))) + (1LL << 27)) >> 28), 0x7FFFFFFFu);
+            const int tab = 2 * j + (fam & 1), rel = i - ifloor(__fma_rn(c0, f, off));
+            s.edge = fam == 0 || fam == 3 ? rel + 32 * sm.sbuild.unit0[tab] : rel * sm.sbuild.nx[tab];
+            s.pad = 0;
+            sm.sh[j][q] = s;
+        }
+        for (int u = far ? sm.sbuild.units : warp; u < sm.sbuild.units; u += OT_NT / 32) {
+            const int tab = ot_find_unit(sm.sbuild, u);
+            const int n = (u - sm.sbuild.unit0[tab]) * 32 + lane;
+            if (n >= sm.sbuild.n[tab]) continue;
+            const int j = tab >> 1, z0 = tab & 1, nx = sm.sbuild.nx[tab];
+            const int k = n * sm.sbuild.inv[tab] >> 16, i = n - k * nx;
+            const MgLattice &L = sm.lat[j];
+            const double f = O.freq[j % nlev];
+            double X = (double)qx0, Z = (double)qz0;
+            if (j >= nlev) { X = X * MG_SECOND_STACK; Z = Z * MG_SECOND_STACK; }
+            const int ib = ifloor(__fma_rn(z0 ? Z : X, f, L.ox)), kb = ifloor(__fma_rn(z0 ? X : Z, f, z0 ? L.oy : L.oz));
+            const int at = 32 * sm.sbuild.unit0[tab] + n;
+            ot_edge(L, z0, sm.sfix[tab], ib + i, kb + k, sm.ep[at], sm.eq[at]);
+        }
+        if (t == 0) {
+            sm.lo[0] = sm.lo[1] = 0x7FFFFFFF;
+            sm.hi[0] = sm.hi[1] = -0x7FFFFFFF;
+            sm.over = far;
+        } else if (t == OT_NT - 1) {
+            sm.depth = (int32_t)__double2ll_rn((depth_grad_d(W, R.qy * 4) + W.off_d) * 0x1.0p28);
+        }
+        __syncthreads();
+        /* ---- 2: the shift noises and the shifted coordinates of the cell (units of 2^-32) */
+        const int ix = tx0 + col, iz = tz0 + row;
+        const bool in = ix < R.nx && iz < R.nz;
+        int64_t x = 0, z = 0;
+        if (!far) {
+            int64_t sa = 0, sb = 0; /* units of 2^-58 */
+#pragma unroll 1
+            for (int k = 0; k < nlev; k++) {
+                int64_t va = 0, vb = 0;
+#pragma unroll
+                for (int st = 0; st < 2; st++) {
+                    const int j = st * nlev + k;
+                    const OtShiftD ax = sm.sh[j][col], by = sm.sh[j][OT_W + col], az = sm.sh[j][2 * OT_W + row],
+                                   bx = sm.sh[j][3 * OT_W + row];
+                    va += ot_octave_d(sm.ep, sm.eq, ax.edge + az.edge, sm.sbuild.nx[2 * j], ax.f, ax.u, az.f, az.u);
+                    vb += ot_octave_d(sm.ep, sm.eq, bx.edge + by.edge, sm.sbuild.nx[2 * j + 1], bx.f, bx.u, by.f, by.u);
+                }
+                const int32_t c = O.c29[k];
+                sa = ot_madw((int32_t)(va >> 31), c, sa);
+                sb = ot_madw((int32_t)(vb >> 31), c, sb);
+            }
+            x = ((int64_t)(qx0 + col) << 32) + (sa >> 24); /* the noise times 4 */
+            z = ((int64_t)(qz0 + row) << 32) + (sb >> 24);
+            const int rx = col * 16 + (int)(sa >> 52), rz = row * 16 + (int)(sb >> 52);
+            const int x0 = __reduce_min_sync(0xFFFFFFFFu, in ? rx : 0x7FFFFFFF), x1 = __reduce_max_sync(0xFFFFFFFFu, in ? rx : -0x7FFFFFFF);
+            const int z0 = __reduce_min_sync(0xFFFFFFFFu, in ? rz : 0x7FFFFFFF), z1 = __reduce_max_sync(0xFFFFFFFFu, in ? rz : -0x7FFFFFFF);
+            if (lane == 0 && x0 <= x1) {
+                atomicMin(&sm.lo[0], x0);
+                atomicMax(&sm.hi[0], x1);
+                atomicMin(&sm.lo[1], z0);
+                atomicMax(&sm.hi[1], z1);
+            }
+        }
+        __syncthreads();
+        /* ---- 3: the climate octaves' edge ranges (warp 0), the next tile (warp 1) */
+        if (warp == 0 && !far) {
+            const int64_t xl = ((int64_t)qx0 << 32) + ((int64_t)sm.lo[0] << 28), xh = ((int64_t)qx0 << 32) + ((int64_t)(sm.hi[0] + 1) << 28);
+            const int64_t zl = ((int64_t)qz0 << 32) + ((int64_t)sm.lo[1] << 28), zh = ((int64_t)qz0 << 32) + ((int64_t)(sm.hi[1] + 1) << 28);
+            const int64_t cxl = xl + __mul64hi(xl, OT_STACK_C), cxh = xh + __mul64hi(xh, OT_STACK_C);
+            const int64_t czl = zl + __mul64hi(zl, OT_STACK_C), czh = zh + __mul64hi(zh, OT_STACK_C);
+            int edges = 0, units = 0, bad = 0;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int e = lane + 32 * h;
+                int n = 0, nx = 0, ib = 0, kb = 0;
+                if (e < nclim) {
+                    const int k = sm.oct[e].k;
+                    const int64_t ox = sm.oct_o[e][0], oz = sm.oct_o[e][1];
+                    ib = ot_hi((((e & 1) ? cxl : xl) >> k) + ox);
+                    kb = ot_hi((((e & 1) ? czl : zl) >> k) + oz);
+                    nx = ot_hi((((e & 1) ? cxh : xh) >> k) + ox) - ib + 1;
+                    const int nz = ot_hi((((e & 1) ? czh : zh) >> k) + oz) - kb + 2;
+                    bad |= nx > 31 || nz > 32;
+                    n = nx * nz;
+                }
+                int a = n, b = (n + 31) / 32;
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int va = __shfl_up_sync(0xFFFFFFFFu, a, d), vb = __shfl_up_sync(0xFFFFFFFFu, b, d);
+                    if (lane >= d) { a += va; b += vb; }
+                }
+                if (e < nclim) {
+                    OtOctD &o = sm.oct[e];
+                    o.ox = sm.oct_o[e][0] - ((int64_t)ib << 32);
+                    o.oz = sm.oct_o[e][1] - ((int64_t)kb << 32);
+                    o.nx = nx;
+                    o.off = edges + a - n;
+                    sm.oct_b[e] = make_int2(ib, kb);
+                }
+                sm.build.unit0[e] = e < nclim ? units + b - (n + 31) / 32 : 0x7FFFFFFF;
+                sm.build.n[e] = (int16_t)n;
+                sm.build.inv[e] = (nx ? (65536 + nx - 1) / nx : 0);
+                edges += __shfl_sync(0xFFFFFFFFu, a, 31);
+                units += __shfl_sync(0xFFFFFFFFu, b, 31);
+            }
+            if (__any_sync(0xFFFFFFFFu, bad) || edges > OT_CAP_D) {
+                if (lane == 0) sm.over = 1;
+            } else if (lane == 0) {
+                sm.build.units = units;
+            }
+        } else if (warp == 1) {
+            ot_next(sm, reqs, nreq, ntiles, counter);
+        } else if (warp == 2) {
+            ot_search_init(sm.rt, lane);
+        }
+        __syncthreads();
+        const bool over = sm.over != 0;
+        /* ---- 4: the climate octaves' edges */
+        if (!over) {
+            for (int u = warp; u < sm.build.units; u += OT_NT / 32) {
+                const int e = ot_find_unit(sm.build, u);
+                const int n = (u - sm.build.unit0[e]) * 32 + lane;
+                if (n >= sm.build.n[e]) continue;
+                const int nx = sm.oct[e].nx, off = sm.oct[e].off;
+                const int k = n * sm.build.inv[e] >> 16, i = n - k * nx;
+                const int2 b = sm.oct_b[e];
+                ot_edge(sm.lat[sm.build.nx[e]], false, sm.fix[e], b.x + i, b.y + k, sm.ep[off + n], sm.eq[off + n]);
+            }
+        }
+        __syncthreads();
+        /* ---- 5: the climate noises, the targets, the R-tree */
+        bool ok = in && !over;
+        int32_t ta[6] = {0, 0, 0, 0, 0, 0}, tb[6] = {0, 0, 0, 0, 0, 0}; /* the targets the cell may have: [ta, tb] */
+        if (ok) {
+            const int64_t xc = x + __mul64hi(x, OT_STACK_C), zc = z + __mul64hi(z, OT_STACK_C);
+            int32_t v[MG_OW_NOISES - 1]; /* units of 2^-29 */
+            int e = 0;
+#pragma unroll
+            for (int n = 0; n < MG_OW_NOISES - 1; n++) {
+                const int end = e + 2 * W.noise[n + 1].nlev;
+                int64_t acc = 0; /* units of 2^-58 */
+#pragma unroll 1
+                for (; e < end; e += 2) {
+                    int64_t lev = 0;
+                    int32_t c = 0;
+#pragma unroll
+                    for (int st = 0; st < 2; st++) {
+                        const OtOctD o = sm.oct[e + st];
+                        const int64_t sx = ((st ? xc : x) >> o.k) + o.ox, sz = ((st ? zc : z) >> o.k) + o.oz;
+                        const int at = o.off + ot_hi(sz) * o.nx + ot_hi(sx);
+                        lev += ot_octave_d(sm.ep, sm.eq, at, o.nx, (int32_t)((uint32_t)sx >> 1), ot_fade31((uint32_t)sx),
+                                           (int32_t)((uint32_t)sz >> 1), ot_fade31((uint32_t)sz));
+                        c = o.c29;
+                    }
+                    acc = ot_madw((int32_t)(lev >> 31), c, acc);
+                }
+                v[n] = (int32_t)(acc >> 29);
+            }
+            const float s29 = 10000.0f * 0x1.0p-29f, s28 = 10000.0f * 0x1.0p-28f;
+            const int32_t ec = W.noise[3].tile_eq, ee = W.noise[4].tile_eq, ew = W.noise[5].tile_eq;
+            ot_target(v[0], W.noise[1].tile_eq, s29, ta[0], tb[0]);
+            ot_target(v[1], W.noise[2].tile_eq, s29, ta[1], tb[1]);
+            ot_target(v[2], ec, s29, ta[2], tb[2]);
+            ot_target(v[3], ee, s29, ta[3], tb[3]);
+            ot_target(v[4], ew, s29, ta[5], tb[5]);
+            /* spline coordinates: floats of the values, of ridges_folded (|(|r| + c0)| + c1) c2 (the sums in units of
+             * 2^-29); each within its noise's bound (times |c2|) and both sides' roundings to float */
+            const float u = 0x1.0p-29f;
+            const int32_t rs = abs(abs(v[4]) + (int32_t)((W.rf_q[0] + (1 << 29)) >> 30)) + (int32_t)((W.rf_q[1] + (1 << 29)) >> 30);
+            const float c2 = (float)W.rf_d[2] * u;
+            SplineIn si;
+            si.c = (float)v[2] * u;
+            si.e = (float)v[3] * u;
+            si.r = (float)v[4] * u;
+            si.f = (float)rs * c2;
+            si.dc = (float)ec * u + fabsf(si.c) * 1.2e-7f;
+            si.de = (float)ee * u + fabsf(si.e) * 1.2e-7f;
+            si.dr = (float)ew * u + fabsf(si.r) * 1.2e-7f;
+            si.df = fabsf(c2) * (float)(ew + 2) + fabsf(si.f) * 1.9e-7f;
+            float es;
+            const float sp = spline_err<MG_SPL_DEPTH>(W.spline, W.spline.root, si, es);
+            ot_target(sm.depth + __float2int_rn(sp * 0x1.0p28f), (int32_t)(es * (1.01f * 0x1.0p28f)) + 4, s28, ta[4], tb[4]);
+            ok = es < 1.0f;
+        }
+        /* at most one target open, between two neighbouring values: both are looked up, and the cell is settled when they
+         * give the same biome (nearly always: a step is 1e-4 of the range) */
+        int amb = 0;
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+            amb += tb[k] - ta[k];
+            ok &= (unsigned)(tb[k] - ta[k]) <= 1u;
+        }
+        ok &= amb <= 1;
+        const MgTreeNode *tree = trees[R.world], *leaves = tree + W.leaf_off;
+        const OtWarpBox box = ot_search_box(sm.rt, ta, tb, ok);
+        __syncthreads();
+        ot_search_list(sm.rt, W, tree);
+        __syncthreads();
+        int biome = 0;
+        if (box.any) {
+            const int n = ot_search_warp(sm.rt, box, tree, leaves, sm.rt.wl[warp]);
+            if (ok) {
+                biome = ot_biome(tree, leaves, sm.rt.wl[warp], n, ta);
+                if (amb) ok = ot_biome(tree, leaves, sm.rt.wl[warp], n, tb) == biome;
+            }
+        }
+        if (in) {
+            const int64_t o = R.out_off + (int64_t)iz * R.nx + ix;
+            if (ok) {
+                put_id(out + o, biome);
+            } else {
+                const unsigned long long k = atomicAdd(nopen, 1ULL);
+                if (k < (unsigned long long)open_cap) open[k] = MgOpenCell{r, iz * R.nx + ix};
+                else put_id(out + o, ot_open_d(W, sm.lat, tree, qx0 + col, R.qy, qz0 + row));
+            }
+        }
+        __syncthreads(); /* the tables are free for the next tile */
+    }
+}
+
+/* the open cells, one per thread: the exact evaluation from the seed's lattices in the pool */
+__global__ void __launch_bounds__(128) k_ow_open(const MgWorldDesc *__restrict__ worlds, const MgTreeNode *const *__restrict__ trees,
+                                                 const MgBatchReq *__restrict__ reqs, const MgLattice *__restrict__ pool,
+                                                 const MgOpenCell *__restrict__ open, const unsigned long long *__restrict__ nopen,
+                                                 long long cap, uint8_t *__restrict__ out) {
+    const long long n = min((long long)*nopen, cap);
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const MgOpenCell c = open[i];
+        const MgBatchReq R = reqs[c.req];
+        const MgWorldDesc &W = worlds[R.world];
+        const int iz = c.cell / R.nx, ix = c.cell - iz * R.nx;
+        put_id(out + R.out_off + c.cell, ot_open_d(W, pool + R.state, trees[R.world], R.qx0 + ix, R.qy, R.qz0 + iz));
+    }
+}
+
+/* ---------------------------------------------------------------- host side */
+/* a world whose Overworld requests the tile kernels take: power-of-two frequencies of at most 1/2 per quart (the wrap is
+ * the identity up to the world border, and the tables' sizes hold), shift levels and nodes within the tables */
+bool ow_tile_supported(const MgWorldDesc &W) {
+    if (W.dim != MG_OVERWORLD) return false;
+    for (int n = 0; n < MG_OW_NOISES && !W.fmode; n++)
+        if (W.noise[n].tile_eq < 0 || W.rf_eq < 0) return false;
+    if (W.noise[0].base != 0 || W.noise[0].nlev > OT_MAXLEV) return false;
+    int base = 0, cap = 0;
+    for (int n = 0; n < MG_OW_NOISES; n++) {
+        const MgNoise &N = W.noise[n];
+        if (N.base != base || N.nlev < 1) return false;
+        base += 2 * N.nlev;
+        for (int k = 0; k < N.nlev; k++)
+            if (N.fexp[k] > -1 || N.fexp[k] < -40) return false;
+    }
+    if (base != W.ntables || base - 2 * W.noise[0].nlev > 64 || base > MG_MAX_TABLES) return false;
+    for (int k = 0; k < W.noise[0].nlev; k++) {
+        const int m = ot_shift_nodes(W.noise[0].freq[k]);
+        cap += 4 * ((m * m + 31) / 32) * 32;
+    }
+    return cap <= (W.fmode ? OT_CAP_F : OT_CAP_D);
+}
+long long ow_tiles(int nx, int nz) { return (long long)((nx + OT_W - 1) / OT_W) * ((nz + OT_W - 1) / OT_W); }
+
+static int g_ow_resident[2] = {0, 0}; /* CTAs per SM x SMs of the double and the float kernel (ow_prepare; callers hold the
+                                       * ABI lock) */
+template <typename K>
+static int prepare_k(K kernel, size_t smem, int sms, int *resident) {
+    int rc = (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int n = 0;
+    if (!rc) rc = (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, OT_NT, smem);
+    *resident = (n > 0 ? n : 1) * sms;
+    return rc;
+}
+int ow_prepare(int sms) {
+    int rc = prepare_k(k_ow_d, sizeof(OtSmemD), sms, &g_ow_resident[0]);
+    return rc ? rc : prepare_k(k_ow_f, sizeof(OtSmemF), sms, &g_ow_resident[1]);
+}
+long long ow_open_cap(long long cells) { return cells > 0 ? cells / 24 + 4096 : 0; }
+
+int launch_ow_tiles(bool fm, const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees, const MgBatchReq *d_reqs, int nreq,
+                    long long ntiles, const MgLattice *d_pool, unsigned long long *d_counter, MgOpenCell *d_open,
+                    unsigned long long *d_nopen, long long open_cap, uint8_t *d_out, cudaStream_t st) {
+    if (ntiles <= 0) return 0;
+    const int resident = g_ow_resident[fm];
+    if (resident <= 0) return (int)cudaErrorInvalidValue;
+    const int grid = (long long)resident < ntiles ? resident : (int)ntiles;
+    {
+        ProfScope ps_(fm ? K_OW_TILE_F : K_OW_TILE_D, st);
+        if (fm) k_ow_f<<<grid, OT_NT, sizeof(OtSmemF), st>>>(d_worlds, d_trees, d_reqs, nreq, ntiles, d_pool, d_counter, d_out);
+        else k_ow_d<<<grid, OT_NT, sizeof(OtSmemD), st>>>(d_worlds, d_trees, d_reqs, nreq, ntiles, d_pool, d_counter, d_open, d_nopen,
+                                                          d_open ? open_cap : 0, d_out);
+    }
+    count_launch_external();
+    return (int)cudaGetLastError();
+}
+int launch_ow_open(const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees, const MgBatchReq *d_reqs, const MgLattice *d_pool,
+                   const MgOpenCell *d_open, const unsigned long long *d_nopen, long long open_cap, uint8_t *d_out, cudaStream_t st) {
+    {
+        ProfScope ps_(K_OW_OPEN, st);
+        k_ow_open<<<4 * 152, 128, 0, st>>>(d_worlds, d_trees, d_reqs, d_pool, d_open, d_nopen, open_cap, d_out);
+    }
+    count_launch_external();
+    return (int)cudaGetLastError();
+}
+
+}  // namespace mg

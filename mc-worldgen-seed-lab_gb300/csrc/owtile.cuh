@@ -1,0 +1,494 @@
+/* owtile.cuh -- Overworld climate of a 16 x 16-cell tile from tables of lattice nodes (device).
+ *
+ * Every NormalNoise on the biome path has one input coordinate that is zero, so an octave is a function of two
+ * coordinates over a plane of its lattice, and a tile of neighbouring cells touches few of the plane's nodes:
+ * 4 to 9 for the octaves below 2^-5 per quart (32 of the climate's 40), about 150 for the finest one.  The
+ * per-cell forms (device.cuh octave_q) look up 14 permutation bytes and 8 gradients per octave sample, which is
+ * most of their time.  Here the CTA builds the nodes once per tile (two gradients of a node: the two lattice
+ * planes around the zero coordinate's fixed offset) into shared memory, and a cell reads its four nodes.
+ *
+ * Phases of a tile (256 threads, one cell each, warps of 8 x 4 cells):
+ *   1  the shift noises' splits per column and row, and their nodes (the inputs are the integer quart grid)
+ *   2  per cell: both shift noises, the shifted coordinates, and their range over the tile
+ *   3  one warp: each climate octave's node range and place in the table; another takes the next tile
+ *   4  the climate octaves' nodes
+ *   5  per cell: the climate noises and what follows from them
+ */
+#ifndef MG_OWTILE_CUH
+#define MG_OWTILE_CUH
+#include "climate.cuh"
+
+namespace mg {
+
+#define OT_W 16                   /* tile width and height in cells */
+#define OT_NT (OT_W * OT_W)       /* threads per CTA */
+#define OT_MAXLEV 3               /* levels of the shift noise (26.x: 3) */
+#define OT_SHIFT_TABS (4 * OT_MAXLEV)
+#define OT_COORD_LIM ((1 << 23) - 4096) /* |quart| below which every wrap of the path is the identity */
+
+/* column and row of this thread's cell: warps take 8 x 4 blocks, so the R-tree walk of a warp has a compact box */
+__device__ __forceinline__ int ot_col() { return ((threadIdx.x >> 5) & 1) * 8 + (threadIdx.x & 7); }
+__device__ __forceinline__ int ot_row() { return (threadIdx.x >> 6) * 4 + ((threadIdx.x >> 3) & 3); }
+
+/* nodes per axis that 16 neighbouring quart columns can touch at frequency f (second stack: 1.0181... f) */
+__host__ __device__ inline int ot_shift_nodes(double f) { return (int)((OT_W - 1) * f * 1.02) + 3; }
+
+/* s = x f + off as the reference rounds it (f a power of two, |x f| < 2^23: the wrap is the identity), floor i and
+ * fraction F in units of 2^-64, from the mantissa of s as a signed 64-bit integer (an arithmetic shift of the negated
+ * mantissa floors): one FP64-pipe operation, of which an SM completes two lanes per clock.  False for |s| < 2^-11,
+ * |s| >= 2^20 and s in (-1, 0), where the reference's difference s - floor(s) rounds. */
+__device__ __forceinline__ bool ot_split(double x, double f, double off, int &i, uint64_t &F) {
+    const double s = __fma_rn(x, f, off);
+    const uint32_t h = (uint32_t)__double2hiint(s);
+    const int e = (int)((h >> 20) & 0x7FFu) - 1023;
+    const int64_t m = (int64_t)(((uint64_t)((h & 0xFFFFFu) | 0x100000u) << 32) | (uint32_t)__double2loint(s));
+    const int64_t neg = (int64_t)((int32_t)h >> 31);
+    const int64_t M = (m ^ neg) - neg; /* s in units of 2^(e - 52) */
+    i = (int32_t)(M >> 32) >> (20 - e);
+    F = (uint64_t)M << (12 + e);
+    return (uint32_t)(e + 11) <= 30u && (e >= 0 || (int32_t)h >= 0);
+}
+/* the rest, out of line; the product is volatile so that the compiler does not compute it ahead of the branch */
+static __device__ __noinline__ SplitF ot_split_f_slow(double x, double f, double off) {
+    SplitF r;
+    double v;
+    asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(v) : "d"(x), "d"(f));
+    split_f_plain(v, off, r.i, r.f);
+    return r;
+}
+/* the float branch's split.  The hardware's u64 -> f32 conversion runs at the FP64 pipe's rate (595 Gop/s; u32 -> f32
+ * 18,700), so the fraction is converted from its upper 32 bits (below 2^-7: its next 32) with the lower ones as a sticky
+ * bit: 26 or more significant bits, whose guard and sticky bits round as the whole fraction does.  Fractions below 2^-14
+ * take the plain path. */
+__device__ __forceinline__ void ot_split_f(double x, double f, double off, int &i, float &fr) {
+    uint64_t F;
+    const bool ok = ot_split(x, f, off, i, F);
+    uint32_t hi = (uint32_t)(F >> 32), lo = (uint32_t)F;
+    float sc = 0x1.0p-32f;
+    if (hi < (1u << 25)) {
+        hi = __funnelshift_l(lo, hi, 7);
+        lo <<= 7;
+        sc = 0x1.0p-39f;
+    }
+    fr = __uint2float_rn(hi | (lo ? 1u : 0u)) * sc;
+    if (!ok || hi < (1u << 25)) {
+        const SplitF r = ot_split_f_slow(x, f, off);
+        i = r.i;
+        fr = r.f;
+    }
+}
+
+/* where the nodes of one octave lie: first node (ib, kb) of the plane, nodes per row, place in the table */
+struct OtRange {
+    int32_t ib, kb, nx, off;
+};
+/* one octave in evaluation order (a noise's levels, first then second stack of each) */
+struct __align__(16) OtOctF {
+    double ox, oz; /* x and z offsets */
+    double f;      /* input factor */
+    float amp;     /* layer amplitude */
+    float uy;      /* smoothstep of the zero coordinate's fraction */
+    OtRange r;
+};
+/* entry of the shift tables: fraction, fraction - 1, smoothstep, node index part */
+struct __align__(16) OtShiftF {
+    float f, g, u;
+    int32_t node;
+};
+
+/* work units of a table build: table t's nodes in units of 32, unit0[t] its first unit (non-decreasing) */
+struct OtBuild {
+    int32_t unit0[64];
+    int16_t n[64], nx[64];
+    int32_t inv[64]; /* ceil(65536 / nx): row = node * inv >> 16 for node < 1024, nx <= 32 */
+    int32_t units;
+};
+/* the table that unit u belongs to (all lanes call it) */
+__device__ __forceinline__ int ot_find_unit(const OtBuild &b, int u) {
+    const int l = threadIdx.x & 31;
+    return __popc(__ballot_sync(0xFFFFFFFFu, b.unit0[l] <= u)) + __popc(__ballot_sync(0xFFFFFFFFu, b.unit0[l + 32] <= u)) - 1;
+}
+
+/* one octave of the float branch from its four nodes (octave_q<float>'s operations on the same values: a node's
+ * gradient dot is fma(g2, y, fma(g1, x, c)) with c the fixed coordinate's exact product; two of the three
+ * components are non-zero, so one operation rounds, whatever the order).  Input (x, 0, z) (Z0 false): the node's two
+ * gradients are those of the planes y and y + 1, t the fixed smoothstep of y; input (x, y, 0) (Z0 true): those of z and
+ * z + 1, t that of z, and (a, b) = (x, y). */
+struct OtNodeF {
+    float4 p; /* g1, g2, c of the lower plane; g1 of the upper */
+    float2 q; /* g2, c of the upper plane */
+};
+__device__ __forceinline__ float ot_dot0(const OtNodeF &n, float a, float b) { return __fmaf_rn(n.p.y, b, __fmaf_rn(n.p.x, a, n.p.z)); }
+__device__ __forceinline__ float ot_dot1(const OtNodeF &n, float a, float b) { return __fmaf_rn(n.q.x, b, __fmaf_rn(n.p.w, a, n.q.y)); }
+template <bool Z0>
+__device__ __forceinline__ float ot_octave_f(const float4 *__restrict__ P, const float2 *__restrict__ Q, int at, int nx, float a,
+                                             float ga, float u, float b, float gb, float v, float t) {
+    const OtNodeF n00{P[at], Q[at]}, n10{P[at + 1], Q[at + 1]}, n01{P[at + nx], Q[at + nx]}, n11{P[at + nx + 1], Q[at + nx + 1]};
+    const float l0 = lerp<float>(u, ot_dot0(n00, a, b), ot_dot0(n10, ga, b));   /* lower plane, row k */
+    const float l1 = lerp<float>(u, ot_dot0(n01, a, gb), ot_dot0(n11, ga, gb)); /* lower plane, row k + 1 */
+    const float h0 = lerp<float>(u, ot_dot1(n00, a, b), ot_dot1(n10, ga, b));
+    const float h1 = lerp<float>(u, ot_dot1(n01, a, gb), ot_dot1(n11, ga, gb));
+    /* the reference lerps x, then y, then z */
+    if (Z0) return lerp<float>(t, lerp<float>(v, l0, l1), lerp<float>(v, h0, h1));
+    return lerp<float>(v, lerp<float>(t, l0, h0), lerp<float>(t, l1, h1));
+}
+
+/* node (i, k) of lattice L: the gradients of its two planes, as the octave above reads them */
+__device__ __forceinline__ void ot_node_f(const MgLattice &L, bool z0, int i, int k, float4 &p, float2 &q) {
+    const PlainPerm P{L.p};
+    const int a = P(i);
+    float4 g0, g1;
+    float c0, c1;
+    if (z0) { /* (i, k) = (x, y) */
+        const int aa = P(a + k);
+        g0 = __ldg(&kGradF[P(aa + L.iz) & 15]);
+        g1 = __ldg(&kGradF[P(aa + L.iz + 1) & 15]);
+        c0 = g0.z * L.z0.f.fz;
+        c1 = g1.z * (L.z0.f.fz - 1.0f);
+        p = make_float4(g0.x, g0.y, c0, g1.x);
+        q = make_float2(g1.y, c1);
+    } else { /* (i, k) = (x, z) */
+        g0 = __ldg(&kGradF[P(P(a + L.iy) + k) & 15]);
+        g1 = __ldg(&kGradF[P(P(a + L.iy + 1) + k) & 15]);
+        c0 = g0.y * L.z0.f.fy;
+        c1 = g1.y * (L.z0.f.fy - 1.0f);
+        p = make_float4(g0.x, g0.z, c0, g1.x);
+        q = make_float2(g1.z, c1);
+    }
+}
+
+/* ============================================================================ R-tree search of a tile
+ * A tile's 256 cells have close targets, so one pruning serves them all (device.cuh warp_tree_candidates has the argument: a
+ * leaf whose distance to the targets' box exceeds the least "largest distance of a leaf to a point of the box" is nearest for
+ * none of them).  The tile's box is tested against the boxes of the leaves' groups (MgWorldDesc::group_off: at most 256 for
+ * the Overworld's 7,600 leaves, one per thread), the groups that may matter leaf by leaf, each warp prunes the list again
+ * with its own 8 x 4 cells' box, and a lane scans what is left (about 30 leaves).  The reference's leaf is the one of least
+ * distance, the first in depth-first order among equals, so the list's order is free: a leaf carries its rank. */
+#define OT_LIST 512      /* leaves a tile's list holds */
+#define OT_WLIST 128     /* leaves a warp's list holds */
+#define OT_GLIST 256     /* groups a tile's list holds */
+struct OtSearch {
+    unsigned long long near; /* distance and number of the group nearest to the tile's box */
+    int lo[6], hi[6];        /* the tile's box */
+    int bad, ngrp, nleaf;
+    uint16_t grp[OT_GLIST];
+    uint16_t leaf[OT_LIST];
+    uint16_t wl[OT_NT / 32][OT_WLIST];
+};
+/* before the block barrier that precedes ot_search_box */
+__device__ __forceinline__ void ot_search_init(OtSearch &s, int t) {
+    if (t < 6) s.lo[t] = 0x7FFFFFFF;
+    else if (t < 12) s.hi[t - 6] = -0x7FFFFFFF;
+    else if (t == 12) s.near = ~0ULL;
+    else if (t == 13) s.bad = s.ngrp = s.nleaf = 0;
+}
+__device__ __forceinline__ void ot_box(const int32_t *lo, const int32_t *hi, RtTarget &lbq, RtTarget &ubq) {
+    for (int k = 0; k < 3; k++) {
+        lbq.p[k] = pack16(lo[2 * k], lo[2 * k + 1]);
+        lbq.n[k] = pack16(-hi[2 * k], -hi[2 * k + 1]);
+        ubq.p[k] = pack16(hi[2 * k], hi[2 * k + 1]);
+        ubq.n[k] = pack16(-lo[2 * k], -lo[2 * k + 1]);
+    }
+}
+struct OtWarpBox {
+    RtTarget lb, ub;
+    bool any;
+};
+/* the warp's box of its active cells' targets [ta, tb] and its part of the tile's; a barrier follows */
+__device__ __forceinline__ OtWarpBox ot_search_box(OtSearch &s, const int32_t *ta, const int32_t *tb, bool active) {
+    const unsigned FULL = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31, lim = 32767 - MG_TREE_PACKED_BOUND;
+    int32_t lo[6], hi[6];
+    int out = 0, mine = 0;
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        lo[k] = __reduce_min_sync(FULL, active ? ta[k] : 0x7FFFFFFF);
+        hi[k] = __reduce_max_sync(FULL, active ? tb[k] : -0x7FFFFFFF);
+        out |= lo[k] < -lim || hi[k] > lim;
+        mine = lane == k ? lo[k] : (lane == k + 6 ? hi[k] : mine);
+    }
+    OtWarpBox b;
+    b.any = lo[0] != 0x7FFFFFFF;
+    if (b.any) {
+        if (lane < 6) atomicMin(&s.lo[lane], mine);
+        else if (lane < 12) atomicMax(&s.hi[lane - 6], mine);
+        else if (lane == 12 && out) s.bad = 1;
+    }
+    ot_box(lo, hi, b.lb, b.ub);
+    return b;
+}
+struct OtNode {
+    uint4 a, b;
+    __device__ __forceinline__ OtNode(const MgTreeNode *n)
+        : a(*reinterpret_cast<const uint4 *>(n)), b(*(reinterpret_cast<const uint4 *>(n) + 1)) {}
+};
+/* the tile's list (all threads; two barriers inside, one must follow) */
+__device__ __forceinline__ void ot_search_list(OtSearch &s, const MgWorldDesc &W, const MgTreeNode *__restrict__ T) {
+    const unsigned FULL = 0xFFFFFFFFu;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    RtTarget lbq, ubq;
+    ot_box(s.lo, s.hi, lbq, ubq);
+    const int ng = W.groups;
+    const MgTreeNode *G = T + W.group_off, *L = T + W.leaf_off;
+    uint32_t lb0 = 0xFFFFFFFFu; /* this thread's first group */
+    {
+        uint32_t m = 0xFFFFFFFFu;
+        int g = 0;
+        for (int i = t; i < ng; i += OT_NT) {
+            const OtNode n(G + i);
+            const uint32_t d = rt_dist(n.a, n.b, lbq);
+            if (i == t) lb0 = d;
+            if (d < m) { m = d; g = i; }
+        }
+        const uint32_t wm = __reduce_min_sync(FULL, m);
+        if (m == wm && wm != 0xFFFFFFFFu) atomicMin(&s.near, (unsigned long long)wm << 16 | (unsigned)g);
+    }
+    __syncthreads();
+    /* the least upper bound over the nearest group's leaves */
+    uint32_t U = 0xFFFFFFFFu;
+    if (s.near != ~0ULL) {
+        const OtNode g(G + (int)(s.near & 0xFFFFu));
+        const int first = (int)(g.b.w & 0xFFFFu), count = (int)((g.b.w >> 16) & 0xFFu);
+        if (lane < count) {
+            const OtNode n(L + first + lane);
+            U = rt_ub_or_inf(n.a, n.b, ubq);
+        }
+    }
+    U = __reduce_min_sync(FULL, U);
+    for (int i = t; i - lane < ng; i += OT_NT) {
+        uint32_t d = lb0;
+        if (i >= OT_NT && i < ng) {
+            const OtNode n(G + i);
+            d = rt_dist(n.a, n.b, lbq);
+        }
+        const bool keep = i < ng && d <= U;
+        const unsigned m = __ballot_sync(FULL, keep);
+        if (!m) continue;
+        int at = 0;
+        if (lane == 0) at = atomicAdd(&s.ngrp, __popc(m));
+        at = __shfl_sync(FULL, at, 0) + __popc(m & ((1u << lane) - 1u));
+        if (keep && at < OT_GLIST) s.grp[at] = (uint16_t)i;
+    }
+    __syncthreads();
+    const int nk = s.ngrp;
+    if (nk > OT_GLIST) { /* every warp sees the same count */
+        s.bad = 1;
+        return;
+    }
+    for (int i = warp; i < nk; i += OT_NT / 32) {
+        const OtNode g(G + s.grp[i]);
+        const int first = (int)(g.b.w & 0xFFFFu), count = (int)((g.b.w >> 16) & 0xFFu);
+        bool keep = false;
+        if (lane < count) {
+            const OtNode n(L + first + lane);
+            keep = rt_dist(n.a, n.b, lbq) <= U;
+        }
+        const unsigned m = __ballot_sync(FULL, keep);
+        if (!m) continue;
+        int at = 0;
+        if (lane == 0) at = atomicAdd(&s.nleaf, __popc(m));
+        at = __shfl_sync(FULL, at, 0) + __popc(m & ((1u << lane) - 1u));
+        if (keep && at < OT_LIST) s.leaf[at] = (uint16_t)(first + lane);
+    }
+}
+/* the warp's list from the tile's: its length, or -1 when the lanes have to search alone */
+__device__ __forceinline__ int ot_search_warp(OtSearch &s, const OtWarpBox &b, const MgTreeNode *__restrict__ T,
+                                               const MgTreeNode *__restrict__ L, uint16_t *wl) {
+    const unsigned FULL = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31, n = s.nleaf;
+    if (s.bad || !rt_packed(T) || n > OT_LIST || n == 0) return -1;
+    uint32_t U = 0xFFFFFFFFu;
+    int nw = 0;
+    for (int c = 0; c < n; c += 32) { /* the least upper bound first: the list is short and its leaves come back from L1 */
+        uint32_t u = 0xFFFFFFFFu;
+        if (c + lane < n) {
+            const OtNode q(L + s.leaf[c + lane]);
+            u = rt_ub_or_inf(q.a, q.b, b.ub);
+        }
+        U = min(U, __reduce_min_sync(FULL, u));
+    }
+    for (int c = 0; c < n; c += 32) {
+        bool keep = false;
+        int at = 0;
+        if (c + lane < n) {
+            at = s.leaf[c + lane];
+            const OtNode q(L + at);
+            keep = rt_dist(q.a, q.b, b.lb) <= U;
+        }
+        const unsigned m = __ballot_sync(FULL, keep);
+        const int p = nw + __popc(m & ((1u << lane) - 1u));
+        if (keep && p < OT_WLIST) wl[p] = (uint16_t)at;
+        nw += __popc(m);
+    }
+    __syncwarp();
+    return nw <= OT_WLIST ? nw : -1;
+}
+/* the lane's leaf (its word: biome in the top byte) among the listed ones; false when a distance was clamped */
+__device__ __forceinline__ bool ot_scan(const MgTreeNode *__restrict__ L, const uint16_t *wl, int n, const RtTarget &q, int &biome) {
+    uint32_t best = 0xFFFFFFFFu, w = 0xFFFFu;
+    for (int k = 0; k < n; k++) {
+        const OtNode c(L + wl[k]);
+        const uint32_t d = rt_dist(c.a, c.b, q);
+        if (d < best || (d == best && (c.b.w & 0xFFFFu) < (w & 0xFFFFu))) { best = d; w = c.b.w; }
+    }
+    biome = (int)(w >> 24);
+    return best < (uint32_t)MG_RT_CLAMP * MG_RT_CLAMP;
+}
+/* the biome at target t: from the warp's list, or alone */
+__device__ __forceinline__ int ot_biome(const MgTreeNode *__restrict__ T, const MgTreeNode *__restrict__ L, const uint16_t *wl, int n,
+                                        const int32_t *t) {
+    RtTarget q;
+    int b;
+    if (n >= 0) {
+        rt_target(t, q);
+        if (ot_scan(L, wl, n, q, b)) return b;
+    }
+    uint64_t d;
+    return T[tree_search(T, t, -1, d)].biome;
+}
+
+/* ============================================================================ double branch
+ * The double branch's five climate noises and ridges_folded reach the biome only through quantised targets (steps of 1e-4),
+ * so the tile form evaluates them in 32-bit fixed point with 64-bit accumulators (no FP64 pipe, which the exact shift octaves
+ * of the per-cell form kept 55 % busy) and takes a target when every value within the form's error bound has it
+ * (MgNoise::tile_eq; about 2 % of the cells keep a target open and go to the exact evaluation of a later launch).
+ *
+ * Over a plane of the lattice an octave is V = (1 - W) L0 + W L1 with a row's value L = P + U Q, P = N0 and Q = N1 - N0
+ * linear in the fractions (X, Z): N = A dx + B dz + C, whose A, B and C mix the two planes' gradients by the fixed
+ * coordinate's smoothstep v: A = (1 - v) g0.x + v g1.x.  (The reference lerps x, then y, then z; the order only matters for
+ * its roundings.)  The table holds one edge per pair of nodes (i, k), (i + 1, k): P's and Q's coefficients. */
+struct OtEdge {
+    int4 p; /* P: X and Z coefficients (units of 2^-29), constant (2^-28); Q: X coefficient (2^-30) */
+    int2 q; /* Q: Z coefficient (2^-30), constant (2^-29) */
+};
+/* the fixed coordinate's part of an octave's edges, in units of 2^-30: v, 1 - v, Y (1 - v), (Y - 1) v */
+struct __align__(16) OtFix {
+    int32_t v, w, c0, c1;
+};
+__device__ __forceinline__ OtFix ot_fix(double y, double v) {
+    OtFix f;
+    f.v = __double2int_rn(v * 0x1.0p30);
+    f.w = (1 << 30) - f.v;
+    f.c0 = __double2int_rn(y * (1.0 - v) * 0x1.0p30);
+    f.c1 = __double2int_rn((y - 1.0) * v * 0x1.0p30);
+    return f;
+}
+/* one climate octave in evaluation order; offsets in units of 2^-32, less the first node's cell */
+struct __align__(16) OtOctD {
+    int64_t ox, oz;
+    int32_t nx, off; /* edges per row, place in the table */
+    int32_t k, c29;  /* input factor 2^-k; level constant */
+};
+__device__ __forceinline__ int64_t ot_madw(int32_t a, int32_t b, int64_t c) {
+    int64_t r;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ int32_t ot_hi(int64_t v) { return (int32_t)(v >> 32); }
+__device__ __forceinline__ int32_t ot_sub_sat(int32_t a, int32_t b) {
+    int32_t r;
+    asm("sub.sat.s32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+/* smoothstep of the fraction t (units of 2^-32) in units of 2^-31, within 3e-9: t > 1/2 as 1 - smoothstep(1 - t), and with
+ * t' = 2 t <= 1, t^3 (10 - 15 t + 6 t^2) = t'^3 / 8 (10 - t' (7.5 - 1.5 t')) */
+__device__ __forceinline__ int32_t ot_fade31(uint32_t t) {
+    const int32_t m = (int32_t)t >> 31;
+    const uint32_t tt = (t ^ (uint32_t)m) << 1;
+    const uint32_t t3 = __umulhi(__umulhi(tt, tt), tt);
+    const uint32_t p = (10u << 28) - __umulhi(tt, 15u * (1u << 27) - (tt >> 5) * 3u);
+    return (int32_t)__umulhi(t3, p) ^ (m & 0x7FFFFFFF);
+}
+/* a row's value in units of 2^-60 from its edge; X and dz in units of 2^-31, dz in [-1, 1] */
+__device__ __forceinline__ int64_t ot_row_d(const OtEdge &e, int32_t X, int32_t dz, int32_t U) {
+    const int64_t q = ot_madw(e.p.w, X, ot_madw(e.q.x, dz, (int64_t)(((uint64_t)(uint32_t)e.q.y << 32) | 0x80000000u)));
+    return ot_madw(U, ot_hi(q), ot_madw(e.p.x, X, ot_madw(e.p.y, dz, (int64_t)((uint64_t)(uint32_t)e.p.z << 32))));
+}
+/* the octave in units of 2^-60; X, Z, U, W in units of 2^-31 */
+__device__ __forceinline__ int64_t ot_octave_d(const int4 *__restrict__ P, const int2 *__restrict__ Q, int at, int nx, int32_t X,
+                                               int32_t U, int32_t Z, int32_t W) {
+    const int64_t l0 = ot_row_d(OtEdge{P[at], Q[at]}, X, Z, U);
+    const int64_t l1 = ot_row_d(OtEdge{P[at + nx], Q[at + nx]}, X, (int32_t)((uint32_t)Z - 0x80000000u), U);
+    return ot_madw(W, ot_hi((int64_t)((uint64_t)(l1 - l0) << 1)), l0);
+}
+/* node (i, k) of lattice L in units of 2^-30: (A, B, C) */
+__device__ __forceinline__ void ot_mix(int h0, int h1, bool z0, const OtFix &f, int32_t &A, int32_t &B, int32_t &C) {
+    const int4 g = __ldg(&kGradI[h0 & 15]), h = __ldg(&kGradI[h1 & 15]);
+    A = g.x * f.w + h.x * f.v;
+    B = z0 ? g.y * f.w + h.y * f.v : g.z * f.w + h.z * f.v;
+    C = z0 ? g.z * f.c0 + h.z * f.c1 : g.y * f.c0 + h.y * f.c1;
+}
+/* edge (i, k) - (i + 1, k) */
+__device__ __forceinline__ void ot_edge(const MgLattice &L, bool z0, const OtFix &f, int i, int k, int4 &p, int2 &q) {
+    const PlainPerm P{L.p};
+    const int a = P(i), b = P(i + 1);
+    int h0, h1, h2, h3;
+    if (z0) {
+        const int aa = P(a + k) + L.iz, bb = P(b + k) + L.iz;
+        h0 = P(aa); h1 = P(aa + 1); h2 = P(bb); h3 = P(bb + 1);
+    } else {
+        h0 = P(P(a + L.iy) + k); h1 = P(P(a + L.iy + 1) + k); h2 = P(P(b + L.iy) + k); h3 = P(P(b + L.iy + 1) + k);
+    }
+    int32_t A0, B0, C0, A1, B1, C1;
+    ot_mix(h0, h1, z0, f, A0, B0, C0);
+    ot_mix(h2, h3, z0, f, A1, B1, C1);
+    p = make_int4((A0 + 1) >> 1, (B0 + 1) >> 1, (C0 + 2) >> 2, ot_sub_sat(A1, A0));
+    q = make_int2(ot_sub_sat(B1, B0), (int32_t)(((int64_t)C1 - A1 - C0 + 1) >> 1));
+}
+/* the targets a value within e of v may have (units of 2^-29, 2^-28 for the depth: `scale` is 10000 times the unit): the
+ * rounding to float, the product by 10000 and the truncation are each monotone, so the ends' targets bound it */
+__device__ __forceinline__ void ot_target(int32_t v, int32_t e, float scale, int32_t &a, int32_t &b) {
+    a = __float2int_rz(__int2float_rn(v - e) * scale);
+    b = __float2int_rz(__int2float_rn(v + e) * scale);
+}
+
+/* The offset spline with a bound: at coordinates within ce of the reference's, the value is within `err` of the reference's.
+ * A Hermite segment's value is a convex combination of its two points' values (so their errors pass through at most) plus
+ * a cubic in t, whose slope in the input is at most (|y2 - y1| + 1.25 (|a| + |b|)) / (x2 - x1); the spline is C1, and a
+ * neighbouring segment's slope differs near the joint by its curvature (below 1e5) times ce (below 1e-6), covered by 0.01 and
+ * 0.1; both evaluations' roundings are within 2^-24 (5 |y2 - y1| + 2 max |y| + 6 (|a| + |b|)) each. */
+struct SplineIn {
+    float c, e, r, f;     /* continents, erosion, ridges, ridges_folded */
+    float dc, de, dr, df; /* their bounds */
+};
+/* the value below reference c.  One copy of the code per nesting level, its state in registers: an explicit stack keeps it in
+ * local memory, and measured three times slower here. */
+template <int D>
+__device__ __forceinline__ float spline_err(const MgSpline &S, int c, const SplineIn &x, float &err) {
+    err = 0.0f;
+    if (c < 0) return S.cval[~c];
+    if constexpr (D == 0) {
+        err = 1e30f; /* not reached: a table nests at most MG_SPL_DEPTH levels */
+        return 0.0f;
+    } else {
+        const int o = S.first[c], n = S.npts[c], k = S.coord[c];
+        const float in = k == 0 ? x.c : (k == 1 ? x.e : (k == 2 ? x.r : x.f));
+        const float de = k == 0 ? x.dc : (k == 1 ? x.de : (k == 2 ? x.dr : x.df));
+        int i = -1; /* last point at or below the input */
+        for (int j = 0; j < n; j++) i += in >= S.loc[o + j] ? 1 : 0;
+        const bool ext = i < 0 || i == n - 1;
+        const int p = o + max(i, 0);
+        float y1 = 0.0f, e1 = 0.0f, y2 = 0.0f, e2 = 0.0f;
+#pragma unroll 1
+        for (int q = 0; q < (ext ? 1 : 2); q++) {
+            y1 = y2;
+            e1 = e2;
+            y2 = spline_err<D - 1>(S, S.child[p + q], x, e2);
+        }
+        const float x1 = S.loc[p], d1 = S.der[p];
+        if (ext) { /* linear extension */
+            const float v = d1 * (in - x1);
+            err = e2 + (fabsf(d1) + 0.1f) * de + 1.2e-7f * (4.0f * fabsf(v) + fabsf(y2));
+            return d1 == 0.0f ? y2 : y2 + v;
+        }
+        const float w = S.loc[p + 1] - x1, t = (in - x1) / w, d2 = S.der[p + 1], dy = y2 - y1;
+        const float a = d1 * w - dy, b = -d2 * w + dy;
+        const float ab = fabsf(a) + fabsf(b), ad = fabsf(dy);
+        err = fmaxf(e1, e2) + (__fdividef(ad + 1.25f * ab, w) * 1.001f + 0.1f) * de +
+              1.2e-7f * (5.0f * ad + 2.0f * fmaxf(fabsf(y1), fabsf(y2)) + 6.0f * ab);
+        return lerp<float>(t, y1, y2) + t * (1.0f - t) * lerp<float>(t, a, b);
+    }
+}
+
+}  // namespace mg
+#endif

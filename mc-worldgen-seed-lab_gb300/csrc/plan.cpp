@@ -23,7 +23,7 @@
 
 struct McGb300Plan {
     int nreq = 0;
-    long long ntiles[BATCH_SHAPES] = {0, 0, 0, 0};
+    mg::BatchGroups groups[BATCH_SHAPES] = {};
     long long out_bytes = 0;
     long long h2d_bytes = 0; /* bytes copied to the device by plan_new */
     std::vector<long long> out_off;
@@ -40,9 +40,9 @@ struct McGb300Plan {
     int *d_first = nullptr; /* Overworld: first lattice of each entry, relative to the Overworld list */
     long long ow_lattices = 0;
     MgLattice *d_pool = nullptr;
-    unsigned long long *d_counter = nullptr; /* tiles taken, cells recorded for the exact pass */
-    MgPending *d_pend = nullptr;             /* records of double-branch Overworld cells left to the exact pass */
-    long long pend_cap = 0;
+    unsigned long long *d_counter = nullptr; /* BATCH_COUNTERS */
+    MgOpenCell *d_open = nullptr;            /* records of double-branch Overworld cells left to the exact evaluation */
+    long long open_cap = 0;
     /* graph of one run */
     cudaStream_t cap = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -103,8 +103,8 @@ int enqueue(McGb300Plan *p, uint8_t *d_out, int shape, cudaStream_t st) {
         int rc = mg::launch_setup_list(p->d_worlds, d, p->d_ent[d], p->nent[d], p->d_first, p->ow_lattices, p->d_pool, st);
         if (rc) return rc;
     }
-    return mg::launch_batch(p->d_worlds, p->d_trees, p->d_reqs[shape], p->nreq, p->ntiles[shape], p->d_pool,
-                            p->d_counter, p->d_pend, p->pend_cap, d_out, p->ctas, shape, st);
+    return mg::launch_batch(p->d_worlds, p->d_trees, p->d_reqs[shape], p->groups[shape], p->d_pool, p->d_counter,
+                            p->d_open, p->open_cap, d_out, p->ctas, shape, st);
 }
 
 /* Order a run on `st` after the plan's previous run (on any stream); caller holds the ABI lock. */
@@ -206,25 +206,25 @@ MCGEN_API int mcgen_gb300_plan_new(const McGb300Request *reqs, int n, int tie_ru
         off += p->cells[(size_t)i];
     }
     p->out_bytes = off;
-    long long dcells = 0; /* double-branch Overworld cells: the ones the exact pass may take */
-    for (int i = 0; i < n; i++) {
-        const MgWorldDesc &W = worlds[(size_t)wof[(size_t)i]]->desc;
-        if (W.dim == MG_OVERWORLD && !W.fmode) dcells += p->cells[(size_t)i];
-    }
-    p->pend_cap = tie_rule == MCGEN_TIE_ENGINE ? mg::batch_pending_cap(dcells) : 0;
-    /* processing order: requests grouped by world, heaviest code path first (Overworld double branch, then
+    /* processing order: the batch's groups (batch.h), within the rest grouped by world, heaviest code path first (Overworld double branch, then
      * float, Nether, End), so that the CTAs resident at any time run the same code (the kernel holds every
      * dimension and branch; mixing them thrashes the instruction cache) and the light tiles come last */
     std::vector<int> order((size_t)n);
     for (int i = 0; i < n; i++) order[(size_t)i] = i;
-    std::vector<int> key((size_t)n); /* code path, then world */
+    std::vector<int> wgroup(worlds.size());
+    for (size_t w = 0; w < worlds.size(); w++) wgroup[w] = mg::batch_group(worlds[w]->desc, tie_rule);
+    long long dcells = 0; /* cells of the double branch's tile kernel: the ones it may leave open */
+    for (int i = 0; i < n; i++)
+        if (wgroup[(size_t)wof[(size_t)i]] == BATCH_OW_D) dcells += p->cells[(size_t)i];
+    p->open_cap = mg::ow_open_cap(dcells);
+    std::vector<int> key((size_t)n); /* group, code path, then world */
     for (int i = 0; i < n; i++) {
-        const MgWorldDesc &W = worlds[(size_t)wof[(size_t)i]]->desc;
-        key[(size_t)i] = (W.dim * 2 + (W.fmode ? 1 : 0)) * (int)(worlds.size() + 1) + wof[(size_t)i];
+        const int wi = wof[(size_t)i];
+        const MgWorldDesc &W = worlds[(size_t)wi]->desc;
+        key[(size_t)i] = ((wgroup[(size_t)wi] * 3 + W.dim) * 2 + (W.fmode ? 1 : 0)) * (int)(worlds.size() + 1) + wi;
     }
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return key[(size_t)a] < key[(size_t)b]; });
     for (int s = 0; s < BATCH_SHAPES; s++) {
-        long long tiles = 0;
         for (int i : order) {
             const McGb300Request &r = reqs[i];
             const int wi = wof[(size_t)i];
@@ -233,12 +233,13 @@ MCGEN_API int mcgen_gb300_plan_new(const McGb300Request *reqs, int n, int tie_ru
             b.state = slot[(size_t)i];
             b.qx0 = r.qx0; b.qz0 = r.qz0; b.nx = r.nx; b.nz = r.nz; b.qy = r.qy;
             b.tie = worlds[(size_t)wi]->desc.dim == MG_END ? MG_TIE_ENGINE : tie_rule;
-            b.tile0 = tiles;
+            const int g = wgroup[(size_t)wi];
+            b.tile0 = p->groups[s].tiles[g];
             b.out_off = p->out_off[(size_t)i];
-            tiles += mg::batch_tiles(worlds[(size_t)wi]->desc.dim, r.qx0, r.qz0, r.nx, r.nz, s);
+            p->groups[s].tiles[g] += mg::batch_tiles(g, worlds[(size_t)wi]->desc.dim, r.qx0, r.qz0, r.nx, r.nz, s);
+            p->groups[s].n[g]++;
             rq[s].push_back(b);
         }
-        p->ntiles[s] = tiles;
     }
     /* device copies: the lists are staged back to back (256-byte aligned) and uploaded in one copy; the
      * lattice pool and the tile counter follow them in the same allocation */
@@ -267,8 +268,8 @@ MCGEN_API int mcgen_gb300_plan_new(const McGb300Request *reqs, int n, int tie_ru
     for (const Part &q : parts) memcpy(host.data() + q.off, q.src, q.bytes);
     const size_t pool_off = (at + 255) & ~(size_t)255;
     const size_t counter_off = pool_off + sizeof(MgLattice) * (size_t)pool;
-    const size_t pend_off = counter_off + 2 * sizeof(unsigned long long);
-    const size_t arena_bytes = pend_off + sizeof(MgPending) * (size_t)p->pend_cap;
+    const size_t open_off = counter_off + BATCH_COUNTERS * sizeof(unsigned long long);
+    const size_t arena_bytes = open_off + sizeof(MgOpenCell) * (size_t)p->open_cap;
     cudaMemPool_t mp = nullptr;
     cudaStream_t ast = mg::abi_stream();
     cudaError_t e = plan_pool(&mp);
@@ -280,7 +281,7 @@ MCGEN_API int mcgen_gb300_plan_new(const McGb300Request *reqs, int n, int tie_ru
         for (const Part &q : parts) *q.dst = base + q.off;
         if (pool) p->d_pool = (MgLattice *)(base + pool_off);
         p->d_counter = (unsigned long long *)(base + counter_off);
-        if (p->pend_cap) p->d_pend = (MgPending *)(base + pend_off);
+        if (p->open_cap) p->d_open = (MgOpenCell *)(base + open_off);
         p->h2d_bytes = (long long)staged;
     }
     if (!e) e = (cudaError_t)mg::batch_prepare(nullptr);

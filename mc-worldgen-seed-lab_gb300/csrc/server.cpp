@@ -80,7 +80,7 @@ struct Batch {
     uint8_t *d_out = nullptr; size_t cap_out = 0;
     uint8_t *h_out = nullptr; size_t cap_hout = 0;
     unsigned long long *d_counter = nullptr; /* tiles taken, cells recorded for the exact pass */
-    MgPending *d_pend = nullptr; size_t cap_pend = 0;
+    MgOpenCell *d_open = nullptr; size_t cap_open = 0;
     std::vector<long long> out_off;
 };
 
@@ -197,7 +197,7 @@ int launch_batch(McGb300Server *s, Batch &b) {
     std::vector<MgBatchReq> reqs;
     std::vector<MgSetupEntry> ent[3];
     std::vector<int> first;
-    long long tiles = 0, out = 0, ow = 0;
+    long long out = 0, ow = 0;
     b.tickets.clear();
     b.held.clear();
     b.out_off.clear();
@@ -246,15 +246,23 @@ int launch_batch(McGb300Server *s, Batch &b) {
         T.state = 1;
     }
     if (b.tickets.empty()) return 0;
-    /* processing order grouped by code path, heaviest first (as in a plan), then the tile numbering */
+    /* processing order: the batch's groups, then by code path, heaviest first (as in a plan), then the tile numbering */
+    std::vector<int> wgroup;
+    for (auto *w : worlds) wgroup.push_back(mg::batch_group(w->desc, MG_TIE_ENGINE));
+    auto path = [&](const MgBatchReq &r) {
+        const MgWorldDesc &d = worlds[(size_t)r.world]->desc;
+        return (wgroup[(size_t)r.world] * 3 + d.dim) * 2 + (d.fmode ? 1 : 0);
+    };
     std::stable_sort(reqs.begin(), reqs.end(), [&](const MgBatchReq &x, const MgBatchReq &y) {
-        const MgWorldDesc &a = worlds[(size_t)x.world]->desc, &c = worlds[(size_t)y.world]->desc;
-        const int wa = a.dim * 2 + (a.fmode ? 1 : 0), wc = c.dim * 2 + (c.fmode ? 1 : 0);
-        return wa != wc ? wa < wc : x.world < y.world;
+        const int px = path(x), py = path(y);
+        return px != py ? px < py : x.world < y.world;
     });
+    mg::BatchGroups groups = {};
     for (auto &r : reqs) {
-        r.tile0 = tiles;
-        tiles += mg::batch_tiles(worlds[(size_t)r.world]->desc.dim, r.qx0, r.qz0, r.nx, r.nz, kServeShape);
+        const int g = wgroup[(size_t)r.world];
+        r.tile0 = groups.tiles[g];
+        groups.tiles[g] += mg::batch_tiles(g, worlds[(size_t)r.world]->desc.dim, r.qx0, r.qz0, r.nx, r.nz, kServeShape);
+        groups.n[g]++;
     }
     cudaError_t e = cudaSuccess;
     std::vector<MgWorldDesc> wd;
@@ -279,14 +287,12 @@ int launch_batch(McGb300Server *s, Batch &b) {
         e = cudaMallocHost((void **)&b.h_out, c);
         b.cap_hout = e ? 0 : c;
     }
-    if (!e && !b.d_counter) e = cudaMalloc(&b.d_counter, 2 * sizeof(unsigned long long));
-    long long dcells = 0; /* double-branch Overworld cells: the ones the exact pass may take */
-    for (const auto &r : reqs) {
-        const MgWorldDesc &W = worlds[(size_t)r.world]->desc;
-        if (W.dim == MG_OVERWORLD && !W.fmode) dcells += (long long)r.nx * r.nz;
-    }
-    const long long pend_cap = mg::batch_pending_cap(dcells);
-    if (!e && pend_cap > 0) e = grow_dev(&b.d_pend, &b.cap_pend, (size_t)pend_cap);
+    if (!e && !b.d_counter) e = cudaMalloc(&b.d_counter, BATCH_COUNTERS * sizeof(unsigned long long));
+    long long dcells = 0; /* cells of the double branch's tile kernel: the ones it may leave open */
+    for (const auto &r : reqs)
+        if (wgroup[(size_t)r.world] == BATCH_OW_D) dcells += (long long)r.nx * r.nz;
+    const long long open_cap = mg::ow_open_cap(dcells);
+    if (!e && open_cap > 0) e = grow_dev(&b.d_open, &b.cap_open, (size_t)open_cap);
     if (e) return crc(e);
     if (s->fail_next) { /* injected failure of this step (tests of the failure path) */
         const int f = s->fail_next;
@@ -317,8 +323,8 @@ int launch_batch(McGb300Server *s, Batch &b) {
     /* hits on states another in-flight batch is still building: order after that batch's setup */
     for (int k : wait_on)
         if ((e = cudaStreamWaitEvent(st, s->batches[(size_t)k].setup_done, 0))) return crc(e);
-    int rc = mg::launch_batch(b.d_worlds, b.d_trees, b.d_reqs, (int)reqs.size(), tiles, s->pool[0].base, b.d_counter,
-                              pend_cap > 0 ? b.d_pend : nullptr, pend_cap, b.d_out, 0, kServeShape, st);
+    int rc = mg::launch_batch(b.d_worlds, b.d_trees, b.d_reqs, groups, s->pool[0].base, b.d_counter,
+                              open_cap > 0 ? b.d_open : nullptr, open_cap, b.d_out, 0, kServeShape, st);
     if (rc) return MCGEN_E_INTERNAL;
     if ((e = cudaMemcpyAsync(b.h_out, b.d_out, (size_t)out, cudaMemcpyDeviceToHost, st))) return crc(e);
     if ((e = cudaEventRecord(b.done, st))) return crc(e);
@@ -493,7 +499,7 @@ MCGEN_API void mcgen_gb300_server_free(McGb300Server *s) {
         cudaFree(b.d_out);
         cudaFreeHost(b.h_out);
         cudaFree(b.d_counter);
-        cudaFree(b.d_pend);
+        cudaFree(b.d_open);
     }
     cudaFree(s->pool[0].base);
     delete s;

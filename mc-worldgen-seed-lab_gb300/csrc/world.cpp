@@ -13,6 +13,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <array>
 #include <memory>
 
 #include "../../include/mcgen.h"
@@ -248,6 +249,51 @@ static double screen_bound32(const MgNoise *s) {
     return 1.25 * e;
 }
 
+/* Bounds of the tile kernels' table form (owtile.cuh ot_octave_d) against the reference's double value, in reals; "q" is
+ * 2^-30.
+ * An octave, given its two coordinates' cells and fractions exactly, is V = (1 - W) L0 + W L1, L = (1 - U) N0 + U N1 over
+ * node values N = A dx + B dz + C with |N| <= 2:
+ *  - A, B, C come from the fixed smoothstep rounded to q (half a unit): A, B within q, C within q: N within 3 q;
+ *  - L = P + U Q: P's coefficients rounded to 2 q (1 q each, two of them), its constant to 4 q (2 q); Q's constant to 2 q
+ *    (1 q), the upper word of Q rounded to 2 q (1 q), a saturated coefficient (1 q): L within 3 + 4 + 3 = 10 q;
+ *  - V's difference L1 - L0 is truncated to 2 q: V within 12 q;
+ *  - a smoothstep error e moves V by at most 2.1 e: |N10 - N00| <= 1 + 2 max(dz, 1/2), so the row-weighted difference is at
+ *    most 2.06.  The tables' smoothsteps of the shift (from 59 bits) are within q; the cells' (ot_fade31, folded to
+ *    t <= 1/2, p = 10 - t'(7.5 - 1.5 t') with t' = 2 t in units of 2^-28 within 4 units, times t^3 <= 1/8; t'^2 and t'^3
+ *    truncated at 2^-32; the result truncated at 2^-31) within 3e-9;
+ *  - a coordinate error e moves V by at most 5 e (|dV/dX| <= 1 + 1.875 x 2.06): the shift's coordinates are exact; a climate
+ *    octave's are truncated at 2^-32 and its offset rounded: within 1.5 x 2^-32, and the reference's own rounding of its sum
+ *    within 2 x 2^-32 (|s| < 2^22 up to the world border): 4 x 2^-32 is taken; the linear forms' 31-bit fractions add 2^-32.
+ * TILE_SHIFT_OCT and TILE_OCT are these sums. */
+static const double TILE_SHIFT_OCT = 12.0 * 0x1.0p-30 + 2.0 * 2.1 * 0x1.0p-30 + 2.0 * 0x1.0p-32;
+static const double TILE_OCT = 12.0 * 0x1.0p-30 + 2.0 * 2.1 * 3e-9 + 2.0 * 5.0 * 4.0 * 0x1.0p-32 + 2.0 * 0x1.0p-32;
+/* sum of the levels' constants of one stack, plain and weighted by frequency */
+static void level_sums(const MgNoise *s, double *c, double *cf) {
+    *c = *cf = 0.0;
+    for (int k = 0; k < s->nlev; k++) {
+        const double v = fabs(s->amp_d[k] * s->vf_d[k] * s->vfac);
+        *c += v;
+        *cf += v * s->freq[k];
+    }
+}
+/* tile_eq of the climate noise s, whose coordinates are shifted by 4 x the noise `shift`: two stacks of octaves, each level's
+ * sum truncated to 2^-29 and its constant rounded to half of that, the reference's own error (screen_bound's terms, far
+ * smaller), and the error of the two shifts times the noise's slope (5 per lattice unit; the second stack 1.0182 steeper).
+ * The values must stay below 4: an octave is at most 1.04 in magnitude (the largest corner dots, max(dx + dz, max(dx, dz) + dy)
+ * per plane, weighted by the smoothsteps, over the unit cube), 1.06 is used. */
+static void tile_bounds(MgNoise *shift, MgNoise *s, int n) {
+    double c, cf, sc, scf;
+    level_sums(shift, &sc, &scf);
+    const double es = 2.0 * sc * TILE_SHIFT_OCT + shift->nlev * (2.0 * 0x1.0p-29 + 2.1 * 0x1.0p-30) + 1e-12;
+    for (int i = 0; i < n; i++) {
+        level_sums(&s[i], &c, &cf);
+        double e = 2.0 * c * TILE_OCT + s[i].nlev * (2.0 * 0x1.0p-29 + 2.1 * 0x1.0p-30) + 1e-12;
+        e += 2.0 * 5.0 * 2.0182 * cf * (4.0 * es + 2.0 * 0x1.0p-32 + 0x1.0p-30);
+        s[i].tile_eq = s[i].fix_err < 0.0 || 2.0 * 1.06 * c > 3.95 ? -1 : (int32_t)ceil(e * 0x1.0p29) + 2;
+    }
+    shift->tile_eq = 2.0 * 1.06 * sc > 3.95 ? -1 : 0;
+}
+
 /* PerlinNoise/NormalNoise constants of 26.1/26.2 (engine/mc_noise.h:178-196) */
 static void noise_double(MgNoise *s, const NoiseParams &P, int legacy) {
     memset(s, 0, sizeof *s);
@@ -275,6 +321,10 @@ static void noise_double(MgNoise *s, const NoiseParams &P, int legacy) {
     s->fix_err = screen_bound(s);
     s->fix_eq = s->fix_err < 0.0 ? -1 : (int64_t)ceil(s->fix_err * 0x1.0p59);
     for (int k = 0; k < s->nlev; k++) s->c31[k] = (int64_t)llround(s->amp_d[k] * s->vf_d[k] * s->vfac * 0x1.0p31);
+    for (int k = 0; k < s->nlev; k++) {
+        const double c = s->amp_d[k] * s->vf_d[k] * s->vfac;
+        s->c29[k] = fabs(c) < 3.9 ? (int32_t)llround(c * 0x1.0p29) : 0;
+    }
     const double e32 = screen_bound32(s);
     s->fix_eq32 = e32 < 0.0 ? -1 : (int64_t)ceil(e32 * 0x1.0p59) + 1;
     octave_seeds(s);
@@ -283,6 +333,7 @@ static void noise_double(MgNoise *s, const NoiseParams &P, int legacy) {
 /* NoiseStack layer constants of 26.3 (engine/mc_noise.h:198-252) */
 static void noise_float(MgNoise *s, const NoiseParams &P, int legacy) {
     memset(s, 0, sizeof *s);
+    s->tile_eq = -1;
     s->fix_eq32 = -1;
     s->legacy = legacy;
     s->octs = P.n;
@@ -412,8 +463,16 @@ struct BNode {
 };
 struct TreeBuilder {
     std::vector<BNode> nodes;
+    std::vector<std::array<int32_t, MG_TREE_DIMS>> centre; /* of each node's box: the sorts read these, not the nodes */
     int cpn;
     static int64_t ctr(const BNode &b, int d) { return (b.lo[d] + b.hi[d]) / 2; }
+    int add(const BNode &n) {
+        nodes.push_back(n);
+        std::array<int32_t, MG_TREE_DIMS> c;
+        for (int d = 0; d < MG_TREE_DIMS; d++) c[(size_t)d] = (int32_t)ctr(n, d);
+        centre.push_back(c);
+        return (int)nodes.size() - 1;
+    }
     void bounds(const std::vector<int> &v, size_t s, size_t e, int64_t *lo, int64_t *hi) const {
         for (int d = 0; d < MG_TREE_DIMS; d++) {
             lo[d] = nodes[v[s]].lo[d];
@@ -424,21 +483,17 @@ struct TreeBuilder {
             }
         }
     }
-    bool less_dims(int a, int b, int dim, bool absolute) const {
-        for (int j = 0; j < MG_TREE_DIMS; j++) {
-            int d = (dim + j) % MG_TREE_DIMS;
-            int64_t x = ctr(nodes[a], d), y = ctr(nodes[b], d);
-            if (absolute) { x = x < 0 ? -x : x; y = y < 0 ? -y : y; }
-            if (x != y) return x < y;
-        }
+    bool less_dims(int a, int b, int dim) const {
+        const auto &ca = centre[(size_t)a], &cb = centre[(size_t)b];
+        for (int j = 0, d = dim; j < MG_TREE_DIMS; j++, d = d + 1 == MG_TREE_DIMS ? 0 : d + 1)
+            if (ca[(size_t)d] != cb[(size_t)d]) return ca[(size_t)d] < cb[(size_t)d];
         return false;
     }
     int subtree(const std::vector<int> &kids) {
         BNode n;
         n.kids = kids;
         bounds(kids, 0, kids.size(), n.lo, n.hi);
-        nodes.push_back(n);
-        return (int)nodes.size() - 1;
+        return add(n);
     }
     int build(std::vector<int> items) {
         size_t n = items.size();
@@ -458,7 +513,7 @@ struct TreeBuilder {
         int64_t best_cost = INT64_MAX;
         int best_dim = -1;
         for (int d = 0; d < MG_TREE_DIMS; d++) {
-            std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return less_dims(a, b, d, false); });
+            std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return less_dims(a, b, d); });
             int64_t cost = 0;
             for (size_t b = 0; b < nb; b++) {
                 int64_t lo[MG_TREE_DIMS], hi[MG_TREE_DIMS];
@@ -512,8 +567,7 @@ static int load_tree(const char *root, int version, int dim, std::vector<MgTreeN
         b.lo[6] = b.hi[6] = atoll(t[12].c_str());
         b.biome = biome_from_key(t[13].c_str());
         if (b.biome < 0) { *err = "unknown biome " + t[13]; return MCGEN_E_DATA; }
-        tb.nodes.push_back(b);
-        leaves.push_back((int)tb.nodes.size() - 1);
+        leaves.push_back(tb.add(b));
     }
     if (leaves.empty()) { *err = "no biome parameters in " + path; return MCGEN_E_DATA; }
     *nleaf = (int)leaves.size();
@@ -569,6 +623,88 @@ static int load_tree(const char *root, int version, int dim, std::vector<MgTreeN
     }
     if (!out->empty() && (*out)[0].count > 0 && packed) (*out)[0].biome = MG_TREE_PACKED;
     return MCGEN_OK;
+}
+
+/* The leaves of a flattened tree clustered into groups of up to 32 (MgWorldDesc::group_off), appended to it.  A set of leaves
+ * is split at a multiple of 32 near its middle by the centre in the dimension whose halves' boxes are smallest. */
+static void append_groups(std::vector<MgTreeNode> *tree, MgWorldDesc *D) {
+    std::vector<MgTreeNode> leaves;
+    std::vector<int> todo{0};
+    while (!todo.empty()) { /* depth first, children in order */
+        const int nd = todo.back();
+        todo.pop_back();
+        const MgTreeNode n = (*tree)[(size_t)nd];
+        if (n.count == 0) {
+            MgTreeNode l = n;
+            l.first = (uint16_t)leaves.size();
+            leaves.push_back(l);
+        }
+        for (int c = n.count - 1; c >= 0; c--) todo.push_back(n.first + c);
+    }
+    std::vector<int> order(leaves.size());
+    for (size_t i = 0; i < order.size(); i++) order[i] = (int)i;
+    auto extent = [&](size_t s, size_t e) {
+        int64_t sum = 0;
+        for (int d = 0; d < 6; d++) {
+            int lo = 32767, hi = -32768;
+            for (size_t i = s; i < e; i++) {
+                lo = std::min(lo, (int)leaves[(size_t)order[i]].lo[d]);
+                hi = std::max(hi, -(int)leaves[(size_t)order[i]].nhi[d]);
+            }
+            sum += hi - lo;
+        }
+        return sum;
+    };
+    std::vector<std::pair<size_t, size_t>> work{{0, order.size()}}, groups;
+    while (!work.empty()) {
+        const auto [s, e] = work.back();
+        work.pop_back();
+        if (e - s <= 32) {
+            groups.push_back({s, e});
+            continue;
+        }
+        const size_t m = s + ((e - s + 32) / 64) * 32;
+        int best = 0;
+        int64_t cost = INT64_MAX;
+        auto split = [&](int d) {
+            std::nth_element(order.begin() + (long)s, order.begin() + (long)m, order.begin() + (long)e, [&](int a, int b) {
+                const int x = leaves[(size_t)a].lo[d] - leaves[(size_t)a].nhi[d], y = leaves[(size_t)b].lo[d] - leaves[(size_t)b].nhi[d];
+                return x != y ? x < y : a < b;
+            });
+        };
+        for (int d = 0; d < 6; d++) {
+            split(d);
+            const int64_t c = extent(s, m) + extent(m, e);
+            if (c < cost) {
+                cost = c;
+                best = d;
+            }
+        }
+        split(best);
+        work.push_back({m, e});
+        work.push_back({s, m});
+    }
+    D->group_off = (int32_t)tree->size();
+    D->groups = (int32_t)groups.size();
+    D->leaf_off = D->group_off + D->groups;
+    for (const auto &g : groups) {
+        MgTreeNode n;
+        memset(&n, 0, sizeof n);
+        n.d7 = 0xFFFFFFFFu;
+        for (int d = 0; d < 6; d++) n.lo[d] = n.nhi[d] = 32767;
+        for (size_t i = g.first; i < g.second; i++) {
+            const MgTreeNode &l = leaves[(size_t)order[i]];
+            for (int d = 0; d < 6; d++) {
+                n.lo[d] = std::min(n.lo[d], l.lo[d]);
+                n.nhi[d] = std::min(n.nhi[d], l.nhi[d]);
+            }
+            n.d7 = std::min(n.d7, l.d7);
+        }
+        n.first = (uint16_t)g.first;
+        n.count = (uint8_t)(g.second - g.first);
+        tree->push_back(n);
+    }
+    for (int i : order) tree->push_back(leaves[(size_t)i]);
 }
 
 int build_world(const char *root, int version, int dim, const char *preset, MgWorldDesc *D,
@@ -677,6 +813,7 @@ int build_world(const char *root, int version, int dim, const char *preset, MgWo
         D->nether[1].base = 2 * D->nether[0].nlev;
         nt = 2 * (D->nether[0].nlev + D->nether[1].nlev);
     }
+    if (dim == MG_OVERWORLD && !D->fmode) tile_bounds(&D->noise[0], &D->noise[1], MG_OW_NOISES - 1);
     if (nt > MG_MAX_TABLES) { *err = "too many octaves"; return MCGEN_E_DATA; }
     D->ntables = nt;
     /* ridges_folded in fixed point (the screen of the ridge noise): the constants must be multiples of 2^-59
@@ -705,6 +842,7 @@ int build_world(const char *root, int version, int dim, const char *preset, MgWo
     D->tree_leaves = nleaf;
     D->tree_fanout = 0;
     for (const MgTreeNode &n : *tree) D->tree_fanout = std::max(D->tree_fanout, (int32_t)n.count);
+    append_groups(tree, D);
     return MCGEN_OK;
 }
 
