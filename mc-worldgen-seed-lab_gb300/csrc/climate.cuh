@@ -591,15 +591,14 @@ __device__ int cell_chunk_chain(const MgWorldDesc &W, const MgSpline &S, const M
  * own search is the warp-shared walk; the chain (rare) runs per lane. */
 template <bool FM, int DIM>
 __device__ __forceinline__ int cell_chunk_warp(const MgWorldDesc &W, const MgSpline &S, const MgLattice *__restrict__ T,
-                                               const MgTreeNode *__restrict__ tree, int qx, int qy, int qz, bool active,
-                                               WarpTreeScratch &ws) {
+                                               const MgTreeNode *__restrict__ tree, int qx, int qy, int qz, bool active) {
     const int qmin = W.min_y >> 2, qh = W.height >> 2;
     const int cy = qy < qmin ? qmin : (qy > qmin + qh - 1 ? qmin + qh - 1 : qy);
     int32_t tg[6] = {0, 0, 0, 0, 0, 0};
     if (active) cell_target<FM, DIM>(W, S, T, qx, cy, qz, tg);
     uint64_t d = 0;
     bool tied = false;
-    const int leaf = tree_search_tie_warp(tree, tg, active, ws, d, tied);
+    const int leaf = tree_search_tie_warp(tree, W, tg, active, d, tied);
     if (!active) return -1;
     return cell_chunk_chain<FM, DIM>(W, S, T, tree, qx, qy, qz, tg, leaf, d, tied);
 }

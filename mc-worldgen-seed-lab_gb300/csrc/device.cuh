@@ -1052,206 +1052,164 @@ __device__ __forceinline__ int tree_search_tie(const MgTreeNode *__restrict__ T,
     return tree_search_tie_stack(T, t, best, tied);
 }
 
-/* ------------------------------------------------------------------ warp-shared R-tree candidates
- * The search's result is the first leaf in depth-first order at the minimum distance (a child is entered
- * iff its box is closer than the best leaf so far, a leaf replaces it iff strictly closer; every ancestor of
- * the first minimal leaf is at most as far, so the walk reaches it, and nothing after it is strictly closer).
- * So any list of leaves, in depth-first order, that holds every leaf able to be at the minimum for a target
- * gives the same leaf when scanned for the first strict minimum.  A warp's 32 cells are neighbours (an 8 x 4
- * block of a tile) with close targets: for the box B spanning them, a leaf whose distance to B (lower bound
- * over B) exceeds U, the least over leaves of their largest distance to a point of B, is farther than some
- * leaf for every target in B.  One walk per warp (the lanes take a node's children, up to 32 at once) lists
- * the leaves with lower bound <= U in depth-first order, U shrinking as leaves are met and starting from the
- * leaf a greedy descent reaches; each lane then scans only that list.  Both bounds use the packed 16-bit
- * distances with B's corners in place of the target (max(lo - Bhi, Blo - hi, 0) and max(lo - Blo, Bhi - hi,
- * 0) per dimension): a clamped lower bound is still a lower bound, and an upper bound is used only when
- * below MG_RT_CLAMP^2, where no dimension was clamped.  A list or stack that would overflow gives up (-1)
- * and the lanes search alone. */
-#define MG_WC_CAND 128
-#define MG_WC_STACK 128
-/* the shared walk pays when a node's children fill most of a warp's lanes: trees built with 19 children per
- * node (26.3 on) take it; with 6 per node (26.1, 26.2) each step would use 6 of 32 lanes, and the lanes'
- * own level-unrolled searches measured faster */
-#define MG_WARP_TREE_FANOUT 12
-struct WarpTreeScratch {
-    uint16_t cand[MG_WC_CAND];
-    uint16_t stack[MG_WC_STACK];
-};
+/* ------------------------------------------------------------------ warp-shared R-tree search
+ * The search's result is the leaf of least distance, the first in depth-first order among equals (a child is entered iff its
+ * box is closer than the best leaf so far, a leaf replaces it iff strictly closer; every ancestor of that leaf is at most as
+ * far, so the walk reaches it, and nothing after it is strictly closer).  So any order of visiting gives the same leaf when
+ * equals are decided by the leaves' depth-first ranks.  A warp of neighbouring cells has close targets, so one pruning serves
+ * its 32 lanes: with B the box of the targets, a leaf or group of leaves whose distance to B (a lower bound for every lane)
+ * exceeds U matters to no lane, where U is the lesser of the least "largest distance of a leaf to a point of B" met and the
+ * largest of the lanes' best distances.  The leaves come in groups of 32 and clusters of 32 groups (MgWorldDesc::group_off;
+ * 238 groups in 8 clusters for the Overworld's 7,600 leaves); lanes test 32 boxes at once, the nearest cluster and its nearest
+ * group are taken first, then what is still within U, and every lane evaluates a group's surviving leaves (about 23 a warp
+ * on real targets, where a lane alone visits 120 to 200 nodes).  It works for any tree shape (26.1's nodes
+ * have 6 children, 26.3's 19).  Both bounds use the packed 16-bit distances with B's corners in place of the target
+ * (max(lo - Bhi, Blo - hi, 0) and max(lo - Blo, Bhi - hi, 0) per dimension): a clamped lower bound is still a lower bound, and
+ * an upper bound is used only when below MG_RT_CLAMP^2, where no dimension was clamped. */
 __device__ __forceinline__ uint32_t rt_ub_or_inf(const uint4 &a, const uint4 &b, const RtTarget &ubq) {
     const uint32_t u = rt_dist(a, b, ubq);
     return u < (uint32_t)MG_RT_CLAMP * MG_RT_CLAMP ? u : 0xFFFFFFFFu;
 }
-/* all 32 lanes call it with the same box; returns the number of candidates in ws.cand, or -1 */
-__device__ __forceinline__ int warp_tree_candidates(const MgTreeNode *__restrict__ T, const RtTarget &lbq,
-                                                    const RtTarget &ubq, WarpTreeScratch &ws) {
+struct RtNode {
+    uint4 a, b;
+    __device__ __forceinline__ RtNode(const MgTreeNode *n)
+        : a(*reinterpret_cast<const uint4 *>(n)), b(*(reinterpret_cast<const uint4 *>(n) + 1)) {}
+};
+/* the nearest leaf (counted from leaf_off), its word and distance, leaves at that distance (capped at 2) */
+struct RtWarp {
+    uint32_t best, word;
+    int leaf, cnt;
+};
+template <bool TIE>
+__device__ __forceinline__ void rt_warp_leaf(const RtNode &n, int at, const RtTarget &q, RtWarp &r) {
+    const uint32_t d = rt_dist(n.a, n.b, q);
+    const bool lt = d < r.best, eq = d == r.best;
+    if (TIE) r.cnt = lt ? 1 : (eq ? min(r.cnt + 1, 2) : r.cnt);
+    if (lt || (eq && (n.b.w & 0xFFFFu) < (r.word & 0xFFFFu))) {
+        r.best = d;
+        r.word = n.b.w;
+        r.leaf = at;
+    }
+}
+/* leaves [32 g, 32 g + 32) of the clustered ones, the last group's fewer; ub: bound U by the group's own upper bounds first */
+template <bool TIE>
+__device__ __forceinline__ void rt_warp_group(const MgTreeNode *__restrict__ L, int leaves, int g, bool ub, const RtTarget &q,
+                                              const RtTarget &lbq, const RtTarget &ubq, bool active, uint32_t &U, RtWarp &r) {
+    const unsigned FULL = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31, first = 32 * g;
+    const MgTreeNode *G = L + first;
+    const bool in = first + lane < leaves;
+    const RtNode n(G + (in ? lane : 0));
+    const uint32_t lb = rt_dist(n.a, n.b, lbq);
+    if (ub) U = min(U, __reduce_min_sync(FULL, rt_ub_or_inf(n.a, n.b, ubq)));
+    unsigned m = __ballot_sync(FULL, in && lb <= U);
+    if (!m) return;
+    while (m) { /* two at a time: their loads and distances overlap */
+        const int i = __ffs((int)m) - 1;
+        m &= m - 1;
+        const int j = m ? __ffs((int)m) - 1 : -1;
+        m &= m - 1;
+        const RtNode n0(G + i), n1(G + max(j, 0));
+        rt_warp_leaf<TIE>(n0, first + i, q, r);
+        if (j >= 0) rt_warp_leaf<TIE>(n1, first + j, q, r);
+    }
+    U = min(U, __reduce_max_sync(FULL, active ? r.best : 0u));
+}
+/* all 32 lanes call it; false (for the whole warp) when the tree or an active lane's target is outside the packed range: the
+ * lanes search alone.  An active lane's best below MG_RT_CLAMP^2 is exact, else it searches alone.  hint: any leaf (counted
+ * from leaf_off), best one near the lane's target (the lane's last result): it bounds the search from the start.  With none
+ * (-1) every group's leaves give upper bounds too (without either, 43 leaves a warp were evaluated instead of 23). */
+template <bool TIE>
+__device__ __forceinline__ bool rt_warp(const MgTreeNode *__restrict__ T, const MgWorldDesc &W, const int32_t *t, bool active,
+                                        int hint, RtWarp &r) {
     const unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
-    const uint32_t rw = reinterpret_cast<const uint4 *>(T)[1].w;
-    /* greedy descent to a leaf (the child nearest to B at each level) for the first bound */
-    uint32_t U = 0xFFFFFFFFu;
-    {
-        int first = (int)(rw & 0xFFFFu), count = (int)((rw >> 16) & 0xFFu);
-        for (int depth = 0; depth < MG_RT_STACK; depth++) {
-            if (count > 32) return -1; /* one lane per child */
-            uint32_t lb = 0xFFFFFFFFu, w = 0;
-            if (lane < count) {
-                const uint4 a = *reinterpret_cast<const uint4 *>(T + first + lane);
-                const uint4 b = *(reinterpret_cast<const uint4 *>(T + first + lane) + 1);
-                lb = rt_dist(a, b, lbq);
-                w = b.w;
-            }
-            const uint32_t m = __reduce_min_sync(FULL, lb);
-            const int pick = __ffs(__ballot_sync(FULL, lb == m)) - 1;
-            const uint32_t pw = __shfl_sync(FULL, w, pick);
-            if (((pw >> 16) & 0xFFu) == 0) {
-                const uint4 a = *reinterpret_cast<const uint4 *>(T + first + pick);
-                const uint4 b = *(reinterpret_cast<const uint4 *>(T + first + pick) + 1);
-                U = rt_ub_or_inf(a, b, ubq);
-                break;
-            }
-            first = (int)(pw & 0xFFFFu);
-            count = (int)((pw >> 16) & 0xFFu);
-        }
-    }
-    /* depth-first walk; the stack holds pending nodes with the earliest in depth-first order on top */
-    int sp = 1, nc = 0;
-    if (lane == 0) ws.stack[0] = 0;
-    __syncwarp();
-    while (sp > 0) {
-        const int node = ws.stack[--sp];
-        const uint32_t nw = reinterpret_cast<const uint4 *>(T + node)[1].w;
-        __syncwarp(); /* every lane has read the top before it is overwritten */
-        const int count = (int)((nw >> 16) & 0xFFu);
-        if (count == 0) { /* a leaf queued behind an internal sibling: it is next in depth-first order */
-            if (nc >= MG_WC_CAND) return -1;
-            if (lane == 0) ws.cand[nc] = (uint16_t)node;
-            nc++;
-            __syncwarp();
-            continue;
-        }
-        if (count > 32) return -1;
-        const int ci = (int)(nw & 0xFFFFu) + lane;
-        bool keep = false, leaf = false;
-        uint32_t ub = 0xFFFFFFFFu;
-        if (lane < count) {
-            const uint4 a = *reinterpret_cast<const uint4 *>(T + ci);
-            const uint4 b = *(reinterpret_cast<const uint4 *>(T + ci) + 1);
-            keep = rt_dist(a, b, lbq) <= U;
-            leaf = ((b.w >> 16) & 0xFFu) == 0;
-            if (keep && leaf) ub = rt_ub_or_inf(a, b, ubq);
-        }
-        U = min(U, __reduce_min_sync(FULL, ub));
-        const unsigned km = __ballot_sync(FULL, keep);
-        const unsigned im = __ballot_sync(FULL, keep && !leaf);
-        /* leaves before the first internal survivor come next in depth-first order: listed now; the first
-         * internal survivor and everything after it are pushed, the first on top */
-        const unsigned em = im ? km & ((1u << (__ffs(im) - 1)) - 1u) : km;
-        const unsigned pm = km & ~em;
-        const unsigned lt = (1u << lane) - 1u;
-        const int ne = __popc(em), np = __popc(pm);
-        if (nc + ne > MG_WC_CAND || sp + np > MG_WC_STACK) return -1;
-        if ((em >> lane) & 1u) ws.cand[nc + __popc(em & lt)] = (uint16_t)ci;
-        if ((pm >> lane) & 1u) ws.stack[sp + np - 1 - __popc(pm & lt)] = (uint16_t)ci;
-        nc += ne;
-        sp += np;
-        __syncwarp();
-    }
-    return nc;
-}
-/* first strict minimum of the packed distance over the listed leaves (the same for every lane's loop); with
- * TIE, also the leaves at that minimum, capped at 2 (the list holds every leaf that can be at the minimum, so
- * the count is the tree's) */
-template <bool TIE = false>
-__device__ __forceinline__ RtState rt_scan(const MgTreeNode *__restrict__ T, const uint16_t *cand, int n,
-                                           const RtTarget &q) {
-    RtState s{0xFFFFFFFFu, -1, 0};
-    for (int k = 0; k < n; k++) {
-        const int ci = cand[k];
-        const uint4 a = *reinterpret_cast<const uint4 *>(T + ci);
-        const uint4 b = *(reinterpret_cast<const uint4 *>(T + ci) + 1);
-        const uint32_t d = rt_dist(a, b, q);
-        if (d < s.best) { s.best = d; s.res = ci; s.cnt = 1; }
-        else if (TIE && d == s.best && s.cnt < 2) s.cnt++;
-    }
-    return s;
-}
-/* tree_search (no candidate) for the 32 cells of a warp, called by all 32 lanes; lanes with active == false
- * take part in the walk and get -1.  Falls back to each lane's own search when the tree or a target is
- * outside the packed range or the list overflows, and to the 64-bit search when a lane's distance was
- * clamped. */
-__device__ __forceinline__ int tree_search_warp(const MgTreeNode *__restrict__ T, const int32_t *t, bool active,
-                                                WarpTreeScratch &ws) {
-    const unsigned FULL = 0xFFFFFFFFu;
+    r.best = 0xFFFFFFFFu;
+    r.word = 0xFFFFu;
+    r.leaf = -1;
+    r.cnt = 0;
     RtTarget q{};
     const bool ok = !active || rt_target(t, q);
-    const unsigned act = __ballot_sync(FULL, active);
-    if (!act) return -1;
-    int n = -1;
-    if (rt_packed(T) && __all_sync(FULL, ok)) {
-        int32_t lo[6], hi[6];
-        for (int k = 0; k < 6; k++) {
-            lo[k] = __reduce_min_sync(FULL, active ? t[k] : 0x7FFFFFFF);
-            hi[k] = __reduce_max_sync(FULL, active ? t[k] : (int32_t)0x80000000);
-        }
-        RtTarget lbq, ubq;
-        for (int k = 0; k < 3; k++) {
-            lbq.p[k] = pack16(lo[2 * k], lo[2 * k + 1]);
-            lbq.n[k] = pack16(-hi[2 * k], -hi[2 * k + 1]);
-            ubq.p[k] = pack16(hi[2 * k], hi[2 * k + 1]);
-            ubq.n[k] = pack16(-lo[2 * k], -lo[2 * k + 1]);
-        }
-        n = warp_tree_candidates(T, lbq, ubq, ws);
+    if (!__all_sync(FULL, ok) || !rt_packed(T)) return false;
+    RtTarget lbq, ubq;
+    bool none = false;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int32_t l0 = __reduce_min_sync(FULL, active ? t[2 * k] : 0x7FFFFFFF), h0 = __reduce_max_sync(FULL, active ? t[2 * k] : -0x7FFFFFFF);
+        const int32_t l1 = __reduce_min_sync(FULL, active ? t[2 * k + 1] : 0x7FFFFFFF), h1 = __reduce_max_sync(FULL, active ? t[2 * k + 1] : -0x7FFFFFFF);
+        none = l0 > h0;
+        lbq.p[k] = pack16(l0, l1);
+        lbq.n[k] = pack16(-h0, -h1);
+        ubq.p[k] = pack16(h0, h1);
+        ubq.n[k] = pack16(-l0, -l1);
     }
-    if (n >= 0) {
-        const RtState s = rt_scan(T, ws.cand, n, q);
-        __syncwarp(); /* the list is read by every lane before the warp's next walk */
-        if (!active) return -1;
-        if (s.res >= 0 && s.best < (uint32_t)MG_RT_CLAMP * MG_RT_CLAMP) return s.res;
-        uint64_t d;
-        return tree_search_stack(T, t, -1, d);
+    if (none) return true; /* no active lane */
+    const int groups = W.groups, leaves = W.tree_leaves;
+    const MgTreeNode *G = T + W.group_off, *L = T + W.leaf_off;
+    uint32_t U = 0xFFFFFFFEu;
+    if (hint >= 0) {
+        /* the hinted leaf's distance bounds the lane's; the leaf itself is met again on the way */
+        const RtNode n(L + hint);
+        const uint32_t d = rt_dist(n.a, n.b, q);
+        r.best = d + 1u;
+        U = min(__reduce_max_sync(FULL, active ? d : 0u), __reduce_min_sync(FULL, active ? rt_ub_or_inf(n.a, n.b, ubq) : 0xFFFFFFFFu));
     }
+    for (int s0 = 0; 32 * s0 < groups; s0 += 32) { /* up to 32 clusters of 32 groups (the Overworld has 8) */
+        const int ns = min((groups + 31) / 32 - s0, 32);
+        uint32_t ls = 0xFFFFFFFFu;
+        if (lane < ns) {
+            const RtNode n(T + W.cluster_off + s0 + lane);
+            ls = rt_dist(n.a, n.b, lbq);
+        }
+        /* the nearest cluster first, and in it the nearest group */
+        const uint32_t wm = __reduce_min_sync(FULL, ls);
+        unsigned todo = __ballot_sync(FULL, ls <= U);
+        int s = __ffs((int)__ballot_sync(FULL, ls == wm)) - 1;
+        bool first = s0 == 0;
+        while (todo) {
+            todo &= ~(1u << s);
+            const int g0 = 32 * (s0 + s), ng = min(groups - g0, 32);
+            uint32_t l = 0xFFFFFFFFu;
+            if (lane < ng) {
+                const RtNode n(G + g0 + lane);
+                l = rt_dist(n.a, n.b, lbq);
+            }
+            unsigned p = __ballot_sync(FULL, l <= U);
+            int j = first ? __ffs((int)__ballot_sync(FULL, l == __reduce_min_sync(FULL, l))) - 1 : __ffs((int)p) - 1;
+            while (p) {
+                p &= ~(1u << j);
+                rt_warp_group<TIE>(L, leaves, g0 + j, first || hint < 0, q, lbq, ubq, active, U, r);
+                first = false;
+                p &= __ballot_sync(FULL, l <= U);
+                j = __ffs((int)p) - 1;
+            }
+            todo &= __ballot_sync(FULL, ls <= U);
+            s = __ffs((int)todo) - 1;
+        }
+    }
+    return true;
+}
+/* tree_search (no candidate) for the 32 neighbouring cells of a warp, called by all 32 lanes; inactive lanes get -1 */
+__device__ __forceinline__ int tree_search_warp(const MgTreeNode *__restrict__ T, const MgWorldDesc &W, const int32_t *t, bool active,
+                                                int hint = -1) {
+    RtWarp r;
+    const bool shared = rt_warp<false>(T, W, t, active, hint, r);
     if (!active) return -1;
     uint64_t d;
-    return tree_search(T, t, -1, d);
+    if (!shared) return tree_search(T, t, -1, d);
+    return r.leaf >= 0 && r.best < (uint32_t)MG_RT_CLAMP * MG_RT_CLAMP ? W.leaf_off + r.leaf : tree_search_stack(T, t, -1, d);
 }
-/* tree_search_tie for the 32 neighbouring cells of a warp (all lanes call it; inactive lanes get -1): the
- * first leaf at the minimum, its distance and whether a second leaf has the same distance */
-__device__ __forceinline__ int tree_search_tie_warp(const MgTreeNode *__restrict__ T, const int32_t *t, bool active,
-                                                    WarpTreeScratch &ws, uint64_t &best, bool &tied) {
-    const unsigned FULL = 0xFFFFFFFFu;
-    RtTarget q{};
-    const bool ok = !active || rt_target(t, q);
-    const unsigned act = __ballot_sync(FULL, active);
-    if (!act) return -1;
-    int n = -1;
-    if (rt_packed(T) && __all_sync(FULL, ok)) {
-        int32_t lo[6], hi[6];
-        for (int k = 0; k < 6; k++) {
-            lo[k] = __reduce_min_sync(FULL, active ? t[k] : 0x7FFFFFFF);
-            hi[k] = __reduce_max_sync(FULL, active ? t[k] : (int32_t)0x80000000);
-        }
-        RtTarget lbq, ubq;
-        for (int k = 0; k < 3; k++) {
-            lbq.p[k] = pack16(lo[2 * k], lo[2 * k + 1]);
-            lbq.n[k] = pack16(-hi[2 * k], -hi[2 * k + 1]);
-            ubq.p[k] = pack16(hi[2 * k], hi[2 * k + 1]);
-            ubq.n[k] = pack16(-lo[2 * k], -lo[2 * k + 1]);
-        }
-        n = warp_tree_candidates(T, lbq, ubq, ws);
-    }
-    if (n >= 0) {
-        const RtState s = rt_scan<true>(T, ws.cand, n, q);
-        __syncwarp();
-        if (!active) return -1;
-        if (s.res >= 0 && s.best < (uint32_t)MG_RT_CLAMP * MG_RT_CLAMP) {
-            best = s.best;
-            tied = s.cnt >= 2;
-            return s.res;
-        }
-        return tree_search_tie_stack(T, t, best, tied);
-    }
+/* tree_search_tie likewise: the nearest leaf, its distance and whether a second leaf has the same distance */
+__device__ __forceinline__ int tree_search_tie_warp(const MgTreeNode *__restrict__ T, const MgWorldDesc &W, const int32_t *t, bool active,
+                                                    uint64_t &best, bool &tied) {
+    RtWarp r;
+    const bool shared = rt_warp<true>(T, W, t, active, -1, r);
     if (!active) return -1;
-    return tree_search_tie(T, t, best, tied);
+    if (!shared) return tree_search_tie(T, t, best, tied);
+    if (r.leaf < 0 || r.best >= (uint32_t)MG_RT_CLAMP * MG_RT_CLAMP) return tree_search_tie_stack(T, t, best, tied);
+    best = r.best;
+    tied = r.cnt >= 2;
+    return W.leaf_off + r.leaf;
 }
 
 /* (long)(v * 10000f) */

@@ -227,14 +227,13 @@ __global__ void __launch_bounds__(128) k_grid(const __grid_constant__ MgWorldDes
     const int ix = tx0 + col, iz = tz0 + row;
     const bool in = ix < nx && iz < nz;
     const long long g = (long long)iz * nx + ix;
-    if (FM && !CHAIN && DIM == MG_OVERWORLD && W.tree_fanout >= MG_WARP_TREE_FANOUT) { /* one pruned walk per warp */
-        __shared__ WarpTreeScratch wt[4];
+    if (FM && !CHAIN && DIM == MG_OVERWORLD) { /* one pruned search per warp */
         int32_t tg[6] = {0, 0, 0, 0, 0, 0};
         if (in) {
             if (FM && tabf) climate_ow_f_tab(W, *S, T, *tabf, col, row, qx0 + ix, qy, qz0 + iz, tg);
             else cell_target<FM, DIM>(W, *S, T, qx0 + ix, qy, qz0 + iz, tg);
         }
-        const int leaf = tree_search_warp(tree, tg, in, wt[threadIdx.x >> 5]);
+        const int leaf = tree_search_warp(tree, W, tg, in);
         if (in) out[g] = tree[leaf].biome;
         return;
     }
@@ -317,19 +316,17 @@ __global__ void __launch_bounds__(128, 6) k_blockgrid(const __grid_constant__ Mg
         stage(W, state, W.ntables, T, S, DIM == MG_OVERWORLD);
         __syncthreads();
     }
-    /* grids of a wide tree (the launcher sizes the grid in tiles for this form): the CTA takes a 16 x 8-cell tile
-     * and each warp an 8 x 4 block of it, neighbours whose targets are close, so the cells' own R-tree searches share one pruned walk (the
-     * chunk-cell chain, rare, stays per lane); not for scattered points or sparse grids, whose warps' targets
-     * are unrelated */
-    if (FM && DIM == MG_OVERWORLD && !xyz && step <= 16 && W.tree_fanout >= MG_WARP_TREE_FANOUT) {
-        __shared__ WarpTreeScratch wt[4];
+    /* grids (the launcher sizes the grid in tiles for this form): the CTA takes a 16 x 8-cell tile and each warp an 8 x 4 block
+     * of it, neighbours whose targets are close, so the cells' own R-tree searches share one pruning (the chunk-cell chain,
+     * rare, stays per lane); not for scattered points or sparse grids, whose warps' targets are unrelated */
+    if (FM && DIM == MG_OVERWORLD && !xyz && step <= 16) {
         const int tw = (nx + 15) / 16, w = threadIdx.x >> 5, l = threadIdx.x & 31;
         const int ix = (int)(blockIdx.x % tw) * 16 + (w & 1) * 8 + (l & 7);
         const int iz = (int)(blockIdx.x / tw) * 8 + (w >> 1) * 4 + (l >> 3);
         const bool in = ix < nx && iz < nz;
         int cx = 0, cy = 0, cz = 0;
         if (in) zoom_cell(zseed, x0 + ix * step, y, z0 + iz * step, cx, cy, cz);
-        const int b = cell_chunk_warp<FM, DIM>(W, *S, T, tree, cx, cy, cz, in, wt[w]);
+        const int b = cell_chunk_warp<FM, DIM>(W, *S, T, tree, cx, cy, cz, in);
         if (in) out[(long long)iz * nx + ix] = (uint8_t)b;
         return;
     }
@@ -546,7 +543,7 @@ static void blockgrid_t(const MgWorldDesc &W, const MgTreeNode *tree, const MgLa
     if (sm) cudaFuncSetAttribute(k_blockgrid<FM, DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     ProfScope ps_(K_BLOCKGRID, st);
     /* the kernel's warp-tile form (its own test of the same condition): one CTA per 16 x 8-cell tile */
-    const bool tiles = FM && DIM == MG_OVERWORLD && !xyz && step <= 16 && W.tree_fanout >= MG_WARP_TREE_FANOUT;
+    const bool tiles = FM && DIM == MG_OVERWORLD && !xyz && step <= 16;
     const unsigned nb = tiles ? (unsigned)(((long long)(nx + 15) / 16) * ((nz + 7) / 8)) : blocks_for((long long)nx * nz, 128);
     k_blockgrid<FM, DIM><<<nb, 128, sm, st>>>(W, tree, state, zseed, x0, z0, nx, nz, step, y, xyz, out, cls, ecx0, ecz0,
                                               encx);

@@ -48,11 +48,11 @@ typedef struct {
      * reference's double value in units of 2^-59 (rounded up; < 0: not screened this way) */
     int64_t c31[MG_MAX_OCT];
     int64_t fix_eq32;
-    /* double branch, the tile kernels' table form: amp_d[k] * vf_d[k] * vfac times 2^29 rounded, and the bound on the
-     * difference between its value and the reference's double value in units of 2^-29 (rounded up; < 0: not available) */
-    int32_t c29[MG_MAX_OCT];
-    int32_t tile_eq;
-    int32_t tile_pad;
+    /* double branch, the tile kernels' table form: amp_d[k] * vf_d[k] * vfac times 2^30 rounded, and the bound on the
+     * difference between its value and the reference's double value in units of 2^-29 (rounded up; < 0: not available),
+     * for cells within 2^17 quarts of the origin and beyond */
+    int32_t c30[MG_MAX_OCT];
+    int32_t tile_eq, tile_eq_far;
 } MgNoise;
 
 /* Offset spline (CubicSpline over continents, erosion, ridges, ridges_folded), float.
@@ -69,7 +69,7 @@ typedef struct __attribute__((aligned(16))) {
 } MgSpline;
 
 /* R-tree node on the device (32 bytes, two 16-byte loads): children of a subtree are contiguous
- * [first, first+count); a leaf has count == 0.  Bounds of the six climate dimensions are quantised values
+ * [first, first+count); a leaf has count == 0 (and its rank in `first`).  Bounds of the six climate dimensions are quantised values
  * (|v| <= 12000 in every table), the upper bounds stored negated (nhi = -hi: packed 16-bit add-max
  * instructions then form t - hi); the seventh dimension ("offset") always meets a target coordinate of 0,
  * so its squared distance max(-hi, lo, 0)^2 is stored instead of its bounds.  The root is never a leaf;
@@ -106,11 +106,10 @@ typedef struct {
     int32_t end_ids[5];            /* the_end, end_highlands, end_midlands, small_end_islands, end_barrens */
     double end_f2, end_g2;         /* 2-D simplex skew 0.5*(sqrt(3)-1) and unskew (3-sqrt(3))/6 */
     int32_t tree_root, tree_nodes, tree_leaves;
-    int32_t tree_fanout;           /* most children of a node (the build's children per node: 6 or 19) */
-    /* the leaves again, clustered, for a search that shares its pruning among a tile's cells: groups of up to 32 leaves with
-     * their box (count, first: the group's leaves counted from node leaf_off) at nodes [group_off, group_off + groups) of the
-     * same array, and the leaves from node leaf_off on, whose `first` is their rank in the tree's depth-first order */
-    int32_t group_off, groups, leaf_off, group_pad;
+    /* the leaves again, clustered, for a search that shares its pruning among a tile's cells: groups of 32 leaves (the last fewer) with
+     * their box at nodes [group_off, group_off + groups) of the same array, the boxes of clusters of 32 groups from node
+     * cluster_off on, and the leaves from node leaf_off on; a leaf's `first` is its rank in the tree's depth-first order (in the tree as well) */
+    int32_t group_off, groups, leaf_off, cluster_off;
     MgSpline spline;
 } MgWorldDesc;
 

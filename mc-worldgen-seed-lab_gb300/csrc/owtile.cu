@@ -14,6 +14,12 @@ namespace mg {
 /* nodes a tile's table holds: the shift noises' (about 610) or the climate octaves' (about 680 on average) */
 #define OT_CAP_F 1024
 
+/* a tile of a request; kept in shared memory so that its fields are read where they are used (held in registers over the
+ * whole tile they made the double branch's kernel spill: 72.1 -> 68.7 ms) */
+struct OtTile {
+    MgBatchReq r;
+    int req, tile;
+};
 struct OtSmemF {
     MgLattice lat[MG_MAX_TABLES];
     float4 np[OT_CAP_F];
@@ -21,9 +27,10 @@ struct OtSmemF {
     OtShiftF sh[2 * OT_MAXLEV][4 * OT_W]; /* per lattice: X + ox, X + oy, Z + oz, Z + ox (16 entries each) */
     OtOctF oct[MG_MAX_TABLES];            /* the climate octaves in evaluation order */
     OtBuild build, sbuild;                /* climate and shift tables */
-    OtSearch rt;
     int lo[2], hi[2];                     /* range of the shifted x and z over the tile, in 1/16 of a quart from its corner */
-    int tile, req, state, over;
+    int state, over;
+    OtTile cur[2]; /* this tile and the next */
+    uint16_t hint[OT_NT]; /* each thread's last leaf: where its next R-tree search starts */
 };
 
 /* the old per-cell form, for a tile whose nodes do not fit (out of line: rare) */
@@ -33,17 +40,23 @@ static __device__ __noinline__ void ot_cell_f(const MgWorldDesc &W, const MgLatt
     for (int k = 0; k < 6; k++) tg[k] = t[k];
 }
 
+/* a search's leaf as the next search's hint (a leaf found by the lane alone is a node of the tree: no hint) */
+__device__ __forceinline__ uint16_t ot_hint(const MgWorldDesc &W, int leaf) {
+    return (uint16_t)(leaf >= W.leaf_off ? leaf - W.leaf_off : 0);
+}
 /* next tile and its request (one whole warp calls it) */
-template <typename SM>
-__device__ __forceinline__ void ot_next(SM &sm, const MgBatchReq *__restrict__ reqs, int nreq, long long ntiles,
+__device__ __forceinline__ void ot_next(OtTile &n, const MgBatchReq *__restrict__ reqs, int nreq, long long ntiles,
                                         unsigned long long *__restrict__ counter) {
     long long tile = 0;
     if ((threadIdx.x & 31) == 0) tile = (long long)atomicAdd(counter, 1ULL);
     tile = __shfl_sync(0xFFFFFFFFu, tile, 0);
     const int r = tile < ntiles ? find_req(reqs, nreq, tile) : -1;
     if ((threadIdx.x & 31) == 0) {
-        sm.tile = r >= 0 ? (int)(tile - reqs[r].tile0) : 0;
-        sm.req = r;
+        n.req = r;
+        if (r >= 0) {
+            n.r = reqs[r];
+            n.tile = (int)(tile - n.r.tile0);
+        }
     }
 }
 
@@ -59,13 +72,13 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const MgWorldDesc *__restrict
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int col = ot_col(), row = ot_row();
     if (t == 0) sm.state = -1;
-    if (warp == 0) ot_next(sm, reqs, nreq, ntiles, counter);
+    sm.hint[t] = 0;
+    if (warp == 0) ot_next(sm.cur[0], reqs, nreq, ntiles, counter);
     __syncthreads();
-    for (;;) {
-        const int r = sm.req;
-        if (r < 0) return;
-        const int tile = sm.tile;
-        const MgBatchReq R = reqs[r];
+    for (int c = 0;; c ^= 1) {
+        if (sm.cur[c].req < 0) return;
+        const int tile = sm.cur[c].tile;
+        const MgBatchReq &R = sm.cur[c].r;
         const MgWorldDesc &W = worlds[R.world];
         const MgNoise &O = W.noise[0];
         const int nlev = O.nlev, nsh = 2 * nlev, nclim = W.ntables - nsh;
@@ -80,6 +93,7 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const MgWorldDesc *__restrict
             for (int i = t; i < W.ntables * (int)(sizeof(MgLattice) / 16); i += OT_NT) b[i] = a[i];
             __syncthreads();
             if (t == 0) sm.state = R.state;
+            sm.hint[t] = 0; /* another request's world may have fewer leaves */
             if (t < nclim) { /* octave t in evaluation order */
                 int n = 1;
                 while (n < MG_OW_NOISES - 1 && t + nsh >= W.noise[n + 1].base) n++;
@@ -150,8 +164,7 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const MgWorldDesc *__restrict
         }
         __syncthreads();
         /* ---- 2: the shift noises and the shifted coordinates of the cell */
-        const int ix = tx0 + col, iz = tz0 + row;
-        const bool in = ix < R.nx && iz < R.nz;
+        const bool in = tx0 + col < R.nx && tz0 + row < R.nz;
         double x = 0.0, z = 0.0;
         if (!far) {
             float sa = 0.0f, sb = 0.0f;
@@ -220,9 +233,7 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const MgWorldDesc *__restrict
                 sm.build.units = units;
             }
         } else if (warp == 1) {
-            ot_next(sm, reqs, nreq, ntiles, counter);
-        } else if (warp == 2) {
-            ot_search_init(sm.rt, lane);
+            ot_next(sm.cur[c ^ 1], reqs, nreq, ntiles, counter);
         }
         __syncthreads();
         const bool over = sm.over != 0;
@@ -247,8 +258,8 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const MgWorldDesc *__restrict
                 asm volatile("" : "+d"(xc), "+d"(zc));
                 float v[MG_OW_NOISES - 1];
                 int e = 0;
-#pragma unroll
-                for (int n = 0; n < MG_OW_NOISES - 1; n++) {
+#pragma unroll 1
+                for (int n = 0; n < MG_OW_NOISES - 1; n++) { /* one copy of the octave's code for the five noises */
                     const int end = e + 2 * W.noise[n + 1].nlev;
                     float acc = 0.0f;
 #pragma unroll 1
@@ -262,22 +273,18 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const MgWorldDesc *__restrict
                         acc += o.amp * ot_octave_f<false>(sm.np, sm.nq, at, o.r.nx, fa, fa - 1.0f, fade<float>(fa), fb, fb - 1.0f,
                                                           fade<float>(fb), o.uy);
                     }
-                    v[n] = acc;
+#pragma unroll
+                    for (int k = 0; k < MG_OW_NOISES - 1; k++) v[k] = n == k ? acc : v[k];
                 }
                 climate_finish_f(W, W.spline, v[0], v[1], v[2], v[3], v[4], R.qy * 4, tg);
             } else {
                 ot_cell_f(W, sm.lat, qx0 + col, R.qy, qz0 + row, tg);
             }
         }
-        const MgTreeNode *tree = trees[R.world], *leaves = tree + W.leaf_off;
-        const OtWarpBox box = ot_search_box(sm.rt, tg, tg, in);
-        __syncthreads();
-        ot_search_list(sm.rt, W, tree);
-        __syncthreads();
-        if (box.any) {
-            const int n = ot_search_warp(sm.rt, box, tree, leaves, sm.rt.wl[warp]);
-            if (in) put_id(out + R.out_off + (int64_t)iz * R.nx + ix, ot_biome(tree, leaves, sm.rt.wl[warp], n, tg));
-        }
+        const MgTreeNode *tree = trees[R.world];
+        const int leaf = tree_search_warp(tree, W, tg, in, sm.hint[t]);
+        if (in) sm.hint[t] = ot_hint(W, leaf);
+        if (in) put_id(out + R.out_off + (int64_t)(qz0 + row - R.qz0) * R.nx + (qx0 + col - R.qx0), tree[leaf].biome);
         __syncthreads(); /* the tables are free for the next tile */
     }
 }
@@ -300,9 +307,10 @@ struct OtSmemD {
     int2 oct_b[MG_MAX_TABLES];       /* their first cells */
     OtFix fix[MG_MAX_TABLES], sfix[OT_SHIFT_TABS]; /* climate octaves; shift tables */
     OtBuild build, sbuild;
-    OtSearch rt;
     int lo[2], hi[2];
-    int tile, req, state, over;
+    int state, over;
+    OtTile cur[2]; /* this tile and the next */
+    uint16_t hint[OT_NT];
     int32_t depth; /* depth gradient and offset constant at the request's y, units of 2^-28 */
 };
 
@@ -328,13 +336,13 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int col = ot_col(), row = ot_row();
     if (t == 0) sm.state = -1;
-    if (warp == 0) ot_next(sm, reqs, nreq, ntiles, counter);
+    sm.hint[t] = 0;
+    if (warp == 0) ot_next(sm.cur[0], reqs, nreq, ntiles, counter);
     __syncthreads();
-    for (;;) {
-        const int r = sm.req;
-        if (r < 0) return;
-        const int tile = sm.tile;
-        const MgBatchReq R = reqs[r];
+    for (int c = 0;; c ^= 1) {
+        if (sm.cur[c].req < 0) return;
+        const int tile = sm.cur[c].tile;
+        const MgBatchReq &R = sm.cur[c].r;
         const MgWorldDesc &W = worlds[R.world];
         const MgNoise &O = W.noise[0];
         const int nlev = O.nlev, nsh = 2 * nlev, nclim = W.ntables - nsh;
@@ -348,6 +356,7 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict
             for (int i = t; i < W.ntables * (int)(sizeof(MgLattice) / 16); i += OT_NT) b[i] = a[i];
             __syncthreads();
             if (t == 0) sm.state = R.state;
+            sm.hint[t] = 0; /* another request's world may have fewer leaves */
             if (t < nclim) { /* octave t in evaluation order */
                 int n = 1;
                 while (n < MG_OW_NOISES - 1 && t + nsh >= W.noise[n + 1].base) n++;
@@ -359,7 +368,7 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict
                 sm.oct_o[t][0] = __double2ll_rn(L.ox * 0x1.0p32);
                 sm.oct_o[t][1] = __double2ll_rn(L.oz * 0x1.0p32);
                 sm.oct[t].k = -N.fexp[k];
-                sm.oct[t].c29 = N.c29[k];
+                sm.oct[t].c30 = N.c30[k];
                 sm.fix[t] = ot_fix(L.fyd, L.uyd);
             } else if (t >= 64 && t < 64 + 2 * nsh) { /* shift tables: lattice j's (x, 0, z) form is 2 j, its (x, y, 0) form 2 j + 1 */
                 const MgLattice &L = sm.lat[(t - 64) >> 1];
@@ -427,11 +436,10 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict
         }
         __syncthreads();
         /* ---- 2: the shift noises and the shifted coordinates of the cell (units of 2^-32) */
-        const int ix = tx0 + col, iz = tz0 + row;
-        const bool in = ix < R.nx && iz < R.nz;
+        const bool in = tx0 + col < R.nx && tz0 + row < R.nz;
         int64_t x = 0, z = 0;
         if (!far) {
-            int64_t sa = 0, sb = 0; /* units of 2^-58 */
+            int64_t sa = 0, sb = 0; /* units of 2^-59 */
 #pragma unroll 1
             for (int k = 0; k < nlev; k++) {
                 int64_t va = 0, vb = 0;
@@ -443,13 +451,13 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict
                     va += ot_octave_d(sm.ep, sm.eq, ax.edge + az.edge, sm.sbuild.nx[2 * j], ax.f, ax.u, az.f, az.u);
                     vb += ot_octave_d(sm.ep, sm.eq, bx.edge + by.edge, sm.sbuild.nx[2 * j + 1], bx.f, bx.u, by.f, by.u);
                 }
-                const int32_t c = O.c29[k];
+                const int32_t c = O.c30[k];
                 sa = ot_madw((int32_t)(va >> 31), c, sa);
                 sb = ot_madw((int32_t)(vb >> 31), c, sb);
             }
-            x = ((int64_t)(qx0 + col) << 32) + (sa >> 24); /* the noise times 4 */
-            z = ((int64_t)(qz0 + row) << 32) + (sb >> 24);
-            const int rx = col * 16 + (int)(sa >> 52), rz = row * 16 + (int)(sb >> 52);
+            x = ((int64_t)(qx0 + col) << 32) + (sa >> 25); /* the noise times 4 */
+            z = ((int64_t)(qz0 + row) << 32) + (sb >> 25);
+            const int rx = col * 16 + (int)(sa >> 53), rz = row * 16 + (int)(sb >> 53);
             const int x0 = __reduce_min_sync(0xFFFFFFFFu, in ? rx : 0x7FFFFFFF), x1 = __reduce_max_sync(0xFFFFFFFFu, in ? rx : -0x7FFFFFFF);
             const int z0 = __reduce_min_sync(0xFFFFFFFFu, in ? rz : 0x7FFFFFFF), z1 = __reduce_max_sync(0xFFFFFFFFu, in ? rz : -0x7FFFFFFF);
             if (lane == 0 && x0 <= x1) {
@@ -506,9 +514,7 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict
                 sm.build.units = units;
             }
         } else if (warp == 1) {
-            ot_next(sm, reqs, nreq, ntiles, counter);
-        } else if (warp == 2) {
-            ot_search_init(sm.rt, lane);
+            ot_next(sm.cur[c ^ 1], reqs, nreq, ntiles, counter);
         }
         __syncthreads();
         const bool over = sm.over != 0;
@@ -532,10 +538,10 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict
             const int64_t xc = x + __mul64hi(x, OT_STACK_C), zc = z + __mul64hi(z, OT_STACK_C);
             int32_t v[MG_OW_NOISES - 1]; /* units of 2^-29 */
             int e = 0;
-#pragma unroll
-            for (int n = 0; n < MG_OW_NOISES - 1; n++) {
+#pragma unroll 1
+            for (int n = 0; n < MG_OW_NOISES - 1; n++) { /* one copy of the octave's code for the five noises */
                 const int end = e + 2 * W.noise[n + 1].nlev;
-                int64_t acc = 0; /* units of 2^-58 */
+                int64_t acc = 0; /* units of 2^-59 */
 #pragma unroll 1
                 for (; e < end; e += 2) {
                     int64_t lev = 0;
@@ -547,16 +553,21 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict
                         const int at = o.off + ot_hi(sz) * o.nx + ot_hi(sx);
                         lev += ot_octave_d(sm.ep, sm.eq, at, o.nx, (int32_t)((uint32_t)sx >> 1), ot_fade31((uint32_t)sx),
                                            (int32_t)((uint32_t)sz >> 1), ot_fade31((uint32_t)sz));
-                        c = o.c29;
+                        c = o.c30;
                     }
                     acc = ot_madw((int32_t)(lev >> 31), c, acc);
                 }
-                v[n] = (int32_t)(acc >> 29);
+#pragma unroll
+                for (int k = 0; k < MG_OW_NOISES - 1; k++) v[k] = n == k ? (int32_t)(acc >> 30) : v[k];
             }
             const float s29 = 10000.0f * 0x1.0p-29f, s28 = 10000.0f * 0x1.0p-28f;
-            const int32_t ec = W.noise[3].tile_eq, ee = W.noise[4].tile_eq, ew = W.noise[5].tile_eq;
-            ot_target(v[0], W.noise[1].tile_eq, s29, ta[0], tb[0]);
-            ot_target(v[1], W.noise[2].tile_eq, s29, ta[1], tb[1]);
+            const bool out17 = max(max(abs(qx0), abs(qz0)) + OT_W, 0) >= 1 << 17;
+            int32_t eq[MG_OW_NOISES];
+#pragma unroll
+            for (int n = 1; n < MG_OW_NOISES; n++) eq[n] = out17 ? W.noise[n].tile_eq_far : W.noise[n].tile_eq;
+            const int32_t ec = eq[3], ee = eq[4], ew = eq[5];
+            ot_target(v[0], eq[1], s29, ta[0], tb[0]);
+            ot_target(v[1], eq[2], s29, ta[1], tb[1]);
             ot_target(v[2], ec, s29, ta[2], tb[2]);
             ot_target(v[3], ee, s29, ta[3], tb[3]);
             ot_target(v[4], ew, s29, ta[5], tb[5]);
@@ -575,8 +586,8 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict
             si.dr = (float)ew * u + fabsf(si.r) * 1.2e-7f;
             si.df = fabsf(c2) * (float)(ew + 2) + fabsf(si.f) * 1.9e-7f;
             float es;
-            const float sp = spline_err<MG_SPL_DEPTH>(W.spline, W.spline.root, si, es);
-            ot_target(sm.depth + __float2int_rn(sp * 0x1.0p28f), (int32_t)(es * (1.01f * 0x1.0p28f)) + 4, s28, ta[4], tb[4]);
+            const float sp = spline_err<OT_SPL_DEPTH>(W.spline, W.spline.root, si, es);
+            ot_target(sm.depth + __float2int_rn(sp * 0x1.0p28f), (int32_t)(es * (1.01f * 0x1.0p28f)) + 3, s28, ta[4], tb[4]);
             ok = es < 1.0f;
         }
         /* at most one target open, between two neighbouring values: both are looked up, and the cell is settled when they
@@ -588,26 +599,31 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict
             ok &= (unsigned)(tb[k] - ta[k]) <= 1u;
         }
         ok &= amb <= 1;
-        const MgTreeNode *tree = trees[R.world], *leaves = tree + W.leaf_off;
-        const OtWarpBox box = ot_search_box(sm.rt, ta, tb, ok);
-        __syncthreads();
-        ot_search_list(sm.rt, W, tree);
-        __syncthreads();
-        int biome = 0;
-        if (box.any) {
-            const int n = ot_search_warp(sm.rt, box, tree, leaves, sm.rt.wl[warp]);
-            if (ok) {
-                biome = ot_biome(tree, leaves, sm.rt.wl[warp], n, ta);
-                if (amb) ok = ot_biome(tree, leaves, sm.rt.wl[warp], n, tb) == biome;
+        const MgTreeNode *tree = trees[R.world];
+        int biome = -1;
+#pragma unroll 1
+        for (int pass = 0; pass < 2; pass++) { /* the lower targets, then the upper ones of the cells that have two */
+            const bool act = ok && (pass == 0 || amb);
+            if (pass && !__any_sync(0xFFFFFFFFu, act)) break;
+            int32_t t6[6];
+#pragma unroll
+            for (int k = 0; k < 6; k++) t6[k] = pass ? tb[k] : ta[k];
+            const int leaf = tree_search_warp(tree, W, t6, act, sm.hint[t]);
+            if (act) {
+                sm.hint[t] = ot_hint(W, leaf);
+                const int b = tree[leaf].biome;
+                ok = pass == 0 || b == biome;
+                biome = b;
             }
         }
         if (in) {
+            const int ix = qx0 + col - R.qx0, iz = qz0 + row - R.qz0;
             const int64_t o = R.out_off + (int64_t)iz * R.nx + ix;
             if (ok) {
                 put_id(out + o, biome);
             } else {
                 const unsigned long long k = atomicAdd(nopen, 1ULL);
-                if (k < (unsigned long long)open_cap) open[k] = MgOpenCell{r, iz * R.nx + ix};
+                if (k < (unsigned long long)open_cap) open[k] = MgOpenCell{sm.cur[c].req, iz * R.nx + ix};
                 else put_id(out + o, ot_open_d(W, sm.lat, tree, qx0 + col, R.qy, qz0 + row));
             }
         }

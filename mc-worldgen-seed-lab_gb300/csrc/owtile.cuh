@@ -157,196 +157,6 @@ __device__ __forceinline__ void ot_node_f(const MgLattice &L, bool z0, int i, in
     }
 }
 
-/* ============================================================================ R-tree search of a tile
- * A tile's 256 cells have close targets, so one pruning serves them all (device.cuh warp_tree_candidates has the argument: a
- * leaf whose distance to the targets' box exceeds the least "largest distance of a leaf to a point of the box" is nearest for
- * none of them).  The tile's box is tested against the boxes of the leaves' groups (MgWorldDesc::group_off: at most 256 for
- * the Overworld's 7,600 leaves, one per thread), the groups that may matter leaf by leaf, each warp prunes the list again
- * with its own 8 x 4 cells' box, and a lane scans what is left (about 30 leaves).  The reference's leaf is the one of least
- * distance, the first in depth-first order among equals, so the list's order is free: a leaf carries its rank. */
-#define OT_LIST 512      /* leaves a tile's list holds */
-#define OT_WLIST 128     /* leaves a warp's list holds */
-#define OT_GLIST 256     /* groups a tile's list holds */
-struct OtSearch {
-    unsigned long long near; /* distance and number of the group nearest to the tile's box */
-    int lo[6], hi[6];        /* the tile's box */
-    int bad, ngrp, nleaf;
-    uint16_t grp[OT_GLIST];
-    uint16_t leaf[OT_LIST];
-    uint16_t wl[OT_NT / 32][OT_WLIST];
-};
-/* before the block barrier that precedes ot_search_box */
-__device__ __forceinline__ void ot_search_init(OtSearch &s, int t) {
-    if (t < 6) s.lo[t] = 0x7FFFFFFF;
-    else if (t < 12) s.hi[t - 6] = -0x7FFFFFFF;
-    else if (t == 12) s.near = ~0ULL;
-    else if (t == 13) s.bad = s.ngrp = s.nleaf = 0;
-}
-__device__ __forceinline__ void ot_box(const int32_t *lo, const int32_t *hi, RtTarget &lbq, RtTarget &ubq) {
-    for (int k = 0; k < 3; k++) {
-        lbq.p[k] = pack16(lo[2 * k], lo[2 * k + 1]);
-        lbq.n[k] = pack16(-hi[2 * k], -hi[2 * k + 1]);
-        ubq.p[k] = pack16(hi[2 * k], hi[2 * k + 1]);
-        ubq.n[k] = pack16(-lo[2 * k], -lo[2 * k + 1]);
-    }
-}
-struct OtWarpBox {
-    RtTarget lb, ub;
-    bool any;
-};
-/* the warp's box of its active cells' targets [ta, tb] and its part of the tile's; a barrier follows */
-__device__ __forceinline__ OtWarpBox ot_search_box(OtSearch &s, const int32_t *ta, const int32_t *tb, bool active) {
-    const unsigned FULL = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31, lim = 32767 - MG_TREE_PACKED_BOUND;
-    int32_t lo[6], hi[6];
-    int out = 0, mine = 0;
-#pragma unroll
-    for (int k = 0; k < 6; k++) {
-        lo[k] = __reduce_min_sync(FULL, active ? ta[k] : 0x7FFFFFFF);
-        hi[k] = __reduce_max_sync(FULL, active ? tb[k] : -0x7FFFFFFF);
-        out |= lo[k] < -lim || hi[k] > lim;
-        mine = lane == k ? lo[k] : (lane == k + 6 ? hi[k] : mine);
-    }
-    OtWarpBox b;
-    b.any = lo[0] != 0x7FFFFFFF;
-    if (b.any) {
-        if (lane < 6) atomicMin(&s.lo[lane], mine);
-        else if (lane < 12) atomicMax(&s.hi[lane - 6], mine);
-        else if (lane == 12 && out) s.bad = 1;
-    }
-    ot_box(lo, hi, b.lb, b.ub);
-    return b;
-}
-struct OtNode {
-    uint4 a, b;
-    __device__ __forceinline__ OtNode(const MgTreeNode *n)
-        : a(*reinterpret_cast<const uint4 *>(n)), b(*(reinterpret_cast<const uint4 *>(n) + 1)) {}
-};
-/* the tile's list (all threads; two barriers inside, one must follow) */
-__device__ __forceinline__ void ot_search_list(OtSearch &s, const MgWorldDesc &W, const MgTreeNode *__restrict__ T) {
-    const unsigned FULL = 0xFFFFFFFFu;
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    RtTarget lbq, ubq;
-    ot_box(s.lo, s.hi, lbq, ubq);
-    const int ng = W.groups;
-    const MgTreeNode *G = T + W.group_off, *L = T + W.leaf_off;
-    uint32_t lb0 = 0xFFFFFFFFu; /* this thread's first group */
-    {
-        uint32_t m = 0xFFFFFFFFu;
-        int g = 0;
-        for (int i = t; i < ng; i += OT_NT) {
-            const OtNode n(G + i);
-            const uint32_t d = rt_dist(n.a, n.b, lbq);
-            if (i == t) lb0 = d;
-            if (d < m) { m = d; g = i; }
-        }
-        const uint32_t wm = __reduce_min_sync(FULL, m);
-        if (m == wm && wm != 0xFFFFFFFFu) atomicMin(&s.near, (unsigned long long)wm << 16 | (unsigned)g);
-    }
-    __syncthreads();
-    /* the least upper bound over the nearest group's leaves */
-    uint32_t U = 0xFFFFFFFFu;
-    if (s.near != ~0ULL) {
-        const OtNode g(G + (int)(s.near & 0xFFFFu));
-        const int first = (int)(g.b.w & 0xFFFFu), count = (int)((g.b.w >> 16) & 0xFFu);
-        if (lane < count) {
-            const OtNode n(L + first + lane);
-            U = rt_ub_or_inf(n.a, n.b, ubq);
-        }
-    }
-    U = __reduce_min_sync(FULL, U);
-    for (int i = t; i - lane < ng; i += OT_NT) {
-        uint32_t d = lb0;
-        if (i >= OT_NT && i < ng) {
-            const OtNode n(G + i);
-            d = rt_dist(n.a, n.b, lbq);
-        }
-        const bool keep = i < ng && d <= U;
-        const unsigned m = __ballot_sync(FULL, keep);
-        if (!m) continue;
-        int at = 0;
-        if (lane == 0) at = atomicAdd(&s.ngrp, __popc(m));
-        at = __shfl_sync(FULL, at, 0) + __popc(m & ((1u << lane) - 1u));
-        if (keep && at < OT_GLIST) s.grp[at] = (uint16_t)i;
-    }
-    __syncthreads();
-    const int nk = s.ngrp;
-    if (nk > OT_GLIST) { /* every warp sees the same count */
-        s.bad = 1;
-        return;
-    }
-    for (int i = warp; i < nk; i += OT_NT / 32) {
-        const OtNode g(G + s.grp[i]);
-        const int first = (int)(g.b.w & 0xFFFFu), count = (int)((g.b.w >> 16) & 0xFFu);
-        bool keep = false;
-        if (lane < count) {
-            const OtNode n(L + first + lane);
-            keep = rt_dist(n.a, n.b, lbq) <= U;
-        }
-        const unsigned m = __ballot_sync(FULL, keep);
-        if (!m) continue;
-        int at = 0;
-        if (lane == 0) at = atomicAdd(&s.nleaf, __popc(m));
-        at = __shfl_sync(FULL, at, 0) + __popc(m & ((1u << lane) - 1u));
-        if (keep && at < OT_LIST) s.leaf[at] = (uint16_t)(first + lane);
-    }
-}
-/* the warp's list from the tile's: its length, or -1 when the lanes have to search alone */
-__device__ __forceinline__ int ot_search_warp(OtSearch &s, const OtWarpBox &b, const MgTreeNode *__restrict__ T,
-                                               const MgTreeNode *__restrict__ L, uint16_t *wl) {
-    const unsigned FULL = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31, n = s.nleaf;
-    if (s.bad || !rt_packed(T) || n > OT_LIST || n == 0) return -1;
-    uint32_t U = 0xFFFFFFFFu;
-    int nw = 0;
-    for (int c = 0; c < n; c += 32) { /* the least upper bound first: the list is short and its leaves come back from L1 */
-        uint32_t u = 0xFFFFFFFFu;
-        if (c + lane < n) {
-            const OtNode q(L + s.leaf[c + lane]);
-            u = rt_ub_or_inf(q.a, q.b, b.ub);
-        }
-        U = min(U, __reduce_min_sync(FULL, u));
-    }
-    for (int c = 0; c < n; c += 32) {
-        bool keep = false;
-        int at = 0;
-        if (c + lane < n) {
-            at = s.leaf[c + lane];
-            const OtNode q(L + at);
-            keep = rt_dist(q.a, q.b, b.lb) <= U;
-        }
-        const unsigned m = __ballot_sync(FULL, keep);
-        const int p = nw + __popc(m & ((1u << lane) - 1u));
-        if (keep && p < OT_WLIST) wl[p] = (uint16_t)at;
-        nw += __popc(m);
-    }
-    __syncwarp();
-    return nw <= OT_WLIST ? nw : -1;
-}
-/* the lane's leaf (its word: biome in the top byte) among the listed ones; false when a distance was clamped */
-__device__ __forceinline__ bool ot_scan(const MgTreeNode *__restrict__ L, const uint16_t *wl, int n, const RtTarget &q, int &biome) {
-    uint32_t best = 0xFFFFFFFFu, w = 0xFFFFu;
-    for (int k = 0; k < n; k++) {
-        const OtNode c(L + wl[k]);
-        const uint32_t d = rt_dist(c.a, c.b, q);
-        if (d < best || (d == best && (c.b.w & 0xFFFFu) < (w & 0xFFFFu))) { best = d; w = c.b.w; }
-    }
-    biome = (int)(w >> 24);
-    return best < (uint32_t)MG_RT_CLAMP * MG_RT_CLAMP;
-}
-/* the biome at target t: from the warp's list, or alone */
-__device__ __forceinline__ int ot_biome(const MgTreeNode *__restrict__ T, const MgTreeNode *__restrict__ L, const uint16_t *wl, int n,
-                                        const int32_t *t) {
-    RtTarget q;
-    int b;
-    if (n >= 0) {
-        rt_target(t, q);
-        if (ot_scan(L, wl, n, q, b)) return b;
-    }
-    uint64_t d;
-    return T[tree_search(T, t, -1, d)].biome;
-}
-
 /* ============================================================================ double branch
  * The double branch's five climate noises and ridges_folded reach the biome only through quantised targets (steps of 1e-4),
  * so the tile form evaluates them in 32-bit fixed point with 64-bit accumulators (no FP64 pipe, which the exact shift octaves
@@ -377,7 +187,7 @@ __device__ __forceinline__ OtFix ot_fix(double y, double v) {
 struct __align__(16) OtOctD {
     int64_t ox, oz;
     int32_t nx, off; /* edges per row, place in the table */
-    int32_t k, c29;  /* input factor 2^-k; level constant */
+    int32_t k, c30;  /* input factor 2^-k; level constant */
 };
 __device__ __forceinline__ int64_t ot_madw(int32_t a, int32_t b, int64_t c) {
     int64_t r;
@@ -390,13 +200,14 @@ __device__ __forceinline__ int32_t ot_sub_sat(int32_t a, int32_t b) {
     asm("sub.sat.s32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
-/* smoothstep of the fraction t (units of 2^-32) in units of 2^-31, within 3e-9: t > 1/2 as 1 - smoothstep(1 - t), and with
- * t' = 2 t <= 1, t^3 (10 - 15 t + 6 t^2) = t'^3 / 8 (10 - t' (7.5 - 1.5 t')) */
+/* smoothstep of the fraction t (units of 2^-32) in units of 2^-31: t > 1/2 as 1 - smoothstep(1 - t), and with t' = 2 t <= 1,
+ * t^3 (10 - 15 t + 6 t^2) = t'^3 / 8 (10 - t' (7.5 - 1.5 t')).  The 2 centres the truncations: within 1.43e-9 (all 2^32
+ * fractions evaluated). */
 __device__ __forceinline__ int32_t ot_fade31(uint32_t t) {
     const int32_t m = (int32_t)t >> 31;
     const uint32_t tt = (t ^ (uint32_t)m) << 1;
     const uint32_t t3 = __umulhi(__umulhi(tt, tt), tt);
-    const uint32_t p = (10u << 28) - __umulhi(tt, 15u * (1u << 27) - (tt >> 5) * 3u);
+    const uint32_t p = (10u << 28) - __umulhi(tt, 15u * (1u << 27) - 2u - (tt >> 5) * 3u);
     return (int32_t)__umulhi(t3, p) ^ (m & 0x7FFFFFFF);
 }
 /* a row's value in units of 2^-60 from its edge; X and dz in units of 2^-31, dz in [-1, 1] */
@@ -446,7 +257,10 @@ __device__ __forceinline__ void ot_target(int32_t v, int32_t e, float scale, int
  * A Hermite segment's value is a convex combination of its two points' values (so their errors pass through at most) plus
  * a cubic in t, whose slope in the input is at most (|y2 - y1| + 1.25 (|a| + |b|)) / (x2 - x1); the spline is C1, and a
  * neighbouring segment's slope differs near the joint by its curvature (below 1e5) times ce (below 1e-6), covered by 0.01 and
- * 0.1; both evaluations' roundings are within 2^-24 (5 |y2 - y1| + 2 max |y| + 6 (|a| + |b|)) each. */
+ * 0.1 (and 2e-9 where a segment is constant); the roundings of one evaluation are within 2^-24 times 2 u_t = 2 (|y2 - y1| +
+ * 1.25 (|a| + |b|)) for t's two, 2 |y2 - y1| + max |y| for the first lerp, a quarter of |y2 - y1| and 1.75 (|a| + |b|) for the
+ * cubic, max |y| + 0.25 (|a| + |b|) for the sum: 4.25 |y2 - y1| + 2 max |y| + 4.5 (|a| + |b|), and both sides round. */
+#define OT_SPL_DEPTH 4 /* nesting levels unrolled (every 26.x table: 4) */
 struct SplineIn {
     float c, e, r, f;     /* continents, erosion, ridges, ridges_folded */
     float dc, de, dr, df; /* their bounds */
@@ -458,7 +272,7 @@ __device__ __forceinline__ float spline_err(const MgSpline &S, int c, const Spli
     err = 0.0f;
     if (c < 0) return S.cval[~c];
     if constexpr (D == 0) {
-        err = 1e30f; /* not reached: a table nests at most MG_SPL_DEPTH levels */
+        err = 1e30f; /* nested deeper: the cell is left open */
         return 0.0f;
     } else {
         const int o = S.first[c], n = S.npts[c], k = S.coord[c];
@@ -478,14 +292,15 @@ __device__ __forceinline__ float spline_err(const MgSpline &S, int c, const Spli
         const float x1 = S.loc[p], d1 = S.der[p];
         if (ext) { /* linear extension */
             const float v = d1 * (in - x1);
-            err = e2 + (fabsf(d1) + 0.1f) * de + 1.2e-7f * (4.0f * fabsf(v) + fabsf(y2));
+            err = d1 == 0.0f ? e2 + 2e-9f : e2 + (fabsf(d1) + 0.1f) * de + 1.2e-7f * (4.0f * fabsf(v) + fabsf(y2));
             return d1 == 0.0f ? y2 : y2 + v;
         }
         const float w = S.loc[p + 1] - x1, t = (in - x1) / w, d2 = S.der[p + 1], dy = y2 - y1;
         const float a = d1 * w - dy, b = -d2 * w + dy;
         const float ab = fabsf(a) + fabsf(b), ad = fabsf(dy);
         err = fmaxf(e1, e2) + (__fdividef(ad + 1.25f * ab, w) * 1.001f + 0.1f) * de +
-              1.2e-7f * (5.0f * ad + 2.0f * fmaxf(fabsf(y1), fabsf(y2)) + 6.0f * ab);
+              1.2e-7f * (4.3f * ad + 2.0f * fmaxf(fabsf(y1), fabsf(y2)) + 4.6f * ab);
+        if (ad + ab + e1 + e2 == 0.0f) err = 2e-9f; /* a constant segment: its value is exact */
         return lerp<float>(t, y1, y2) + t * (1.0f - t) * lerp<float>(t, a, b);
     }
 }

@@ -305,9 +305,8 @@ __global__ void k_check_tree(const MgTreeNode *__restrict__ T, long long n, uint
  * neighbouring cells has: per warp a centre in the tables' range and per lane a spread of 50, 400, 2,000 or
  * 6,000 around it; about one lane in eight inactive; in one warp in sixteen one lane far outside the packed
  * range (the warp's fallback).  Case i is lane i % 32 of warp case i / 32.  out[0]: differing leaves. */
-__global__ void __launch_bounds__(128) k_check_tree_warp(const MgTreeNode *__restrict__ T, long long n, uint64_t seed,
-                                                         unsigned long long *out) {
-    __shared__ WarpTreeScratch ws[4];
+__global__ void __launch_bounds__(128) k_check_tree_warp(const __grid_constant__ MgWorldDesc W, const MgTreeNode *__restrict__ T,
+                                                         long long n, uint64_t seed, unsigned long long *out) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     unsigned long long bad = 0;
     const long long nw = (n + 31) / 32, step = (long long)gridDim.x * 4;
@@ -325,10 +324,15 @@ __global__ void __launch_bounds__(128) k_check_tree_warp(const MgTreeNode *__res
             const int32_t c = (int32_t)(r % 24001) - 12000;
             t[k] = far_lane ? (int32_t)(q % 80001) - 40000 : c + (int32_t)(q % (uint64_t)(2 * spread + 1)) - spread;
         }
-        const int lw = tree_search_warp(T, t, active, ws[wib]);
-        if (active) {
+        const int lw = tree_search_warp(T, W, t, active);
+        uint64_t dt = 0;
+        bool tied = false;
+        const int lt = tree_search_tie_warp(T, W, t, active, dt, tied);
+        if (active) { /* leaves are compared by their depth-first rank */
             uint64_t d;
-            bad += lw != tree_search_stack(T, t, -1, d);
+            bool tie0;
+            const int l0 = tree_search_tie_stack(T, t, d, tie0);
+            bad += (T[lw].first != T[l0].first) + (T[lt].first != T[l0].first) + (dt != d) + (tied != tie0);
         }
     }
     atomicAdd(&out[0], bad);
@@ -434,7 +438,7 @@ extern "C" MCGEN_API int mcgen_gb300_check_tree(const McWorld *w, long long n, u
     if (cudaMalloc(&d, 2 * sizeof(unsigned long long)) != cudaSuccess) return MCGEN_E_NOMEM;
     cudaMemset(d, 0, 2 * sizeof(unsigned long long));
     k_check_tree<<<152 * 4, 128>>>(w->d_tree, n, seed, d);
-    k_check_tree_warp<<<152 * 4, 128>>>(w->d_tree, n, seed ^ 0xA5A5A5A5ULL, d);
+    k_check_tree_warp<<<152 * 4, 128>>>(w->desc, w->d_tree, n, seed ^ 0xA5A5A5A5ULL, d);
     unsigned long long h[2] = {0, 0};
     cudaError_t e = cudaMemcpy(h, d, sizeof h, cudaMemcpyDeviceToHost);
     cudaFree(d);

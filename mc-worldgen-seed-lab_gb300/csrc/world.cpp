@@ -249,24 +249,24 @@ static double screen_bound32(const MgNoise *s) {
     return 1.25 * e;
 }
 
-/* Bounds of the tile kernels' table form (owtile.cuh ot_octave_d) against the reference's double value, in reals; "q" is
- * 2^-30.
+/* Bounds of the tile kernels' table form (owtile.cuh ot_octave_d) against the reference's double value, in reals; q = 2^-30,
+ * u = 2^-32.
  * An octave, given its two coordinates' cells and fractions exactly, is V = (1 - W) L0 + W L1, L = (1 - U) N0 + U N1 over
  * node values N = A dx + B dz + C with |N| <= 2:
- *  - A, B, C come from the fixed smoothstep rounded to q (half a unit): A, B within q, C within q: N within 3 q;
- *  - L = P + U Q: P's coefficients rounded to 2 q (1 q each, two of them), its constant to 4 q (2 q); Q's constant to 2 q
- *    (1 q), the upper word of Q rounded to 2 q (1 q), a saturated coefficient (1 q): L within 3 + 4 + 3 = 10 q;
- *  - V's difference L1 - L0 is truncated to 2 q: V within 12 q;
- *  - a smoothstep error e moves V by at most 2.1 e: |N10 - N00| <= 1 + 2 max(dz, 1/2), so the row-weighted difference is at
- *    most 2.06.  The tables' smoothsteps of the shift (from 59 bits) are within q; the cells' (ot_fade31, folded to
- *    t <= 1/2, p = 10 - t'(7.5 - 1.5 t') with t' = 2 t in units of 2^-28 within 4 units, times t^3 <= 1/8; t'^2 and t'^3
- *    truncated at 2^-32; the result truncated at 2^-31) within 3e-9;
- *  - a coordinate error e moves V by at most 5 e (|dV/dX| <= 1 + 1.875 x 2.06): the shift's coordinates are exact; a climate
- *    octave's are truncated at 2^-32 and its offset rounded: within 1.5 x 2^-32, and the reference's own rounding of its sum
- *    within 2 x 2^-32 (|s| < 2^22 up to the world border): 4 x 2^-32 is taken; the linear forms' 31-bit fractions add 2^-32.
- * TILE_SHIFT_OCT and TILE_OCT are these sums. */
-static const double TILE_SHIFT_OCT = 12.0 * 0x1.0p-30 + 2.0 * 2.1 * 0x1.0p-30 + 2.0 * 0x1.0p-32;
-static const double TILE_OCT = 12.0 * 0x1.0p-30 + 2.0 * 2.1 * 3e-9 + 2.0 * 5.0 * 4.0 * 0x1.0p-32 + 2.0 * 0x1.0p-32;
+ *  - the fixed smoothstep is rounded to q (half a unit each in A and B per unit of gradient difference, at most 2; |dx| + |dz|
+ *    weighted by the smoothsteps is at most 1) and C's two products to q: V within 2 q;
+ *  - P's X coefficient is rounded to 2 q (1 q), its Z coefficient likewise (|dz| weighted: 0.5 q), its constant to 4 q (2 q);
+ *    Q's constant to 2 q (1 q), Q's upper word to 2 q (1 q), a saturated coefficient (1 q): 6.5 q;
+ *  - the difference L1 - L0 is truncated to 2 q: 2 q.  Together 10.5 q; 11 q is used.
+ *  - a smoothstep error e moves V by at most 2.52 e, a coordinate error e by at most 3.8 e (the sums over the four nodes of the
+ *    largest |dV/dU| and |dV/dX| any gradients give, maximised over the unit cube; 2.511 and 3.750).  The shift tables'
+ *    smoothsteps are within u of the exact ones and their coordinates exact; the cells' smoothsteps (ot_fade31, all 2^32
+ *    fractions evaluated) within 1.53e-9, their coordinates truncated at u and the offset rounded: 1.5 u, with the
+ *    reference's own rounding of its sum: 0.1 u for |quart| < 2^17, 2 u up to the world border.  The linear forms' 31-bit
+ *    fractions add u each. */
+static const double TILE_Q = 0x1.0p-30, TILE_U = 0x1.0p-32;
+static const double TILE_SHIFT_OCT = 11.0 * TILE_Q + 2.0 * 2.52 * TILE_U + 2.0 * TILE_U;
+static double tile_oct(bool far) { return 11.0 * TILE_Q + 2.0 * 2.52 * 1.53e-9 + 2.0 * 3.8 * (far ? 3.5 : 1.6) * TILE_U + 2.0 * TILE_U; }
 /* sum of the levels' constants of one stack, plain and weighted by frequency */
 static void level_sums(const MgNoise *s, double *c, double *cf) {
     *c = *cf = 0.0;
@@ -276,22 +276,32 @@ static void level_sums(const MgNoise *s, double *c, double *cf) {
         *cf += v * s->freq[k];
     }
 }
-/* tile_eq of the climate noise s, whose coordinates are shifted by 4 x the noise `shift`: two stacks of octaves, each level's
- * sum truncated to 2^-29 and its constant rounded to half of that, the reference's own error (screen_bound's terms, far
- * smaller), and the error of the two shifts times the noise's slope (5 per lattice unit; the second stack 1.0182 steeper).
- * The values must stay below 4: an octave is at most 1.04 in magnitude (the largest corner dots, max(dx + dz, max(dx, dz) + dy)
- * per plane, weighted by the smoothsteps, over the unit cube), 1.06 is used. */
+/* a noise from octaves within `oct`: two stacks, each level's sum (below 2.1) truncated at 2^-29 and its constant rounded at
+ * 2^-30, the reference's own roundings (screen_bound's terms, below 1e-12) */
+static double tile_noise(const MgNoise *s, double c, double oct) {
+    return 2.0 * c * oct + c * 0x1.0p-29 + s->nlev * 2.1 * 0x1.0p-31 + 1e-12;
+}
+/* tile_eq and tile_eq_far of the climate noises s, whose coordinates are shifted by 4 x the noise `shift`: the noise itself,
+ * and the error of the two shifted coordinates (both sides' roundings of them too) times its slope, 3.8 per lattice unit and
+ * stack (the second 1.0182 steeper).  The values must stay below 4: an octave is at most 1.04 in magnitude (the largest corner
+ * dots weighted by the smoothsteps, over the unit cube); 1.06 is used. */
 static void tile_bounds(MgNoise *shift, MgNoise *s, int n) {
     double c, cf, sc, scf;
     level_sums(shift, &sc, &scf);
-    const double es = 2.0 * sc * TILE_SHIFT_OCT + shift->nlev * (2.0 * 0x1.0p-29 + 2.1 * 0x1.0p-30) + 1e-12;
+    const double es = tile_noise(shift, sc, TILE_SHIFT_OCT);
+    bool ok = 2.0 * 1.06 * sc < 3.95;
+    for (int k = 0; k < shift->nlev; k++) ok = ok && shift->c30[k] != 0;
+    shift->tile_eq = shift->tile_eq_far = ok ? 0 : -1;
     for (int i = 0; i < n; i++) {
         level_sums(&s[i], &c, &cf);
-        double e = 2.0 * c * TILE_OCT + s[i].nlev * (2.0 * 0x1.0p-29 + 2.1 * 0x1.0p-30) + 1e-12;
-        e += 2.0 * 5.0 * 2.0182 * cf * (4.0 * es + 2.0 * 0x1.0p-32 + 0x1.0p-30);
-        s[i].tile_eq = s[i].fix_err < 0.0 || 2.0 * 1.06 * c > 3.95 ? -1 : (int32_t)ceil(e * 0x1.0p29) + 2;
+        bool in = ok && s[i].fix_err >= 0.0 && 2.0 * 1.06 * c < 3.95;
+        for (int k = 0; k < s[i].nlev; k++) in = in && s[i].c30[k] != 0;
+        for (int far = 0; far < 2; far++) {
+            const double e = tile_noise(&s[i], c, tile_oct(far != 0)) +
+                             2.0 * 3.8 * 2.0182 * cf * (4.0 * es + (far ? 6.0 : 2.2) * TILE_U);
+            (far ? s[i].tile_eq_far : s[i].tile_eq) = in ? (int32_t)ceil(e * 0x1.0p29) + 2 : -1;
+        }
     }
-    shift->tile_eq = 2.0 * 1.06 * sc > 3.95 ? -1 : 0;
 }
 
 /* PerlinNoise/NormalNoise constants of 26.1/26.2 (engine/mc_noise.h:178-196) */
@@ -323,7 +333,7 @@ static void noise_double(MgNoise *s, const NoiseParams &P, int legacy) {
     for (int k = 0; k < s->nlev; k++) s->c31[k] = (int64_t)llround(s->amp_d[k] * s->vf_d[k] * s->vfac * 0x1.0p31);
     for (int k = 0; k < s->nlev; k++) {
         const double c = s->amp_d[k] * s->vf_d[k] * s->vfac;
-        s->c29[k] = fabs(c) < 3.9 ? (int32_t)llround(c * 0x1.0p29) : 0;
+        s->c30[k] = fabs(c) < 1.99 ? (int32_t)llround(c * 0x1.0p30) : 0; /* 0: the table form is not available */
     }
     const double e32 = screen_bound32(s);
     s->fix_eq32 = e32 < 0.0 ? -1 : (int64_t)ceil(e32 * 0x1.0p59) + 1;
@@ -333,7 +343,7 @@ static void noise_double(MgNoise *s, const NoiseParams &P, int legacy) {
 /* NoiseStack layer constants of 26.3 (engine/mc_noise.h:198-252) */
 static void noise_float(MgNoise *s, const NoiseParams &P, int legacy) {
     memset(s, 0, sizeof *s);
-    s->tile_eq = -1;
+    s->tile_eq = s->tile_eq_far = -1;
     s->fix_eq32 = -1;
     s->legacy = legacy;
     s->octs = P.n;
@@ -625,8 +635,8 @@ static int load_tree(const char *root, int version, int dim, std::vector<MgTreeN
     return MCGEN_OK;
 }
 
-/* The leaves of a flattened tree clustered into groups of up to 32 (MgWorldDesc::group_off), appended to it.  A set of leaves
- * is split at a multiple of 32 near its middle by the centre in the dimension whose halves' boxes are smallest. */
+/* The leaves of a flattened tree clustered into groups of 32, the last fewer (MgWorldDesc::group_off), appended to it.  A set of leaves
+ * is split at a multiple of 32 near its middle by the centre in the dimension whose halves' boxes have the least volume. */
 static void append_groups(std::vector<MgTreeNode> *tree, MgWorldDesc *D) {
     std::vector<MgTreeNode> leaves;
     std::vector<int> todo{0};
@@ -635,25 +645,24 @@ static void append_groups(std::vector<MgTreeNode> *tree, MgWorldDesc *D) {
         todo.pop_back();
         const MgTreeNode n = (*tree)[(size_t)nd];
         if (n.count == 0) {
-            MgTreeNode l = n;
-            l.first = (uint16_t)leaves.size();
-            leaves.push_back(l);
+            (*tree)[(size_t)nd].first = (uint16_t)leaves.size();
+            leaves.push_back((*tree)[(size_t)nd]);
         }
         for (int c = n.count - 1; c >= 0; c--) todo.push_back(n.first + c);
     }
     std::vector<int> order(leaves.size());
     for (size_t i = 0; i < order.size(); i++) order[i] = (int)i;
-    auto extent = [&](size_t s, size_t e) {
-        int64_t sum = 0;
+    auto volume = [&](size_t s, size_t e) { /* leaves times the logarithm of their box's volume (each side widened by 1000) */
+        double sum = 0.0;
         for (int d = 0; d < 6; d++) {
             int lo = 32767, hi = -32768;
             for (size_t i = s; i < e; i++) {
                 lo = std::min(lo, (int)leaves[(size_t)order[i]].lo[d]);
                 hi = std::max(hi, -(int)leaves[(size_t)order[i]].nhi[d]);
             }
-            sum += hi - lo;
+            sum += log2((double)(hi - lo) + 1000.0);
         }
-        return sum;
+        return sum * (double)(e - s);
     };
     std::vector<std::pair<size_t, size_t>> work{{0, order.size()}}, groups;
     while (!work.empty()) {
@@ -665,7 +674,7 @@ static void append_groups(std::vector<MgTreeNode> *tree, MgWorldDesc *D) {
         }
         const size_t m = s + ((e - s + 32) / 64) * 32;
         int best = 0;
-        int64_t cost = INT64_MAX;
+        double cost = 1e300;
         auto split = [&](int d) {
             std::nth_element(order.begin() + (long)s, order.begin() + (long)m, order.begin() + (long)e, [&](int a, int b) {
                 const int x = leaves[(size_t)a].lo[d] - leaves[(size_t)a].nhi[d], y = leaves[(size_t)b].lo[d] - leaves[(size_t)b].nhi[d];
@@ -674,7 +683,7 @@ static void append_groups(std::vector<MgTreeNode> *tree, MgWorldDesc *D) {
         };
         for (int d = 0; d < 6; d++) {
             split(d);
-            const int64_t c = extent(s, m) + extent(m, e);
+            const double c = volume(s, m) + volume(m, e);
             if (c < cost) {
                 cost = c;
                 best = d;
@@ -684,15 +693,17 @@ static void append_groups(std::vector<MgTreeNode> *tree, MgWorldDesc *D) {
         work.push_back({m, e});
         work.push_back({s, m});
     }
+    const size_t ng = groups.size();
     D->group_off = (int32_t)tree->size();
-    D->groups = (int32_t)groups.size();
-    D->leaf_off = D->group_off + D->groups;
-    for (const auto &g : groups) {
+    D->groups = (int32_t)ng;
+    D->cluster_off = D->group_off + D->groups;
+    D->leaf_off = D->cluster_off + (int32_t)((ng + 31) / 32);
+    auto push_box = [&](size_t s, size_t e) { /* of the leaves order[s..e) */
         MgTreeNode n;
         memset(&n, 0, sizeof n);
         n.d7 = 0xFFFFFFFFu;
         for (int d = 0; d < 6; d++) n.lo[d] = n.nhi[d] = 32767;
-        for (size_t i = g.first; i < g.second; i++) {
+        for (size_t i = s; i < e; i++) {
             const MgTreeNode &l = leaves[(size_t)order[i]];
             for (int d = 0; d < 6; d++) {
                 n.lo[d] = std::min(n.lo[d], l.lo[d]);
@@ -700,10 +711,10 @@ static void append_groups(std::vector<MgTreeNode> *tree, MgWorldDesc *D) {
             }
             n.d7 = std::min(n.d7, l.d7);
         }
-        n.first = (uint16_t)g.first;
-        n.count = (uint8_t)(g.second - g.first);
         tree->push_back(n);
-    }
+    };
+    for (const auto &g : groups) push_box(g.first, g.second);
+    for (size_t c = 0; c < ng; c += 32) push_box(groups[c].first, groups[std::min(c + 32, ng) - 1].second);
     for (int i : order) tree->push_back(leaves[(size_t)i]);
 }
 
@@ -840,8 +851,6 @@ int build_world(const char *root, int version, int dim, const char *preset, MgWo
     D->tree_root = 0;
     D->tree_nodes = (int)tree->size();
     D->tree_leaves = nleaf;
-    D->tree_fanout = 0;
-    for (const MgTreeNode &n : *tree) D->tree_fanout = std::max(D->tree_fanout, (int32_t)n.count);
     append_groups(tree, D);
     return MCGEN_OK;
 }
