@@ -24,6 +24,7 @@ struct McWorld {
     /* device copies, created on first GPU use */
     int dev_ready;
     MgTreeNode *d_tree;
+    MgWorldDesc *d_desc;
     MgLattice *d_state;
     /* identity that no other world of the process ever has (caches key on it, never on the address) */
     uint64_t uid;

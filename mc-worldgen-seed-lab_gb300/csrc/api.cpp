@@ -95,12 +95,17 @@ int device_ready_locked() {
 int world_device_locked(McWorld *w) {
     if (w->dev_ready) return MCGEN_OK;
     cudaError_t e = cudaSuccess;
-    size_t tb = sizeof(MgTreeNode) * (w->tree.empty() ? 1 : w->tree.size());
-    if ((e = cudaMalloc(&w->d_tree, tb)) != cudaSuccess) return cuda_code(e);
-    if (!w->tree.empty() && (e = cudaMemcpy(w->d_tree, w->tree.data(), sizeof(MgTreeNode) * w->tree.size(),
-                                            cudaMemcpyHostToDevice)) != cudaSuccess)
-        return cuda_code(e);
-    if ((e = cudaMalloc(&w->d_state, sizeof(MgLattice) * (size_t)w->desc.ntables)) != cudaSuccess) return cuda_code(e);
+    /* one allocation: the tree, the description, the seed's lattices (each a multiple of 16 bytes) */
+    const size_t tb = sizeof(MgTreeNode) * w->tree.size(), wb = (sizeof(MgWorldDesc) + 15) & ~(size_t)15;
+    if (!w->d_tree) {
+        uint8_t *base = nullptr;
+        if ((e = cudaMalloc(&base, tb + wb + sizeof(MgLattice) * (size_t)w->desc.ntables)) != cudaSuccess) return cuda_code(e);
+        w->d_tree = (MgTreeNode *)base;
+        w->d_desc = (MgWorldDesc *)(base + tb);
+        w->d_state = (MgLattice *)(base + tb + wb);
+    }
+    if (tb && (e = cudaMemcpy(w->d_tree, w->tree.data(), tb, cudaMemcpyHostToDevice)) != cudaSuccess) return cuda_code(e);
+    if ((e = cudaMemcpy(w->d_desc, &w->desc, sizeof(MgWorldDesc), cudaMemcpyHostToDevice)) != cudaSuccess) return cuda_code(e);
     int64_t *d_seed = nullptr;
     if ((e = cudaMallocAsync(&d_seed, sizeof(int64_t), g_stream)) != cudaSuccess) return cuda_code(e);
     cudaMemcpyAsync(d_seed, &w->seeds.climate, sizeof(int64_t), cudaMemcpyHostToDevice, g_stream);
@@ -114,8 +119,7 @@ int world_device_locked(McWorld *w) {
 
 /* cudaFree waits for the device work that may still read the tree */
 void world_destroy_locked(McWorld *w) {
-    if (w->d_tree) cudaFree(w->d_tree);
-    if (w->d_state) cudaFree(w->d_state);
+    if (w->d_tree) cudaFree(w->d_tree); /* with the description and the lattices behind it */
     delete w;
 }
 
@@ -138,6 +142,14 @@ struct DevBuf { /* stream-ordered scratch, freed on the same stream */
     cudaStream_t s;
     explicit DevBuf(cudaStream_t st) : s(st) {}
     cudaError_t alloc(size_t n) { return n ? cudaMallocAsync(&p, n, s) : cudaSuccess; }
+    /* scratch that the launch can do without: null when there is no memory */
+    cudaError_t alloc_optional(size_t n) {
+        const cudaError_t e = alloc(n);
+        if (e != cudaErrorMemoryAllocation) return e;
+        cudaGetLastError();
+        p = nullptr;
+        return cudaSuccess;
+    }
     ~DevBuf() { if (p) cudaFreeAsync(p, s); }
 };
 
@@ -156,8 +168,9 @@ void end_chunk_range(long long xmin, long long xmax, long long zmin, long long z
 int block_biomes_dev(const McWorld *w, int x0, int z0, int nx, int nz, int step, int y, const int32_t *d_xyz,
                      long long xmin, long long xmax, long long zmin, long long zmax, uint8_t *d_out, cudaStream_t st) {
     int cx0 = 0, cz0 = 0, ncx = 0, ncz = 0;
-    DevBuf cls(st);
+    DevBuf cls(st); /* the End's chunk classes, or the Overworld's scratch */
     const long long n = (long long)nx * nz;
+    if (cudaError_t e = cls.alloc_optional(mg::block_scratch_bytes(w->desc, x0, z0, nx, nz, step, d_xyz != nullptr))) return cuda_code(e);
     if (w->desc.dim == MG_END) {
         end_chunk_range(xmin, xmax, zmin, zmax, &cx0, &cz0, &ncx, &ncz);
         /* a table is worth it when samples share chunks; sparse samples evaluate their chunk directly */
@@ -166,7 +179,7 @@ int block_biomes_dev(const McWorld *w, int x0, int z0, int nx, int nz, int step,
             if (e) return cuda_code(e);
         }
     }
-    int rc = mg::launch_block_biomes(w->desc, w->d_tree, w->d_state, w->zoom_seed, x0, z0, nx, nz, step, y, d_xyz,
+    int rc = mg::launch_block_biomes(w->desc, w->d_desc, w->d_tree, w->d_state, w->zoom_seed, x0, z0, nx, nz, step, y, d_xyz,
                                      d_out, cls.p, cx0, cz0, ncx, ncz, st);
     return rc ? cuda_code((cudaError_t)rc) : MCGEN_OK;
 }
@@ -455,16 +468,13 @@ MCGEN_API int mcgen_gb300_world_info(const McWorld *w, int *version, int *dimens
     return MCGEN_OK;
 }
 
-static int quart_grid_on(const McWorld *w, int qx0, int qz0, int nx, int nz, int qy, int rule, uint8_t *d_out,
+static int quart_grid_on(const McWorld *w, const MgLattice *state, int qx0, int qz0, int nx, int nz, int qy, int rule, uint8_t *d_out,
                          cudaStream_t st) {
-    const long long n = (long long)nx * nz;
     DevBuf scratch(st);
-    size_t sb = 0;
-    if (w->dim == MG_END) sb = (size_t)(nx / 4 + 3) * (size_t)(nz / 4 + 3);
-    else if (rule == MCGEN_TIE_GRID_CHAIN || rule == MCGEN_TIE_CHUNK_ORDER) sb = mg::chain_scratch_bytes(n);
-    cudaError_t e = scratch.alloc(sb);
+    const size_t need = mg::quart_scratch_bytes(w->desc, rule, nx, nz);
+    cudaError_t e = mg::quart_scratch_optional(w->desc, rule) ? scratch.alloc_optional(need) : scratch.alloc(need);
     if (e) return cuda_code(e);
-    int rc = mg::launch_quart_grid(w->desc, w->d_tree, w->d_state, qx0, qz0, nx, nz, qy, rule, d_out, scratch.p, st);
+    int rc = mg::launch_quart_grid(w->desc, w->d_desc, w->d_tree, state, qx0, qz0, nx, nz, qy, rule, d_out, scratch.p, st);
     return rc ? cuda_code((cudaError_t)rc) : MCGEN_OK;
 }
 
@@ -480,7 +490,7 @@ MCGEN_API int mcgen_gb300_quart_grid(const McWorld *w, int qx0, int qz0, int nx,
     DevBuf d_out(g_stream);
     cudaError_t e = d_out.alloc((size_t)nx * (size_t)nz);
     if (e) return cuda_code(e);
-    rc = quart_grid_on(w, qx0, qz0, nx, nz, qy, tie_rule, (uint8_t *)d_out.p, g_stream);
+    rc = quart_grid_on(w, w->d_state, qx0, qz0, nx, nz, qy, tie_rule, (uint8_t *)d_out.p, g_stream);
     if (rc) return rc;
     if ((e = cudaMemcpyAsync(out, d_out.p, (size_t)nx * (size_t)nz, cudaMemcpyDeviceToHost, g_stream))) return cuda_code(e);
     return cuda_code(cudaStreamSynchronize(g_stream));
@@ -494,7 +504,7 @@ MCGEN_API int mcgen_gb300_quart_grid_dev(const McWorld *w, int qx0, int qz0, int
     if (!device_ready_locked()) return MCGEN_E_UNSUPPORTED;
     int rc = world_device_locked(const_cast<McWorld *>(w));
     if (rc) return rc;
-    return quart_grid_on(w, qx0, qz0, nx, nz, qy, tie_rule, d_out, (cudaStream_t)stream);
+    return quart_grid_on(w, w->d_state, qx0, qz0, nx, nz, qy, tie_rule, d_out, (cudaStream_t)stream);
 }
 
 static int seed_points_on(const McWorld *w, const int64_t *d_seeds, int ns, const int32_t *d_pts, int np,
@@ -603,19 +613,13 @@ MCGEN_API int mcgen_gb300_quart_grid_seed_dev(const McWorld *w, int64_t seed, in
     int rc = world_device_locked(const_cast<McWorld *>(w));
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    DevBuf state(st), d_seed(st), scratch(st);
+    DevBuf state(st), d_seed(st);
     cudaError_t e;
     if ((e = state.alloc(sizeof(MgLattice) * (size_t)w->desc.ntables)) || (e = d_seed.alloc(sizeof(int64_t))))
         return cuda_code(e);
     if ((e = cudaMemcpyAsync(d_seed.p, &seed, sizeof seed, cudaMemcpyHostToDevice, st))) return cuda_code(e);
     if ((rc = mg::launch_setup(w->desc, (const int64_t *)d_seed.p, 1, (MgLattice *)state.p, st))) return cuda_code((cudaError_t)rc);
-    size_t sb = 0;
-    if (w->dim == MG_END) sb = (size_t)(nx / 4 + 3) * (size_t)(nz / 4 + 3);
-    else if (tie_rule == MCGEN_TIE_GRID_CHAIN || tie_rule == MCGEN_TIE_CHUNK_ORDER) sb = mg::chain_scratch_bytes((long long)nx * nz);
-    if ((e = scratch.alloc(sb))) return cuda_code(e);
-    rc = mg::launch_quart_grid(w->desc, w->d_tree, (const MgLattice *)state.p, qx0, qz0, nx, nz, qy, tie_rule, d_out,
-                               scratch.p, st);
-    return rc ? cuda_code((cudaError_t)rc) : MCGEN_OK;
+    return quart_grid_on(w, (const MgLattice *)state.p, qx0, qz0, nx, nz, qy, tie_rule, d_out, st);
 }
 
 MCGEN_API long long mcgen_gb300_launch_count(void) { return mg::launch_count(); }

@@ -253,7 +253,7 @@ const int kBatchTileWidths[BATCH_SHAPES] = {8, 8, 8, 8};
 static int g_resident[BATCH_SHAPES] = {0, 0, 0, 0}; /* CTAs per SM x SMs, per shape (batch_prepare) */
 
 int batch_group(const MgWorldDesc &W, int tie) {
-    if (tie != MG_TIE_ENGINE || !ow_tile_supported(W)) return BATCH_REST;
+    if ((tie != MG_TIE_ENGINE && tie != MG_TIE_CHUNK_CELL) || !ow_tile_supported(W)) return BATCH_REST;
     return W.fmode ? BATCH_OW_F : BATCH_OW_D;
 }
 
@@ -306,23 +306,29 @@ int batch_prepare(int *ctas_per_sm) {
     if (!rc) rc = prepare_t<8, 7>(1, sms);
     if (!rc) rc = prepare_t<8, 6>(2, sms);
     if (!rc) rc = prepare_t<8, 8>(3, sms);
-    if (!rc) rc = ow_prepare(sms);
+    if (!rc) rc = ow_prepare();
     if (!rc) prepared_dev = dev;
     if (ctas_per_sm) *ctas_per_sm = g_resident[0] / (sms > 0 ? sms : 1);
     return rc;
 }
 
+void batch_open_cap(const long long cells[2], int tie, long long open_cap[2]) {
+    open_cap[0] = ow_open_cap(cells[0]);
+    open_cap[1] = tie == MG_TIE_CHUNK_CELL ? ow_open_cap(cells[1]) : 0; /* the float branch leaves tied cells only */
+}
 int launch_batch(const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees, const MgBatchReq *d_reqs,
-                 const BatchGroups &g, const MgLattice *d_pool, unsigned long long *d_counter, MgOpenCell *d_open,
-                 long long open_cap, uint8_t *d_out, int ctas, int shape, cudaStream_t st) {
+                 const BatchGroups &g, int tie, const MgLattice *d_pool, unsigned long long *d_counter, MgOpenCell *d_open,
+                 const long long open_cap[2], uint8_t *d_out, int ctas, int shape, cudaStream_t st) {
     if (g.tiles[0] + g.tiles[1] + g.tiles[2] <= 0) return 0;
     if (shape < 0 || shape >= BATCH_SHAPES || g_resident[shape] <= 0) return (int)cudaErrorInvalidValue;
     cudaError_t e = cudaMemsetAsync(d_counter, 0, BATCH_COUNTERS * sizeof(unsigned long long), st);
     if (e) return (int)e;
-    unsigned long long *nopen = d_counter + BATCH_GROUPS;
-    int rc = launch_ow_tiles(false, d_worlds, d_trees, d_reqs, g.n[0], g.tiles[0], d_pool, d_counter, d_open, nopen, open_cap, d_out, st);
-    if (!rc) rc = launch_ow_tiles(true, d_worlds, d_trees, d_reqs + g.n[0], g.n[1], g.tiles[1], d_pool, d_counter + 1, nullptr,
-                                  nullptr, 0, d_out, st);
+    auto group = [&](int i, bool open_pass) {
+        return launch_ow_batch(i == 1, tie, open_pass, d_worlds, d_trees, d_reqs + (i ? g.n[0] : 0), g.n[i], g.tiles[i], d_pool, d_counter + i,
+                               d_open ? d_open + (i ? open_cap[0] : 0) : nullptr, d_counter + BATCH_GROUPS + i, open_cap[i], d_out, st);
+    };
+    int rc = group(0, false);
+    if (!rc) rc = group(1, false);
     if (rc) return rc;
     if (g.tiles[BATCH_REST] > 0) {
         const MgBatchReq *rq = d_reqs + g.n[0] + g.n[1];
@@ -345,8 +351,8 @@ int launch_batch(const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees, 
         count_launch_external();
         if ((e = cudaGetLastError())) return (int)e;
     }
-    if (g.tiles[0] > 0 && d_open && open_cap > 0) rc = launch_ow_open(d_worlds, d_trees, d_reqs, d_pool, d_open, nopen, open_cap, d_out, st);
-    return rc;
+    rc = group(0, true);
+    return rc ? rc : group(1, true);
 }
 
 }  // namespace mg

@@ -25,30 +25,29 @@ typedef struct {
 
 #define BATCH_SHAPES 4
 /* The requests of a batch come in three groups, each contiguous and with a tile numbering of its own: Overworld
- * requests under the ENGINE rule by branch (owtile.cu: 16 x 16-cell tiles), then everything else (batch.cu). */
+ * requests by branch (owtile.cu: 16 x 16-cell tiles), then everything else (batch.cu). */
 enum { BATCH_OW_D = 0, BATCH_OW_F = 1, BATCH_REST = 2, BATCH_GROUPS = 3 };
 namespace mg {
 struct BatchGroups {
     int n[BATCH_GROUPS];
     long long tiles[BATCH_GROUPS];
 };
-/* device counters of a batch: tiles taken per group, cells recorded as open */
-#define BATCH_COUNTERS (BATCH_GROUPS + 1)
+/* device counters of a batch: tiles taken per group, cells recorded as open per Overworld group */
+#define BATCH_COUNTERS (BATCH_GROUPS + 2)
 int batch_group(const MgWorldDesc &W, int tie);
-/* owtile.cu: tiles of a request, the worlds it takes, attributes, launch */
+
+/* ---- owtile.cu: worlds the tile kernels take, a request's tiles, attributes (call before any capture) */
 bool ow_tile_supported(const MgWorldDesc &W);
 long long ow_tiles(int nx, int nz);
-int ow_prepare(int sms);
-/* records to provide for a batch with `cells` double-branch Overworld cells (about 2 % keep a target open; cells beyond the
- * record are evaluated in place) */
+int ow_prepare();
+/* records to provide for `cells` cells some of which are left to the exact evaluation (the double branch's with a target
+ * open, well below 1 %; under the chunk-cell rule the tied ones too; cells beyond the record are evaluated in place) */
 long long ow_open_cap(long long cells);
-/* fm: the float branch's kernel; the double branch's records the cells it leaves open */
-int launch_ow_tiles(bool fm, const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees, const MgBatchReq *d_reqs, int nreq,
-                    long long ntiles, const MgLattice *d_pool, unsigned long long *d_counter, MgOpenCell *d_open,
-                    unsigned long long *d_nopen, long long open_cap, uint8_t *d_out, cudaStream_t st);
-/* the exact evaluation of the recorded cells */
-int launch_ow_open(const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees, const MgBatchReq *d_reqs, const MgLattice *d_pool,
-                   const MgOpenCell *d_open, const unsigned long long *d_nopen, long long open_cap, uint8_t *d_out, cudaStream_t st);
+/* a group's requests (fm: the float branch's); open_pass: the recorded cells, after the tiles */
+int launch_ow_batch(bool fm, int tie, bool open_pass, const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees,
+                    const MgBatchReq *d_reqs, int nreq, long long ntiles, const MgLattice *d_pool, unsigned long long *d_counter,
+                    MgOpenCell *d_open, unsigned long long *d_nopen, long long open_cap, uint8_t *d_out, cudaStream_t st);
+
 /* tile widths of the four Overworld/Nether tile shapes (128 cells each; the shapes also differ in the
  * register budget: 9, 7, 6 and 8 resident CTAs per SM) */
 extern const int kBatchTileWidths[BATCH_SHAPES];
@@ -60,11 +59,13 @@ int launch_setup_list(const MgWorldDesc *d_worlds, int dim, const MgSetupEntry *
                       long long total_lattices, MgLattice *d_pool, cudaStream_t st);
 /* kernel attributes and resident grid sizes; call before any stream capture */
 int batch_prepare(int *ctas_per_sm);
-/* d_reqs: the requests in group order.  ctas: upper bound on the rest's persistent grid, 0 = every resident CTA of
- * the shape.  d_counter: BATCH_COUNTERS counters; with d_open (open_cap records) the double-branch Overworld cells the tile
- * kernel leaves open are recorded and finished by a last launch, without it in place. */
+/* d_reqs: the requests in group order, all under one tie rule.  ctas: upper bound on the rest's persistent grid, 0 = every
+ * resident CTA of the shape.  d_counter: BATCH_COUNTERS counters.  d_open: open_cap[0] + open_cap[1] records for the open cells
+ * of the double and the float group, finished by launches after the tiles (null: evaluated in place). */
 int launch_batch(const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees, const MgBatchReq *d_reqs,
-                 const BatchGroups &g, const MgLattice *d_pool, unsigned long long *d_counter, MgOpenCell *d_open,
-                 long long open_cap, uint8_t *d_out, int ctas, int shape, cudaStream_t st);
+                 const BatchGroups &g, int tie, const MgLattice *d_pool, unsigned long long *d_counter, MgOpenCell *d_open,
+                 const long long open_cap[2], uint8_t *d_out, int ctas, int shape, cudaStream_t st);
+/* open_cap of a batch whose Overworld groups have `cells` cells */
+void batch_open_cap(const long long cells[2], int tie, long long open_cap[2]);
 }  // namespace mg
 #endif

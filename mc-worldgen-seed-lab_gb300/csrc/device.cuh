@@ -924,11 +924,23 @@ struct RtTarget {
     uint32_t p[3], n[3];
 };
 __device__ __forceinline__ uint32_t pack16(int32_t lo, int32_t hi) { return (uint32_t)(lo & 0xFFFF) | ((uint32_t)hi << 16); }
-/* false when a coordinate is outside +-(32767 - MG_TREE_PACKED_BOUND) */
-__device__ __forceinline__ bool rt_target(const int32_t *t, RtTarget &q) {
+/* a coordinate beyond +-(32767 - MG_TREE_PACKED_BOUND) may still be within 16 bits of all bounds of its dimension, which lie in
+ * the root's box or, an exclusive upper bound of an empty range, one below it (amplified depths: 25,000 against bounds from 0 to
+ * 11,000; on the 64-bit search they cost a tile 350 us) */
+__device__ __noinline__ static bool rt_target_far(const MgTreeNode *__restrict__ T, const int32_t t0, const int32_t t1, const int32_t t2,
+                                                  const int32_t t3, const int32_t t4, const int32_t t5) {
+    const int32_t t[6] = {t0, t1, t2, t3, t4, t5};
+    bool ok = true;
+    for (int k = 0; k < 6; k++)
+        ok &= t[k] >= -32767 && t[k] <= 32767 && t[k] <= 32766 + T->lo[k] && t[k] >= -T->nhi[k] - 32766;
+    return ok;
+}
+/* false when a coordinate is too far from the bounds of its dimension for the packed distances */
+__device__ __forceinline__ bool rt_target(const MgTreeNode *__restrict__ T, const int32_t *t, RtTarget &q) {
     const int32_t lim = 32767 - MG_TREE_PACKED_BOUND;
     bool ok = true;
     for (int k = 0; k < 6; k++) ok &= t[k] >= -lim && t[k] <= lim;
+    if (!ok) ok = rt_target_far(T, t[0], t[1], t[2], t[3], t[4], t[5]);
     for (int k = 0; k < 3; k++) {
         q.p[k] = pack16(t[2 * k], t[2 * k + 1]);
         q.n[k] = pack16(-t[2 * k], -t[2 * k + 1]);
@@ -1022,7 +1034,7 @@ __device__ __forceinline__ bool rt_packed(const MgTreeNode *__restrict__ T) {
 template <bool FLAT>
 __device__ __forceinline__ int tree_search_t(const MgTreeNode *__restrict__ T, const int32_t *t, int cand, uint64_t &best) {
     RtTarget q;
-    if (cand < 0 && rt_packed(T) && rt_target(t, q)) {
+    if (cand < 0 && rt_packed(T) && rt_target(T, t, q)) {
         const RtState s = FLAT ? rt_find_flat<false>(T, q) : rt_find<false>(T, q);
         if (s.res >= 0 && s.best < (uint32_t)MG_RT_CLAMP * MG_RT_CLAMP) {
             best = s.best;
@@ -1041,7 +1053,7 @@ __device__ __forceinline__ int tree_search_scattered(const MgTreeNode *__restric
 __device__ __forceinline__ int tree_search_tie(const MgTreeNode *__restrict__ T, const int32_t *t, uint64_t &best,
                                                bool &tied) {
     RtTarget q;
-    if (rt_packed(T) && rt_target(t, q)) {
+    if (rt_packed(T) && rt_target(T, t, q)) {
         const RtState s = rt_find<true>(T, q);
         if (s.res >= 0 && s.best < (uint32_t)MG_RT_CLAMP * MG_RT_CLAMP) {
             best = s.best;
@@ -1075,61 +1087,132 @@ struct RtNode {
     __device__ __forceinline__ RtNode(const MgTreeNode *n)
         : a(*reinterpret_cast<const uint4 *>(n)), b(*(reinterpret_cast<const uint4 *>(n) + 1)) {}
 };
-/* the nearest leaf (counted from leaf_off), its word and distance, leaves at that distance (capped at 2) */
+/* the nearest leaf (counted from leaf_off), its word and distance, leaves at that distance (capped at 2; not by rt_warp<NEXT>);
+ * rt_warp<NEXT>: the least distance of the other leaves met (RT_OTHER), or of those of another biome (RT_BIOME) */
+enum { RT_OTHER = 1, RT_BIOME = 2 };
 struct RtWarp {
     uint32_t best, word;
     int leaf, cnt;
+    uint32_t next;
 };
-template <bool TIE>
-__device__ __forceinline__ void rt_warp_leaf(const RtNode &n, int at, const RtTarget &q, RtWarp &r) {
-    const uint32_t d = rt_dist(n.a, n.b, q);
+/* The root of a leaf's distance changes by at most 1 when the target moves by one unit in one dimension.  So a leaf that is
+ * nearest at t, all others being farther than (sqrt(best) + 2)^2, is nearest at the neighbouring targets too, and untied; with
+ * only the leaves of other biomes that far, the neighbours' nearest has its biome.
+ * rt_beyond(d) >= (sqrt(d) + 2)^2 (d + 4 sqrt(d) + 4, the root by rsqrtf, within 2 ulp; 0 rsqrtf(0) is a NaN, cast to 0). */
+__device__ __forceinline__ uint32_t rt_beyond(uint32_t d) {
+    return d < 0x80000000u ? d + (uint32_t)(4.01f * ((float)d * rsqrtf((float)d))) + 6u : d;
+}
+template <bool TIE, int NEXT = 0>
+__device__ __forceinline__ void rt_warp_leaf_at(uint32_t d, uint32_t word, int at, RtWarp &r) {
+    if (NEXT == RT_OTHER || (NEXT == RT_BIOME && (word ^ r.word) > 0xFFFFFFu)) r.next = min(r.next, max(r.best, d));
     const bool lt = d < r.best, eq = d == r.best;
     if (TIE) r.cnt = lt ? 1 : (eq ? min(r.cnt + 1, 2) : r.cnt);
-    if (lt || (eq && (n.b.w & 0xFFFFu) < (r.word & 0xFFFFu))) {
+    if (lt || (eq && (word & 0xFFFFu) < (r.word & 0xFFFFu))) {
         r.best = d;
-        r.word = n.b.w;
+        r.word = word;
         r.leaf = at;
     }
 }
+template <bool TIE, int NEXT>
+__device__ __forceinline__ void rt_warp_leaf(const RtNode &n, int at, const RtTarget &q, RtWarp &r) {
+    rt_warp_leaf_at<TIE, NEXT>(rt_dist(n.a, n.b, q), n.b.w, at, r);
+}
+/* One target's search by the whole warp, a cluster, group or leaf per lane, nearest first; all lanes pass the same q and U (a
+ * distance that some leaf does not exceed).  The result is the same in all lanes; leaf -1 when the distance is not exact. */
+__device__ __noinline__ static RtWarp rt_point(const MgTreeNode *__restrict__ T, const MgWorldDesc &W, const RtTarget q, uint32_t U) {
+    const unsigned FULL = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    RtWarp r{0xFFFFFFFFu, 0, -1, 0, 0xFFFFFFFFu};
+    const int groups = W.groups, leaves = W.tree_leaves;
+    const MgTreeNode *G = T + W.group_off, *L = T + W.leaf_off;
+    for (int s0 = 0; 32 * s0 < groups; s0 += 32) {
+        uint32_t ls = 0xFFFFFFFFu;
+        if (32 * (s0 + lane) < groups) {
+            const RtNode n(T + W.cluster_off + s0 + lane);
+            ls = rt_dist(n.a, n.b, q);
+        }
+        for (;;) {
+            const uint32_t ms = __reduce_min_sync(FULL, ls);
+            if (ms > U) break;
+            const int s = __ffs((int)__ballot_sync(FULL, ls == ms)) - 1;
+            if (lane == s) ls = 0xFFFFFFFFu;
+            const int g0 = 32 * (s0 + s);
+            uint32_t lg = 0xFFFFFFFFu;
+            if (g0 + lane < groups) {
+                const RtNode n(G + g0 + lane);
+                lg = rt_dist(n.a, n.b, q);
+            }
+            for (;;) {
+                const uint32_t mg = __reduce_min_sync(FULL, lg);
+                if (mg > U) break;
+                const int g = __ffs((int)__ballot_sync(FULL, lg == mg)) - 1;
+                if (lane == g) lg = 0xFFFFFFFFu;
+                const int at = 32 * (g0 + g) + lane;
+                uint32_t d = 0xFFFFFFFFu;
+                if (at < leaves) {
+                    const RtNode n(L + at);
+                    d = rt_dist(n.a, n.b, q);
+                    rt_warp_leaf_at<true>(d, n.b.w, at, r);
+                }
+                U = min(U, __reduce_min_sync(FULL, d));
+            }
+        }
+    }
+    const bool at = r.best == U && r.leaf >= 0;
+    const unsigned rank = at ? r.word & 0xFFFFu : 0xFFFFFFFFu, first = __reduce_min_sync(FULL, rank);
+    const unsigned who = __ballot_sync(FULL, at && rank == first);
+    const bool exact = who && U < (uint32_t)MG_RT_CLAMP * MG_RT_CLAMP;
+    const int src = who ? __ffs((int)who) - 1 : 0;
+    return RtWarp{U, __shfl_sync(FULL, r.word, src), exact ? __shfl_sync(FULL, r.leaf, src) : -1,
+                  (int)__reduce_add_sync(FULL, at ? min(r.cnt, 2) : 0), 0};
+}
 /* leaves [32 g, 32 g + 32) of the clustered ones, the last group's fewer; ub: bound U by the group's own upper bounds first */
-template <bool TIE>
-__device__ __forceinline__ void rt_warp_group(const MgTreeNode *__restrict__ L, int leaves, int g, bool ub, const RtTarget &q,
-                                              const RtTarget &lbq, const RtTarget &ubq, bool active, uint32_t &U, RtWarp &r) {
+template <bool TIE, int NEXT>
+__device__ __forceinline__ void rt_warp_group(const MgTreeNode *__restrict__ L, const MgTreeNode *__restrict__ box, int leaves, int g, bool ub, const RtTarget &q,
+                                              const RtTarget &lbq, const RtTarget &ubq, bool active, bool near, uint32_t bound, uint32_t &U, RtWarp &r) {
     const unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31, first = 32 * g;
     const MgTreeNode *G = L + first;
     const bool in = first + lane < leaves;
     const RtNode n(G + (in ? lane : 0));
     const uint32_t lb = rt_dist(n.a, n.b, lbq);
-    if (ub) U = min(U, __reduce_min_sync(FULL, rt_ub_or_inf(n.a, n.b, ubq)));
+    auto within = [&](uint32_t d) { return NEXT && near ? rt_beyond(d) : d; };
+    if (ub) U = min(U, within(__reduce_min_sync(FULL, rt_ub_or_inf(n.a, n.b, ubq))));
     unsigned m = __ballot_sync(FULL, in && lb <= U);
     if (!m) return;
+    if (m & (m - 1)) { /* does any lane need it?  Where terrain breaks (amplified heights) the targets' box meets up to 95 groups
+                        * and 870 leaves of which each lane needs 5 groups: 310 -> 170 us for 256 x 256 such cells */
+        const RtNode b(box);
+        const uint32_t own = min(r.best, bound);
+        if (!__any_sync(FULL, active && rt_dist(b.a, b.b, q) <= within(own))) return;
+    }
     while (m) { /* two at a time: their loads and distances overlap */
         const int i = __ffs((int)m) - 1;
         m &= m - 1;
         const int j = m ? __ffs((int)m) - 1 : -1;
         m &= m - 1;
         const RtNode n0(G + i), n1(G + max(j, 0));
-        rt_warp_leaf<TIE>(n0, first + i, q, r);
-        if (j >= 0) rt_warp_leaf<TIE>(n1, first + j, q, r);
+        rt_warp_leaf<TIE, NEXT>(n0, first + i, q, r);
+        if (j >= 0) rt_warp_leaf<TIE, NEXT>(n1, first + j, q, r);
     }
-    U = min(U, __reduce_max_sync(FULL, active ? r.best : 0u));
+    U = min(U, within(__reduce_max_sync(FULL, active ? min(r.best, bound) : 0u)));
 }
 /* all 32 lanes call it; false (for the whole warp) when the tree or an active lane's target is outside the packed range: the
  * lanes search alone.  An active lane's best below MG_RT_CLAMP^2 is exact, else it searches alone.  hint: any leaf (counted
  * from leaf_off), best one near the lane's target (the lane's last result): it bounds the search from the start.  With none
  * (-1) every group's leaves give upper bounds too (without either, 43 leaves a warp were evaluated instead of 23). */
-template <bool TIE>
+template <bool TIE, int NEXT>
 __device__ __forceinline__ bool rt_warp(const MgTreeNode *__restrict__ T, const MgWorldDesc &W, const int32_t *t, bool active,
-                                        int hint, RtWarp &r) {
+                                        int hint, RtWarp &r, bool near = false) {
     const unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
     r.best = 0xFFFFFFFFu;
     r.word = 0xFFFFu;
     r.leaf = -1;
     r.cnt = 0;
+    r.next = 0xFFFFFFFFu;
     RtTarget q{};
-    const bool ok = !active || rt_target(t, q);
+    const bool ok = !active || rt_target(T, t, q);
     if (!__all_sync(FULL, ok) || !rt_packed(T)) return false;
     RtTarget lbq, ubq;
     bool none = false;
@@ -1146,13 +1229,13 @@ __device__ __forceinline__ bool rt_warp(const MgTreeNode *__restrict__ T, const 
     if (none) return true; /* no active lane */
     const int groups = W.groups, leaves = W.tree_leaves;
     const MgTreeNode *G = T + W.group_off, *L = T + W.leaf_off;
-    uint32_t U = 0xFFFFFFFEu;
+    uint32_t U = 0xFFFFFFFEu, bound = 0xFFFFFFFFu;
     if (hint >= 0) {
         /* the hinted leaf's distance bounds the lane's; the leaf itself is met again on the way */
         const RtNode n(L + hint);
-        const uint32_t d = rt_dist(n.a, n.b, q);
-        r.best = d + 1u;
-        U = min(__reduce_max_sync(FULL, active ? d : 0u), __reduce_min_sync(FULL, active ? rt_ub_or_inf(n.a, n.b, ubq) : 0xFFFFFFFFu));
+        bound = rt_dist(n.a, n.b, q);
+        const uint32_t u = min(__reduce_max_sync(FULL, active ? bound : 0u), __reduce_min_sync(FULL, active ? rt_ub_or_inf(n.a, n.b, ubq) : 0xFFFFFFFFu));
+        U = min(U, NEXT && near ? rt_beyond(u) : u);
     }
     for (int s0 = 0; 32 * s0 < groups; s0 += 32) { /* up to 32 clusters of 32 groups (the Overworld has 8) */
         const int ns = min((groups + 31) / 32 - s0, 32);
@@ -1178,7 +1261,7 @@ __device__ __forceinline__ bool rt_warp(const MgTreeNode *__restrict__ T, const 
             int j = first ? __ffs((int)__ballot_sync(FULL, l == __reduce_min_sync(FULL, l))) - 1 : __ffs((int)p) - 1;
             while (p) {
                 p &= ~(1u << j);
-                rt_warp_group<TIE>(L, leaves, g0 + j, first || hint < 0, q, lbq, ubq, active, U, r);
+                rt_warp_group<TIE, NEXT>(L, G + g0 + j, leaves, g0 + j, first || hint < 0, q, lbq, ubq, active, near, bound, U, r);
                 first = false;
                 p &= __ballot_sync(FULL, l <= U);
                 j = __ffs((int)p) - 1;
@@ -1189,26 +1272,39 @@ __device__ __forceinline__ bool rt_warp(const MgTreeNode *__restrict__ T, const 
     }
     return true;
 }
-/* tree_search (no candidate) for the 32 neighbouring cells of a warp, called by all 32 lanes; inactive lanes get -1 */
+/* tree_search (no candidate) for the 32 neighbouring cells of a warp, called by all 32 lanes; inactive lanes get -1.
+ * NEAR: in the lanes that ask for it (sure), sure = every target one unit away in one dimension has this biome too. */
+template <bool NEAR = false>
 __device__ __forceinline__ int tree_search_warp(const MgTreeNode *__restrict__ T, const MgWorldDesc &W, const int32_t *t, bool active,
-                                                int hint = -1) {
+                                                int hint = -1, bool *sure = nullptr) {
     RtWarp r;
-    const bool shared = rt_warp<false>(T, W, t, active, hint, r);
+    const bool near = NEAR && __any_sync(0xFFFFFFFFu, active && *sure);
+    const bool shared = rt_warp<false, NEAR ? RT_BIOME : 0>(T, W, t, active, hint, r, near);
+    const bool ask = NEAR && *sure;
+    if (NEAR) *sure = false;
     if (!active) return -1;
     uint64_t d;
     if (!shared) return tree_search(T, t, -1, d);
-    return r.leaf >= 0 && r.best < (uint32_t)MG_RT_CLAMP * MG_RT_CLAMP ? W.leaf_off + r.leaf : tree_search_stack(T, t, -1, d);
+    if (r.leaf < 0 || r.best >= (uint32_t)MG_RT_CLAMP * MG_RT_CLAMP) return tree_search_stack(T, t, -1, d);
+    if (ask) *sure = r.next > rt_beyond(r.best);
+    return W.leaf_off + r.leaf;
 }
-/* tree_search_tie likewise: the nearest leaf, its distance and whether a second leaf has the same distance */
+/* tree_search_tie likewise: the nearest leaf, its distance and whether a second leaf has the same distance.  NEAR: in
+ * the lanes that ask for it, sure = the leaf is the nearest one of every target one unit away in one dimension too, no other as near. */
+template <bool NEAR = false>
 __device__ __forceinline__ int tree_search_tie_warp(const MgTreeNode *__restrict__ T, const MgWorldDesc &W, const int32_t *t, bool active,
-                                                    uint64_t &best, bool &tied) {
+                                                    uint64_t &best, bool &tied, int hint = -1, bool *sure = nullptr) {
     RtWarp r;
-    const bool shared = rt_warp<true>(T, W, t, active, -1, r);
+    const bool near = NEAR && __any_sync(0xFFFFFFFFu, active && *sure);
+    const bool shared = rt_warp<!NEAR, NEAR ? RT_OTHER : 0>(T, W, t, active, hint, r, near);
+    const bool ask = NEAR && *sure;
+    if (NEAR) *sure = false;
     if (!active) return -1;
     if (!shared) return tree_search_tie(T, t, best, tied);
     if (r.leaf < 0 || r.best >= (uint32_t)MG_RT_CLAMP * MG_RT_CLAMP) return tree_search_tie_stack(T, t, best, tied);
     best = r.best;
-    tied = r.cnt >= 2;
+    tied = NEAR ? r.next == r.best : r.cnt >= 2;
+    if (ask) *sure = r.next > rt_beyond(r.best);
     return W.leaf_off + r.leaf;
 }
 

@@ -19,7 +19,9 @@
 #include "endtile.cuh"
 #include "device.cuh"
 #include "launch.h"
+#include "batch.h"
 #include "prof.h"
+#include "warpcell.cuh"
 
 using namespace mgd;
 
@@ -195,7 +197,6 @@ __global__ void __launch_bounds__(128) k_points(const __grid_constant__ MgWorldD
 
 /* One seed's quart grid.  ENGINE: biome ids.  GRID_CHAIN: first minimum leaf, its fitness, tie flag and
  * the target of every cell, for k_chain_resolve. */
-struct ChainRec { int32_t tg[6]; uint64_t d; int32_t leaf; int32_t tie; };
 template <bool FM, int DIM, bool CHAIN>
 __global__ void __launch_bounds__(128) k_grid(const __grid_constant__ MgWorldDesc W, const MgTreeNode *__restrict__ tree,
                                               const MgLattice *__restrict__ state, int qx0, int qz0, int nx, int nz,
@@ -347,6 +348,23 @@ __global__ void __launch_bounds__(128, 6) k_blockgrid(const __grid_constant__ Mg
     }
     out[g] = (uint8_t)cell_chunk<FM, DIM>(W, *S, T, tree, cx, cy, cz);
 }
+/* Block points, one per warp (wc_*): a point's octaves, zoom candidates and tree nodes over the lanes.  A thread per point ran
+ * them in series: one point took 90 us, and a warp of unrelated points diverged in every search. */
+template <bool FM, int DIM>
+__global__ void __launch_bounds__(128) k_block_points(const __grid_constant__ MgWorldDesc W, const MgTreeNode *__restrict__ tree,
+                                                      const MgLattice *__restrict__ state, int64_t zseed,
+                                                      const int32_t *__restrict__ xyz, int n, uint8_t *__restrict__ out) {
+    extern __shared__ uint4 smem_raw[];
+    WcStage &st = *reinterpret_cast<WcStage *>(smem_raw);
+    wc_stage(st, W, state, threadIdx.x, blockDim.x);
+    __syncthreads();
+    for (int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < n; i += (int)((gridDim.x * blockDim.x) >> 5)) {
+        int cx, cy, cz;
+        wc_zoom(zseed, xyz[3 * (size_t)i], xyz[3 * (size_t)i + 1], xyz[3 * (size_t)i + 2], cx, cy, cz);
+        const int b = wc_cell_chunk<FM, DIM>(W, st.spline, st.lat, tree, cx, cy, cz);
+        if ((threadIdx.x & 31) == 0) out[i] = (uint8_t)b;
+    }
+}
 /* End class of chunks [cx0, cx0+ncx) x [cz0, cz0+ncz) */
 template <bool FM>
 __global__ void __launch_bounds__(128) k_end_chunks(const MgLattice *__restrict__ state, int cx0, int cz0, int ncx,
@@ -487,8 +505,18 @@ int launch_end_lookup(const MgWorldDesc &W, const uint8_t *cls, int cx0, int cz0
     count_launch();
     return (int)cudaGetLastError();
 }
-size_t chain_scratch_bytes(long long ncells) { return (size_t)ncells * (sizeof(ChainRec) + sizeof(int32_t)); }
-int launch_quart_grid(const MgWorldDesc &W, const MgTreeNode *tree, const MgLattice *state, int qx0, int qz0, int nx, int nz, int qy, int rule, uint8_t *out, void *scratch, cudaStream_t st) {
+/* chain records and their order, then (Overworld) the tile kernels' scratch */
+static size_t chain_bytes(long long n) { return ((size_t)n * (sizeof(ChainRec) + sizeof(int32_t)) + 15) & ~(size_t)15; }
+static bool chain_rule(int rule) { return rule == MG_TIE_GRID_CHAIN || rule == MG_TIE_CHUNK_ORDER; }
+/* cell indices of a tile grid are 32-bit */
+static bool quart_tiles(const MgWorldDesc &W, long long n) { return ow_tile_supported(W) && n < (1LL << 31); }
+size_t quart_scratch_bytes(const MgWorldDesc &W, int rule, int nx, int nz) {
+    if (W.dim == MG_END) return (size_t)(nx / 4 + 3) * (size_t)(nz / 4 + 3);
+    const long long n = (long long)nx * nz;
+    return (chain_rule(rule) ? chain_bytes(n) : 0) + (quart_tiles(W, n) ? ow_grid_scratch_bytes(W, false, n) : 0);
+}
+int launch_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const MgLattice *state, int qx0, int qz0,
+                      int nx, int nz, int qy, int rule, uint8_t *out, void *scratch, cudaStream_t st) {
     long long n = (long long)nx * nz;
     if (n <= 0) return 0;
     if (W.dim == MG_END) {
@@ -502,9 +530,14 @@ int launch_quart_grid(const MgWorldDesc &W, const MgTreeNode *tree, const MgLatt
         count_launch();
         return launch_end_lookup(W, cls, cx0, cz0, ncx, qx0, qz0, nx, nz, out, st);
     }
-    bool chain = rule == MG_TIE_GRID_CHAIN || rule == MG_TIE_CHUNK_ORDER;
+    const bool chain = chain_rule(rule);
     ChainRec *rec = (ChainRec *)scratch;
-    if (W.fmode) {
+    if (quart_tiles(W, n)) {
+        uint8_t *more = chain ? (uint8_t *)scratch + chain_bytes(n) : (uint8_t *)scratch;
+        const int rc = launch_ow_quart_grid(W, d_world, tree, state, qx0, qz0, nx, nz, qy, chain ? rec : nullptr, out,
+                                            ow_grid_scratch_bytes(W, false, n) ? more : nullptr, st);
+        if (rc) return rc;
+    } else if (W.fmode) {
         if (W.dim == MG_OVERWORLD) {
             if (chain) grid_t<true, MG_OVERWORLD, true>(W, tree, state, qx0, qz0, nx, nz, qy, out, rec, st);
             else grid_t<true, MG_OVERWORLD, false>(W, tree, state, qx0, qz0, nx, nz, qy, out, rec, st);
@@ -540,20 +573,35 @@ static void blockgrid_t(const MgWorldDesc &W, const MgTreeNode *tree, const MgLa
                         int z0, int nx, int nz, int step, int y, const int32_t *xyz, uint8_t *out, const uint8_t *cls,
                         int ecx0, int ecz0, int encx, cudaStream_t st) {
     size_t sm = DIM == MG_END ? 0 : grid_smem(W);
-    if (sm) cudaFuncSetAttribute(k_blockgrid<FM, DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     ProfScope ps_(K_BLOCKGRID, st);
+    if constexpr (DIM != MG_END) {
+        if (xyz) {
+            const long long nb = ((long long)nx + 3) / 4;
+            k_block_points<FM, DIM><<<(unsigned)(nb < 16 * 152 ? nb : 16 * 152), 128, sizeof(WcStage), st>>>(W, tree, state, zseed, xyz, nx,
+                                                                                                          out);
+            return;
+        }
+    }
+    if (sm) cudaFuncSetAttribute(k_blockgrid<FM, DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     /* the kernel's warp-tile form (its own test of the same condition): one CTA per 16 x 8-cell tile */
     const bool tiles = FM && DIM == MG_OVERWORLD && !xyz && step <= 16;
     const unsigned nb = tiles ? (unsigned)(((long long)(nx + 15) / 16) * ((nz + 7) / 8)) : blocks_for((long long)nx * nz, 128);
     k_blockgrid<FM, DIM><<<nb, 128, sm, st>>>(W, tree, state, zseed, x0, z0, nx, nz, step, y, xyz, out, cls, ecx0, ecz0,
                                               encx);
 }
+/* the scratch holds only the record of open cells, and without it (null) those are evaluated where they occur */
+bool quart_scratch_optional(const MgWorldDesc &W, int rule) { return W.dim == MG_OVERWORLD && !chain_rule(rule); }
+size_t block_scratch_bytes(const MgWorldDesc &W, int x0, int z0, int nx, int nz, int step, bool points) {
+    return W.dim == MG_OVERWORLD && !points && ow_block_grid_supported(W, x0, z0, step) ? ow_grid_scratch_bytes(W, true, (long long)nx * nz) : 0;
+}
 /* Block-coordinate biomes: a grid (xyz == nullptr) or n = nx points (nz == 1) at xyz. For the End,
  * `scratch` holds the chunk classes of [ecx0, ecx0+encx) x [ecz0, ecz0+encz). */
-int launch_block_biomes(const MgWorldDesc &W, const MgTreeNode *tree, const MgLattice *state, int64_t zseed, int x0,
-                        int z0, int nx, int nz, int step, int y, const int32_t *xyz, uint8_t *out, void *scratch,
+int launch_block_biomes(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const MgLattice *state, int64_t zseed,
+                        int x0, int z0, int nx, int nz, int step, int y, const int32_t *xyz, uint8_t *out, void *scratch,
                         int ecx0, int ecz0, int encx, int encz, cudaStream_t st) {
     if ((long long)nx * nz <= 0) return 0;
+    if (W.dim == MG_OVERWORLD && !xyz && ow_block_grid_supported(W, x0, z0, step))
+        return launch_ow_block_grid(W, d_world, tree, state, zseed, x0, z0, nx, nz, step, y, out, scratch, st);
     uint8_t *cls = (uint8_t *)scratch; /* End chunk classes, or null: evaluate per sample */
     if (W.dim == MG_END && cls) {
         if (W.fmode) { ProfScope ps_(K_END_CHUNKS, st); k_end_chunks<true><<<end_tiles(encx, encz), 128, 0, st>>>(state, ecx0, ecz0, encx, encz, cls, W.end_f2, W.end_g2); }

@@ -9,6 +9,9 @@
 
 namespace mg {
 
+/* GRID_CHAIN and CHUNK_ORDER: a cell's target, its first minimum leaf (a node index), fitness and tie flag */
+struct ChainRec { int32_t tg[6]; uint64_t d; int32_t leaf; int32_t tie; };
+
 long long launch_count();
 void count_launch_external(); /* for launchers outside kernels.cu */
 
@@ -33,18 +36,28 @@ int launch_ow_search_first(const MgWorldDesc &W, const MgTreeNode *tree, const i
                            const MgObs &o, int ties, void *scratch, int64_t *surv, unsigned *nsurv,
                            unsigned long long *fail, cudaStream_t st);
 
-/* one seed's quart grid.  Scratch: chain_scratch_bytes(nx*nz) for GRID_CHAIN and CHUNK_ORDER; for the End,
- * (nx/4 + 2) * (nz/4 + 2) bytes of chunk classes. */
-size_t chain_scratch_bytes(long long ncells);
-int launch_quart_grid(const MgWorldDesc &W, const MgTreeNode *tree, const MgLattice *state, int qx0, int qz0, int nx,
-                      int nz, int qy, int rule, uint8_t *out, void *scratch, cudaStream_t st);
+/* one seed's quart grid.  d_world: the description's device copy.  Scratch: quart_scratch_bytes. */
+size_t quart_scratch_bytes(const MgWorldDesc &W, int rule, int nx, int nz);
+bool quart_scratch_optional(const MgWorldDesc &W, int rule); /* may be null when there is no memory for it */
+int launch_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const MgLattice *state, int qx0, int qz0,
+                      int nx, int nz, int qy, int rule, uint8_t *out, void *scratch, cudaStream_t st);
 
 /* block-coordinate biomes (zoom + chunk-cell ties): a grid when xyz == nullptr, else nx points at xyz
- * (nz == 1).  End: scratch = chunk classes of [ecx0, ecx0+encx) x [ecz0, ecz0+encz), or null to evaluate
- * the class per sample. */
-int launch_block_biomes(const MgWorldDesc &W, const MgTreeNode *tree, const MgLattice *state, int64_t zseed, int x0,
-                        int z0, int nx, int nz, int step, int y, const int32_t *xyz, uint8_t *out, void *scratch,
+ * (nz == 1).  d_world: the description's device copy.  Scratch: block_scratch_bytes; for the End the chunk classes of
+ * [ecx0, ecx0+encx) x [ecz0, ecz0+encz), or null to evaluate the class per sample. */
+size_t block_scratch_bytes(const MgWorldDesc &W, int x0, int z0, int nx, int nz, int step, bool points);
+int launch_block_biomes(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const MgLattice *state, int64_t zseed,
+                        int x0, int z0, int nx, int nz, int step, int y, const int32_t *xyz, uint8_t *out, void *scratch,
                         int ecx0, int ecz0, int encx, int encz, cudaStream_t st);
+
+/* the same through the tile kernels (owtile.cu), for worlds ow_tile_supported takes and blocks at most 4 apart.  rec: the
+ * cells' chain records, or null.  Scratch: ow_grid_scratch_bytes. */
+bool ow_block_grid_supported(const MgWorldDesc &W, int x0, int z0, int step);
+size_t ow_grid_scratch_bytes(const MgWorldDesc &W, bool chunk_rule, long long cells);
+int launch_ow_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const MgLattice *state, int qx0,
+                         int qz0, int nx, int nz, int qy, ChainRec *rec, uint8_t *out, void *scratch, cudaStream_t st);
+int launch_ow_block_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const MgLattice *state, int64_t zseed,
+                         int x0, int z0, int nx, int nz, int step, int y, uint8_t *out, void *scratch, cudaStream_t st);
 
 /* Overworld density functions (continents, erosion, ridges, offset, depth) at n block points xyz[3i..3i+2] of
  * one seed's lattices: out[5i + k] (cudaErrorInvalidValue for other dimensions) */

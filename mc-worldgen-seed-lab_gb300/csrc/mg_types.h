@@ -73,8 +73,9 @@ typedef struct __attribute__((aligned(16))) {
  * (|v| <= 12000 in every table), the upper bounds stored negated (nhi = -hi: packed 16-bit add-max
  * instructions then form t - hi); the seventh dimension ("offset") always meets a target coordinate of 0,
  * so its squared distance max(-hi, lo, 0)^2 is stored instead of its bounds.  The root is never a leaf;
- * its biome byte holds MG_TREE_PACKED when every bound lies within +-MG_TREE_PACKED_BOUND (the packed
- * 16-bit distances are then exact for targets within +-(32767 - MG_TREE_PACKED_BOUND)). */
+ * its biome byte holds MG_TREE_PACKED when every bound lies within +-MG_TREE_PACKED_BOUND and hi >= lo - 1 (the packed
+ * 16-bit distances are then exact for targets within +-(32767 - MG_TREE_PACKED_BOUND), and for those within 32,766 of the
+ * root's box). */
 typedef struct __attribute__((aligned(16))) {
     int16_t lo[6];
     int16_t nhi[6];

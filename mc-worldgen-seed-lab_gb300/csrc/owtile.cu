@@ -1,5 +1,5 @@
-/* owtile.cu -- the batched form's Overworld requests (ENGINE rule): persistent kernels over 16 x 16-cell tiles whose
- * octaves read tables of lattice nodes (owtile.cuh). */
+/* owtile.cu -- the Overworld over areas: the batched form's requests, quart grids and the drop-in block map, by persistent
+ * kernels over 16 x 16-cell tiles whose octaves read tables of lattice nodes (owtile.cuh). */
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -8,6 +8,7 @@
 #include "launch.h"
 #include "owtile.cuh"
 #include "prof.h"
+#include "warpcell.cuh"
 
 namespace mg {
 
@@ -24,7 +25,7 @@ struct OtSmemF {
     MgLattice lat[MG_MAX_TABLES];
     float4 np[OT_CAP_F];
     float2 nq[OT_CAP_F];
-    OtShiftF sh[2 * OT_MAXLEV][4 * OT_W]; /* per lattice: X + ox, X + oy, Z + oz, Z + ox (16 entries each) */
+    OtShiftF sh[2 * OT_MAXLEV][4 * OT_TABW]; /* per lattice: X + ox, X + oy, Z + oz, Z + ox (a column or row each) */
     OtOctF oct[MG_MAX_TABLES];            /* the climate octaves in evaluation order */
     OtBuild build, sbuild;                /* climate and shift tables */
     int lo[2], hi[2];                     /* range of the shifted x and z over the tile, in 1/16 of a quart from its corner */
@@ -44,51 +45,124 @@ static __device__ __noinline__ void ot_cell_f(const MgWorldDesc &W, const MgLatt
 __device__ __forceinline__ uint16_t ot_hint(const MgWorldDesc &W, int leaf) {
     return (uint16_t)(leaf >= W.leaf_off ? leaf - W.leaf_off : 0);
 }
-/* next tile and its request (one whole warp calls it) */
-__device__ __forceinline__ void ot_next(OtTile &n, const MgBatchReq *__restrict__ reqs, int nreq, long long ntiles,
-                                        unsigned long long *__restrict__ counter) {
+/* where tiles come from: a batch's requests through its work queue, or one grid's tiles in turn (reqs null) */
+struct OtWork {
+    const MgWorldDesc *worlds;
+    const MgTreeNode *const *trees; /* per world; or, for one grid, null and `tree` */
+    const MgTreeNode *tree;
+    const MgBatchReq *reqs;
+    int nreq;
+    long long ntiles;
+    const MgLattice *pool;
+    unsigned long long *counter;
+    MgOpenCell *open; /* cells left to the exact evaluation, their counter and the room for them */
+    unsigned long long *nopen;
+    long long open_cap;
+    uint8_t *out;
+    MgBatchReq one;             /* one grid */
+    int64_t zseed;              /* OT_BLOCK: zoom seed, first block, spacing, block y */
+    int32_t x0, z0, step, y;
+    ChainRec *rec;              /* OT_CHAIN */
+};
+/* next tile and its request (one whole warp calls it); prev: the CTA's last tile of one grid, -1 at first */
+__device__ __forceinline__ void ot_next(OtTile &n, const OtWork &K, int prev) {
+    if (!K.reqs) {
+        if ((threadIdx.x & 31) == 0) {
+            const long long tile = prev < 0 ? (long long)blockIdx.x : (long long)prev + gridDim.x;
+            n.r = K.one;
+            n.req = tile < K.ntiles ? 0 : -1;
+            n.tile = (int)tile;
+        }
+        return;
+    }
     long long tile = 0;
-    if ((threadIdx.x & 31) == 0) tile = (long long)atomicAdd(counter, 1ULL);
+    if ((threadIdx.x & 31) == 0) tile = (long long)atomicAdd(K.counter, 1ULL);
     tile = __shfl_sync(0xFFFFFFFFu, tile, 0);
-    const int r = tile < ntiles ? find_req(reqs, nreq, tile) : -1;
+    const int r = tile < K.ntiles ? find_req(K.reqs, K.nreq, tile) : -1;
     if ((threadIdx.x & 31) == 0) {
         n.req = r;
         if (r >= 0) {
-            n.r = reqs[r];
+            n.r = K.reqs[r];
             n.tile = (int)(tile - n.r.tile0);
         }
     }
+}
+/* the quart cell of tile cell (tx, tz) of the grid, counted from (qx0, qz0) and quart y0 */
+template <int MODE>
+__device__ __forceinline__ void ot_cell(const OtWork &K, int tx, int tz, int qx0, int qz0, int qy0, int &dx, int &dz, int &dy) {
+    int cx, cy, cz;
+    zoom_cell(K.zseed, K.x0 + tx * K.step, K.y, K.z0 + tz * K.step, cx, cy, cz);
+    dx = cx - qx0;
+    dz = cz - qz0;
+    dy = cy - qy0;
+}
+__device__ __forceinline__ int ot_clamp_y(const MgWorldDesc &W, int qy) {
+    const int lo = W.min_y >> 2, hi = lo + (W.height >> 2) - 1;
+    return qy < lo ? lo : (qy > hi ? hi : qy);
+}
+/* one cell by the per-lane exact forms: a cell left open that has no room in the record, or one of many recorded ones */
+template <bool FM, int MODE>
+__device__ __noinline__ void ot_exact(const OtWork &K, const MgWorldDesc &W, const MgLattice *T, const MgTreeNode *tree, int qx, int qy,
+                                      int qz, long long o) {
+    if (MODE == OT_CHUNK || MODE == OT_BLOCK) {
+        put_id(K.out + o, cell_chunk<FM, MG_OVERWORLD>(W, W.spline, T, tree, qx, qy, qz));
+        return;
+    }
+    int32_t tg[6];
+    climate_ow<FM>(W, W.spline, T, qx, qy, qz, tg);
+    uint64_t d;
+    if (MODE == OT_CHAIN) {
+        bool tied;
+        const int leaf = tree_search_tie(tree, tg, d, tied);
+        ChainRec &r = K.rec[o];
+        for (int k = 0; k < 6; k++) r.tg[k] = tg[k];
+        r.d = d;
+        r.leaf = leaf;
+        r.tie = tied;
+        put_id(K.out + o, tree[leaf].biome);
+    } else {
+        put_id(K.out + o, tree[tree_search_scattered(tree, tg, -1, d)].biome);
+    }
+}
+/* leave a cell open: recorded, or evaluated here when the record is full */
+template <bool FM, int MODE>
+__device__ __forceinline__ void ot_leave_open(const OtWork &K, const MgWorldDesc &W, const MgLattice *T, const MgTreeNode *tree, int req,
+                                              int cell, int qx, int qy, int qz, long long o) {
+    const unsigned long long k = K.open_cap > 0 ? atomicAdd(K.nopen, 1ULL) : ~0ULL;
+    if (k < (unsigned long long)K.open_cap) K.open[k] = MgOpenCell{req, cell};
+    else ot_exact<FM, MODE>(K, W, T, tree, qx, qy, qz, o);
 }
 
 /* Float branch (26.3 on), bit for bit the per-cell form's operations.  Bound by instruction issue (66 % of peak; the octaves'
  * separately rounded lerps, the splits' mantissa shifts, the tree scan).  64 registers and 55 KB of shared memory: 4 CTAs,
  * 32 warps per SM.  The uneven batch's 70.8 M float-branch cells: 47.6 ms in the per-cell form, 37.9 ms here. */
-__global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const MgWorldDesc *__restrict__ worlds, const MgTreeNode *const *__restrict__ trees,
-                                                   const MgBatchReq *__restrict__ reqs, int nreq, long long ntiles,
-                                                   const MgLattice *__restrict__ pool, unsigned long long *__restrict__ counter,
-                                                   uint8_t *__restrict__ out) {
+template <int MODE>
+__global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const __grid_constant__ OtWork K) {
     extern __shared__ uint4 smem_raw[];
     OtSmemF &sm = *reinterpret_cast<OtSmemF *>(smem_raw);
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int col = ot_col(), row = ot_row();
     if (t == 0) sm.state = -1;
     sm.hint[t] = 0;
-    if (warp == 0) ot_next(sm.cur[0], reqs, nreq, ntiles, counter);
+    if (warp == 0) ot_next(sm.cur[0], K, -1);
     __syncthreads();
     for (int c = 0;; c ^= 1) {
         if (sm.cur[c].req < 0) return;
         const int tile = sm.cur[c].tile;
         const MgBatchReq &R = sm.cur[c].r;
-        const MgWorldDesc &W = worlds[R.world];
+        const MgWorldDesc &W = K.worlds[R.world];
         const MgNoise &O = W.noise[0];
         const int nlev = O.nlev, nsh = 2 * nlev, nclim = W.ntables - nsh;
         const int tw = (R.nx + OT_W - 1) / OT_W;
         const int tx0 = (tile % tw) * OT_W, tz0 = (tile / tw) * OT_W;
-        const int qx0 = R.qx0 + tx0, qz0 = R.qz0 + tz0;
+        /* first quart cell of the tile (of a block map: the lowest the zoom can give) */
+        const int qx0 = MODE == OT_BLOCK ? (K.x0 + tx0 * K.step - 2) >> 2 : R.qx0 + tx0;
+        const int qz0 = MODE == OT_BLOCK ? (K.z0 + tz0 * K.step - 2) >> 2 : R.qz0 + tz0;
+        const int qy0 = MODE == OT_BLOCK ? (K.y - 2) >> 2 : R.qy;
         /* beyond the world border the wrap may move a cell: the per-cell form takes the tile */
         const bool far = qx0 <= -OT_COORD_LIM || qz0 <= -OT_COORD_LIM || qx0 >= OT_COORD_LIM || qz0 >= OT_COORD_LIM;
         if (R.state != sm.state) { /* the request's lattices, octave constants and shift table layout */
-            const uint4 *a = reinterpret_cast<const uint4 *>(pool + R.state);
+            const uint4 *a = reinterpret_cast<const uint4 *>(K.pool + R.state);
             uint4 *b = reinterpret_cast<uint4 *>(sm.lat);
             for (int i = t; i < W.ntables * (int)(sizeof(MgLattice) / 16); i += OT_NT) b[i] = a[i];
             __syncthreads();
@@ -126,8 +200,8 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const MgWorldDesc *__restrict
             __syncthreads();
         }
         /* ---- 1: the shift noises' splits per column and row, and their nodes */
-        for (int e = far ? nsh * 4 * OT_W : t; e < nsh * 4 * OT_W; e += OT_NT) {
-            const int j = e / (4 * OT_W), q = e % (4 * OT_W), fam = q / OT_W, idx = q % OT_W;
+        for (int e = far ? nsh * 4 * OT_TABW : t; e < nsh * 4 * OT_TABW; e += OT_NT) {
+            const int j = e / (4 * OT_TABW), q = e % (4 * OT_TABW), fam = q / OT_TABW, idx = q % OT_TABW;
             const MgLattice &L = sm.lat[j];
             const double f = O.freq[j % nlev];
             const double off = fam == 0 || fam == 3 ? L.ox : (fam == 1 ? L.oy : L.oz);
@@ -165,14 +239,19 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const MgWorldDesc *__restrict
         __syncthreads();
         /* ---- 2: the shift noises and the shifted coordinates of the cell */
         const bool in = tx0 + col < R.nx && tz0 + row < R.nz;
+        int dx = col, dz = row, dy = 0; /* the cell, from the tile's first */
+        if (MODE == OT_BLOCK) {
+            if (in) ot_cell<MODE>(K, tx0 + col, tz0 + row, qx0, qz0, qy0, dx, dz, dy);
+            else dx = dz = 0;
+        }
         double x = 0.0, z = 0.0;
         if (!far) {
             float sa = 0.0f, sb = 0.0f;
 #pragma unroll 1
             for (int q = 0; q < nsh; q++) { /* level by level, first stack then second: each sum in its order */
                 const int k = q >> 1, j = (q & 1) * nlev + k;
-                const OtShiftF ax = sm.sh[j][col], by = sm.sh[j][OT_W + col], az = sm.sh[j][2 * OT_W + row],
-                               bx = sm.sh[j][3 * OT_W + row];
+                const OtShiftF ax = sm.sh[j][dx], by = sm.sh[j][OT_TABW + dx], az = sm.sh[j][2 * OT_TABW + dz],
+                               bx = sm.sh[j][3 * OT_TABW + dz];
                 const float amp = O.amp_f[k];
                 sa += amp * ot_octave_f<false>(sm.np, sm.nq, ax.node + az.node, sm.sbuild.nx[2 * j], ax.f, ax.g, ax.u, az.f,
                                                az.g, az.u, sm.lat[j].z0.f.uy);
@@ -180,9 +259,9 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const MgWorldDesc *__restrict
                                               by.g, by.u, sm.lat[j].z0.f.uz);
             }
             const float sx = sa * 4.0f, sz = sb * 4.0f;
-            x = (double)(qx0 + col) + (double)sx;
-            z = (double)(qz0 + row) + (double)sz;
-            const int rx = __float2int_rd(((float)col + sx) * 16.0f), rz = __float2int_rd(((float)row + sz) * 16.0f);
+            x = (double)(qx0 + dx) + (double)sx;
+            z = (double)(qz0 + dz) + (double)sz;
+            const int rx = __float2int_rd(((float)dx + sx) * 16.0f), rz = __float2int_rd(((float)dz + sz) * 16.0f);
             const int x0 = __reduce_min_sync(0xFFFFFFFFu, in ? rx : 0x7FFFFFFF), x1 = __reduce_max_sync(0xFFFFFFFFu, in ? rx : -0x7FFFFFFF);
             const int z0 = __reduce_min_sync(0xFFFFFFFFu, in ? rz : 0x7FFFFFFF), z1 = __reduce_max_sync(0xFFFFFFFFu, in ? rz : -0x7FFFFFFF);
             if (lane == 0 && x0 <= x1) {
@@ -233,7 +312,7 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const MgWorldDesc *__restrict
                 sm.build.units = units;
             }
         } else if (warp == 1) {
-            ot_next(sm.cur[c ^ 1], reqs, nreq, ntiles, counter);
+            ot_next(sm.cur[c ^ 1], K, tile);
         }
         __syncthreads();
         const bool over = sm.over != 0;
@@ -276,15 +355,34 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const MgWorldDesc *__restrict
 #pragma unroll
                     for (int k = 0; k < MG_OW_NOISES - 1; k++) v[k] = n == k ? acc : v[k];
                 }
-                climate_finish_f(W, W.spline, v[0], v[1], v[2], v[3], v[4], R.qy * 4, tg);
+                climate_finish_f(W, W.spline, v[0], v[1], v[2], v[3], v[4],
+                                 (MODE == OT_CHUNK || MODE == OT_BLOCK ? ot_clamp_y(W, qy0 + dy) : qy0) * 4, tg);
             } else {
-                ot_cell_f(W, sm.lat, qx0 + col, R.qy, qz0 + row, tg);
+                ot_cell_f(W, sm.lat, qx0 + dx, MODE == OT_CHUNK || MODE == OT_BLOCK ? ot_clamp_y(W, qy0 + dy) : qy0, qz0 + dz, tg);
             }
         }
-        const MgTreeNode *tree = trees[R.world];
-        const int leaf = tree_search_warp(tree, W, tg, in, sm.hint[t]);
-        if (in) sm.hint[t] = ot_hint(W, leaf);
-        if (in) put_id(out + R.out_off + (int64_t)(qz0 + row - R.qz0) * R.nx + (qx0 + col - R.qx0), tree[leaf].biome);
+        const MgTreeNode *tree = K.trees ? K.trees[R.world] : K.tree;
+        uint64_t d = 0;
+        bool tied = false;
+        int leaf;
+        if (MODE == OT_ENGINE) leaf = tree_search_warp(tree, W, tg, in, sm.hint[t]);
+        else leaf = tree_search_tie_warp(tree, W, tg, in, d, tied, sm.hint[t]);
+        if (in) {
+            sm.hint[t] = ot_hint(W, leaf);
+            const int cell = (tile / tw * OT_W + row) * R.nx + tile % tw * OT_W + col;
+            const int64_t o = R.out_off + cell;
+            if (MODE == OT_CHAIN) {
+                ChainRec &q = K.rec[o];
+                for (int k = 0; k < 6; k++) q.tg[k] = tg[k];
+                q.d = d;
+                q.leaf = leaf;
+                q.tie = tied;
+            }
+            /* a tied cell's candidate chain is left to the launch that follows */
+            if ((MODE == OT_CHUNK || MODE == OT_BLOCK) && tied)
+                ot_leave_open<true, MODE>(K, W, sm.lat, tree, sm.cur[c].req, cell, qx0 + dx, qy0 + dy, qz0 + dz, o);
+            else put_id(K.out + o, tree[leaf].biome);
+        }
         __syncthreads(); /* the tables are free for the next tile */
     }
 }
@@ -301,7 +399,7 @@ struct OtSmemD {
     MgLattice lat[MG_MAX_TABLES];
     int4 ep[OT_CAP_D];
     int2 eq[OT_CAP_D];
-    OtShiftD sh[2 * OT_MAXLEV][4 * OT_W];
+    OtShiftD sh[2 * OT_MAXLEV][4 * OT_TABW];
     OtOctD oct[MG_MAX_TABLES];
     int64_t oct_o[MG_MAX_TABLES][2]; /* the climate octaves' offsets in units of 2^-32 */
     int2 oct_b[MG_MAX_TABLES];       /* their first cells */
@@ -311,47 +409,39 @@ struct OtSmemD {
     int state, over;
     OtTile cur[2]; /* this tile and the next */
     uint16_t hint[OT_NT];
-    int32_t depth; /* depth gradient and offset constant at the request's y, units of 2^-28 */
+    int32_t depth[2]; /* depth gradient and offset constant at quart y0 and y0 + 1, units of 2^-28 */
 };
-
-/* a cell left open: recorded for the later launch, or evaluated here when the record is full */
-static __device__ __noinline__ int ot_open_d(const MgWorldDesc &W, const MgLattice *T, const MgTreeNode *tree, int qx, int qy, int qz) {
-    int32_t tg[6];
-    climate_ow<false>(W, W.spline, T, qx, qy, qz, tg);
-    uint64_t d;
-    return tree[tree_search_scattered(tree, tg, -1, d)].biome;
-}
 
 /* Double branch (26.1, 26.2).  The per-cell form was bound by the FP64 pipe (12 exact shift octaves, 348 operations of 446 a
  * cell at two lanes per SM and clock) beside 40 octaves of 64 x 64-bit products; here nothing per cell uses FP64 and an octave
  * is 11 32 x 32-bit products.  Bound by instruction issue and the wide multiplies.  The uneven batch's 151.6 M double-branch
  * cells: 222.5 ms in the per-cell form, 79.2 ms here (k_ow_open 0.6 ms of it). */
-__global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict__ worlds, const MgTreeNode *const *__restrict__ trees,
-                                                   const MgBatchReq *__restrict__ reqs, int nreq, long long ntiles,
-                                                   const MgLattice *__restrict__ pool, unsigned long long *__restrict__ counter,
-                                                   MgOpenCell *__restrict__ open, unsigned long long *__restrict__ nopen,
-                                                   long long open_cap, uint8_t *__restrict__ out) {
+template <int MODE>
+__global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const __grid_constant__ OtWork K) {
     extern __shared__ uint4 smem_raw[];
     OtSmemD &sm = *reinterpret_cast<OtSmemD *>(smem_raw);
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int col = ot_col(), row = ot_row();
     if (t == 0) sm.state = -1;
     sm.hint[t] = 0;
-    if (warp == 0) ot_next(sm.cur[0], reqs, nreq, ntiles, counter);
+    if (warp == 0) ot_next(sm.cur[0], K, -1);
     __syncthreads();
     for (int c = 0;; c ^= 1) {
         if (sm.cur[c].req < 0) return;
         const int tile = sm.cur[c].tile;
         const MgBatchReq &R = sm.cur[c].r;
-        const MgWorldDesc &W = worlds[R.world];
+        const MgWorldDesc &W = K.worlds[R.world];
         const MgNoise &O = W.noise[0];
         const int nlev = O.nlev, nsh = 2 * nlev, nclim = W.ntables - nsh;
         const int tw = (R.nx + OT_W - 1) / OT_W;
         const int tx0 = (tile % tw) * OT_W, tz0 = (tile / tw) * OT_W;
-        const int qx0 = R.qx0 + tx0, qz0 = R.qz0 + tz0;
+        /* first quart cell of the tile (of a block map: the lowest the zoom can give) */
+        const int qx0 = MODE == OT_BLOCK ? (K.x0 + tx0 * K.step - 2) >> 2 : R.qx0 + tx0;
+        const int qz0 = MODE == OT_BLOCK ? (K.z0 + tz0 * K.step - 2) >> 2 : R.qz0 + tz0;
+        const int qy0 = MODE == OT_BLOCK ? (K.y - 2) >> 2 : R.qy;
         const bool far = qx0 <= -OT_COORD_LIM || qz0 <= -OT_COORD_LIM || qx0 >= OT_COORD_LIM || qz0 >= OT_COORD_LIM;
         if (R.state != sm.state) { /* the request's lattices, octave constants and shift table layout */
-            const uint4 *a = reinterpret_cast<const uint4 *>(pool + R.state);
+            const uint4 *a = reinterpret_cast<const uint4 *>(K.pool + R.state);
             uint4 *b = reinterpret_cast<uint4 *>(sm.lat);
             for (int i = t; i < W.ntables * (int)(sizeof(MgLattice) / 16); i += OT_NT) b[i] = a[i];
             __syncthreads();
@@ -391,8 +481,8 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict
             __syncthreads();
         }
         /* ---- 1: the shift noises' splits per column and row, and their edges */
-        for (int e = far ? nsh * 4 * OT_W : t; e < nsh * 4 * OT_W; e += OT_NT) {
-            const int j = e / (4 * OT_W), q = e % (4 * OT_W), fam = q / OT_W, idx = q % OT_W;
+        for (int e = far ? nsh * 4 * OT_TABW : t; e < nsh * 4 * OT_TABW; e += OT_NT) {
+            const int j = e / (4 * OT_TABW), q = e % (4 * OT_TABW), fam = q / OT_TABW, idx = q % OT_TABW;
             const MgLattice &L = sm.lat[j];
             const double f = O.freq[j % nlev];
             const double off = fam == 0 || fam == 3 ? L.ox : (fam == 1 ? L.oy : L.oz);
@@ -431,12 +521,18 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict
             sm.lo[0] = sm.lo[1] = 0x7FFFFFFF;
             sm.hi[0] = sm.hi[1] = -0x7FFFFFFF;
             sm.over = far;
-        } else if (t == OT_NT - 1) {
-            sm.depth = (int32_t)__double2ll_rn((depth_grad_d(W, R.qy * 4) + W.off_d) * 0x1.0p28);
+        } else if (t >= OT_NT - 2) { /* a block map's cells lie at two heights */
+            const int i = OT_NT - 1 - t, qy = MODE == OT_CHUNK || MODE == OT_BLOCK ? ot_clamp_y(W, qy0 + i) : qy0;
+            sm.depth[i] = (int32_t)__double2ll_rn((depth_grad_d(W, qy * 4) + W.off_d) * 0x1.0p28);
         }
         __syncthreads();
         /* ---- 2: the shift noises and the shifted coordinates of the cell (units of 2^-32) */
         const bool in = tx0 + col < R.nx && tz0 + row < R.nz;
+        int dx = col, dz = row, dy = 0; /* the cell, from the tile's first */
+        if (MODE == OT_BLOCK) {
+            if (in) ot_cell<MODE>(K, tx0 + col, tz0 + row, qx0, qz0, qy0, dx, dz, dy);
+            else dx = dz = 0;
+        }
         int64_t x = 0, z = 0;
         if (!far) {
             int64_t sa = 0, sb = 0; /* units of 2^-59 */
@@ -446,8 +542,8 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict
 #pragma unroll
                 for (int st = 0; st < 2; st++) {
                     const int j = st * nlev + k;
-                    const OtShiftD ax = sm.sh[j][col], by = sm.sh[j][OT_W + col], az = sm.sh[j][2 * OT_W + row],
-                                   bx = sm.sh[j][3 * OT_W + row];
+                    const OtShiftD ax = sm.sh[j][dx], by = sm.sh[j][OT_TABW + dx], az = sm.sh[j][2 * OT_TABW + dz],
+                                   bx = sm.sh[j][3 * OT_TABW + dz];
                     va += ot_octave_d(sm.ep, sm.eq, ax.edge + az.edge, sm.sbuild.nx[2 * j], ax.f, ax.u, az.f, az.u);
                     vb += ot_octave_d(sm.ep, sm.eq, bx.edge + by.edge, sm.sbuild.nx[2 * j + 1], bx.f, bx.u, by.f, by.u);
                 }
@@ -455,9 +551,9 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict
                 sa = ot_madw((int32_t)(va >> 31), c, sa);
                 sb = ot_madw((int32_t)(vb >> 31), c, sb);
             }
-            x = ((int64_t)(qx0 + col) << 32) + (sa >> 25); /* the noise times 4 */
-            z = ((int64_t)(qz0 + row) << 32) + (sb >> 25);
-            const int rx = col * 16 + (int)(sa >> 53), rz = row * 16 + (int)(sb >> 53);
+            x = ((int64_t)(qx0 + dx) << 32) + (sa >> 25); /* the noise times 4 */
+            z = ((int64_t)(qz0 + dz) << 32) + (sb >> 25);
+            const int rx = dx * 16 + (int)(sa >> 53), rz = dz * 16 + (int)(sb >> 53);
             const int x0 = __reduce_min_sync(0xFFFFFFFFu, in ? rx : 0x7FFFFFFF), x1 = __reduce_max_sync(0xFFFFFFFFu, in ? rx : -0x7FFFFFFF);
             const int z0 = __reduce_min_sync(0xFFFFFFFFu, in ? rz : 0x7FFFFFFF), z1 = __reduce_max_sync(0xFFFFFFFFu, in ? rz : -0x7FFFFFFF);
             if (lane == 0 && x0 <= x1) {
@@ -514,7 +610,7 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict
                 sm.build.units = units;
             }
         } else if (warp == 1) {
-            ot_next(sm.cur[c ^ 1], reqs, nreq, ntiles, counter);
+            ot_next(sm.cur[c ^ 1], K, tile);
         }
         __syncthreads();
         const bool over = sm.over != 0;
@@ -587,7 +683,7 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict
             si.df = fabsf(c2) * (float)(ew + 2) + fabsf(si.f) * 1.9e-7f;
             float es;
             const float sp = spline_err<OT_SPL_DEPTH>(W.spline, W.spline.root, si, es);
-            ot_target(sm.depth + __float2int_rn(sp * 0x1.0p28f), (int32_t)(es * (1.01f * 0x1.0p28f)) + 3, s28, ta[4], tb[4]);
+            ot_target(sm.depth[MODE == OT_BLOCK ? dy : 0] + __float2int_rn(sp * 0x1.0p28f), (int32_t)(es * (1.01f * 0x1.0p28f)) + 3, s28, ta[4], tb[4]);
             ok = es < 1.0f;
         }
         /* at most one target open, between two neighbouring values: both are looked up, and the cell is settled when they
@@ -599,50 +695,111 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const MgWorldDesc *__restrict
             ok &= (unsigned)(tb[k] - ta[k]) <= 1u;
         }
         ok &= amb <= 1;
-        const MgTreeNode *tree = trees[R.world];
-        int biome = -1;
+        const MgTreeNode *tree = K.trees ? K.trees[R.world] : K.tree;
+        const int cell = (tile / tw * OT_W + row) * R.nx + tile % tw * OT_W + col;
+        const int64_t o = R.out_off + cell;
+        int biome = -1; /* (OT_CHAIN: the leaf) */
 #pragma unroll 1
-        for (int pass = 0; pass < 2; pass++) { /* the lower targets, then the upper ones of the cells that have two */
+        for (int pass = 0; pass < 2; pass++) { /* the lower targets, then the upper ones of cells with two */
             const bool act = ok && (pass == 0 || amb);
             if (pass && !__any_sync(0xFFFFFFFFu, act)) break;
             int32_t t6[6];
 #pragma unroll
             for (int k = 0; k < 6; k++) t6[k] = pass ? tb[k] : ta[k];
-            const int leaf = tree_search_warp(tree, W, t6, act, sm.hint[t]);
+            uint64_t d = 0;
+            bool tied = false;
+            int leaf;
+            bool sure = pass == 0 && amb;
+            if (MODE == OT_ENGINE) leaf = tree_search_warp<true>(tree, W, t6, act, sm.hint[t], &sure);
+            else leaf = tree_search_tie_warp<true>(tree, W, t6, act, d, tied, sm.hint[t], &sure);
+            if (sure) amb = 0; /* the upper target's leaf is the same */
             if (act) {
                 sm.hint[t] = ot_hint(W, leaf);
-                const int b = tree[leaf].biome;
+                if (MODE == OT_CHAIN) {
+                    ChainRec &q = K.rec[o];
+                    for (int k = 0; k < 6; k++) q.tg[k] = t6[k];
+                    q.d = d;
+                    q.leaf = leaf;
+                    q.tie = tied;
+                }
+                const int b = MODE == OT_CHAIN ? leaf : tree[leaf].biome;
                 ok = pass == 0 || b == biome;
+                /* a tied cell's chain needs the target (OT_CHAIN: a record's target is read only for tied cells) */
+                if (MODE == OT_CHUNK || MODE == OT_BLOCK) ok &= !tied;
+                if (MODE == OT_CHAIN) ok &= !(tied && amb);
                 biome = b;
             }
         }
         if (in) {
-            const int ix = qx0 + col - R.qx0, iz = qz0 + row - R.qz0;
-            const int64_t o = R.out_off + (int64_t)iz * R.nx + ix;
-            if (ok) {
-                put_id(out + o, biome);
-            } else {
-                const unsigned long long k = atomicAdd(nopen, 1ULL);
-                if (k < (unsigned long long)open_cap) open[k] = MgOpenCell{sm.cur[c].req, iz * R.nx + ix};
-                else put_id(out + o, ot_open_d(W, sm.lat, tree, qx0 + col, R.qy, qz0 + row));
-            }
+            if (ok) put_id(K.out + o, MODE == OT_CHAIN ? tree[biome].biome : biome);
+            else ot_leave_open<false, MODE>(K, W, sm.lat, tree, sm.cur[c].req, cell, qx0 + dx, qy0 + dy, qz0 + dz, o);
         }
         __syncthreads(); /* the tables are free for the next tile */
     }
 }
 
-/* the open cells, one per thread: the exact evaluation from the seed's lattices in the pool */
-__global__ void __launch_bounds__(128) k_ow_open(const MgWorldDesc *__restrict__ worlds, const MgTreeNode *const *__restrict__ trees,
-                                                 const MgBatchReq *__restrict__ reqs, const MgLattice *__restrict__ pool,
-                                                 const MgOpenCell *__restrict__ open, const unsigned long long *__restrict__ nopen,
-                                                 long long cap, uint8_t *__restrict__ out) {
-    const long long n = min((long long)*nopen, cap);
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const MgOpenCell c = open[i];
-        const MgBatchReq R = reqs[c.req];
-        const MgWorldDesc &W = worlds[R.world];
+/* the open cells: up to 65,536 by a warp each (25 us for the first, then its throughput), more by a thread each (200 us for any
+ * number).  One grid's lattices and spline are copied to shared memory by each block; a batch's are read through L1.  24 warps
+ * per SM: a cell by a warp is a chain of latencies, so its rate is the warps in flight.  Under the chunk-cell rule a block takes
+ * each cell: its tied chain's cells at once (wc_block_chunk). */
+#define OT_OPEN_NT 128
+#define OT_OPEN_SMEM sizeof(WcStage)
+template <bool FM, int MODE>
+__global__ void __launch_bounds__(OT_OPEN_NT, 6) k_ow_open(const __grid_constant__ OtWork K) {
+    extern __shared__ uint4 smem_raw[];
+    const long long n = min((long long)*K.nopen, K.open_cap);
+    const bool by_warp = n <= 65536 || MODE == OT_CHUNK || MODE == OT_BLOCK;
+    const int lane = threadIdx.x & 31;
+    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x, threads = (long long)gridDim.x * blockDim.x;
+    if (!by_warp) {
+        for (long long i = id; i < n; i += threads) {
+            const MgOpenCell c = K.open[i];
+            const MgBatchReq R = K.reqs ? K.reqs[c.req] : K.one;
+            const int iz = c.cell / R.nx, ix = c.cell - iz * R.nx;
+            ot_exact<FM, MODE>(K, K.worlds[R.world], K.pool + R.state, K.trees ? K.trees[R.world] : K.tree, R.qx0 + ix, R.qy, R.qz0 + iz,
+                               R.out_off + c.cell);
+        }
+        return;
+    }
+    if ((long long)blockIdx.x * (MODE == OT_CHUNK || MODE == OT_BLOCK ? 1 : OT_OPEN_NT / 32) >= n) return;
+    WcStage &s = *reinterpret_cast<WcStage *>(smem_raw);
+    if (!K.reqs) {
+        wc_stage(s, K.worlds[0], K.pool, threadIdx.x, OT_OPEN_NT);
+        __syncthreads();
+    }
+    __shared__ WcStep steps[MODE == OT_CHUNK || MODE == OT_BLOCK ? WC_STEPS : 1];
+    constexpr bool chains = MODE == OT_CHUNK || MODE == OT_BLOCK; /* a block per cell, else a warp */
+    for (long long i = chains ? (long long)blockIdx.x : id >> 5; i < n; i += chains ? (long long)gridDim.x : threads >> 5) {
+        const MgOpenCell c = K.open[i];
+        const MgBatchReq R = K.reqs ? K.reqs[c.req] : K.one;
+        const MgWorldDesc &W = K.worlds[R.world];
+        const MgTreeNode *tree = K.trees ? K.trees[R.world] : K.tree;
+        const MgLattice *T = K.reqs ? K.pool + R.state : s.lat;
+        const MgSpline &S = K.reqs ? W.spline : s.spline;
         const int iz = c.cell / R.nx, ix = c.cell - iz * R.nx;
-        put_id(out + R.out_off + c.cell, ot_open_d(W, pool + R.state, trees[R.world], R.qx0 + ix, R.qy, R.qz0 + iz));
+        int qx = R.qx0 + ix, qy = R.qy, qz = R.qz0 + iz;
+        const long long o = R.out_off + c.cell;
+        if (MODE == OT_BLOCK) wc_zoom(K.zseed, K.x0 + ix * K.step, K.y, K.z0 + iz * K.step, qx, qy, qz);
+        if (chains) {
+            const int b = wc_block_chunk<FM, MG_OVERWORLD, OT_OPEN_NT / 32>(W, S, T, tree, qx, qy, qz, steps);
+            if (threadIdx.x == 0) put_id(K.out + o, b);
+            __syncthreads();
+            continue;
+        }
+        int32_t tg[6];
+        wc_target<FM, MG_OVERWORLD>(W, S, T, qx, qy, qz, tg);
+        uint64_t d;
+        bool tied;
+        const int leaf = wc_search(tree, W, tg, d, tied);
+        if (lane) continue;
+        if (MODE == OT_CHAIN) {
+            ChainRec &r = K.rec[o];
+            for (int k = 0; k < 6; k++) r.tg[k] = tg[k];
+            r.d = d;
+            r.leaf = leaf;
+            r.tie = tied;
+        }
+        put_id(K.out + o, tree[leaf].biome);
     }
 }
 
@@ -671,46 +828,151 @@ bool ow_tile_supported(const MgWorldDesc &W) {
 }
 long long ow_tiles(int nx, int nz) { return (long long)((nx + OT_W - 1) / OT_W) * ((nz + OT_W - 1) / OT_W); }
 
-static int g_ow_resident[2] = {0, 0}; /* CTAs per SM x SMs of the double and the float kernel (ow_prepare; callers hold the
-                                       * ABI lock) */
-template <typename K>
-static int prepare_k(K kernel, size_t smem, int sms, int *resident) {
-    int rc = (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    int n = 0;
-    if (!rc) rc = (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, OT_NT, smem);
-    *resident = (n > 0 ? n : 1) * sms;
+static int g_ow_resident[2][4]; /* CTAs per SM x SMs by branch and mode (ow_prepare; callers hold the ABI lock) */
+template <int MODE>
+static int prepare_mode(int sms) {
+    int rc = (int)cudaFuncSetAttribute(k_ow_d<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(OtSmemD)), n = 0;
+    if (!rc) rc = (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_ow_d<MODE>, OT_NT, sizeof(OtSmemD));
+    g_ow_resident[0][MODE] = (n > 0 ? n : 1) * sms;
+    if (!rc) rc = (int)cudaFuncSetAttribute(k_ow_f<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(OtSmemF));
+    if (!rc) rc = (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_ow_f<MODE>, OT_NT, sizeof(OtSmemF));
+    g_ow_resident[1][MODE] = (n > 0 ? n : 1) * sms;
     return rc;
 }
-int ow_prepare(int sms) {
-    int rc = prepare_k(k_ow_d, sizeof(OtSmemD), sms, &g_ow_resident[0]);
-    return rc ? rc : prepare_k(k_ow_f, sizeof(OtSmemF), sms, &g_ow_resident[1]);
+int ow_prepare() {
+    static int prepared_dev = -1; /* the attributes are per device and set once */
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    if (prepared_dev == dev) return 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int rc = prepare_mode<OT_ENGINE>(sms);
+    if (!rc) rc = prepare_mode<OT_CHUNK>(sms);
+    if (!rc) rc = prepare_mode<OT_BLOCK>(sms);
+    if (!rc) rc = prepare_mode<OT_CHAIN>(sms);
+    if (!rc) prepared_dev = dev;
+    return rc;
 }
-long long ow_open_cap(long long cells) { return cells > 0 ? cells / 24 + 4096 : 0; }
+long long ow_open_cap(long long cells) { return cells > 0 ? cells / 32 + 4096 : 0; }
 
-int launch_ow_tiles(bool fm, const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees, const MgBatchReq *d_reqs, int nreq,
-                    long long ntiles, const MgLattice *d_pool, unsigned long long *d_counter, MgOpenCell *d_open,
-                    unsigned long long *d_nopen, long long open_cap, uint8_t *d_out, cudaStream_t st) {
-    if (ntiles <= 0) return 0;
-    const int resident = g_ow_resident[fm];
+template <int MODE>
+static void tiles_t(bool fm, const OtWork &K, int grid, cudaStream_t st) {
+    if (fm) k_ow_f<MODE><<<grid, OT_NT, sizeof(OtSmemF), st>>>(K);
+    else k_ow_d<MODE><<<grid, OT_NT, sizeof(OtSmemD), st>>>(K);
+}
+static int launch_tiles(bool fm, int mode, const OtWork &K, cudaStream_t st) {
+    const int resident = g_ow_resident[fm][mode];
     if (resident <= 0) return (int)cudaErrorInvalidValue;
-    const int grid = (long long)resident < ntiles ? resident : (int)ntiles;
+    const int grid = (long long)resident < K.ntiles ? resident : (int)K.ntiles;
     {
         ProfScope ps_(fm ? K_OW_TILE_F : K_OW_TILE_D, st);
-        if (fm) k_ow_f<<<grid, OT_NT, sizeof(OtSmemF), st>>>(d_worlds, d_trees, d_reqs, nreq, ntiles, d_pool, d_counter, d_out);
-        else k_ow_d<<<grid, OT_NT, sizeof(OtSmemD), st>>>(d_worlds, d_trees, d_reqs, nreq, ntiles, d_pool, d_counter, d_open, d_nopen,
-                                                          d_open ? open_cap : 0, d_out);
+        switch (mode) {
+        case OT_CHUNK: tiles_t<OT_CHUNK>(fm, K, grid, st); break;
+        case OT_BLOCK: tiles_t<OT_BLOCK>(fm, K, grid, st); break;
+        case OT_CHAIN: tiles_t<OT_CHAIN>(fm, K, grid, st); break;
+        default: tiles_t<OT_ENGINE>(fm, K, grid, st); break;
+        }
     }
     count_launch_external();
     return (int)cudaGetLastError();
 }
-int launch_ow_open(const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees, const MgBatchReq *d_reqs, const MgLattice *d_pool,
-                   const MgOpenCell *d_open, const unsigned long long *d_nopen, long long open_cap, uint8_t *d_out, cudaStream_t st) {
+template <int MODE>
+static void open_t(bool fm, const OtWork &K, int grid, cudaStream_t st) {
+    if (fm) k_ow_open<true, MODE><<<grid, OT_OPEN_NT, OT_OPEN_SMEM, st>>>(K);
+    else k_ow_open<false, MODE><<<grid, OT_OPEN_NT, OT_OPEN_SMEM, st>>>(K);
+}
+static int launch_open(bool fm, int mode, const OtWork &K, cudaStream_t st) {
+    if (!K.open || K.open_cap <= 0) return 0;
+    const int grid = 6 * 152;
     {
         ProfScope ps_(K_OW_OPEN, st);
-        k_ow_open<<<4 * 152, 128, 0, st>>>(d_worlds, d_trees, d_reqs, d_pool, d_open, d_nopen, open_cap, d_out);
+        switch (mode) {
+        case OT_CHUNK: open_t<OT_CHUNK>(fm, K, grid, st); break;
+        case OT_BLOCK: open_t<OT_BLOCK>(fm, K, grid, st); break;
+        case OT_CHAIN: if (!fm) k_ow_open<false, OT_CHAIN><<<grid, OT_OPEN_NT, OT_OPEN_SMEM, st>>>(K); break;
+        default: if (!fm) k_ow_open<false, OT_ENGINE><<<grid, OT_OPEN_NT, OT_OPEN_SMEM, st>>>(K); break;
+        }
     }
     count_launch_external();
     return (int)cudaGetLastError();
+}
+
+int launch_ow_batch(bool fm, int tie, bool open_pass, const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees,
+                    const MgBatchReq *d_reqs, int nreq, long long ntiles, const MgLattice *d_pool, unsigned long long *d_counter,
+                    MgOpenCell *d_open, unsigned long long *d_nopen, long long open_cap, uint8_t *d_out, cudaStream_t st) {
+    if (ntiles <= 0) return 0;
+    OtWork K{};
+    K.worlds = d_worlds;
+    K.trees = d_trees;
+    K.reqs = d_reqs;
+    K.nreq = nreq;
+    K.ntiles = ntiles;
+    K.pool = d_pool;
+    K.counter = d_counter;
+    K.open = d_open;
+    K.nopen = d_nopen;
+    K.open_cap = d_open ? open_cap : 0;
+    K.out = d_out;
+    const int mode = tie == MG_TIE_CHUNK_CELL ? OT_CHUNK : OT_ENGINE;
+    return open_pass ? (fm && mode == OT_ENGINE ? 0 : launch_open(fm, mode, K, st)) : launch_tiles(fm, mode, K, st);
+}
+
+/* ---- one grid: scratch for the open cells' record (a counter, then the cells) */
+static long long grid_open_cap(bool fm, int mode, long long cells) {
+    return fm && (mode == OT_ENGINE || mode == OT_CHAIN) ? 0 : ow_open_cap(cells);
+}
+size_t ow_grid_scratch_bytes(const MgWorldDesc &W, bool chunk_rule, long long cells) {
+    const long long cap = grid_open_cap(W.fmode != 0, chunk_rule ? OT_BLOCK : OT_CHAIN, cells);
+    return cap > 0 ? 16 + (size_t)cap * sizeof(MgOpenCell) : 0;
+}
+static int grid_run(const MgWorldDesc &W, int mode, OtWork &K, void *scratch, cudaStream_t st) {
+    const bool fm = W.fmode != 0;
+    const long long cells = (long long)K.one.nx * K.one.nz;
+    K.ntiles = ow_tiles(K.one.nx, K.one.nz);
+    K.open_cap = scratch ? grid_open_cap(fm, mode, cells) : 0;
+    int rc = ow_prepare();
+    if (rc) return rc;
+    if (K.open_cap > 0) {
+        K.nopen = (unsigned long long *)scratch;
+        K.open = (MgOpenCell *)((uint8_t *)scratch + 16);
+        const cudaError_t e = cudaMemsetAsync(K.nopen, 0, sizeof(unsigned long long), st);
+        if (e) return (int)e;
+    }
+    rc = launch_tiles(fm, mode, K, st);
+    return rc ? rc : launch_open(fm, mode, K, st);
+}
+int launch_ow_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const MgLattice *state, int qx0,
+                         int qz0, int nx, int nz, int qy, ChainRec *rec, uint8_t *out, void *scratch, cudaStream_t st) {
+    OtWork K{};
+    K.worlds = d_world;
+    K.tree = tree;
+    K.pool = state;
+    K.out = out;
+    K.rec = rec;
+    K.one.qx0 = qx0;
+    K.one.qz0 = qz0;
+    K.one.nx = nx;
+    K.one.nz = nz;
+    K.one.qy = qy;
+    return grid_run(W, rec ? OT_CHAIN : OT_ENGINE, K, scratch, st);
+}
+bool ow_block_grid_supported(const MgWorldDesc &W, int x0, int z0, int step) {
+    return ow_tile_supported(W) && step <= 4 && x0 >= INT32_MIN + 16 && z0 >= INT32_MIN + 16;
+}
+int launch_ow_block_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const MgLattice *state, int64_t zseed,
+                         int x0, int z0, int nx, int nz, int step, int y, uint8_t *out, void *scratch, cudaStream_t st) {
+    OtWork K{};
+    K.worlds = d_world;
+    K.tree = tree;
+    K.pool = state;
+    K.out = out;
+    K.one.nx = nx;
+    K.one.nz = nz;
+    K.zseed = zseed;
+    K.x0 = x0;
+    K.z0 = z0;
+    K.step = step;
+    K.y = y;
+    return grid_run(W, OT_BLOCK, K, scratch, st);
 }
 
 }  // namespace mg

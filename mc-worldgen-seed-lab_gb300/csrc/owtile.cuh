@@ -21,6 +21,7 @@
 namespace mg {
 
 #define OT_W 16                   /* tile width and height in cells */
+#define OT_TABW 17                /* quart columns a tile's cells may lie in (BiomeManager's zoom of blocks up to 4 apart: one more) */
 #define OT_NT (OT_W * OT_W)       /* threads per CTA */
 #define OT_MAXLEV 3               /* levels of the shift noise (26.x: 3) */
 #define OT_SHIFT_TABS (4 * OT_MAXLEV)
@@ -30,8 +31,16 @@ namespace mg {
 __device__ __forceinline__ int ot_col() { return ((threadIdx.x >> 5) & 1) * 8 + (threadIdx.x & 7); }
 __device__ __forceinline__ int ot_row() { return (threadIdx.x >> 6) * 4 + ((threadIdx.x >> 3) & 3); }
 
-/* nodes per axis that 16 neighbouring quart columns can touch at frequency f (second stack: 1.0181... f) */
-__host__ __device__ inline int ot_shift_nodes(double f) { return (int)((OT_W - 1) * f * 1.02) + 3; }
+/* nodes per axis that OT_TABW neighbouring quart columns can touch at frequency f (second stack: 1.0181... f) */
+__host__ __device__ inline int ot_shift_nodes(double f) { return (int)((OT_TABW - 1) * f * 1.02) + 3; }
+
+/* what a tile's cells are and what is wanted of them */
+enum {
+    OT_ENGINE = 0, /* quart cells; the first leaf in tree order at the minimum */
+    OT_CHUNK = 1,  /* quart cells; the chunk-cell rule (cell_chunk) */
+    OT_BLOCK = 2,  /* blocks `step` <= 4 apart, zoomed to quart cells; the chunk-cell rule */
+    OT_CHAIN = 3   /* quart cells; ENGINE's leaf with its target, distance and tie flag for the candidate chains */
+};
 
 /* s = x f + off as the reference rounds it (f a power of two, |x f| < 2^23: the wrap is the identity), floor i and
  * fraction F in units of 2^-64, from the mantissa of s as a signed 64-bit integer (an arithmetic shift of the negated

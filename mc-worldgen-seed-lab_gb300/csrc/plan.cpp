@@ -41,8 +41,9 @@ struct McGb300Plan {
     long long ow_lattices = 0;
     MgLattice *d_pool = nullptr;
     unsigned long long *d_counter = nullptr; /* BATCH_COUNTERS */
-    MgOpenCell *d_open = nullptr;            /* records of double-branch Overworld cells left to the exact evaluation */
-    long long open_cap = 0;
+    MgOpenCell *d_open = nullptr;            /* records of Overworld cells left to the exact evaluation, double then float branch */
+    long long open_cap[2] = {0, 0};
+    int tie = 0;
     /* graph of one run */
     cudaStream_t cap = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -103,7 +104,7 @@ int enqueue(McGb300Plan *p, uint8_t *d_out, int shape, cudaStream_t st) {
         int rc = mg::launch_setup_list(p->d_worlds, d, p->d_ent[d], p->nent[d], p->d_first, p->ow_lattices, p->d_pool, st);
         if (rc) return rc;
     }
-    return mg::launch_batch(p->d_worlds, p->d_trees, p->d_reqs[shape], p->groups[shape], p->d_pool, p->d_counter,
+    return mg::launch_batch(p->d_worlds, p->d_trees, p->d_reqs[shape], p->groups[shape], p->tie, p->d_pool, p->d_counter,
                             p->d_open, p->open_cap, d_out, p->ctas, shape, st);
 }
 
@@ -213,10 +214,13 @@ MCGEN_API int mcgen_gb300_plan_new(const McGb300Request *reqs, int n, int tie_ru
     for (int i = 0; i < n; i++) order[(size_t)i] = i;
     std::vector<int> wgroup(worlds.size());
     for (size_t w = 0; w < worlds.size(); w++) wgroup[w] = mg::batch_group(worlds[w]->desc, tie_rule);
-    long long dcells = 0; /* cells of the double branch's tile kernel: the ones it may leave open */
-    for (int i = 0; i < n; i++)
-        if (wgroup[(size_t)wof[(size_t)i]] == BATCH_OW_D) dcells += p->cells[(size_t)i];
-    p->open_cap = mg::ow_open_cap(dcells);
+    long long ow_cells[2] = {0, 0}; /* of the Overworld groups: the cells the tile kernels may leave open */
+    for (int i = 0; i < n; i++) {
+        const int g = wgroup[(size_t)wof[(size_t)i]];
+        if (g != BATCH_REST) ow_cells[g] += p->cells[(size_t)i];
+    }
+    p->tie = tie_rule;
+    mg::batch_open_cap(ow_cells, tie_rule, p->open_cap);
     std::vector<int> key((size_t)n); /* group, code path, then world */
     for (int i = 0; i < n; i++) {
         const int wi = wof[(size_t)i];
@@ -269,7 +273,7 @@ MCGEN_API int mcgen_gb300_plan_new(const McGb300Request *reqs, int n, int tie_ru
     const size_t pool_off = (at + 255) & ~(size_t)255;
     const size_t counter_off = pool_off + sizeof(MgLattice) * (size_t)pool;
     const size_t open_off = counter_off + BATCH_COUNTERS * sizeof(unsigned long long);
-    const size_t arena_bytes = open_off + sizeof(MgOpenCell) * (size_t)p->open_cap;
+    const size_t arena_bytes = open_off + sizeof(MgOpenCell) * (size_t)(p->open_cap[0] + p->open_cap[1]);
     cudaMemPool_t mp = nullptr;
     cudaStream_t ast = mg::abi_stream();
     cudaError_t e = plan_pool(&mp);
@@ -281,7 +285,7 @@ MCGEN_API int mcgen_gb300_plan_new(const McGb300Request *reqs, int n, int tie_ru
         for (const Part &q : parts) *q.dst = base + q.off;
         if (pool) p->d_pool = (MgLattice *)(base + pool_off);
         p->d_counter = (unsigned long long *)(base + counter_off);
-        if (p->open_cap) p->d_open = (MgOpenCell *)(base + open_off);
+        if (p->open_cap[0] + p->open_cap[1]) p->d_open = (MgOpenCell *)(base + open_off);
         p->h2d_bytes = (long long)staged;
     }
     if (!e) e = (cudaError_t)mg::batch_prepare(nullptr);

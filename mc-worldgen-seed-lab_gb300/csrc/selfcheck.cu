@@ -304,7 +304,7 @@ __global__ void k_check_tree(const MgTreeNode *__restrict__ T, long long n, uint
 /* The warp-shared search (tree_search_warp) against the 64-bit stack search on targets of the kind a warp of
  * neighbouring cells has: per warp a centre in the tables' range and per lane a spread of 50, 400, 2,000 or
  * 6,000 around it; about one lane in eight inactive; in one warp in sixteen one lane far outside the packed
- * range (the warp's fallback).  Case i is lane i % 32 of warp case i / 32.  out[0]: differing leaves. */
+ * range (the warp's fallback); with what NEAR says of the neighbouring targets, and rt_point.  Case i is lane i % 32 of warp case i / 32.  out[0]: differing leaves. */
 __global__ void __launch_bounds__(128) k_check_tree_warp(const __grid_constant__ MgWorldDesc W, const MgTreeNode *__restrict__ T,
                                                          long long n, uint64_t seed, unsigned long long *out) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -333,6 +333,32 @@ __global__ void __launch_bounds__(128) k_check_tree_warp(const __grid_constant__
             bool tie0;
             const int l0 = tree_search_tie_stack(T, t, d, tie0);
             bad += (T[lw].first != T[l0].first) + (T[lt].first != T[l0].first) + (dt != d) + (tied != tie0);
+        }
+        /* the same with a hint, asking whether the neighbouring targets give the same biome and leaf: half of the lanes ask */
+        bool sure = lane & 1, sure1 = lane & 1, tied1 = false;
+        const int hint = (int)(q % (uint64_t)W.tree_leaves);
+        const int ln = tree_search_warp<true>(T, W, t, active, __shfl_sync(0xFFFFFFFFu, hint, 0), &sure);
+        const int ln1 = tree_search_tie_warp<true>(T, W, t, active, dt, tied1, __shfl_sync(0xFFFFFFFFu, hint, 0), &sure1);
+        if (active) {
+            bad += (T[ln].first != T[lw].first) + (T[ln1].first != T[lw].first) + (tied1 != tied);
+            for (int k = 0; k < 12 && (sure || sure1); k++) {
+                uint64_t d;
+                bool tie0;
+                t[k >> 1] += k & 1 ? 1 : -1;
+                const int l0 = tree_search_tie_stack(T, t, d, tie0);
+                t[k >> 1] -= k & 1 ? 1 : -1;
+                bad += (sure && T[l0].biome != T[ln].biome) + (sure1 && (T[l0].first != T[ln1].first || tie0));
+            }
+        }
+        /* one lane's target by the whole warp (rt_point) */
+        int32_t t1[6];
+        const int src = __ffs((int)__ballot_sync(0xFFFFFFFFu, active)) - 1;
+        if (src < 0) continue;
+        for (int k = 0; k < 6; k++) t1[k] = __shfl_sync(0xFFFFFFFFu, t[k], src);
+        RtTarget q1;
+        if (rt_target(T, t1, q1) && rt_packed(T)) {
+            const RtWarp p = rt_point(T, W, q1, 0xFFFFFFFEu);
+            if (lane == src && p.leaf >= 0) bad += (T[W.leaf_off + p.leaf].first != T[lt].first) + (p.best != dt) + ((p.cnt >= 2) != tied);
         }
     }
     atomicAdd(&out[0], bad);

@@ -288,11 +288,12 @@ int launch_batch(McGb300Server *s, Batch &b) {
         b.cap_hout = e ? 0 : c;
     }
     if (!e && !b.d_counter) e = cudaMalloc(&b.d_counter, BATCH_COUNTERS * sizeof(unsigned long long));
-    long long dcells = 0; /* cells of the double branch's tile kernel: the ones it may leave open */
+    long long ow_cells[2] = {0, 0}, open_cap[2]; /* of the Overworld groups: the cells the tile kernels may leave open */
     for (const auto &r : reqs)
-        if (wgroup[(size_t)r.world] == BATCH_OW_D) dcells += (long long)r.nx * r.nz;
-    const long long open_cap = mg::ow_open_cap(dcells);
-    if (!e && open_cap > 0) e = grow_dev(&b.d_open, &b.cap_open, (size_t)open_cap);
+        if (wgroup[(size_t)r.world] != BATCH_REST) ow_cells[wgroup[(size_t)r.world]] += (long long)r.nx * r.nz;
+    mg::batch_open_cap(ow_cells, MG_TIE_ENGINE, open_cap);
+    const long long nopen = open_cap[0] + open_cap[1];
+    if (!e && nopen > 0) e = grow_dev(&b.d_open, &b.cap_open, (size_t)nopen);
     if (e) return crc(e);
     if (s->fail_next) { /* injected failure of this step (tests of the failure path) */
         const int f = s->fail_next;
@@ -323,8 +324,8 @@ int launch_batch(McGb300Server *s, Batch &b) {
     /* hits on states another in-flight batch is still building: order after that batch's setup */
     for (int k : wait_on)
         if ((e = cudaStreamWaitEvent(st, s->batches[(size_t)k].setup_done, 0))) return crc(e);
-    int rc = mg::launch_batch(b.d_worlds, b.d_trees, b.d_reqs, groups, s->pool[0].base, b.d_counter,
-                              open_cap > 0 ? b.d_open : nullptr, open_cap, b.d_out, 0, kServeShape, st);
+    int rc = mg::launch_batch(b.d_worlds, b.d_trees, b.d_reqs, groups, MG_TIE_ENGINE, s->pool[0].base, b.d_counter,
+                              nopen > 0 ? b.d_open : nullptr, open_cap, b.d_out, 0, kServeShape, st);
     if (rc) return MCGEN_E_INTERNAL;
     if ((e = cudaMemcpyAsync(b.h_out, b.d_out, (size_t)out, cudaMemcpyDeviceToHost, st))) return crc(e);
     if ((e = cudaEventRecord(b.done, st))) return crc(e);

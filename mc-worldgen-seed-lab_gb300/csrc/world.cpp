@@ -598,7 +598,7 @@ static int load_tree(const char *root, int version, int dim, std::vector<MgTreeN
     std::vector<int> src;
     src.push_back(root_id);
     out->push_back(MgTreeNode());
-    bool packed = true; /* every bound within +-MG_TREE_PACKED_BOUND (the root's flag) */
+    bool packed = true; /* every bound within +-MG_TREE_PACKED_BOUND, hi >= lo - 1 (the root's flag) */
     for (size_t h = 0; h < src.size(); h++) {
         const BNode &b = tb.nodes[(size_t)src[h]];
         MgTreeNode &o = (*out)[h];
@@ -614,7 +614,7 @@ static int load_tree(const char *root, int version, int dim, std::vector<MgTreeN
                 o.lo[d] = (int16_t)lo;
                 o.nhi[d] = (int16_t)(-hi);
                 if (lo < -MG_TREE_PACKED_BOUND || lo > MG_TREE_PACKED_BOUND || hi < -MG_TREE_PACKED_BOUND ||
-                    hi > MG_TREE_PACKED_BOUND)
+                    hi > MG_TREE_PACKED_BOUND || hi < lo - 1)
                     packed = false;
             } else {
                 int64_t x = std::max(std::max(-hi, lo), (int64_t)0);

@@ -29,3 +29,52 @@ def test_overworld_tiles(version, preset):
     for r, got in zip(reqs, plan.split(plan.run())):
         exp = ow.quart_grid(*r[1:], O.TIE_ENGINE)
         assert np.array_equal(got, exp), (r[1:], int((got != exp).sum()))
+
+
+GRIDS = [("26.3", "normal"), ("26.3", "amplified"), ("26.1", "amplified"), ("26.2", "normal")]
+
+
+def world_pair(version, preset, seed):
+    mg = ge.package()
+    mg.load()
+    if mg.device_count() < 1:
+        pytest.fail("no CUDA device")
+    return mg, mg.Generator.open(ge.data_root(), version).world("minecraft:overworld", preset, seed), \
+        O.World(ge.data_root(), version, "overworld", preset)
+
+
+@pytest.mark.parametrize("version,preset", GRIDS)
+def test_block_maps_and_points(version, preset):
+    """Block maps: the tile form (steps 1 to 4) and the form for sparser samples, at tile edges, at the origin, the world
+    border, the coordinate beyond which the tables hand over, and heights inside, at the ends of and outside the build range
+    (where the chunk-cell chain is longest); then the same blocks as a list of points."""
+    seed = -2757711463728365141
+    mg, w, ow = world_pair(version, preset, seed)
+    for step in (1, 2, 3, 4, 5, 17):
+        for x, z in [(0, 0), (-23, -9), (29999984, -29999984), (4 * 8388608 - 4 * 4096 - 30, 11), (-2000000000, 2000000000)]:
+            nx, nz = {1: (67, 35), 2: (33, 18), 3: (1, 40), 4: (50, 7)}.get(step, (17, 16))
+            for y in (63, -64, 319, 2000):
+                x0, z0 = x - step * nx // 2, z - step * nz // 2
+                got, exp = w.biome_grid(x0, z0, nx, nz, step, y), ow.biome_grid(seed, x0, z0, nx, nz, step, y)
+                assert np.array_equal(got, exp), (step, x, z, y, int((got != exp).sum()))
+        xyz = np.array([(x0 + step * i, y, z0 + step * j) for y in (-80, 40) for j in range(nz) for i in range(nx)], np.int32)
+        assert np.array_equal(w.biome_points(xyz), ow.block_points(seed, xyz)), step
+
+
+@pytest.mark.parametrize("version,preset", GRIDS)
+def test_quart_grids_and_chunk_plans(version, preset):
+    """Every tie rule's grid form and the chunk-cell plan, one request per world, at the sizes and corners of the batch."""
+    seed = 7415553284403671009
+    mg, w, ow = world_pair(version, preset, seed)
+    shapes = [(1, 1), (17, 33), (250, 40)]
+    for x, z in CORNERS:
+        for nx, nz in shapes:
+            for qy in (16, -17, 90):
+                q = (x - nx // 2, z - nz // 2, nx, nz, qy)
+                for rule in (mg.TIE_ENGINE, mg.TIE_GRID_CHAIN):
+                    assert np.array_equal(w.quart_grid(*q, rule), ow.quart_grid(seed, *q, rule)), (q, rule)
+                assert np.array_equal(w.quart_grid(*q, mg.TIE_CHUNK_ORDER), ow.chunk_order_grid(seed, *q)), q
+    reqs = [(w, seed, x - nx // 2, z - nz // 2, nx, nz, 15) for x, z in CORNERS for nx, nz in shapes]
+    plan = mg.Plan(reqs, tie_rule=mg.TIE_CHUNK_CELL)
+    for r, got in zip(reqs, plan.split(plan.run())):
+        assert np.array_equal(got, ow.chunk_grid(*r[1:])), r[1:]
