@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(LNT) k_setup_list_xo(const MgWorldDesc *__rest
     h.oz = xo_double(x) * 256.0;
     for (int w = 0; w < 64; w++) perm[w][t] = 0x03020100u + 0x04040404u * (uint32_t)w;
     uint8_t *mine = reinterpret_cast<uint8_t *>(&perm[0][t]);
-    for (int q = 0; q < 256; q++) lst_swap(mine, q, q + xo_int(x, 256u - (uint32_t)q));
+    xo_shuffle<LNT>(mine, x);
     lst_store(perm, t, h, pool + E.slot + j, !W.fmode);
 }
 /* Nether entries: one thread per (entry, noise); End entries: one thread per entry. */

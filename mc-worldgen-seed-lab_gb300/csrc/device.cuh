@@ -54,6 +54,53 @@ __device__ __forceinline__ int xo_int(Xo &r, uint32_t bound) {
 }
 __device__ __forceinline__ double xo_double(Xo &r) { return (double)(xo_next(r) >> 11) * 0x1.0p-53; }
 
+/* The 256-step Fisher-Yates shuffle of a lattice by one thread: byte i of its permutation at mine + (i >> 2) * 4 ROW + (i & 3),
+ * identity at the start.  The generator's state is kept in 32-bit halves (of a draw only the low word is used), and the draws
+ * that nextInt might reject (low word of the product below the bound: 3e-8 a draw) are found by the least low word of all
+ * steps, after which the shuffle is done again with the test at each step.  Bound by the integer pipe (79 %): with 64-bit state
+ * and the test's branch at every step it took 36 instructions a step instead of 26 (2^20 seeds' lattices 16.5 -> 14.7 ms).
+ * Moving shifts to multiply-adds did not help (they are at the issue limit then). */
+template <int ROW>
+__device__ __forceinline__ void xo_shuffle(uint8_t *mine, const Xo x) {
+    uint32_t a0 = (uint32_t)x.lo, a1 = (uint32_t)(x.lo >> 32), b0 = (uint32_t)x.hi, b1 = (uint32_t)(x.hi >> 32), least = 0xFFFFFFFFu;
+#pragma unroll 1
+    for (uint32_t qw = 0; qw < 64; qw++) {
+#pragma unroll
+        for (uint32_t r = 0; r < 4; r++) {
+            const uint32_t q = 4 * qw + r;
+            uint32_t s0, s1;
+            asm("{\n\tadd.cc.u32 %0, %2, %4;\n\taddc.u32 %1, %3, %5;\n\t}" : "=r"(s0), "=r"(s1) : "r"(a0), "r"(a1), "r"(b0), "r"(b1));
+            const uint64_t m = (uint64_t)(__funnelshift_l(s1, s0, 17) + a0) * (256u - q);
+            least = min(least, (uint32_t)m);
+            b0 ^= a0;
+            b1 ^= a1;
+            const uint32_t c0 = a1, c1 = a0; /* rotl 49 = halves exchanged, then 17 */
+            a0 = __funnelshift_l(c1, c0, 17) ^ b0 ^ (b0 << 21);
+            a1 = __funnelshift_l(c0, c1, 17) ^ b1 ^ __funnelshift_l(b0, b1, 21);
+            const uint32_t d0 = __funnelshift_l(b1, b0, 28);
+            b1 = __funnelshift_l(b0, b1, 28);
+            b0 = d0;
+            const uint32_t k = q + (uint32_t)(m >> 32);
+            uint8_t *pa = mine + qw * (4 * ROW) + r, *pb = mine + (k + (k >> 2) * (4 * ROW - 4));
+            const uint8_t va = *pa, vb = *pb;
+            *pa = vb;
+            *pb = va;
+        }
+    }
+    if (least >= 256u) return;
+    Xo y = x;
+#pragma unroll 1
+    for (int w = 0; w < 64; w++) *reinterpret_cast<uint32_t *>(mine + w * (4 * ROW)) = 0x03020100u + 0x04040404u * (uint32_t)w;
+#pragma unroll 1
+    for (uint32_t q = 0; q < 256; q++) {
+        const uint32_t k = q + (uint32_t)xo_int(y, 256u - q);
+        uint8_t *pa = mine + (q + (q >> 2) * (4 * ROW - 4)), *pb = mine + (k + (k >> 2) * (4 * ROW - 4));
+        const uint8_t va = *pa, vb = *pb;
+        *pa = vb;
+        *pb = va;
+    }
+}
+
 /* java.util.Random LCG */
 #define MG_LCG_MUL 0x5DEECE66DULL
 #define MG_LCG_MASK 0xFFFFFFFFFFFFULL
@@ -1086,7 +1133,12 @@ struct RtNode {
     uint4 a, b;
     __device__ __forceinline__ RtNode(const MgTreeNode *n)
         : a(*reinterpret_cast<const uint4 *>(n)), b(*(reinterpret_cast<const uint4 *>(n) + 1)) {}
+    /* node i of blocks of 32 nodes, 32 first halves before 32 second halves: a warp reads a block in 8 wavefronts (whole nodes
+     * in a row, 32 bytes apart, took 16) */
+    __device__ __forceinline__ RtNode(const uint4 *blocks, int i)
+        : a(blocks[(i >> 5) * 64 + (i & 31)]), b(blocks[(i >> 5) * 64 + 32 + (i & 31)]) {}
 };
+__device__ __forceinline__ const uint4 *rt_blocks(const MgTreeNode *T, int off) { return reinterpret_cast<const uint4 *>(T + off); }
 /* the nearest leaf (counted from leaf_off), its word and distance, leaves at that distance (capped at 2; not by rt_warp<NEXT>);
  * rt_warp<NEXT>: the least distance of the other leaves met (RT_OTHER), or of those of another biome (RT_BIOME) */
 enum { RT_OTHER = 1, RT_BIOME = 2 };
@@ -1118,17 +1170,20 @@ __device__ __forceinline__ void rt_warp_leaf(const RtNode &n, int at, const RtTa
     rt_warp_leaf_at<TIE, NEXT>(rt_dist(n.a, n.b, q), n.b.w, at, r);
 }
 /* One target's search by the whole warp, a cluster, group or leaf per lane, nearest first; all lanes pass the same q and U (a
- * distance that some leaf does not exceed).  The result is the same in all lanes; leaf -1 when the distance is not exact. */
-__device__ __noinline__ static RtWarp rt_point(const MgTreeNode *__restrict__ T, const MgWorldDesc &W, const RtTarget q, uint32_t U) {
+ * distance that some leaf does not exceed).  The result is the same in all lanes; leaf -1 when the distance is not exact.
+ * MASK: instead of the leaf's word, whether any leaf at the least distance has a biome of m0 | m1 << 64. */
+template <bool MASK = false>
+__device__ __noinline__ static RtWarp rt_point(const MgTreeNode *__restrict__ T, const MgWorldDesc &W, const RtTarget q, uint32_t U,
+                                               uint64_t m0 = 0, uint64_t m1 = 0) {
     const unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
     RtWarp r{0xFFFFFFFFu, 0, -1, 0, 0xFFFFFFFFu};
     const int groups = W.groups, leaves = W.tree_leaves;
-    const MgTreeNode *G = T + W.group_off, *L = T + W.leaf_off;
+    const uint4 *C = rt_blocks(T, W.cluster_off), *G = rt_blocks(T, W.group_off), *L = rt_blocks(T, W.block_off);
     for (int s0 = 0; 32 * s0 < groups; s0 += 32) {
         uint32_t ls = 0xFFFFFFFFu;
         if (32 * (s0 + lane) < groups) {
-            const RtNode n(T + W.cluster_off + s0 + lane);
+            const RtNode n(C, s0 + lane);
             ls = rt_dist(n.a, n.b, q);
         }
         for (;;) {
@@ -1139,7 +1194,7 @@ __device__ __noinline__ static RtWarp rt_point(const MgTreeNode *__restrict__ T,
             const int g0 = 32 * (s0 + s);
             uint32_t lg = 0xFFFFFFFFu;
             if (g0 + lane < groups) {
-                const RtNode n(G + g0 + lane);
+                const RtNode n(G, g0 + lane);
                 lg = rt_dist(n.a, n.b, q);
             }
             for (;;) {
@@ -1150,15 +1205,26 @@ __device__ __noinline__ static RtWarp rt_point(const MgTreeNode *__restrict__ T,
                 const int at = 32 * (g0 + g) + lane;
                 uint32_t d = 0xFFFFFFFFu;
                 if (at < leaves) {
-                    const RtNode n(L + at);
+                    const RtNode n(L, at);
                     d = rt_dist(n.a, n.b, q);
-                    rt_warp_leaf_at<true>(d, n.b.w, at, r);
+                    if (MASK) {
+                        const uint32_t b = n.b.w >> 24, in = (uint32_t)((b & 64 ? m1 : m0) >> (b & 63)) & 1u;
+                        r.word = d < r.best ? in : (d == r.best ? r.word | in : r.word);
+                        r.leaf = d < r.best ? at : r.leaf;
+                        r.best = min(r.best, d);
+                    } else {
+                        rt_warp_leaf_at<true>(d, n.b.w, at, r);
+                    }
                 }
                 U = min(U, __reduce_min_sync(FULL, d));
             }
         }
     }
     const bool at = r.best == U && r.leaf >= 0;
+    if (MASK) {
+        const int found = __any_sync(FULL, at) && U < (uint32_t)MG_RT_CLAMP * MG_RT_CLAMP ? 0 : -1;
+        return RtWarp{U, __any_sync(FULL, at && r.word) ? 1u : 0u, found, 0, 0};
+    }
     const unsigned rank = at ? r.word & 0xFFFFu : 0xFFFFFFFFu, first = __reduce_min_sync(FULL, rank);
     const unsigned who = __ballot_sync(FULL, at && rank == first);
     const bool exact = who && U < (uint32_t)MG_RT_CLAMP * MG_RT_CLAMP;
@@ -1168,13 +1234,13 @@ __device__ __noinline__ static RtWarp rt_point(const MgTreeNode *__restrict__ T,
 }
 /* leaves [32 g, 32 g + 32) of the clustered ones, the last group's fewer; ub: bound U by the group's own upper bounds first */
 template <bool TIE, int NEXT>
-__device__ __forceinline__ void rt_warp_group(const MgTreeNode *__restrict__ L, const MgTreeNode *__restrict__ box, int leaves, int g, bool ub, const RtTarget &q,
-                                              const RtTarget &lbq, const RtTarget &ubq, bool active, bool near, uint32_t bound, uint32_t &U, RtWarp &r) {
+__device__ __forceinline__ void rt_warp_group(const uint4 *__restrict__ L, const uint4 *__restrict__ G, int leaves, int g, bool ub,
+                                              const RtTarget &q, const RtTarget &lbq, const RtTarget &ubq, bool active, bool near,
+                                              uint32_t bound, uint32_t &U, RtWarp &r) {
     const unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31, first = 32 * g;
-    const MgTreeNode *G = L + first;
     const bool in = first + lane < leaves;
-    const RtNode n(G + (in ? lane : 0));
+    const RtNode n(L, first + lane);
     const uint32_t lb = rt_dist(n.a, n.b, lbq);
     auto within = [&](uint32_t d) { return NEXT && near ? rt_beyond(d) : d; };
     if (ub) U = min(U, within(__reduce_min_sync(FULL, rt_ub_or_inf(n.a, n.b, ubq))));
@@ -1182,7 +1248,7 @@ __device__ __forceinline__ void rt_warp_group(const MgTreeNode *__restrict__ L, 
     if (!m) return;
     if (m & (m - 1)) { /* does any lane need it?  Where terrain breaks (amplified heights) the targets' box meets up to 95 groups
                         * and 870 leaves of which each lane needs 5 groups: 310 -> 170 us for 256 x 256 such cells */
-        const RtNode b(box);
+        const RtNode b(G, g);
         const uint32_t own = min(r.best, bound);
         if (!__any_sync(FULL, active && rt_dist(b.a, b.b, q) <= within(own))) return;
     }
@@ -1191,7 +1257,7 @@ __device__ __forceinline__ void rt_warp_group(const MgTreeNode *__restrict__ L, 
         m &= m - 1;
         const int j = m ? __ffs((int)m) - 1 : -1;
         m &= m - 1;
-        const RtNode n0(G + i), n1(G + max(j, 0));
+        const RtNode n0(L, first + i), n1(L, first + max(j, 0));
         rt_warp_leaf<TIE, NEXT>(n0, first + i, q, r);
         if (j >= 0) rt_warp_leaf<TIE, NEXT>(n1, first + j, q, r);
     }
@@ -1228,11 +1294,11 @@ __device__ __forceinline__ bool rt_warp(const MgTreeNode *__restrict__ T, const 
     }
     if (none) return true; /* no active lane */
     const int groups = W.groups, leaves = W.tree_leaves;
-    const MgTreeNode *G = T + W.group_off, *L = T + W.leaf_off;
+    const uint4 *C = rt_blocks(T, W.cluster_off), *G = rt_blocks(T, W.group_off), *L = rt_blocks(T, W.block_off);
     uint32_t U = 0xFFFFFFFEu, bound = 0xFFFFFFFFu;
     if (hint >= 0) {
         /* the hinted leaf's distance bounds the lane's; the leaf itself is met again on the way */
-        const RtNode n(L + hint);
+        const RtNode n(T + W.leaf_off + hint);
         bound = rt_dist(n.a, n.b, q);
         const uint32_t u = min(__reduce_max_sync(FULL, active ? bound : 0u), __reduce_min_sync(FULL, active ? rt_ub_or_inf(n.a, n.b, ubq) : 0xFFFFFFFFu));
         U = min(U, NEXT && near ? rt_beyond(u) : u);
@@ -1241,7 +1307,7 @@ __device__ __forceinline__ bool rt_warp(const MgTreeNode *__restrict__ T, const 
         const int ns = min((groups + 31) / 32 - s0, 32);
         uint32_t ls = 0xFFFFFFFFu;
         if (lane < ns) {
-            const RtNode n(T + W.cluster_off + s0 + lane);
+            const RtNode n(C, s0 + lane);
             ls = rt_dist(n.a, n.b, lbq);
         }
         /* the nearest cluster first, and in it the nearest group */
@@ -1254,14 +1320,14 @@ __device__ __forceinline__ bool rt_warp(const MgTreeNode *__restrict__ T, const 
             const int g0 = 32 * (s0 + s), ng = min(groups - g0, 32);
             uint32_t l = 0xFFFFFFFFu;
             if (lane < ng) {
-                const RtNode n(G + g0 + lane);
+                const RtNode n(G, g0 + lane);
                 l = rt_dist(n.a, n.b, lbq);
             }
             unsigned p = __ballot_sync(FULL, l <= U);
             int j = first ? __ffs((int)__ballot_sync(FULL, l == __reduce_min_sync(FULL, l))) - 1 : __ffs((int)p) - 1;
             while (p) {
                 p &= ~(1u << j);
-                rt_warp_group<TIE, NEXT>(L, G + g0 + j, leaves, g0 + j, first || hint < 0, q, lbq, ubq, active, near, bound, U, r);
+                rt_warp_group<TIE, NEXT>(L, G, leaves, g0 + j, first || hint < 0, q, lbq, ubq, active, near, bound, U, r);
                 first = false;
                 p &= __ballot_sync(FULL, l <= U);
                 j = __ffs((int)p) - 1;
@@ -1271,6 +1337,29 @@ __device__ __forceinline__ bool rt_warp(const MgTreeNode *__restrict__ T, const 
         }
     }
     return true;
+}
+/* tree_search (no candidate) for 32 unrelated targets, called by all 32 lanes (inactive ones get -1): one after another, each
+ * by the whole warp.  A lane alone visits 120 to 200 nodes, and lanes with unrelated targets diverge at most of them (2,000
+ * instructions per target); the warp looks at 32 boxes at once (10 steps of 40). */
+__device__ __forceinline__ int tree_search_lanes(const MgTreeNode *__restrict__ T, const MgWorldDesc &W, const int32_t *t, bool active) {
+    const unsigned FULL = 0xFFFFFFFFu;
+    RtTarget q{};
+    const bool ok = active && rt_packed(T) && rt_target(T, t, q);
+    int leaf = -1;
+    for (unsigned m = __ballot_sync(FULL, ok); m; m &= m - 1) {
+        const int src = __ffs((int)m) - 1;
+        RtTarget s;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            s.p[k] = __shfl_sync(FULL, q.p[k], src);
+            s.n[k] = __shfl_sync(FULL, q.n[k], src);
+        }
+        const RtWarp r = rt_point(T, W, s, 0xFFFFFFFEu);
+        if ((int)(threadIdx.x & 31) == src) leaf = r.leaf;
+    }
+    if (!active) return -1;
+    uint64_t d;
+    return leaf >= 0 ? W.leaf_off + leaf : tree_search_stack(T, t, -1, d);
 }
 /* tree_search (no candidate) for the 32 neighbouring cells of a warp, called by all 32 lanes; inactive lanes get -1.
  * NEAR: in the lanes that ask for it (sure), sure = every target one unit away in one dimension has this biome too. */

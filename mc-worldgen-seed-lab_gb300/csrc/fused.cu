@@ -7,7 +7,8 @@
  * to shared memory, and one thread per (seed, point) sums them in the reference's order
  * (engine/mc_noise.h:285-324), forms the shifted coordinates after the ShiftA/ShiftB pass
  * (engine/mc_climate.h:113-164) and writes the five noise values.  k_ow_finish_tree then finishes the
- * climate and searches the R-tree (ENGINE rule) with one thread per sample, at full occupancy: inside the
+ * climate with one thread per sample and searches the R-tree (ENGINE rule) for a warp's 32 samples one after another, 32
+ * boxes at a time (tree_search_lanes: 957 -> 470 us for 65,536 seeds x 8 points), at full occupancy: inside the
  * fused kernel that serial per-point work would leave most of a CTA idle at its barriers.
  *
  * Phases per chunk of NPC points:  B  offset lattices: ShiftA and ShiftB octaves
@@ -111,18 +112,7 @@ __global__ void __launch_bounds__(FNT) k_ow_seed_climate(const __grid_constant__
         oz = xo_double(x) * 256.0;
         for (int w = 0; w < 64; w++) sm.perm[w][t] = 0x03020100u + 0x04040404u * (uint32_t)w;
         uint8_t *mine = reinterpret_cast<uint8_t *>(&sm.perm[0][t]); /* byte i at mine + (i>>2)*4*FPS + (i&3) */
-        for (int qw = 0; qw < 64; qw++) {
-#pragma unroll
-            for (int r4 = 0; r4 < 4; r4++) {
-                const int q = 4 * qw + r4;
-                const int k = q + xo_int(x, 256u - (uint32_t)q);
-                uint8_t *pa = mine + qw * (4 * FPS) + r4;
-                uint8_t *pb = mine + (k >> 2) * (4 * FPS) + (k & 3);
-                uint8_t va = *pa, vb = *pb;
-                *pa = vb;
-                *pb = va;
-            }
-        }
+        xo_shuffle<FPS>(mine, x);
     }
     /* split of the offsets used by a zero input coordinate */
     OffHdr h;
@@ -280,15 +270,17 @@ __global__ void __launch_bounds__(128) k_ow_finish_tree(const __grid_constant__ 
     }
     __syncthreads();
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= (long long)ns * np) return;
-    const int p = (int)(g % np);
-    const int by = pts[(size_t)(g / np) * pstride + 3 * p + 1] * 4;
-    int32_t tg[6];
-    const auto *v = clim + (size_t)g * 5;
-    if (FM) climate_finish_f(W, S, (float)v[0], (float)v[1], (float)v[2], (float)v[3], (float)v[4], by, tg);
-    else climate_finish_d(W, S, (double)v[0], (double)v[1], (double)v[2], (double)v[3], (double)v[4], by, tg);
-    uint64_t d;
-    const int leaf = tree_search_scattered(tree, tg, -1, d);
+    const bool in = g < (long long)ns * np;
+    int32_t tg[6] = {0, 0, 0, 0, 0, 0};
+    if (in) {
+        const int p = (int)(g % np);
+        const int by = pts[(size_t)(g / np) * pstride + 3 * p + 1] * 4;
+        const auto *v = clim + (size_t)g * 5;
+        if (FM) climate_finish_f(W, S, (float)v[0], (float)v[1], (float)v[2], (float)v[3], (float)v[4], by, tg);
+        else climate_finish_d(W, S, (double)v[0], (double)v[1], (double)v[2], (double)v[3], (double)v[4], by, tg);
+    }
+    const int leaf = tree_search_lanes(tree, W, tg, in);
+    if (!in) return;
     out[g] = tree[leaf].biome;
     if (targets)
         for (int k = 0; k < 6; k++) targets[g * 6 + k] = tg[k];
@@ -313,17 +305,17 @@ __global__ void __launch_bounds__(128) k_ow_search_first(const __grid_constant__
     }
     __syncthreads();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    bool failed = false;
-    if (g < ns) {
-        int32_t tg[6];
+    const bool in = g < ns;
+    int32_t tg[6] = {0, 0, 0, 0, 0, 0};
+    if (in) {
         const auto *v = clim + (size_t)g * 5;
         const int by = pts[3 * g + 1] * 4;
         if (FM) climate_finish_f(W, S, (float)v[0], (float)v[1], (float)v[2], (float)v[3], (float)v[4], by, tg);
         else climate_finish_d(W, S, (double)v[0], (double)v[1], (double)v[2], (double)v[3], (double)v[4], by, tg);
-        if (obs_accept(o, tree, tg, ties != 0)) surv[atomicAdd(nsurv, 1u)] = seeds[g];
-        else failed = true;
     }
-    const int nf = __syncthreads_count(failed);
+    const bool met = obs_accept(o, tree, W, tg, ties != 0, in);
+    if (met) surv[atomicAdd(nsurv, 1u)] = seeds[g];
+    const int nf = __syncthreads_count(in && !met);
     if (threadIdx.x == 0 && nf) atomicAdd(fail, (unsigned long long)nf);
 }
 

@@ -90,8 +90,7 @@ __global__ void __launch_bounds__(SETUP_NT) k_setup_xo(const __grid_constant__ M
     h.oy = xo_double(x) * 256.0;
     h.oz = xo_double(x) * 256.0;
     perm_identity(perm, t);
-    uint8_t *base = reinterpret_cast<uint8_t *>(&perm[0][0]);
-    for (int q = 0; q < 256; q++) perm_swap(base, t, q, q + xo_int(x, 256u - (uint32_t)q));
+    xo_shuffle<SETUP_NT>(reinterpret_cast<uint8_t *>(&perm[0][t]), x);
     MgLattice *L = out + g;
     header_store(h, L, !W.fmode);
     perm_store(perm, t, L);

@@ -107,10 +107,11 @@ typedef struct {
     int32_t end_ids[5];            /* the_end, end_highlands, end_midlands, small_end_islands, end_barrens */
     double end_f2, end_g2;         /* 2-D simplex skew 0.5*(sqrt(3)-1) and unskew (3-sqrt(3))/6 */
     int32_t tree_root, tree_nodes, tree_leaves;
-    /* the leaves again, clustered, for a search that shares its pruning among a tile's cells: groups of 32 leaves (the last fewer) with
-     * their box at nodes [group_off, group_off + groups) of the same array, the boxes of clusters of 32 groups from node
-     * cluster_off on, and the leaves from node leaf_off on; a leaf's `first` is its rank in the tree's depth-first order (in the tree as well) */
-    int32_t group_off, groups, leaf_off, cluster_off;
+    /* The leaves again, clustered, for searches by a whole warp: groups of 32 leaves (the last fewer), clusters of 32 groups.
+     * Offsets are nodes of the tree's array: the leaves as nodes in clustered order at leaf_off (a leaf's `first` is its rank in
+     * the tree's depth-first order, there and in the tree), and the groups' boxes, the clusters' boxes and the leaves once more in
+     * blocks of 32 nodes whose first 16 bytes precede their second 16 bytes. */
+    int32_t groups, leaf_off, group_off, cluster_off, block_off;
     MgSpline spline;
 } MgWorldDesc;
 

@@ -65,26 +65,28 @@ __global__ void __launch_bounds__(128) k_search_rest(const __grid_constant__ MgW
     }
     __syncthreads();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g < ns) {
-        const int64_t seed = seeds[g];
-        const MgLattice *T = states + (size_t)g * W.ntables;
-        int64_t hs = 0;
-        bool have = false;
-        int j = j0;
-        for (; j < nobs; j++) {
-            const MgObs &o = obs[j];
-            int qx, qy, qz;
-            obs_cell(o, seed, hs, have, qx, qy, qz);
-            bool ok;
-            if (DIM == MG_END) {
-                ok = end_accept<FM>(W, T->p, o, qx, qz);
-            } else {
-                int32_t tg[6];
-                cell_target<FM, DIM>(W, S, T, qx, qy, qz, tg);
-                ok = obs_accept(o, tree, tg, ties != 0);
-            }
-            if (!ok) break;
+    const int64_t seed = g < ns ? seeds[g] : 0;
+    const MgLattice *T = states + (size_t)(g < ns ? g : 0) * W.ntables;
+    int64_t hs = 0;
+    bool have = false;
+    int j = j0;
+    bool alive = g < ns && j < nobs;
+    while (__any_sync(0xFFFFFFFFu, alive)) { /* the warp searches the tree together */
+        const MgObs &o = obs[alive ? j : 0];
+        int qx = 0, qy = 0, qz = 0;
+        if (alive) obs_cell(o, seed, hs, have, qx, qy, qz);
+        bool ok;
+        if (DIM == MG_END) {
+            ok = alive && end_accept<FM>(W, T->p, o, qx, qz);
+        } else {
+            int32_t tg[6] = {0, 0, 0, 0, 0, 0};
+            if (alive) cell_target<FM, DIM>(W, S, T, qx, qy, qz, tg);
+            ok = obs_accept(o, tree, W, tg, ties != 0, alive);
         }
+        if (alive && ok) j++;
+        alive = alive && ok && j < nobs;
+    }
+    if (g < ns) {
         atomicAdd(&hist[j], 1u);
         if (j == nobs) {
             const unsigned k = atomicAdd(nfound, 1u);

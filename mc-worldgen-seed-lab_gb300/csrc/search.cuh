@@ -93,15 +93,44 @@ __device__ __forceinline__ void tree_ties(const MgTreeNode *__restrict__ T, cons
 
 /* observation met by a target: its ENGINE biome is in the mask, or (ties) any equal-fitness leaf's is.  The
  * ENGINE leaf is one of the equal-fitness leaves, so in ties mode the one traversal that collects their
- * biomes decides alone. */
-__device__ __forceinline__ bool obs_accept(const MgObs &o, const MgTreeNode *__restrict__ T, const int32_t *tg, bool ties) {
-    if (!ties) {
-        uint64_t d;
-        return obs_in(o, T[tree_search_scattered(T, tg, -1, d)].biome);
+ * biomes decides alone.  Called by all 32 lanes; the active ones' targets one after another, each by the whole warp. */
+__device__ __forceinline__ bool obs_accept(const MgObs &o, const MgTreeNode *__restrict__ T, const MgWorldDesc &W, const int32_t *tg,
+                                           bool ties, bool active) {
+    if (W.groups <= 1) { /* the Nether's five leaves: 32 searches at once */
+        uint64_t m[2], d;
+        if (!active) return false;
+        if (!ties) return obs_in(o, T[tree_search_scattered(T, tg, -1, d)].biome);
+        tree_ties(T, tg, m);
+        return ((m[0] & o.mask[0]) | (m[1] & o.mask[1])) != 0;
     }
-    uint64_t m[2];
-    tree_ties(T, tg, m);
-    return ((m[0] & o.mask[0]) | (m[1] & o.mask[1])) != 0;
+    if (!ties) {
+        const int leaf = tree_search_lanes(T, W, tg, active);
+        return active && obs_in(o, T[leaf].biome);
+    }
+    const unsigned FULL = 0xFFFFFFFFu;
+    RtTarget q{};
+    const bool ok = active && rt_packed(T) && rt_target(T, tg, q);
+    bool met = false, alone = active;
+    for (unsigned m = __ballot_sync(FULL, ok); m; m &= m - 1) {
+        const int src = __ffs((int)m) - 1;
+        RtTarget s;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            s.p[k] = __shfl_sync(FULL, q.p[k], src);
+            s.n[k] = __shfl_sync(FULL, q.n[k], src);
+        }
+        const RtWarp r = rt_point<true>(T, W, s, 0xFFFFFFFEu, __shfl_sync(FULL, o.mask[0], src), __shfl_sync(FULL, o.mask[1], src));
+        if ((int)(threadIdx.x & 31) == src) {
+            met = r.word != 0;
+            alone = r.leaf < 0;
+        }
+    }
+    if (alone) {
+        uint64_t m[2];
+        tree_ties(T, tg, m);
+        met = ((m[0] & o.mask[0]) | (m[1] & o.mask[1])) != 0;
+    }
+    return met;
 }
 
 /* The End check of an observation, deciding early (same answer as the full window).

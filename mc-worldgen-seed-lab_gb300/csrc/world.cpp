@@ -694,11 +694,22 @@ static void append_groups(std::vector<MgTreeNode> *tree, MgWorldDesc *D) {
         work.push_back({s, m});
     }
     const size_t ng = groups.size();
-    D->group_off = (int32_t)tree->size();
     D->groups = (int32_t)ng;
-    D->cluster_off = D->group_off + D->groups;
-    D->leaf_off = D->cluster_off + (int32_t)((ng + 31) / 32);
-    auto push_box = [&](size_t s, size_t e) { /* of the leaves order[s..e) */
+    D->leaf_off = (int32_t)tree->size();
+    for (int i : order) tree->push_back(leaves[(size_t)i]);
+    while (tree->size() % 4) tree->push_back(MgTreeNode()); /* 128-byte lines */
+    auto split = [&](const std::vector<MgTreeNode> &v) { /* blocks of 32 nodes: their first halves, then their second halves */
+        const size_t at = tree->size();
+        tree->resize(at + (v.size() + 31) / 32 * 32);
+        uint8_t *p = reinterpret_cast<uint8_t *>(tree->data() + at);
+        for (size_t i = 0; i < v.size(); i++) {
+            uint8_t *q = p + i / 32 * 1024 + i % 32 * 16;
+            memcpy(q, &v[i], 16);
+            memcpy(q + 512, reinterpret_cast<const uint8_t *>(&v[i]) + 16, 16);
+        }
+        return (int32_t)at;
+    };
+    auto box = [&](size_t s, size_t e) { /* of the leaves order[s..e) */
         MgTreeNode n;
         memset(&n, 0, sizeof n);
         n.d7 = 0xFFFFFFFFu;
@@ -711,11 +722,15 @@ static void append_groups(std::vector<MgTreeNode> *tree, MgWorldDesc *D) {
             }
             n.d7 = std::min(n.d7, l.d7);
         }
-        tree->push_back(n);
+        return n;
     };
-    for (const auto &g : groups) push_box(g.first, g.second);
-    for (size_t c = 0; c < ng; c += 32) push_box(groups[c].first, groups[std::min(c + 32, ng) - 1].second);
-    for (int i : order) tree->push_back(leaves[(size_t)i]);
+    std::vector<MgTreeNode> gs, cs, ls;
+    for (const auto &g : groups) gs.push_back(box(g.first, g.second));
+    for (size_t c = 0; c < ng; c += 32) cs.push_back(box(groups[c].first, groups[std::min(c + 32, ng) - 1].second));
+    for (int i : order) ls.push_back(leaves[(size_t)i]);
+    D->group_off = split(gs);
+    D->cluster_off = split(cs);
+    D->block_off = split(ls);
 }
 
 int build_world(const char *root, int version, int dim, const char *preset, MgWorldDesc *D,

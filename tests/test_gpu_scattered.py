@@ -1,0 +1,39 @@
+"""Scattered samples searched by whole warps: many seeds at points of any number (last warps partly empty, targets far from
+the tree's boxes at extreme heights), and the seed search's observations in both tie modes, against the oracle."""
+import numpy as np
+import pytest
+
+import __graft_entry__ as ge
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("version,preset,dim", [("26.1", "normal", "overworld"), ("26.3", "amplified", "overworld"),
+                                                ("26.4-snapshot-2", "large_biomes", "overworld"), ("26.2", "normal", "the_nether")])
+def test_scattered(version, preset, dim):
+    mg = ge.package()
+    mg.load()
+    if mg.device_count() < 1:
+        pytest.fail("no CUDA device")
+    w = mg.Generator.open(ge.data_root(), version).world("minecraft:" + dim, preset, 0)
+    ow = O.World(ge.data_root(), version, dim, preset)
+    rng = np.random.default_rng(11)
+    for ns, npt in ((1, 1), (1, 31), (3, 11), (129, 1), (17, 9)):
+        seeds = rng.integers(-2**63, 2**63 - 1, ns)
+        pts = rng.integers(-7000, 7000, (npt, 3)).astype(np.int32)
+        pts[:, 1] = rng.integers(-600, 600, npt)
+        got, tg = w.seed_points(seeds, pts, want_targets=True)
+        exp, et = ow.points(seeds, pts, want_targets=True)
+        assert np.array_equal(np.asarray(got).reshape(-1), np.asarray(exp).reshape(-1)), (ns, npt)
+        assert np.array_equal(np.asarray(tg).reshape(-1), np.asarray(et).reshape(-1)), (ns, npt)
+    seeds = rng.integers(-2**63, 2**63 - 1, 777)
+    at = rng.integers(-3000, 3000, (3, 3)).astype(np.int32)
+    at[:, 1] = (16, -200, 300)
+    ids = np.asarray(ow.points(seeds[:1], at)).reshape(-1)
+    obs = mg.make_obs([(int(x), int(y), int(z), [int(b)]) for (x, y, z), b in zip(at, ids)])
+    oobs = O.make_obs([(int(x), int(y), int(z), [int(b)]) for (x, y, z), b in zip(at, ids)])
+    for ties in (False, True):
+        got = w.search(obs, kind=mg.SEEDS_LIST, seeds=seeds, ties=ties)
+        exp = ow.search(oobs, kind=O.SEEDS_LIST, seeds=seeds, ties=ties)
+        assert np.array_equal(got[0], exp[0]) and np.array_equal(got[1], exp[1]), (ties, got[1], exp[1])
