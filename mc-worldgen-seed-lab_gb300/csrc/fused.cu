@@ -71,13 +71,37 @@ struct FusedSmem {
     typename std::conditional<std::is_same<V, float>::value, OffHdrF, OffHdr>::type hdr[FMAXOFF];
 };
 
+/* lattice j of a seed (engine/mc_climate.h:95-106, engine/mc_noise.h:29-41), its permutation into a column of FusedSmem::perm */
+struct FusedOwn {
+    int noise = 0, st = 0, lev = 0;
+    double ox = 0.0, oy = 0.0, oz = 0.0;
+};
+__device__ __forceinline__ void fused_lattice(const MgWorldDesc &W, int64_t seed, int j, uint32_t *col, FusedOwn &o) {
+    while (o.noise < MG_OW_NOISES - 1 && j >= W.noise[o.noise + 1].base) o.noise++;
+    const MgNoise &N = W.noise[o.noise];
+    const int r = j - N.base;
+    o.st = r >= N.nlev;
+    o.lev = r - o.st * N.nlev;
+    Xo root = xo_from_seed(seed);
+    uint64_t plo = xo_next(root), phi = xo_next(root);
+    Xo nr = xo_make(W.nhl[o.noise] ^ plo, W.nhh[o.noise] ^ phi);
+    uint64_t a = xo_next(nr), b = xo_next(nr);
+    if (o.st) { a = xo_next(nr); b = xo_next(nr); }
+    Xo x = xo_make(N.hlo[o.lev] ^ a, N.hhi[o.lev] ^ b);
+    o.ox = xo_double(x) * 256.0;
+    o.oy = xo_double(x) * 256.0;
+    o.oz = xo_double(x) * 256.0;
+    for (int w = 0; w < 64; w++) col[w * FPS] = 0x03020100u + 0x04040404u * (uint32_t)w;
+    xo_shuffle<FPS>(reinterpret_cast<uint8_t *>(col), x); /* byte i at col + (i >> 2) * 4 FPS + (i & 3) */
+}
+
 /* Threads are lattice-major: thread t owns lattice j = t / spc of local seed t % spc, so the offset-noise
  * lattices of all the CTA's seeds are threads 0 .. noff*spc-1 and their shift octaves (16 per point) can be
  * spread over every thread of the CTA in phase B. */
 template <bool FM>
 __global__ void __launch_bounds__(FNT) k_ow_seed_climate(const __grid_constant__ MgWorldDesc W,
                                                          const int64_t *__restrict__ seeds, int ns,
-                                                         const int32_t *__restrict__ pts, int np, int pstride,
+                                                         const int32_t *__restrict__ pts, int np,
                                                          typename std::conditional<FM, float, double>::type *__restrict__ clim) {
     typedef typename std::conditional<FM, float, double>::type V;
     extern __shared__ uint4 smem_raw[];
@@ -92,28 +116,11 @@ __global__ void __launch_bounds__(FNT) k_ow_seed_climate(const __grid_constant__
     const int noff = 2 * O.nlev;              /* offset-noise lattices per seed (noise 0 is first) */
     const int nown = noff * spc;              /* offset-noise lattice owners in the CTA */
 
-    /* ---- phase A: this thread's lattice (engine/mc_climate.h:95-106, engine/mc_noise.h:29-41) */
-    int noise = 0, st = 0, lev = 0;
-    double ox = 0.0, oy = 0.0, oz = 0.0;
-    if (active) {
-        while (noise < MG_OW_NOISES - 1 && j >= W.noise[noise + 1].base) noise++;
-        const MgNoise &N = W.noise[noise];
-        const int r = j - N.base;
-        st = r >= N.nlev;
-        lev = r - st * N.nlev;
-        Xo root = xo_from_seed(seeds[s0 + ls]);
-        uint64_t plo = xo_next(root), phi = xo_next(root);
-        Xo nr = xo_make(W.nhl[noise] ^ plo, W.nhh[noise] ^ phi);
-        uint64_t a = xo_next(nr), b = xo_next(nr);
-        if (st) { a = xo_next(nr); b = xo_next(nr); }
-        Xo x = xo_make(N.hlo[lev] ^ a, N.hhi[lev] ^ b);
-        ox = xo_double(x) * 256.0;
-        oy = xo_double(x) * 256.0;
-        oz = xo_double(x) * 256.0;
-        for (int w = 0; w < 64; w++) sm.perm[w][t] = 0x03020100u + 0x04040404u * (uint32_t)w;
-        uint8_t *mine = reinterpret_cast<uint8_t *>(&sm.perm[0][t]); /* byte i at mine + (i>>2)*4*FPS + (i&3) */
-        xo_shuffle<FPS>(mine, x);
-    }
+    /* ---- phase A: this thread's lattice */
+    FusedOwn own;
+    if (active) fused_lattice(W, seeds[s0 + ls], j, &sm.perm[0][t], own);
+    const int noise = own.noise, st = own.st, lev = own.lev;
+    const double ox = own.ox, oy = own.oy, oz = own.oz;
     /* split of the offsets used by a zero input coordinate */
     OffHdr h;
     h.ox = ox; h.oy = oy; h.oz = oz;
@@ -135,7 +142,7 @@ __global__ void __launch_bounds__(FNT) k_ow_seed_climate(const __grid_constant__
             if (s0 + o % spc >= ns) continue;
             const auto &oh = sm.hdr[o];
             const IlvPerm<FPS> perm{pbase, o};
-            const int32_t *pp = pts + (size_t)(s0 + o % spc) * pstride + 3 * (p0 + p);
+            const int32_t *pp = pts + 3 * (p0 + p);
             double X = (double)pp[0], Z = (double)pp[2];
             if (ost) { X = X * MG_SECOND_STACK; Z = Z * MG_SECOND_STACK; }
             const double of = O.freq[olev];
@@ -168,7 +175,7 @@ __global__ void __launch_bounds__(FNT) k_ow_seed_climate(const __grid_constant__
         if (t < spc * FNPC) {
             const int cs = t / FNPC, p = t % FNPC;
             if (p < npc && s0 + cs < ns) {
-                const int32_t *pp = pts + (size_t)(s0 + cs) * pstride + 3 * (p0 + p);
+                const int32_t *pp = pts + 3 * (p0 + p);
                 const double X = (double)pp[0], Z = (double)pp[2];
                 double x, z;
                 if (FM) {
@@ -260,7 +267,7 @@ template <bool FM>
 __global__ void __launch_bounds__(128) k_ow_finish_tree(const __grid_constant__ MgWorldDesc W,
                                                         const MgTreeNode *__restrict__ tree,
                                                         const typename std::conditional<FM, float, double>::type *__restrict__ clim,
-                                                        int ns, const int32_t *__restrict__ pts, int np, int pstride,
+                                                        int ns, const int32_t *__restrict__ pts, int np,
                                                         uint8_t *__restrict__ out, int32_t *__restrict__ targets) {
     __shared__ MgSpline S;
     {
@@ -274,7 +281,7 @@ __global__ void __launch_bounds__(128) k_ow_finish_tree(const __grid_constant__ 
     int32_t tg[6] = {0, 0, 0, 0, 0, 0};
     if (in) {
         const int p = (int)(g % np);
-        const int by = pts[(size_t)(g / np) * pstride + 3 * p + 1] * 4;
+        const int by = pts[3 * p + 1] * 4;
         const auto *v = clim + (size_t)g * 5;
         if (FM) climate_finish_f(W, S, (float)v[0], (float)v[1], (float)v[2], (float)v[3], (float)v[4], by, tg);
         else climate_finish_d(W, S, (double)v[0], (double)v[1], (double)v[2], (double)v[3], (double)v[4], by, tg);
@@ -286,16 +293,235 @@ __global__ void __launch_bounds__(128) k_ow_finish_tree(const __grid_constant__ 
         for (int k = 0; k < 6; k++) targets[g * 6 + k] = tg[k];
 }
 
-/* Seed search, Overworld, first observation of every candidate: finish the climate at the candidate's own
- * cell, check the observation (mask, or any equal-fitness leaf in ties mode); passing candidates are
- * appended to `surv`, failures counted into *fail (engine/cuda/mc_gpu.cuh:476-493, stage [0]). */
+/* ---- seed search, Overworld, one observation of every candidate (engine/cuda/mc_gpu.cuh:476-493, stage [0]), in three kernels.
+ * The shuffles bound it (46 of 256 steps per candidate, the integer pipe), so it builds no more lattices than decide a candidate:
+ * k_ow_search_th those of the offset, temperature and humidity (14 of 46), after which a table (k_search_possible) says whether
+ * any leaf with an observed biome can still be nearest (about 29 % of the candidates); k_ow_search_rest the others' for those,
+ * k_ow_search_first the target and the tree.  2^20 candidates: 14.7 + 0.9 ms in one stage, 8.6 ms in three. */
+
+/* possible[r] bit c: a leaf with a biome of the mask can be nearest to a target of temperature class r and humidity class c
+ * (class: cuts at or below the value).  It cannot when some other leaf holds the whole class while it does not, and holds its box
+ * in every other dimension: then that leaf is closer, whatever the other coordinates.  One block per leaf (a warp per leaf took 75 us,
+ * a chain of loads). */
+__global__ void __launch_bounds__(256) k_search_possible(const __grid_constant__ MgWorldDesc W, const MgTreeNode *__restrict__ tree,
+                                                         MgObs o, uint32_t *__restrict__ possible) {
+    const int lane = threadIdx.x & 31;
+    const MgTreeNode *L = tree + W.leaf_off;
+    auto cls = [&](int d, int v) {
+        int k = 0;
+        for (int i = 0; i < W.cuts[d]; i++) k += W.cut[d][i] <= v;
+        return k;
+    };
+    auto bits = [](int a, int b) { return b < a ? 0u : (0xFFFFFFFFu >> (31 - (b - a))) << a; };
+    if (W.cuts[0] < 0 || W.cuts[1] < 0) { /* too many bounds for the table: everything is possible */
+        if (blockIdx.x == 0 && threadIdx.x < 32) possible[threadIdx.x] = 0xFFFFFFFFu;
+        return;
+    }
+    __shared__ uint32_t row[32];
+    {
+        const MgTreeNode n = L[blockIdx.x];
+        if (!obs_in(o, n.biome)) return;
+        if (threadIdx.x < 32) row[threadIdx.x] = 0;
+        __syncthreads();
+        uint32_t covered = 0; /* of row `lane` */
+        for (int m0 = (int)(threadIdx.x & ~31u); m0 < W.tree_leaves; m0 += (int)blockDim.x) {
+            bool over = m0 + lane < W.tree_leaves;
+            const MgTreeNode m = L[over ? m0 + lane : 0];
+            for (int d = 2; d < 6; d++) over &= m.lo[d] <= n.lo[d] && m.nhi[d] <= n.nhi[d];
+            over &= m.d7 <= n.d7;
+            for (unsigned w = __ballot_sync(0xFFFFFFFFu, over); w; w &= w - 1) {
+                const MgTreeNode &c = L[m0 + __ffs((int)w) - 1];
+                if (lane >= cls(0, c.lo[0]) && lane <= cls(0, -c.nhi[0])) covered |= bits(cls(1, c.lo[1]), cls(1, -c.nhi[1]));
+            }
+        }
+        atomicOr(&row[lane], covered);
+        __syncthreads();
+        if (threadIdx.x >= 32) return;
+        const uint32_t own = lane >= cls(0, n.lo[0]) && lane <= cls(0, -n.nhi[0]) ? bits(cls(1, n.lo[1]), cls(1, -n.nhi[1])) : 0u;
+        atomicOr(&possible[lane], own | ~row[lane]);
+    }
+}
+
+/* candidates that are left after the first stage: their index, shifted coordinates and (in clim) first two noise values */
+template <typename V>
+struct SearchList {
+    unsigned *count;
+    int32_t *index;
+    double2 *coord;
+    V *clim; /* 5 per entry */
+};
+template <typename V>
+struct SearchSmem {
+    uint32_t perm[64][FPS];
+    V val[FPS], valb[FPS]; /* octave values by owner */
+    double coord[FPS / 2][4];
+};
+/* lattices [j0, j1) of each seed, spc seeds per CTA: thread t owns lattice j0 + t / spc of local seed t % spc */
+template <bool FM, typename V>
+__device__ __forceinline__ V search_octave(const MgWorldDesc &W, const FusedOwn &own, const OffHdr &h, const IlvPerm<FPS> &perm,
+                                           const double *c) {
+    const MgNoise &N = W.noise[own.noise];
+    const double x = c[own.st ? 2 : 0], z = c[own.st ? 3 : 1], f = N.freq[own.lev];
+    const int k = N.fexp[own.lev];
+    int ix, iz;
+    if constexpr (FM) {
+        float fx, fz;
+        split_fk(x, f, k, own.ox, ix, fx);
+        split_fk(z, f, k, own.oz, iz, fz);
+        return (V)octave_y0<float>(perm, h, ix, fx, iz, fz);
+    } else {
+        double fx, fz;
+        int64_t FX, FZ;
+        split_dk(x, f, k, own.ox, ix, fx, FX);
+        split_dk(z, f, k, own.oz, iz, fz, FZ);
+        return (V)octave_d_y0(perm, h, ix, fx, FX, iz, fz, FZ);
+    }
+}
+/* a noise's sum of its octaves, in the reference's order (engine/mc_noise.h:285-324); first: val index of its first lattice */
+template <bool FM, typename V>
+__device__ __forceinline__ V search_sum(const MgNoise &N, const V *val, int first, int spc, int s) {
+    if constexpr (FM) {
+        float acc = 0.0f;
+        for (int k = 0; k < N.nlev; k++) {
+            acc += N.amp_f[k] * val[(first + k) * spc + s];
+            acc += N.amp_f[k] * val[(first + N.nlev + k) * spc + s];
+        }
+        return acc;
+    } else {
+        double a1 = 0.0, a2 = 0.0;
+        for (int k = 0; k < N.nlev; k++) a1 += N.amp_d[k] * val[(first + k) * spc + s] * N.vf_d[k];
+        for (int k = 0; k < N.nlev; k++) a2 += N.amp_d[k] * val[(first + N.nlev + k) * spc + s] * N.vf_d[k];
+        return (a1 + a2) * N.vfac;
+    }
+}
 template <bool FM>
-__global__ void __launch_bounds__(128) k_ow_search_first(const __grid_constant__ MgWorldDesc W,
-                                                         const MgTreeNode *__restrict__ tree,
-                                                         const typename std::conditional<FM, float, double>::type *__restrict__ clim,
-                                                         int ns, const int64_t *__restrict__ seeds,
-                                                         const int32_t *__restrict__ pts, MgObs o, int ties,
-                                                         int64_t *__restrict__ surv, unsigned *__restrict__ nsurv,
+__global__ void __launch_bounds__(FPS) k_ow_search_th(const __grid_constant__ MgWorldDesc W, const int64_t *__restrict__ seeds, int ns,
+                                                      const int32_t *__restrict__ pts, const uint32_t *__restrict__ possible,
+                                                      SearchList<typename std::conditional<FM, float, double>::type> out,
+                                                      unsigned long long *__restrict__ fail) {
+    typedef typename std::conditional<FM, float, double>::type V;
+    extern __shared__ uint4 smem_raw[];
+    SearchSmem<V> &sm = *reinterpret_cast<SearchSmem<V> *>(smem_raw);
+    const int t = threadIdx.x, nt = W.noise[3].base, spc = FPS / nt, s0 = blockIdx.x * spc, ls = t % spc;
+    const bool active = t / spc < nt && s0 + ls < ns;
+    FusedOwn own;
+    OffHdr h;
+    if (active) {
+        fused_lattice(W, seeds[s0 + ls], t / spc, &sm.perm[0][t], own);
+        h.ox = own.ox; h.oy = own.oy; h.oz = own.oz;
+        lattice_header(h, !FM);
+    }
+    const IlvPerm<FPS> perm{reinterpret_cast<const uint8_t *>(&sm.perm[0][0]), t};
+    const MgNoise &O = W.noise[0];
+    if (active && own.noise == 0) { /* ShiftA (x, 0, z) and ShiftB (z, x, 0) */
+        const int32_t *pp = pts + (size_t)(s0 + ls) * 3;
+        double X = (double)pp[0], Z = (double)pp[2];
+        if (own.st) { X = X * MG_SECOND_STACK; Z = Z * MG_SECOND_STACK; }
+        const double f = O.freq[own.lev];
+        const int k = O.fexp[own.lev];
+        int ix, iz, iy;
+        if constexpr (FM) {
+            float fx, fz, fy;
+            split_fk(X, f, k, own.ox, ix, fx);
+            split_fk(Z, f, k, own.oz, iz, fz);
+            sm.val[t] = (V)octave_y0<float>(perm, h, ix, fx, iz, fz);
+            split_fk(Z, f, k, own.ox, ix, fx);
+            split_fk(X, f, k, own.oy, iy, fy);
+            sm.valb[t] = (V)octave_z0<float>(perm, h, ix, fx, iy, fy);
+        } else {
+            double fx, fz, fy;
+            int64_t FX, FZ, FY;
+            split_dk(X, f, k, own.ox, ix, fx, FX);
+            split_dk(Z, f, k, own.oz, iz, fz, FZ);
+            sm.val[t] = (V)octave_d_y0(perm, h, ix, fx, FX, iz, fz, FZ);
+            split_dk(Z, f, k, own.ox, ix, fx, FX);
+            split_dk(X, f, k, own.oy, iy, fy, FY);
+            sm.valb[t] = (V)octave_d_z0(perm, h, ix, fx, FX, iy, fy, FY);
+        }
+    }
+    __syncthreads();
+    const bool mine = t < spc && s0 + t < ns;
+    double2 at = make_double2(0.0, 0.0);
+    if (mine) {
+        const int32_t *pp = pts + (size_t)(s0 + t) * 3;
+        at.x = (double)pp[0] + (double)(search_sum<FM, V>(O, sm.val, 0, spc, t) * (V)4.0);
+        at.y = (double)pp[2] + (double)(search_sum<FM, V>(O, sm.valb, 0, spc, t) * (V)4.0);
+        sm.coord[t][0] = at.x;
+        sm.coord[t][1] = at.y;
+        sm.coord[t][2] = at.x * MG_SECOND_STACK;
+        sm.coord[t][3] = at.y * MG_SECOND_STACK;
+    }
+    __syncthreads();
+    if (active && own.noise != 0) sm.val[t] = search_octave<FM, V>(W, own, h, perm, sm.coord[ls]);
+    __syncthreads();
+    if (t < 32 * ((spc + 31) / 32)) {
+        bool left = false;
+        V th[2] = {0, 0};
+        if (mine) {
+            int c[2] = {0, 0};
+            for (int d = 0; d < 2; d++) {
+                th[d] = search_sum<FM, V>(W.noise[1 + d], sm.val, W.noise[1 + d].base, spc, t);
+                const int v = quantize((float)th[d]);
+                for (int i = 0; i < W.cuts[d]; i++) c[d] += W.cut[d][i] <= v;
+            }
+            left = possible[c[0]] >> c[1] & 1;
+        }
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, left), f = __ballot_sync(0xFFFFFFFFu, mine && !left);
+        unsigned k = 0;
+        if ((t & 31) == 0) {
+            if (m) k = atomicAdd(out.count, (unsigned)__popc(m));
+            if (f) atomicAdd(fail, (unsigned long long)__popc(f));
+        }
+        k = __shfl_sync(0xFFFFFFFFu, k, 0) + (unsigned)__popc(m & ((1u << (t & 31)) - 1));
+        if (left) {
+            out.index[k] = s0 + t;
+            out.coord[k] = at;
+            out.clim[(size_t)k * 5] = th[0];
+            out.clim[(size_t)k * 5 + 1] = th[1];
+        }
+    }
+}
+/* the other three noises of the candidates in the list */
+template <bool FM>
+__global__ void __launch_bounds__(FPS) k_ow_search_rest(const __grid_constant__ MgWorldDesc W, const int64_t *__restrict__ seeds,
+                                                        SearchList<typename std::conditional<FM, float, double>::type> list) {
+    typedef typename std::conditional<FM, float, double>::type V;
+    extern __shared__ uint4 smem_raw[];
+    SearchSmem<V> &sm = *reinterpret_cast<SearchSmem<V> *>(smem_raw);
+    const int t = threadIdx.x, j0 = W.noise[3].base, nt = W.ntables - j0, spc = FPS / nt, ls = t % spc;
+    const int ns = (int)*list.count;
+    const IlvPerm<FPS> perm{reinterpret_cast<const uint8_t *>(&sm.perm[0][0]), t};
+    for (int s0 = (int)blockIdx.x * spc; s0 < ns; s0 += (int)gridDim.x * spc) {
+        if (t < spc && s0 + t < ns) {
+            const double2 at = list.coord[s0 + t];
+            sm.coord[t][0] = at.x;
+            sm.coord[t][1] = at.y;
+            sm.coord[t][2] = at.x * MG_SECOND_STACK;
+            sm.coord[t][3] = at.y * MG_SECOND_STACK;
+        }
+        __syncthreads();
+        if (t / spc < nt && s0 + ls < ns) {
+            FusedOwn own;
+            OffHdr h;
+            fused_lattice(W, seeds[list.index[s0 + ls]], j0 + t / spc, &sm.perm[0][t], own);
+            h.ox = own.ox; h.oy = own.oy; h.oz = own.oz;
+            lattice_header(h, !FM);
+            sm.val[t] = search_octave<FM, V>(W, own, h, perm, sm.coord[ls]);
+        }
+        __syncthreads();
+        if (t < 3 * spc) {
+            const int q = 3 + t / spc, s = t % spc;
+            if (s0 + s < ns) list.clim[(size_t)(s0 + s) * 5 + q - 1] = search_sum<FM, V>(W.noise[q], sm.val, W.noise[q].base - j0, spc, s);
+        }
+        __syncthreads();
+    }
+}
+/* the target and the tree; passing candidates are appended to `surv`, failures counted into *fail */
+template <bool FM>
+__global__ void __launch_bounds__(128) k_ow_search_first(const __grid_constant__ MgWorldDesc W, const MgTreeNode *__restrict__ tree,
+                                                         SearchList<typename std::conditional<FM, float, double>::type> list,
+                                                         const int64_t *__restrict__ seeds, const int32_t *__restrict__ pts, MgObs o,
+                                                         int ties, int64_t *__restrict__ surv, unsigned *__restrict__ nsurv,
                                                          unsigned long long *__restrict__ fail) {
     __shared__ MgSpline S;
     {
@@ -304,42 +530,68 @@ __global__ void __launch_bounds__(128) k_ow_search_first(const __grid_constant__
         for (int i = threadIdx.x; i < (int)(sizeof(MgSpline) / 16); i += blockDim.x) d[i] = c[i];
     }
     __syncthreads();
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool in = g < ns;
-    int32_t tg[6] = {0, 0, 0, 0, 0, 0};
-    if (in) {
-        const auto *v = clim + (size_t)g * 5;
-        const int by = pts[3 * g + 1] * 4;
-        if (FM) climate_finish_f(W, S, (float)v[0], (float)v[1], (float)v[2], (float)v[3], (float)v[4], by, tg);
-        else climate_finish_d(W, S, (double)v[0], (double)v[1], (double)v[2], (double)v[3], (double)v[4], by, tg);
+    const int n = (int)*list.count;
+    int nf = 0;
+    for (int b = (int)blockIdx.x * 128; b < n; b += (int)gridDim.x * 128) {
+        const int k = b + (int)threadIdx.x;
+        const bool in = k < n;
+        const int g = in ? list.index[k] : 0;
+        int32_t tg[6] = {0, 0, 0, 0, 0, 0};
+        if (in) {
+            const auto *v = list.clim + (size_t)k * 5;
+            const int by = pts[3 * (size_t)g + 1] * 4;
+            if (FM) climate_finish_f(W, S, (float)v[0], (float)v[1], (float)v[2], (float)v[3], (float)v[4], by, tg);
+            else climate_finish_d(W, S, (double)v[0], (double)v[1], (double)v[2], (double)v[3], (double)v[4], by, tg);
+        }
+        const bool met = obs_accept(o, tree, W, tg, ties != 0, in);
+        if (met) surv[atomicAdd(nsurv, 1u)] = seeds[g];
+        nf += __syncthreads_count(in && !met);
     }
-    const bool met = obs_accept(o, tree, W, tg, ties != 0, in);
-    if (met) surv[atomicAdd(nsurv, 1u)] = seeds[g];
-    const int nf = __syncthreads_count(in && !met);
     if (threadIdx.x == 0 && nf) atomicAdd(fail, (unsigned long long)nf);
 }
 
+/* scratch: the table, the list's counter, index, coordinates and noise values */
+size_t search_scratch_bytes(const MgWorldDesc &W, long long n) {
+    return 256 + (size_t)n * (sizeof(double2) + 5 * (W.fmode ? sizeof(float) : sizeof(double)) + sizeof(int32_t));
+}
 template <bool FM>
 static int search_first_t(const MgWorldDesc &W, const MgTreeNode *tree, const int64_t *seeds, int ns, const int32_t *pts,
                           const MgObs &o, int ties, void *scratch, int64_t *surv, unsigned *nsurv,
                           unsigned long long *fail, cudaStream_t st) {
     typedef typename std::conditional<FM, float, double>::type V;
-    const size_t sm = sizeof(FusedSmem<V>);
-    cudaError_t e = cudaFuncSetAttribute(k_ow_seed_climate<FM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (!e) e = cudaFuncSetAttribute(k_ow_seed_climate<FM>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     (int)cudaSharedmemCarveoutMaxShared); /* room for 4 CTAs per SM */
+    const int sm = (int)sizeof(SearchSmem<V>);
+    cudaError_t e = cudaFuncSetAttribute(k_ow_search_th<FM>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    if (!e) e = cudaFuncSetAttribute(k_ow_search_rest<FM>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    if (!e) e = cudaFuncSetAttribute(k_ow_search_th<FM>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    if (!e) e = cudaFuncSetAttribute(k_ow_search_rest<FM>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    uint8_t *p = (uint8_t *)scratch;
+    uint32_t *possible = (uint32_t *)p;
+    SearchList<V> list;
+    list.count = (unsigned *)(p + 128);
+    list.coord = (double2 *)(p + 256);
+    list.clim = (V *)(list.coord + ns);
+    list.index = (int32_t *)(list.clim + (size_t)ns * 5);
+    if (!e) e = cudaMemsetAsync(p, 0, 256, st);
     if (e) return (int)e;
-    const int spc = FNT / W.ntables;
-    V *clim = (V *)scratch;
+    {
+        ProfScope ps_(K_SEARCH_CELLS, st);
+        k_search_possible<<<(unsigned)W.tree_leaves, 256, 0, st>>>(W, tree, o, possible);
+    }
+    count_launch_external();
+    const int spc = FPS / W.noise[3].base;
     {
         ProfScope ps_(K_OW_SEED_CLIMATE, st);
-        k_ow_seed_climate<FM><<<(unsigned)((ns + spc - 1) / spc), FNT, sm, st>>>(W, seeds, ns, pts, 1, 3, clim);
+        k_ow_search_th<FM><<<(unsigned)((ns + spc - 1) / spc), FPS, sm, st>>>(W, seeds, ns, pts, possible, list, fail);
+    }
+    count_launch_external();
+    {
+        ProfScope ps_(K_OW_SEED_CLIMATE, st);
+        k_ow_search_rest<FM><<<4 * 152, FPS, sm, st>>>(W, seeds, list);
     }
     count_launch_external();
     {
         ProfScope ps_(K_SEARCH_FIRST, st);
-        k_ow_search_first<FM><<<(unsigned)((ns + 127) / 128), 128, 0, st>>>(W, tree, clim, ns, seeds, pts, o, ties, surv,
-                                                                             nsurv, fail);
+        k_ow_search_first<FM><<<8 * 152, 128, 0, st>>>(W, tree, list, seeds, pts, o, ties, surv, nsurv, fail);
     }
     count_launch_external();
     return 0;
@@ -376,13 +628,13 @@ static int fused_t(const MgWorldDesc &W, const MgTreeNode *tree, const int64_t *
     V *clim = (V *)scratch;
     {
         ProfScope ps_(K_OW_SEED_CLIMATE, st);
-        k_ow_seed_climate<FM><<<(unsigned)((ns + spc - 1) / spc), FNT, sm, st>>>(W, seeds, ns, pts, np, 0, clim);
+        k_ow_seed_climate<FM><<<(unsigned)((ns + spc - 1) / spc), FNT, sm, st>>>(W, seeds, ns, pts, np, clim);
     }
     count_launch_external();
     const long long n = (long long)ns * np;
     {
         ProfScope ps_(K_OW_FINISH_TREE, st);
-        k_ow_finish_tree<FM><<<(unsigned)((n + 127) / 128), 128, 0, st>>>(W, tree, clim, ns, pts, np, 0, out, tg);
+        k_ow_finish_tree<FM><<<(unsigned)((n + 127) / 128), 128, 0, st>>>(W, tree, clim, ns, pts, np, out, tg);
     }
     count_launch_external();
     return 0;

@@ -85,6 +85,7 @@ typedef struct __attribute__((aligned(16))) {
     uint8_t biome;
 } MgTreeNode;
 #define MG_TREE_PACKED 1
+#define MG_MAX_CUTS 31
 #define MG_TREE_PACKED_BOUND 12767
 
 /* Seed-independent world description, copied once to the device. */
@@ -112,6 +113,9 @@ typedef struct {
      * the tree's depth-first order, there and in the tree), and the groups' boxes, the clusters' boxes and the leaves once more in
      * blocks of 32 nodes whose first 16 bytes precede their second 16 bytes. */
     int32_t groups, leaf_off, group_off, cluster_off, block_off;
+    /* temperature and humidity bounds of the leaves (lo and hi + 1), ascending: a leaf holds all of the values between two
+     * neighbouring cuts or none.  cuts[d] = -1: more than MG_MAX_CUTS. */
+    int32_t cuts[2], cut[2][MG_MAX_CUTS];
     MgSpline spline;
 } MgWorldDesc;
 

@@ -23,7 +23,9 @@
 #include "launch.h"
 #include "prof.h"
 #include "search.cuh"
+#include "warpcell.cuh"
 
+#define SEARCH_STAGED 4096 /* survivors above which the next observation is checked by launch_ow_search_first too */
 static_assert(sizeof(MgObs) == sizeof(McGb300Obs) && sizeof(MgObs) == 32, "observation layout");
 
 namespace mg {
@@ -47,8 +49,8 @@ __global__ void k_search_cells(int kind, const int64_t *__restrict__ list, uint6
     }
 }
 
-/* observations j0 .. nobs-1 of every seed, stopping at the first that fails; one thread per seed, its
- * lattices from `states` through L1 */
+/* observations j0 .. nobs-1 of every seed, stopping at the first that fails; its lattices from `states` through L1.  Overworld:
+ * the few candidates that are left, a warp each (wc_target, rt_point; a thread each took 500 us for 5,000); else a thread each. */
 template <bool FM, int DIM>
 __global__ void __launch_bounds__(128) k_search_rest(const __grid_constant__ MgWorldDesc W, const MgTreeNode *__restrict__ tree,
                                                      const MgLattice *__restrict__ states, const int64_t *__restrict__ seeds,
@@ -64,7 +66,7 @@ __global__ void __launch_bounds__(128) k_search_rest(const __grid_constant__ MgW
         for (int i = threadIdx.x; i < (int)(sizeof(MgSpline) / 16); i += blockDim.x) d[i] = c[i];
     }
     __syncthreads();
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    const int g = DIM == MG_OVERWORLD ? (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) : (int)(blockIdx.x * blockDim.x + threadIdx.x);
     const int64_t seed = g < ns ? seeds[g] : 0;
     const MgLattice *T = states + (size_t)(g < ns ? g : 0) * W.ntables;
     int64_t hs = 0;
@@ -76,7 +78,12 @@ __global__ void __launch_bounds__(128) k_search_rest(const __grid_constant__ MgW
         int qx = 0, qy = 0, qz = 0;
         if (alive) obs_cell(o, seed, hs, have, qx, qy, qz);
         bool ok;
-        if (DIM == MG_END) {
+        if (DIM == MG_OVERWORLD) { /* one candidate, the same in all lanes */
+            int32_t tg[6];
+            wc_target<FM, DIM>(W, S, T, qx, qy, qz, tg);
+            ok = obs_accept(o, tree, W, tg, ties != 0, (threadIdx.x & 31) == 0);
+            ok = __shfl_sync(0xFFFFFFFFu, ok, 0);
+        } else if (DIM == MG_END) {
             ok = alive && end_accept<FM>(W, T->p, o, qx, qz);
         } else {
             int32_t tg[6] = {0, 0, 0, 0, 0, 0};
@@ -86,7 +93,7 @@ __global__ void __launch_bounds__(128) k_search_rest(const __grid_constant__ MgW
         if (alive && ok) j++;
         alive = alive && ok && j < nobs;
     }
-    if (g < ns) {
+    if (g < ns && (DIM != MG_OVERWORLD || (threadIdx.x & 31) == 0)) {
         atomicAdd(&hist[j], 1u);
         if (j == nobs) {
             const unsigned k = atomicAdd(nfound, 1u);
@@ -102,7 +109,7 @@ template <bool FM>
 int rest_t(const MgWorldDesc &W, const MgTreeNode *tree, const MgLattice *states, const int64_t *seeds, int ns,
            const MgObs *obs, int nobs, int j0, int ties, int64_t *found, unsigned *nfound, unsigned maxfound,
            unsigned long long *reached, cudaStream_t st) {
-    const unsigned grid = (unsigned)((ns + 127) / 128);
+    const unsigned grid = W.dim == MG_OVERWORLD ? (unsigned)((ns + 3) / 4) : (unsigned)((ns + 127) / 128);
     ProfScope ps_(K_SEARCH_REST, st);
     if (W.dim == MG_OVERWORLD)
         k_search_rest<FM, MG_OVERWORLD><<<grid, 128, 0, st>>>(W, tree, states, seeds, ns, obs, nobs, j0, ties, found, nfound, maxfound, reached);
@@ -184,7 +191,7 @@ MCGEN_API int mcgen_gb300_search(const McWorld *w, int kind, const int64_t *list
     if (!e && ow) {
         e = sc.get(&d_pts, (size_t)CH * 3);
         if (!e) e = sc.get(&d_surv, (size_t)CH);
-        if (!e) e = sc.get((uint8_t **)&d_clim, mg::fused_scratch_bytes(W, CH));
+        if (!e) e = sc.get((uint8_t **)&d_clim, mg::search_scratch_bytes(W, CH));
         if (!e) e = sc.get(&d_states, (size_t)SB * W.ntables);
     } else if (!e) {
         e = sc.get(&d_states, (size_t)CH * W.ntables);
@@ -218,15 +225,27 @@ MCGEN_API int mcgen_gb300_search(const McWorld *w, int kind, const int64_t *list
                                           max_found, d_reached, st);
             continue;
         }
-        e = cudaMemsetAsync(d_cnt, 0, sizeof(unsigned), st);
-        if (!e) rc = mg::launch_ow_search_first(W, w->d_tree, d_seeds, m, d_pts, o0, ties, d_clim, d_surv, d_cnt, d_reached, st);
-        unsigned ns = 0;
-        if (!e && !rc) e = cudaMemcpyAsync(&ns, d_cnt, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
-        if (!e && !rc) e = cudaStreamSynchronize(st);
+        /* the observations one by one while many candidates are left, then lattices in memory for the rest */
+        unsigned ns = (unsigned)m;
+        int j = 0;
+        while (!e && !rc && j < nobs && (j == 0 || ns > (unsigned)SEARCH_STAGED)) {
+            MgObs o;
+            memcpy(&o, &obs[j], sizeof o);
+            if (j > 0) {
+                mg::ProfScope ps_(mg::K_SEARCH_CELLS, st);
+                mg::k_search_cells<<<(ns + 127) / 128, 128, 0, st>>>(MCGEN_SEEDS_LIST, d_surv, 0, 0, (int)ns, o, d_seeds, d_pts);
+                mg::count_launch_external();
+            }
+            e = cudaMemsetAsync(d_cnt, 0, sizeof(unsigned), st);
+            if (!e) rc = mg::launch_ow_search_first(W, w->d_tree, d_seeds, (int)ns, d_pts, o, ties, d_clim, d_surv, d_cnt, d_reached + j, st);
+            if (!e && !rc) e = cudaMemcpyAsync(&ns, d_cnt, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+            if (!e && !rc) e = cudaStreamSynchronize(st);
+            j++;
+        }
         for (unsigned b0 = 0; !e && !rc && b0 < ns; b0 += (unsigned)SB) {
             const int mb = (int)std::min<unsigned>((unsigned)SB, ns - b0);
-            if (nobs > 1) rc = mg::launch_setup(W, d_surv + b0, mb, d_states, st);
-            if (!rc) rc = mg::launch_rest(W, w->d_tree, d_states, d_surv + b0, mb, d_obs, nobs, 1, ties, d_found, d_cnt + 1,
+            if (j < nobs) rc = mg::launch_setup(W, d_surv + b0, mb, d_states, st);
+            if (!rc) rc = mg::launch_rest(W, w->d_tree, d_states, d_surv + b0, mb, d_obs, nobs, j, ties, d_found, d_cnt + 1,
                                           max_found, d_reached, st);
         }
     }

@@ -724,6 +724,17 @@ static void append_groups(std::vector<MgTreeNode> *tree, MgWorldDesc *D) {
         }
         return n;
     };
+    for (int d = 0; d < 2; d++) {
+        std::vector<int> c;
+        for (const MgTreeNode &l : leaves) {
+            c.push_back(l.lo[d]);
+            c.push_back(1 - l.nhi[d]);
+        }
+        std::sort(c.begin(), c.end());
+        c.erase(std::unique(c.begin(), c.end()), c.end());
+        D->cuts[d] = c.size() <= MG_MAX_CUTS ? (int32_t)c.size() : -1;
+        for (int k = 0; k < D->cuts[d]; k++) D->cut[d][k] = c[(size_t)k];
+    }
     std::vector<MgTreeNode> gs, cs, ls;
     for (const auto &g : groups) gs.push_back(box(g.first, g.second));
     for (size_t c = 0; c < ng; c += 32) cs.push_back(box(groups[c].first, groups[std::min(c + 32, ng) - 1].second));

@@ -37,3 +37,28 @@ def test_scattered(version, preset, dim):
         got = w.search(obs, kind=mg.SEEDS_LIST, seeds=seeds, ties=ties)
         exp = ow.search(oobs, kind=O.SEEDS_LIST, seeds=seeds, ties=ties)
         assert np.array_equal(got[0], exp[0]) and np.array_equal(got[1], exp[1]), (ties, got[1], exp[1])
+
+
+@pytest.mark.parametrize("version,preset", [("26.1", "normal"), ("26.3", "amplified"), ("26.4-snapshot-2", "normal")])
+def test_search_stages(version, preset):
+    """Enough candidates for several staged observations and the rest by a warp each; masks of one common biome, of many and of
+    none (the table of possible biomes all clear), block observations."""
+    mg = ge.package()
+    mg.load()
+    if mg.device_count() < 1:
+        pytest.fail("no CUDA device")
+    w = mg.Generator.open(ge.data_root(), version).world("minecraft:overworld", preset, 0)
+    ow = O.World(ge.data_root(), version, "overworld", preset)
+    rng = np.random.default_rng(5)
+    n, base = 6001, int(rng.integers(-2**63, 2**63 - 1))
+    for block in (False, True):
+        scale = 4 if block else 1
+        at = rng.integers(-3000, 3000, (4, 3)) * scale
+        at[:, 1] = np.array([16, 16, -9, 60]) * scale
+        ids = [int(b) for b in np.asarray(ow.points([base + 7], at // scale)).reshape(-1)]
+        masks = [sorted(set(ids) | set(range(0, 60, 2))), list(range(60)), [ids[2], ids[0]], [ids[3]]]
+        for rows in (masks, [[127]] + masks[1:]):
+            r = [(int(x), int(y), int(z), m) for (x, y, z), m in zip(at, rows)]
+            got = w.search(mg.make_obs(r, block), kind=mg.SEEDS_RANGE, base=base, n=n)
+            exp = ow.search(O.make_obs(r, block), kind=O.SEEDS_RANGE, base=base, n=n)
+            assert np.array_equal(got[0], exp[0]) and np.array_equal(got[1], exp[1]), (block, got[1], exp[1])
