@@ -166,20 +166,18 @@ __device__ __noinline__ void batch_cells(const MgWorldDesc &W, const MgSpline &S
     put_id(out + R.out_off + (size_t)iz * R.nx + ix, b);
 }
 
-/* End tile: chunks [cx0, cx0 + END_TC) x [cz0, cz0 + END_TC) counted from the chunk of the request's
- * first cell; the tile writes the request's cells that lie in those chunks. */
+/* End tile t of a request (tiles counted from the chunk of its first cell): the classes of its chunks, then the request's cells
+ * in them */
 template <bool FM>
-__device__ __noinline__ void batch_end(const MgWorldDesc &W, BatchSmem &sm, const MgBatchReq &R, int tcx, int tcz,
-                                          uint8_t *out) {
-    const int cx0 = (R.qx0 >> 2) + tcx * END_TC, cz0 = (R.qz0 >> 2) + tcz * END_TC;
-    end_tile_classes<FM>(sm.end.endp, W.end_f2, W.end_g2, cx0, cz0, sm.end.tile);
-    for (int i = threadIdx.x; i < 16 * END_TC * END_TC; i += blockDim.x) {
-        const int qx = 4 * cx0 + i % (4 * END_TC), qz = 4 * cz0 + i / (4 * END_TC);
-        const int ix = qx - R.qx0, iz = qz - R.qz0;
-        if (ix < 0 || iz < 0 || ix >= R.nx || iz >= R.nz) continue;
-        put_id(out + R.out_off + (size_t)iz * R.nx + ix,
-               W.end_ids[sm.end.tile.cls[(i / (16 * END_TC)) * END_TC + (i % (4 * END_TC)) / 4]]);
-    }
+__device__ __noinline__ void batch_end(const MgWorldDesc &W, BatchSmem &sm, const MgBatchReq &R, int t, uint8_t *out) {
+    const int c0 = R.qx0 >> 2, d0 = R.qz0 >> 2, ncx = ((R.qx0 + R.nx - 1) >> 2) - c0 + 1, ncz = ((R.qz0 + R.nz - 1) >> 2) - d0 + 1;
+    const int w = end_tile_side(ncx, END_TC), h = end_tile_side(ncz, END_TC), tw = (ncx + w - 1) / w;
+    const int cx0 = c0 + t % tw * w, cz0 = d0 + t / tw * h;
+    end_tile_classes<FM>(sm.end.endp, W.end_f2, W.end_g2, cx0, cz0, w, h, sm.end.tile);
+    for (int iz = max(4 * cz0 - R.qz0, 0) + (int)(threadIdx.x >> 5); iz < min(4 * (cz0 + h) - R.qz0, R.nz); iz += BNT / 32)
+        for (int ix = max(4 * cx0 - R.qx0, 0) + (int)(threadIdx.x & 31); ix < min(4 * (cx0 + w) - R.qx0, R.nx); ix += 32)
+            put_id(out + R.out_off + (size_t)iz * R.nx + ix,
+                   W.end_ids[sm.end.tile.cls[(((R.qz0 + iz) >> 2) - cz0) * w + ((R.qx0 + ix) >> 2) - cx0]]);
 }
 
 /* TILE_W: tile width in cells (tiles are 128 cells); MINB: resident CTAs per SM the register allocation
@@ -215,6 +213,7 @@ __global__ void __launch_bounds__(BNT, MINB) k_batch(const MgWorldDesc *__restri
         if (new_state) {
             if (W.dim == MG_END) {
                 for (int i = threadIdx.x; i < 256; i += BNT) sm.end.endp[i] = pool[R.state].p[i];
+                end_tile_grad(pool[R.state].p, sm.end.tile);
             } else {
                 const uint4 *a = reinterpret_cast<const uint4 *>(pool + R.state);
                 uint4 *b = reinterpret_cast<uint4 *>(sm.lat);
@@ -225,10 +224,8 @@ __global__ void __launch_bounds__(BNT, MINB) k_batch(const MgWorldDesc *__restri
         if (threadIdx.x == 0) sm.state = R.state;
         const int tile = sm.tile;
         if (W.dim == MG_END) {
-            const int ncx = ((R.qx0 + R.nx - 1) >> 2) - (R.qx0 >> 2) + 1;
-            const int tw = (ncx + END_TC - 1) / END_TC;
-            if (W.fmode) batch_end<true>(W, sm, R, tile % tw, tile / tw, out);
-            else batch_end<false>(W, sm, R, tile % tw, tile / tw, out);
+            if (W.fmode) batch_end<true>(W, sm, R, tile, out);
+            else batch_end<false>(W, sm, R, tile, out);
             continue;
         }
         constexpr int TILE_H = BNT / TILE_W;
@@ -261,7 +258,8 @@ long long batch_tiles(int group, int dim, int qx0, int qz0, int nx, int nz, int 
     if (group != BATCH_REST) return ow_tiles(nx, nz);
     if (dim == MG_END) {
         const long long ncx = ((qx0 + nx - 1) >> 2) - (qx0 >> 2) + 1, ncz = ((qz0 + nz - 1) >> 2) - (qz0 >> 2) + 1;
-        return ((ncx + END_TC - 1) / END_TC) * ((ncz + END_TC - 1) / END_TC);
+        const int w = end_tile_side((int)ncx, END_TC), h = end_tile_side((int)ncz, END_TC);
+        return ((ncx + w - 1) / w) * ((ncz + h - 1) / h);
     }
     const int tw = kBatchTileWidths[shape], th = BNT / tw;
     return (long long)((nx + tw - 1) / tw) * ((nz + th - 1) / th);

@@ -390,43 +390,94 @@ __device__ __forceinline__ double simplex2(const uint8_t *__restrict__ p, double
 }
 /* End island test, screened: the reference decides an island cell by nv < -0.9f (double branch, the float
  * constant widened) or (float)nv < -0.9f (float branch), nv = simplex2 in double (about 60 FP64-pipe
- * operations).  Here the skew, the cell (i, j), the corner choice and the first corner's offsets x0, y0 are
- * the reference's double arithmetic (exact same values), and the three corner terms are evaluated in float
- * from those offsets: |float value - nv| <= END_ISLAND_E (a forward error bound: offsets within 5 u of the
+ * operations).  Here the three corner terms are evaluated in float from the first corner's offsets x0, y0:
+ * |float value - nv| <= END_ISLAND_E (a forward error bound: offsets within 5 u of the
  * double ones, u = 2^-24; tt = 0.5 - x^2 - y^2 within 32 u; tt^4 within 18 u; the gradient dot within 12 u;
  * each term tt^4 * dot within 26 u for |x|, |y| < 0.71 (tt > 0); three terms and their sums within 78 u; times
  * 70: 5,500 u = 3.3e-4 plus the reference's own double roundings, taken as 5e-4).  A value farther than that
  * from the threshold settles the test (with one more float ulp for the float branch's rounding); the rest
  * (a few in 10^4) take the exact double evaluation.  mcgen_gb300_check_end checks the bound and the decisions
- * on the device. */
+ * on the device.
+ *
+ * The coordinates are whole numbers, so within END_FAR the skew is fixed point (2^-40) in place of the reference's doubles
+ * (9 FP64 operations): x0, y0 come within 3 u (G2's rounding, up to 2^-41 a cell, is added back in float).  Where the cell or the
+ * corner choice is nearly ambiguous it may be the reference's neighbour; the corners that the two choices do not share are then
+ * at the edge of their terms' support (tt <= 2e-6, cut off at 0), so the value is within the bound all the same. */
 #define END_ISLAND_E 5e-4f
-__device__ __forceinline__ bool end_island(const uint8_t *__restrict__ p, double xin, double yin, double F2, double G2,
-                                           bool fm) {
-    const double s = (xin + yin) * F2;
-    const int i = ifloor(xin + s), j = ifloor(yin + s);
-    const double t = (double)(i + j) * G2;
-    const double x0 = xin - ((double)i - t), y0 = yin - ((double)j - t);
-    const int i1 = x0 > y0 ? 1 : 0, j1 = 1 - i1;
-    const float g2 = (float)G2, xf = (float)x0, yf = (float)y0;
-    const float xs[3] = {xf, xf - (float)i1 + g2, xf - 1.0f + 2.0f * g2};
-    const float ys[3] = {yf, yf - (float)j1 + g2, yf - 1.0f + 2.0f * g2};
-    const int ii = i & 255, jj = j & 255;
-    const int gs[3] = {p[(ii + p[jj]) & 255] % 12, p[(ii + i1 + p[(jj + j1) & 255]) & 255] % 12,
-                       p[(ii + 1 + p[(jj + 1) & 255]) & 255] % 12};
+#define END_FAR (1 << 21)
+#define END_Q 40
+#define END_F2Q ((int64_t)(0.36602540378443865 * (double)(1LL << END_Q)))
+#define END_G2Q ((int64_t)(0.21132486540518713 * (double)(1LL << END_Q)))
+struct EndCell {
+    int i, j;
+    float x0, y0;
+};
+/* |tx|, |tz| < END_FAR */
+__device__ __forceinline__ EndCell end_cell(int tx, int tz, double G2) {
+    const float g2e = (float)(G2 - (double)END_G2Q * 0x1.0p-40);
+    const int64_t s = (int64_t)(tx + tz) * END_F2Q;
+    EndCell c;
+    c.i = (int)((((int64_t)tx << END_Q) + s) >> END_Q);
+    c.j = (int)((((int64_t)tz << END_Q) + s) >> END_Q);
+    const int64_t t = (int64_t)(c.i + c.j) * END_G2Q;
+    const float te = (float)(c.i + c.j) * g2e;
+    c.x0 = (float)(int32_t)((((int64_t)(tx - c.i) << END_Q) + t) >> 10) * 0x1.0p-30f + te;
+    c.y0 = (float)(int32_t)((((int64_t)(tz - c.j) << END_Q) + t) >> 10) * 0x1.0p-30f + te;
+    return c;
+}
+/* the gradient of a permutation value, its third component dropped */
+__device__ __forceinline__ float2 end_grad(int v) {
+    const int g = v % 12;
+    return make_float2(gdot<float>(g, 1.0f, 0.0f, 0.0f), gdot<float>(g, 0.0f, 1.0f, 0.0f));
+}
+/* the three terms times 70; G(k): the gradient of p[k] */
+template <typename GRAD>
+__device__ __forceinline__ float end_simplex_f(const uint8_t *__restrict__ p, const GRAD &G, const EndCell &e, float g2) {
+    const int i1 = e.x0 > e.y0 ? 1 : 0, j1 = 1 - i1;
+    const float xs[3] = {e.x0, e.x0 - (float)i1 + g2, e.x0 - 1.0f + 2.0f * g2};
+    const float ys[3] = {e.y0, e.y0 - (float)j1 + g2, e.y0 - 1.0f + 2.0f * g2};
+    const int ii = e.i & 255, jj = e.j & 255;
+    const float2 gs[3] = {G((ii + p[jj]) & 255), G((ii + i1 + p[(jj + j1) & 255]) & 255), G((ii + 1 + p[(jj + 1) & 255]) & 255)};
     float n = 0.0f;
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-        float tt = 0.5f - xs[c] * xs[c] - ys[c] * ys[c];
-        if (tt > 0.0f) {
-            tt *= tt;
-            n += tt * tt * gdot<float>(gs[c], xs[c], ys[c], 0.0f);
-        }
+        float tt = fmaxf(0.5f - xs[c] * xs[c] - ys[c] * ys[c], 0.0f);
+        tt *= tt;
+        n += tt * tt * (gs[c].x * xs[c] + gs[c].y * ys[c]);
     }
-    n *= 70.0f;
-    if (n < -0.9f - (END_ISLAND_E + 1e-4f)) return true; /* nv < -0.9f - ulp: an island in both branches */
-    if (n >= -0.9f + (END_ISLAND_E + 1e-4f)) return false; /* nv > -0.9f: none */
-    const double nv = simplex2(p, xin, yin, F2, G2);
+    return n * 70.0f;
+}
+template <typename GRAD>
+__device__ __forceinline__ bool end_island_g(const uint8_t *__restrict__ p, const GRAD &G, long long tx, long long tz, double F2, double G2,
+                                             bool fm) {
+    EndCell e;
+    if (tx > -END_FAR && tx < END_FAR && tz > -END_FAR && tz < END_FAR) {
+        e = end_cell((int)tx, (int)tz, G2);
+    } else {
+        const double xin = (double)tx, yin = (double)tz, s = (xin + yin) * F2;
+        e.i = ifloor(xin + s);
+        e.j = ifloor(yin + s);
+        const double t = (double)(e.i + e.j) * G2;
+        e.x0 = (float)(xin - ((double)e.i - t));
+        e.y0 = (float)(yin - ((double)e.j - t));
+    }
+    const float n = end_simplex_f(p, G, e, (float)G2);
+    if (fabsf(n + 0.9f) > END_ISLAND_E + 1e-4f) return n < -0.9f;
+    const double nv = simplex2(p, (double)tx, (double)tz, F2, G2);
     return fm ? ((float)nv < -0.9f) : (nv < (double)-0.9f);
+}
+__device__ __forceinline__ bool end_island(const uint8_t *__restrict__ p, long long tx, long long tz, double F2, double G2, bool fm) {
+    return end_island_g(p, [&](int k) { return end_grad(p[k]); }, tx, tz, F2, G2, fm);
+}
+/* (float)sqrt((double)v): rounding the double root to float is the float root correctly rounded, since a double has more than
+ * twice a float's bits plus two; the double root costs 20 operations of the FP64 pipe */
+__device__ __forceinline__ float end_sqrt(float v) { return __fsqrt_rn(v); }
+/* island size fmod(|x| 3439 + |z| 147, 13) + 9: the sum is a whole number (its parts are, rounded or not), below 2^32 within
+ * 1.2 million chunk cells */
+__device__ __forceinline__ float end_size(float tx, float tz) {
+    const float a = fabsf(tx) * 3439.0f + fabsf(tz) * 147.0f;
+    if (a < 4294967040.0f) return (float)((uint32_t)a % 13u) + 9.0f;
+    return fmodf(a, 13.0f) + 9.0f;
 }
 __device__ __forceinline__ float clampf(float v, float lo, float hi) { return v < lo ? lo : (v < hi ? v : hi); }
 /* EndIslandDensityFunction.getHeightValue at (sx, sz) = (block / 8); rad: half-width of the island window in
@@ -437,17 +488,17 @@ inline __device__ float end_height(const uint8_t *__restrict__ p, bool fm, int s
     float best;
     if (!fm) {
         int32_t sq = (int32_t)((uint32_t)sx * (uint32_t)sx + (uint32_t)sz * (uint32_t)sz); /* Java int overflow */
-        float len = (float)sqrt((double)(float)sq);
+        float len = end_sqrt((float)sq);
         best = clampf(100.0f - len * 8.0f, -100.0f, 80.0f);
     } else best = -100.0f;
     for (int dx = -rad; dx <= rad; dx++)
         for (int dz = -rad; dz <= rad; dz++) {
             long long tx = (long long)cx + dx, tz = (long long)cz + dz;
             if (tx * tx + tz * tz <= 4096LL) continue;
-            if (!end_island(p, (double)tx, (double)tz, F2, G2, fm)) continue;
-            float size = fmodf(fabsf((float)tx) * 3439.0f + fabsf((float)tz) * 147.0f, 13.0f) + 9.0f;
+            if (!end_island(p, tx, tz, F2, G2, fm)) continue;
+            float size = end_size((float)tx, (float)tz);
             float xd = (float)(ox - dx * 2), zd = (float)(oz - dz * 2);
-            float h = clampf(100.0f - (float)sqrt((double)(xd * xd + zd * zd)) * size, -100.0f, 80.0f);
+            float h = clampf(100.0f - end_sqrt(xd * xd + zd * zd) * size, -100.0f, 80.0f);
             best = best > h ? best : h;
         }
     return best;
@@ -462,7 +513,7 @@ inline __device__ int end_chunk_class(const uint8_t *__restrict__ p, bool fm, in
     if (!fm) e = ((double)h - 8.0) / 128.0;
     else {
         float dx = (float)(0 - bx), dz = (float)(0 - bz);
-        float len = (float)sqrt((double)(dx * dx + 0.0f * 0.0f + dz * dz));
+        float len = end_sqrt(dx * dx + 0.0f * 0.0f + dz * dz);
         float c = (clampf(100.0f - len, -100.0f, 80.0f) - 8.0f) * 0.0078125f;
         float o = (h - 8.0f) / 128.0f;
         e = (double)(c > o ? c : o);

@@ -364,28 +364,35 @@ __global__ void __launch_bounds__(128) k_block_points(const __grid_constant__ Mg
         if ((threadIdx.x & 31) == 0) out[i] = (uint8_t)b;
     }
 }
-/* End class of chunks [cx0, cx0+ncx) x [cz0, cz0+ncz) */
+/* End class of chunks [cx0, cx0+ncx) x [cz0, cz0+ncz): one w x h-chunk tile per block (endtile.cuh) */
 template <bool FM>
 __global__ void __launch_bounds__(128) k_end_chunks(const MgLattice *__restrict__ state, int cx0, int cz0, int ncx,
-                                                    int ncz, uint8_t *__restrict__ cls, double F2, double G2) {
-    /* one 8 x 8-chunk tile per block (endtile.cuh) */
+                                                    int ncz, int w, int h, uint8_t *__restrict__ cls, double F2, double G2) {
     __shared__ uint8_t p[256];
     __shared__ EndTile tile;
     for (int i = threadIdx.x; i < 256; i += blockDim.x) p[i] = state->p[i];
+    end_tile_grad(state->p, tile);
     __syncthreads();
-    const int tw = (ncx + END_TC - 1) / END_TC;
-    const int tx0 = cx0 + (int)(blockIdx.x % tw) * END_TC, tz0 = cz0 + (int)(blockIdx.x / tw) * END_TC;
-    end_tile_classes<FM>(p, F2, G2, tx0, tz0, tile);
-    if (threadIdx.x < END_TC * END_TC) {
-        const int cx = tx0 + threadIdx.x % END_TC, cz = tz0 + threadIdx.x / END_TC;
-        if (cx < cx0 + ncx && cz < cz0 + ncz) cls[(size_t)(cz - cz0) * ncx + (cx - cx0)] = tile.cls[threadIdx.x];
+    const int tw = (ncx + w - 1) / w;
+    const int tx0 = cx0 + (int)(blockIdx.x % tw) * w, tz0 = cz0 + (int)(blockIdx.x / tw) * h;
+    end_tile_classes<FM>(p, F2, G2, tx0, tz0, w, h, tile);
+    for (int i = threadIdx.x; i < w * h; i += blockDim.x) {
+        const int cx = tx0 + i % w, cz = tz0 + i / w;
+        if (cx < cx0 + ncx && cz < cz0 + ncz) cls[(size_t)(cz - cz0) * ncx + (cx - cx0)] = tile.cls[i];
     }
 }
 
 /* ============================================================================ host launchers */
 static inline unsigned blocks_for(long long n, int nt) { return (unsigned)((n + nt - 1) / nt); }
-static unsigned end_tiles(int ncx, int ncz) {
-    return (unsigned)(((long long)(ncx + END_TC - 1) / END_TC) * ((ncz + END_TC - 1) / END_TC));
+/* one grid's classes: large tiles (fewer window cells a chunk) once they fill the chip, else tiles of 8 x 8 */
+static void end_chunks(const MgWorldDesc &W, const MgLattice *state, int cx0, int cz0, int ncx, int ncz, uint8_t *cls, cudaStream_t st) {
+    const int cap = (long long)ncx * ncz >= 152LL * END_TC * END_TC ? END_TC : 8;
+    const int w = end_tile_side(ncx, cap), h = end_tile_side(ncz, cap);
+    const unsigned tiles = (unsigned)((long long)((ncx + w - 1) / w) * ((ncz + h - 1) / h));
+    ProfScope ps_(K_END_CHUNKS, st);
+    if (W.fmode) k_end_chunks<true><<<tiles, 128, 0, st>>>(state, cx0, cz0, ncx, ncz, w, h, cls, W.end_f2, W.end_g2);
+    else k_end_chunks<false><<<tiles, 128, 0, st>>>(state, cx0, cz0, ncx, ncz, w, h, cls, W.end_f2, W.end_g2);
+    count_launch();
 }
 static size_t grid_smem(const MgWorldDesc &W) { return sizeof(MgSpline) + (size_t)W.ntables * sizeof(MgLattice); }
 /* k_grid's: the Overworld adds its tiles' shift table */
@@ -524,9 +531,7 @@ int launch_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const Mg
         int cx1 = ((qx0 + nx - 1) * 4) >> 4, cz1 = ((qz0 + nz - 1) * 4) >> 4;
         int ncx = cx1 - cx0 + 1, ncz = cz1 - cz0 + 1;
         uint8_t *cls = (uint8_t *)scratch;
-        if (W.fmode) { ProfScope ps_(K_END_CHUNKS, st); k_end_chunks<true><<<end_tiles(ncx, ncz), 128, 0, st>>>(state, cx0, cz0, ncx, ncz, cls, W.end_f2, W.end_g2); }
-        else { ProfScope ps_(K_END_CHUNKS, st); k_end_chunks<false><<<end_tiles(ncx, ncz), 128, 0, st>>>(state, cx0, cz0, ncx, ncz, cls, W.end_f2, W.end_g2); }
-        count_launch();
+        end_chunks(W, state, cx0, cz0, ncx, ncz, cls, st);
         return launch_end_lookup(W, cls, cx0, cz0, ncx, qx0, qz0, nx, nz, out, st);
     }
     const bool chain = chain_rule(rule);
@@ -574,7 +579,9 @@ static void blockgrid_t(const MgWorldDesc &W, const MgTreeNode *tree, const MgLa
     size_t sm = DIM == MG_END ? 0 : grid_smem(W);
     ProfScope ps_(K_BLOCKGRID, st);
     if constexpr (DIM != MG_END) {
-        if (xyz) {
+        /* the Nether's cells are cheap enough for a thread each once there are enough of them (26.1: 3,000 points 19.8 us by warps,
+         * 22.0 by threads; 14,108 points 67.6 and 30.5) */
+        if (xyz && (DIM == MG_OVERWORLD || nx <= 3072)) {
             const long long nb = ((long long)nx + 3) / 4;
             k_block_points<FM, DIM><<<(unsigned)(nb < 16 * 152 ? nb : 16 * 152), 128, sizeof(WcStage), st>>>(W, tree, state, zseed, xyz, nx,
                                                                                                           out);
@@ -603,9 +610,7 @@ int launch_block_biomes(const MgWorldDesc &W, const MgWorldDesc *d_world, const 
         return launch_ow_block_grid(W, d_world, tree, state, zseed, x0, z0, nx, nz, step, y, out, scratch, st);
     uint8_t *cls = (uint8_t *)scratch; /* End chunk classes, or null: evaluate per sample */
     if (W.dim == MG_END && cls) {
-        if (W.fmode) { ProfScope ps_(K_END_CHUNKS, st); k_end_chunks<true><<<end_tiles(encx, encz), 128, 0, st>>>(state, ecx0, ecz0, encx, encz, cls, W.end_f2, W.end_g2); }
-        else { ProfScope ps_(K_END_CHUNKS, st); k_end_chunks<false><<<end_tiles(encx, encz), 128, 0, st>>>(state, ecx0, ecz0, encx, encz, cls, W.end_f2, W.end_g2); }
-        count_launch();
+        end_chunks(W, state, ecx0, ecz0, encx, encz, cls, st);
     }
     if (W.fmode) {
         if (W.dim == MG_OVERWORLD) blockgrid_t<true, MG_OVERWORLD>(W, tree, state, zseed, x0, z0, nx, nz, step, y, xyz, out, cls, ecx0, ecz0, encx, st);

@@ -187,12 +187,12 @@ __device__ __forceinline__ bool end_accept(const MgWorldDesc &W, const uint8_t *
     float cdist = 0.0f;
     if (!FM) {
         int32_t sq = (int32_t)((uint32_t)sx * (uint32_t)sx + (uint32_t)sz * (uint32_t)sz);
-        float len = (float)sqrt((double)(float)sq);
+        float len = end_sqrt((float)sq);
         best = clampf(100.0f - len * 8.0f, -100.0f, 80.0f);
     } else {
         best = -100.0f;
         const float ddx = (float)(0 - bx), ddz = (float)(0 - bz);
-        const float len = (float)sqrt((double)(ddx * ddx + 0.0f * 0.0f + ddz * ddz));
+        const float len = end_sqrt(ddx * ddx + 0.0f * 0.0f + ddz * ddz);
         cdist = (clampf(100.0f - len, -100.0f, 80.0f) - 8.0f) * 0.0078125f;
     }
     auto rank_now = [&]() {
@@ -212,10 +212,10 @@ __device__ __forceinline__ bool end_accept(const MgWorldDesc &W, const uint8_t *
         if (dx < -rad || dx > rad || dz < -rad || dz > rad) continue;
         const long long tx = (long long)ccx + dx, tz = (long long)ccz + dz;
         if (tx * tx + tz * tz <= 4096LL) continue;
-        if (!end_island(p, (double)tx, (double)tz, W.end_f2, W.end_g2, FM)) continue;
-        const float size = fmodf(fabsf((float)tx) * 3439.0f + fabsf((float)tz) * 147.0f, 13.0f) + 9.0f;
+        if (!end_island(p, tx, tz, W.end_f2, W.end_g2, FM)) continue;
+        const float size = end_size((float)tx, (float)tz);
         const float xd = (float)(ox - dx * 2), zd = (float)(oz - dz * 2);
-        const float h = clampf(100.0f - (float)sqrt((double)(xd * xd + zd * zd)) * size, -100.0f, 80.0f);
+        const float h = clampf(100.0f - end_sqrt(xd * xd + zd * zd) * size, -100.0f, 80.0f);
         best = best > h ? best : h;
     }
     return in[rank_now()];

@@ -399,30 +399,12 @@ __global__ void __launch_bounds__(128) k_check_end(long long n, uint64_t seed, d
             const bool fm = (r >> 4) & 1;
             const double nv = mg::simplex2(perm, x, z, F2, G2);
             const bool exact = fm ? ((float)nv < -0.9f) : (nv < (double)-0.9f);
-            bad += mg::end_island(perm, x, z, F2, G2, fm) != exact;
+            bad += mg::end_island(perm, (long long)x, (long long)z, F2, G2, fm) != exact;
             /* the float evaluation alone, as end_island forms it, for the bound */
-            const double s = (x + z) * F2;
-            const int ci = mgd::ifloor(x + s), cj = mgd::ifloor(z + s);
-            const double t = (double)(ci + cj) * G2;
-            const double x0 = x - ((double)ci - t), y0 = z - ((double)cj - t);
-            const int i1 = x0 > y0 ? 1 : 0, j1 = 1 - i1;
-            const float g2 = (float)G2, xf = (float)x0, yf = (float)y0;
-            const float xs[3] = {xf, xf - (float)i1 + g2, xf - 1.0f + 2.0f * g2};
-            const float ys[3] = {yf, yf - (float)j1 + g2, yf - 1.0f + 2.0f * g2};
-            const int ii = ci & 255, jj = cj & 255;
-            const int gs[3] = {perm[(ii + perm[jj]) & 255] % 12, perm[(ii + i1 + perm[(jj + j1) & 255]) & 255] % 12,
-                               perm[(ii + 1 + perm[(jj + 1) & 255]) & 255] % 12};
-            float nf = 0.0f;
-            for (int c = 0; c < 3; c++) {
-                float tt = 0.5f - xs[c] * xs[c] - ys[c] * ys[c];
-                if (tt > 0.0f) {
-                    tt *= tt;
-                    nf += tt * tt * mgd::gdot<float>(gs[c], xs[c], ys[c], 0.0f);
-                }
-            }
-            nf *= 70.0f;
+            if (x <= -END_FAR || z <= -END_FAR) continue;
+            const float nf = mg::end_simplex_f(perm, [&](int k) { return mg::end_grad(perm[k]); }, mg::end_cell((int)x, (int)z, G2), (float)G2);
             worst = fmax(worst, fabs((double)nf - nv) / (double)END_ISLAND_E);
-            left += !(nf < -0.9f - (END_ISLAND_E + 1e-4f) || nf >= -0.9f + (END_ISLAND_E + 1e-4f));
+            left += fabsf(nf + 0.9f) <= END_ISLAND_E + 1e-4f;
         }
     }
     atomicAdd(&out[0], bad);

@@ -62,3 +62,24 @@ def test_search_stages(version, preset):
             got = w.search(mg.make_obs(r, block), kind=mg.SEEDS_RANGE, base=base, n=n)
             exp = ow.search(O.make_obs(r, block), kind=O.SEEDS_RANGE, base=base, n=n)
             assert np.array_equal(got[0], exp[0]) and np.array_equal(got[1], exp[1]), (block, got[1], exp[1])
+
+
+@pytest.mark.parametrize("version", ["26.1", "26.3"])
+def test_end_tiles(version):
+    """End grids of every tile shape: one chunk, sides around a tile's 24 chunks and their equal parts, corners inside a chunk, at the
+    central disc, at the world border and beyond the fixed-point skew's range; batched and alone."""
+    mg = ge.package()
+    mg.load()
+    if mg.device_count() < 1:
+        pytest.fail("no CUDA device")
+    seed = 7126353871628162251
+    w = mg.Generator.open(ge.data_root(), version).world("minecraft:the_end", "normal", seed)
+    ow = O.World(ge.data_root(), version, "the_end", "normal")
+    shapes = [(1, 1), (3, 97), (96, 97), (101, 5), (200, 130)]
+    corners = [(0, 0), (-257, 250), (1001, -3002), (7499990, -7499990), (4 * (1 << 21) - 60, 77), (-20000003, 30000001)]
+    reqs = [(w, seed, x - nx // 2, z - nz // 2, nx, nz, 16) for x, z in corners for nx, nz in shapes]
+    plan = mg.Plan(reqs)
+    for r, got in zip(reqs, plan.split(plan.run())):
+        exp = ow.quart_grid(*r[1:], O.TIE_ENGINE)
+        assert np.array_equal(got, exp), r[1:]
+        assert np.array_equal(w.quart_grid(*r[2:]), exp), r[1:]
