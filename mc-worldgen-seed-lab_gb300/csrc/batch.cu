@@ -25,6 +25,8 @@
 #include "climate.cuh"
 #include "endtile.cuh"
 #include "launch.h"
+#include "legacy.cuh"
+#include "nethertile.cuh"
 #include "prof.h"
 
 namespace mg {
@@ -33,13 +35,6 @@ namespace mg {
 
 /* ---------------------------------------------------------------- setup of a list of (world, seed) */
 #define LNT 128
-__device__ __forceinline__ void lst_swap(uint8_t *mine, int i, int j) {
-    uint8_t *a = mine + (i >> 2) * (4 * LNT) + (i & 3);
-    uint8_t *b = mine + (j >> 2) * (4 * LNT) + (j & 3);
-    uint8_t x = *a, y = *b;
-    *a = y;
-    *b = x;
-}
 __device__ __forceinline__ void lst_store(uint32_t (*perm)[LNT], int t, MgLattice &h, MgLattice *L, bool dbl) {
     lattice_header(h, dbl);
     const uint4 *src = reinterpret_cast<const uint4 *>(&h);
@@ -83,50 +78,27 @@ __global__ void __launch_bounds__(LNT) k_setup_list_xo(const MgWorldDesc *__rest
     xo_shuffle<LNT>(mine, x);
     lst_store(perm, t, h, pool + E.slot + j, !W.fmode);
 }
-/* Nether entries: one thread per (entry, noise); End entries: one thread per entry. */
-__device__ __forceinline__ void lst_legacy(uint64_t &s, uint32_t (*perm)[LNT], int t, MgLattice *L, bool dbl) {
-    MgLattice h;
-    h.ox = lcg_double(s) * 256.0;
-    h.oy = lcg_double(s) * 256.0;
-    h.oz = lcg_double(s) * 256.0;
-    for (int w = 0; w < 64; w++) perm[w][t] = 0x03020100u + 0x04040404u * (uint32_t)w;
-    uint8_t *mine = reinterpret_cast<uint8_t *>(&perm[0][t]);
-    for (int q = 0; q < 256; q++) lst_swap(mine, q, q + lcg_int(s, 256 - q));
-    if (L) lst_store(perm, t, h, L, dbl);
-}
-__global__ void __launch_bounds__(LNT) k_setup_list_legacy(const MgWorldDesc *__restrict__ worlds,
-                                                           const MgSetupEntry *__restrict__ ent, int n,
+/* Nether entries: LEGACY_GROUP threads per (entry, noise); End entries: one thread per entry. */
+__global__ void __launch_bounds__(LNT) k_setup_list_legacy(const MgWorldDesc *__restrict__ worlds, const MgSetupEntry *__restrict__ ent, int n,
                                                            MgLattice *__restrict__ pool) {
     __shared__ uint32_t perm[64][LNT];
     const int t = threadIdx.x;
-    const long long g = (long long)blockIdx.x * LNT + t;
+    const long long g = ((long long)blockIdx.x * LNT + t) / LEGACY_GROUP;
     if (g >= 2LL * n) return;
     const MgSetupEntry &E = ent[g >> 1];
     const MgWorldDesc &W = worlds[E.world];
-    const int nz = (int)(g & 1);
-    const MgNoise &N = W.nether[nz];
-    uint64_t st = lcg_init((int64_t)((uint64_t)E.seed + (uint64_t)nz));
+    const MgNoise &N = W.nether[g & 1];
     MgLattice *T = pool + E.slot + N.base;
-    int slot[MG_MAX_OCT];
-    for (int q = 0; q < MG_MAX_OCT; q++) slot[q] = -1;
-    for (int k = 0; k < N.nlev; k++) slot[N.idx[k]] = k;
-    const int zero = -N.first;
-    for (int stack = 0; stack < 2; stack++) {
-        MgLattice *S = T + stack * N.nlev;
-        const bool keep_zero = zero >= 0 && zero < N.octs && slot[zero] >= 0;
-        lst_legacy(st, perm, t, keep_zero ? S + slot[zero] : nullptr, !W.fmode);
-        for (int q = zero - 1; q >= 0; q--) {
-            if (q < N.octs && slot[q] >= 0) lst_legacy(st, perm, t, S + slot[q], !W.fmode);
-            else st = lcg_jump(st, 262);
-        }
-    }
+    legacy_noise<LNT>(N, (int)(g & 1), E.seed, &perm[0][t], [&](int i, MgLattice &h) { lst_store(perm, t, h, T + i, !W.fmode); });
 }
 __global__ void __launch_bounds__(LNT) k_setup_list_end(const MgSetupEntry *__restrict__ ent, int n, MgLattice *__restrict__ pool) {
     __shared__ uint32_t perm[64][LNT];
-    const long long g = (long long)blockIdx.x * LNT + threadIdx.x;
+    const int t = threadIdx.x;
+    const long long g = (long long)blockIdx.x * LNT + t;
     if (g >= n) return;
-    uint64_t st = lcg_jump(lcg_init(ent[g].seed), 17292);
-    lst_legacy(st, perm, threadIdx.x, pool + ent[g].slot, false); /* the End reads the permutation only */
+    MgLattice h;
+    legacy_end<LNT>(ent[g].seed, &perm[0][t], h);
+    lst_store(perm, t, h, pool + ent[g].slot, false); /* the End reads the permutation only */
 }
 
 /* ---------------------------------------------------------------- the persistent batch kernel */
@@ -140,6 +112,7 @@ struct BatchSmem {
     union {
         MgLattice lat[MG_MAX_TABLES];
         BatchEnd end;
+        NetherTile nether;
     };
     int tile, req, state;
 };
@@ -214,6 +187,8 @@ __global__ void __launch_bounds__(BNT, MINB) k_batch(const MgWorldDesc *__restri
             if (W.dim == MG_END) {
                 for (int i = threadIdx.x; i < 256; i += BNT) sm.end.endp[i] = pool[R.state].p[i];
                 end_tile_grad(pool[R.state].p, sm.end.tile);
+            } else if (nether_tile_supported(W)) {
+                nether_stage(W, pool + R.state, trees[R.world], sm.nether);
             } else {
                 const uint4 *a = reinterpret_cast<const uint4 *>(pool + R.state);
                 uint4 *b = reinterpret_cast<uint4 *>(sm.lat);
@@ -226,6 +201,12 @@ __global__ void __launch_bounds__(BNT, MINB) k_batch(const MgWorldDesc *__restri
         if (W.dim == MG_END) {
             if (W.fmode) batch_end<true>(W, sm, R, tile, out);
             else batch_end<false>(W, sm, R, tile, out);
+            continue;
+        }
+        if (nether_tile_supported(W)) {
+            const int tw = (R.nx + NT_W - 1) / NT_W;
+            if (W.fmode) nether_tile<true>(W, sm.nether, trees[R.world], R, tile % tw * NT_W, tile / tw * NT_W, out);
+            else nether_tile<false>(W, sm.nether, trees[R.world], R, tile % tw * NT_W, tile / tw * NT_W, out);
             continue;
         }
         constexpr int TILE_H = BNT / TILE_W;
@@ -254,13 +235,14 @@ int batch_group(const MgWorldDesc &W, int tie) {
     return W.fmode ? BATCH_OW_F : BATCH_OW_D;
 }
 
-long long batch_tiles(int group, int dim, int qx0, int qz0, int nx, int nz, int shape) {
+long long batch_tiles(int group, const MgWorldDesc &W, int qx0, int qz0, int nx, int nz, int shape) {
     if (group != BATCH_REST) return ow_tiles(nx, nz);
-    if (dim == MG_END) {
+    if (W.dim == MG_END) {
         const long long ncx = ((qx0 + nx - 1) >> 2) - (qx0 >> 2) + 1, ncz = ((qz0 + nz - 1) >> 2) - (qz0 >> 2) + 1;
         const int w = end_tile_side((int)ncx, END_TC), h = end_tile_side((int)ncz, END_TC);
         return ((ncx + w - 1) / w) * ((ncz + h - 1) / h);
     }
+    if (nether_tile_supported(W)) return (long long)((nx + NT_W - 1) / NT_W) * ((nz + NT_W - 1) / NT_W);
     const int tw = kBatchTileWidths[shape], th = BNT / tw;
     return (long long)((nx + tw - 1) / tw) * ((nz + th - 1) / th);
 }
@@ -273,7 +255,7 @@ int launch_setup_list(const MgWorldDesc *d_worlds, int dim, const MgSetupEntry *
         k_setup_list_xo<<<(unsigned)((total_lattices + LNT - 1) / LNT), LNT, 0, st>>>(d_worlds, d_ent, n, d_first, total_lattices, d_pool);
     } else if (dim == MG_NETHER) {
         ProfScope ps_(K_SETUP_LEGACY, st);
-        k_setup_list_legacy<<<(unsigned)((2LL * n + LNT - 1) / LNT), LNT, 0, st>>>(d_worlds, d_ent, n, d_pool);
+        k_setup_list_legacy<<<(unsigned)((2LL * LEGACY_GROUP * n + LNT - 1) / LNT), LNT, 0, st>>>(d_worlds, d_ent, n, d_pool);
     } else {
         ProfScope ps_(K_SETUP_END, st);
         k_setup_list_end<<<(unsigned)((n + LNT - 1) / LNT), LNT, 0, st>>>(d_ent, n, d_pool);

@@ -53,7 +53,7 @@ int launch_ow_batch(bool fm, int tie, bool open_pass, const MgWorldDesc *d_world
 extern const int kBatchTileWidths[BATCH_SHAPES];
 /* tiles of a request of group `group`: 16 x 16 cells (owtile.cu); in the rest, 128 quart cells of shape `shape`
  * (Overworld, Nether) or 8 x 8 chunks (End) */
-long long batch_tiles(int group, int dim, int qx0, int qz0, int nx, int nz, int shape);
+long long batch_tiles(int group, const MgWorldDesc &W, int qx0, int qz0, int nx, int nz, int shape);
 /* lattices of a list of entries of one dimension; Overworld needs the prefix sums of lattices per entry */
 int launch_setup_list(const MgWorldDesc *d_worlds, int dim, const MgSetupEntry *d_ent, int n, const int *d_first,
                       long long total_lattices, MgLattice *d_pool, cudaStream_t st);

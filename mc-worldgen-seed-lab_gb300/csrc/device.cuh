@@ -131,13 +131,35 @@ __device__ __forceinline__ int32_t mod_small(int32_t u, int32_t d) {
     const uint32_t q = __umulhi((uint32_t)u, kDivMagic.m[d]) >> kDivMagic.sh[d];
     return u - (int32_t)q * d;
 }
-/* java.util.Random.nextInt(bound) for 1 <= bound <= 256 (the permutation shuffles) */
-__device__ __forceinline__ int lcg_int(uint64_t &s, int32_t bound) {
-    if ((bound & -bound) == bound) return (int)(((int64_t)bound * (int64_t)lcg_bits(s, 31)) >> 31);
-    for (;;) {
-        int32_t b = lcg_bits(s, 31), v = mod_small(b, bound);
-        if ((int32_t)((uint32_t)b - (uint32_t)v + (uint32_t)(bound - 1)) >= 0) return v;
+/* the 256-step shuffle of a column (xo_shuffle's layout, identity at the start) by java.util.Random.nextInt(256 - q); returns the draws it
+ * rejected */
+template <int ROW>
+__device__ __forceinline__ int lcg_shuffle(uint8_t *mine, uint64_t &s) {
+    int rejected = 0;
+#pragma unroll 1
+    for (int qw = 0; qw < 64; qw++) {
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const int bound = 256 - (4 * qw + r);
+            uint32_t b = (uint32_t)lcg_bits(s, 31), v;
+            if ((bound & -bound) == bound) { /* the same for every lane */
+                v = __umulhi(b << 1, (uint32_t)bound);
+            } else {
+                v = (uint32_t)mod_small((int32_t)b, bound);
+                while ((int32_t)(b - v + (uint32_t)(bound - 1)) < 0) { /* 3e-8 a draw */
+                    b = (uint32_t)lcg_bits(s, 31);
+                    v = (uint32_t)mod_small((int32_t)b, bound);
+                    rejected++;
+                }
+            }
+            const uint32_t k = (uint32_t)(4 * qw + r) + v;
+            uint8_t *pa = mine + qw * (4 * ROW) + r, *pb = mine + (k + (k >> 2) * (4 * ROW - 4));
+            const uint8_t va = *pa, vb = *pb;
+            *pa = vb;
+            *pb = va;
+        }
     }
+    return rejected;
 }
 __device__ __forceinline__ double lcg_double(uint64_t &s) {
     int64_t hi = lcg_bits(s, 26), lo = lcg_bits(s, 27);

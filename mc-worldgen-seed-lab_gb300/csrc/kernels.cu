@@ -19,6 +19,7 @@
 #include "endtile.cuh"
 #include "device.cuh"
 #include "launch.h"
+#include "legacy.cuh"
 #include "batch.h"
 #include "prof.h"
 #include "warpcell.cuh"
@@ -44,13 +45,6 @@ void count_launch_external() { count_launch(); }
  * thread hits bank t % 32 whatever i is: the 32 lanes of a warp never conflict. */
 __device__ __forceinline__ void perm_identity(uint32_t (*perm)[SETUP_NT], int t) {
     for (int w = 0; w < 64; w++) perm[w][t] = 0x03020100u + 0x04040404u * (uint32_t)w;
-}
-__device__ __forceinline__ void perm_swap(uint8_t *base, int t, int i, int j) {
-    uint8_t *a = base + (((i >> 2) * SETUP_NT + t) << 2) + (i & 3);
-    uint8_t *b = base + (((j >> 2) * SETUP_NT + t) << 2) + (j & 3);
-    uint8_t x = *a, y = *b;
-    *a = y;
-    *b = x;
 }
 __device__ __forceinline__ void perm_store(uint32_t (*perm)[SETUP_NT], int t, MgLattice *L) {
     uint4 *dst = reinterpret_cast<uint4 *>(L->p);
@@ -96,55 +90,29 @@ __global__ void __launch_bounds__(SETUP_NT) k_setup_xo(const __grid_constant__ M
     perm_store(perm, t, L);
 }
 
-/* one legacy lattice from the LCG into the thread's shuffle slot, then to `L` (if non-null) */
-__device__ __forceinline__ void legacy_lattice(uint64_t &s, uint32_t (*perm)[SETUP_NT], int t, MgLattice *L, bool dbl) {
-    MgLattice h;
-    h.ox = lcg_double(s) * 256.0;
-    h.oy = lcg_double(s) * 256.0;
-    h.oz = lcg_double(s) * 256.0;
-    perm_identity(perm, t);
-    uint8_t *base = reinterpret_cast<uint8_t *>(&perm[0][0]);
-    for (int q = 0; q < 256; q++) perm_swap(base, t, q, q + lcg_int(s, 256 - q));
-    if (L) {
-        header_store(h, L, dbl);
-        perm_store(perm, t, L);
-    }
-}
-/* Nether biome noises: temperature from LCG(seed), vegetation from LCG(seed + 1); each stack builds the
- * zero octave first, then octaves zero-1 .. 0, skipping 262 draws for an absent one
- * (engine/mc_noise.h:266-282, engine/cuda/mcg_host.c:49-51). */
+/* Nether biome noises: temperature from LCG(seed), vegetation from LCG(seed + 1); LEGACY_GROUP threads per (seed, noise) */
 __global__ void __launch_bounds__(SETUP_NT) k_setup_legacy(const __grid_constant__ MgWorldDesc W, const int64_t *__restrict__ seeds,
                                                            int ns, MgLattice *__restrict__ out) {
     __shared__ uint32_t perm[64][SETUP_NT];
     const int t = threadIdx.x;
-    const long long g = (long long)blockIdx.x * SETUP_NT + t;
+    const long long g = ((long long)blockIdx.x * SETUP_NT + t) / LEGACY_GROUP;
     if (g >= 2LL * ns) return;
-    const int s = (int)(g >> 1), n = (int)(g & 1);
-    const MgNoise &N = W.nether[n];
-    uint64_t st = lcg_init((int64_t)((uint64_t)seeds[s] + (uint64_t)n));
-    MgLattice *T = out + (size_t)s * W.ntables + N.base;
-    int slot[MG_MAX_OCT];
-    for (int q = 0; q < MG_MAX_OCT; q++) slot[q] = -1;
-    for (int k = 0; k < N.nlev; k++) slot[N.idx[k]] = k;
-    const int zero = -N.first;
-    for (int stack = 0; stack < 2; stack++) {
-        MgLattice *S = T + stack * N.nlev;
-        bool keep_zero = zero >= 0 && zero < N.octs && slot[zero] >= 0;
-        legacy_lattice(st, perm, t, keep_zero ? S + slot[zero] : nullptr, !W.fmode);
-        for (int q = zero - 1; q >= 0; q--) {
-            if (q < N.octs && slot[q] >= 0) legacy_lattice(st, perm, t, S + slot[q], !W.fmode);
-            else st = lcg_jump(st, 262);
-        }
-    }
+    const MgNoise &N = W.nether[g & 1];
+    MgLattice *T = out + (size_t)(g >> 1) * W.ntables + N.base;
+    legacy_noise<SETUP_NT>(N, (int)(g & 1), seeds[g >> 1], &perm[0][t], [&](int i, MgLattice &h) {
+        header_store(h, T + i, !W.fmode);
+        perm_store(perm, t, T + i);
+    });
 }
-/* End: LegacyRandomSource(seed).consumeCount(17292), then the simplex lattice (engine/mc_end.h:18-22) */
 __global__ void __launch_bounds__(SETUP_NT) k_setup_end(const int64_t *__restrict__ seeds, int ns, MgLattice *__restrict__ out) {
     __shared__ uint32_t perm[64][SETUP_NT];
     const int t = threadIdx.x;
     const long long g = (long long)blockIdx.x * SETUP_NT + t;
     if (g >= ns) return;
-    uint64_t st = lcg_jump(lcg_init(seeds[g]), 17292);
-    legacy_lattice(st, perm, t, out + g, false); /* the End reads the permutation only */
+    MgLattice h;
+    legacy_end<SETUP_NT>(seeds[g], &perm[0][t], h);
+    header_store(h, out + g, false); /* the End reads the permutation only */
+    perm_store(perm, t, out + g);
 }
 
 /* ============================================================================ sampling kernels */
@@ -406,7 +374,7 @@ int launch_setup(const MgWorldDesc &W, const int64_t *d_seeds, int ns, MgLattice
         long long n = (long long)ns * W.ntables;
         { ProfScope ps_(K_SETUP_XO, st); k_setup_xo<<<blocks_for(n, SETUP_NT), SETUP_NT, 0, st>>>(W, d_seeds, ns, d_states); }
     } else if (W.dim == MG_NETHER) {
-        { ProfScope ps_(K_SETUP_LEGACY, st); k_setup_legacy<<<blocks_for(2LL * ns, SETUP_NT), SETUP_NT, 0, st>>>(W, d_seeds, ns, d_states); }
+        { ProfScope ps_(K_SETUP_LEGACY, st); k_setup_legacy<<<blocks_for(2LL * LEGACY_GROUP * ns, SETUP_NT), SETUP_NT, 0, st>>>(W, d_seeds, ns, d_states); }
     } else {
         { ProfScope ps_(K_SETUP_END, st); k_setup_end<<<blocks_for(ns, SETUP_NT), SETUP_NT, 0, st>>>(d_seeds, ns, d_states); }
     }

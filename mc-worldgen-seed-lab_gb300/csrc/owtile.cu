@@ -391,10 +391,6 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const __grid_constant__ OtWor
 #define OT_CAP_D 896 /* edges a tile's table holds */
 #define OT_STACK_C ((int64_t)((MG_SECOND_STACK - 1.0) * 0x1.0p64)) /* exact */
 
-/* entry of the shift tables: fraction and smoothstep (units of 2^-31), edge index part */
-struct __align__(16) OtShiftD {
-    int32_t f, u, edge, pad;
-};
 struct OtSmemD {
     MgLattice lat[MG_MAX_TABLES];
     int4 ep[OT_CAP_D];

@@ -192,6 +192,10 @@ __device__ __forceinline__ OtFix ot_fix(double y, double v) {
     f.c1 = __double2int_rn((y - 1.0) * v * 0x1.0p30);
     return f;
 }
+/* entry of the shift tables: fraction and smoothstep (units of 2^-31), edge index part */
+struct __align__(16) OtShiftD {
+    int32_t f, u, edge, pad;
+};
 /* one climate octave in evaluation order; offsets in units of 2^-32, less the first node's cell */
 struct __align__(16) OtOctD {
     int64_t ox, oz;

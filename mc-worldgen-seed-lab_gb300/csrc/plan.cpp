@@ -240,7 +240,7 @@ MCGEN_API int mcgen_gb300_plan_new(const McGb300Request *reqs, int n, int tie_ru
             const int g = wgroup[(size_t)wi];
             b.tile0 = p->groups[s].tiles[g];
             b.out_off = p->out_off[(size_t)i];
-            p->groups[s].tiles[g] += mg::batch_tiles(g, worlds[(size_t)wi]->desc.dim, r.qx0, r.qz0, r.nx, r.nz, s);
+            p->groups[s].tiles[g] += mg::batch_tiles(g, worlds[(size_t)wi]->desc, r.qx0, r.qz0, r.nx, r.nz, s);
             p->groups[s].n[g]++;
             rq[s].push_back(b);
         }

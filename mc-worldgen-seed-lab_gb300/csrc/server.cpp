@@ -261,7 +261,7 @@ int launch_batch(McGb300Server *s, Batch &b) {
     for (auto &r : reqs) {
         const int g = wgroup[(size_t)r.world];
         r.tile0 = groups.tiles[g];
-        groups.tiles[g] += mg::batch_tiles(g, worlds[(size_t)r.world]->desc.dim, r.qx0, r.qz0, r.nx, r.nz, kServeShape);
+        groups.tiles[g] += mg::batch_tiles(g, worlds[(size_t)r.world]->desc, r.qx0, r.qz0, r.nx, r.nz, kServeShape);
         groups.n[g]++;
     }
     cudaError_t e = cudaSuccess;

@@ -304,6 +304,15 @@ static void tile_bounds(MgNoise *shift, MgNoise *s, int n) {
     }
 }
 
+/* the same of a Nether noise, whose coordinates are whole numbers: its octaves come from tables of splits, like the shift's */
+static void tile_bounds_nether(MgNoise *s) {
+    double c, cf;
+    level_sums(s, &c, &cf);
+    bool in = s->fix_err >= 0.0 && 2.0 * 1.06 * c < 3.95;
+    for (int k = 0; k < s->nlev; k++) in = in && s->c30[k] != 0;
+    s->tile_eq = s->tile_eq_far = in ? (int32_t)ceil(tile_noise(s, c, TILE_SHIFT_OCT) * 0x1.0p29) + 2 : -1;
+}
+
 /* PerlinNoise/NormalNoise constants of 26.1/26.2 (engine/mc_noise.h:178-196) */
 static void noise_double(MgNoise *s, const NoiseParams &P, int legacy) {
     memset(s, 0, sizeof *s);
@@ -845,7 +854,12 @@ int build_world(const char *root, int version, int dim, const char *preset, MgWo
         const NoiseParams *t = find("nether/temperature"), *v = find("nether/vegetation");
         if (!t || !v) { *err = "nether biome noises not found"; return MCGEN_E_DATA; }
         if (D->fmode) { noise_float(&D->nether[0], *t, 1); noise_float(&D->nether[1], *v, 1); }
-        else { noise_double(&D->nether[0], *t, 1); noise_double(&D->nether[1], *v, 1); }
+        else {
+            noise_double(&D->nether[0], *t, 1);
+            noise_double(&D->nether[1], *v, 1);
+            tile_bounds_nether(&D->nether[0]);
+            tile_bounds_nether(&D->nether[1]);
+        }
         D->nether[0].base = 0;
         D->nether[1].base = 2 * D->nether[0].nlev;
         nt = 2 * (D->nether[0].nlev + D->nether[1].nlev);

@@ -83,3 +83,18 @@ def test_end_tiles(version):
         exp = ow.quart_grid(*r[1:], O.TIE_ENGINE)
         assert np.array_equal(got, exp), r[1:]
         assert np.array_equal(w.quart_grid(*r[2:]), exp), r[1:]
+
+
+def test_nether_rejected_draws():
+    """About one seed in 12,000 rejects a draw in a shuffle of its Nether noises, which moves the octaves built after it."""
+    mg = ge.package()
+    mg.load()
+    if mg.device_count() < 1:
+        pytest.fail("no CUDA device")
+    w = mg.Generator.open(ge.data_root(), "26.3").world("minecraft:the_nether", "normal", 0)
+    ow = O.World(ge.data_root(), "26.3", "the_nether", "normal")
+    seeds = np.random.default_rng(2).integers(-2**63, 2**63 - 1, 120000)
+    pts = np.array([[137, 16, -911]], np.int32)
+    _, tg = w.seed_points(seeds, pts, want_targets=True)
+    _, et = ow.points(seeds, pts, want_targets=True)
+    assert np.array_equal(np.asarray(tg).reshape(-1, 6), np.asarray(et).reshape(-1, 6))
