@@ -142,14 +142,17 @@ __global__ void __launch_bounds__(128) k_points(const __grid_constant__ MgWorldD
         for (int i = threadIdx.x; i < (int)(sizeof(MgSpline) / 16); i += blockDim.x) d[i] = c[i];
         __syncthreads();
     }
-    const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (DIM == MG_END) g >>= 5; /* a warp per sample */
     if (g >= (long long)ns * np) return;
     const int s = (int)(g / np), p = (int)(g % np);
     const int qx = pts[3 * p], qy = pts[3 * p + 1], qz = pts[3 * p + 2];
     const MgLattice *T = states + (size_t)s * W.ntables;
     int32_t tg[6];
     if (DIM == MG_END) {
-        out[g] = (uint8_t)W.end_ids[end_chunk_class(T->p, FM, (qx * 4) >> 4, (qz * 4) >> 4, W.end_f2, W.end_g2)];
+        const int c = end_chunk_class(T->p, FM, (qx * 4) >> 4, (qz * 4) >> 4, W.end_f2, W.end_g2);
+        if (threadIdx.x & 31) return;
+        out[g] = (uint8_t)W.end_ids[c];
         if (targets)
             for (int k = 0; k < 6; k++) targets[g * 6 + k] = 0;
         return;
@@ -308,9 +311,7 @@ __global__ void __launch_bounds__(128, 6) k_blockgrid(const __grid_constant__ Mg
     zoom_cell(zseed, bxk, byk, bzk, cx, cy, cz);
     if (DIM == MG_END) {
         int chx = (cx * 4) >> 4, chz = (cz * 4) >> 4;
-        int c = end_cls ? end_cls[(size_t)(chz - ecz0) * encx + (chx - ecx0)]
-                        : end_chunk_class(state->p, FM, chx, chz, W.end_f2, W.end_g2);
-        out[g] = (uint8_t)W.end_ids[c];
+        out[g] = (uint8_t)W.end_ids[end_cls[(size_t)(chz - ecz0) * encx + (chx - ecx0)]];
         return;
     }
     out[g] = (uint8_t)cell_chunk<FM, DIM>(W, *S, T, tree, cx, cy, cz);
@@ -330,6 +331,22 @@ __global__ void __launch_bounds__(128) k_block_points(const __grid_constant__ Mg
         wc_zoom(zseed, xyz[3 * (size_t)i], xyz[3 * (size_t)i + 1], xyz[3 * (size_t)i + 2], cx, cy, cz);
         const int b = wc_cell_chunk<FM, DIM>(W, st.spline, st.lat, tree, cx, cy, cz);
         if ((threadIdx.x & 31) == 0) out[i] = (uint8_t)b;
+    }
+}
+/* sparse End samples (a grid, or nx points at xyz), whose chunks are not worth a table of classes: one per warp */
+template <bool FM>
+__global__ void __launch_bounds__(128) k_end_samples(const __grid_constant__ MgWorldDesc W, const MgLattice *__restrict__ state,
+                                                     int64_t zseed, int x0, int z0, int nx, long long n, int step, int y,
+                                                     const int32_t *__restrict__ xyz, uint8_t *__restrict__ out) {
+    __shared__ uint8_t p[256];
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) p[i] = state->p[i];
+    __syncthreads();
+    for (long long g = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < n; g += (long long)gridDim.x * blockDim.x >> 5) {
+        const int x = xyz ? xyz[3 * g] : x0 + (int)(g % nx) * step, z = xyz ? xyz[3 * g + 2] : z0 + (int)(g / nx) * step;
+        int cx, cy, cz;
+        zoom_cell(zseed, x, xyz ? xyz[3 * g + 1] : y, z, cx, cy, cz);
+        const int c = end_chunk_class(p, FM, (cx * 4) >> 4, (cz * 4) >> 4, W.end_f2, W.end_g2);
+        if ((threadIdx.x & 31) == 0) out[g] = (uint8_t)W.end_ids[c];
     }
 }
 /* End class of chunks [cx0, cx0+ncx) x [cz0, cz0+ncz): one w x h-chunk tile per block (endtile.cuh) */
@@ -427,7 +444,7 @@ template <bool FM, int DIM>
 static void points_t(const MgWorldDesc &W, const MgTreeNode *tree, const MgLattice *states, int ns, const int32_t *pts,
                      int np, uint8_t *out, int32_t *tg, cudaStream_t st) {
     long long n = (long long)ns * np;
-    { ProfScope ps_(K_POINTS, st); k_points<FM, DIM><<<blocks_for(n, 128), 128, 0, st>>>(W, tree, states, ns, pts, np, out, tg); }
+    { ProfScope ps_(K_POINTS, st); k_points<FM, DIM><<<blocks_for(DIM == MG_END ? 32 * n : n, 128), 128, 0, st>>>(W, tree, states, ns, pts, np, out, tg); }
 }
 int launch_points(const MgWorldDesc &W, const MgTreeNode *tree, const MgLattice *states, int ns, const int32_t *pts,
                   int np, uint8_t *out, int32_t *tg, cudaStream_t st) {
@@ -546,6 +563,11 @@ static void blockgrid_t(const MgWorldDesc &W, const MgTreeNode *tree, const MgLa
                         int ecx0, int ecz0, int encx, cudaStream_t st) {
     size_t sm = DIM == MG_END ? 0 : grid_smem(W);
     ProfScope ps_(K_BLOCKGRID, st);
+    if (DIM == MG_END && !cls) {
+        const long long n = (long long)nx * nz, nb = (n + 3) / 4;
+        k_end_samples<FM><<<(unsigned)(nb < 16 * 152 ? nb : 16 * 152), 128, 0, st>>>(W, state, zseed, x0, z0, nx, n, step, y, xyz, out);
+        return;
+    }
     if constexpr (DIM != MG_END) {
         /* the Nether's cells are cheap enough for a thread each once there are enough of them (26.1: 3,000 points 19.8 us by warps,
          * 22.0 by threads; 14,108 points 67.6 and 30.5) */
