@@ -43,8 +43,9 @@ int ow_prepare();
 /* records to provide for `cells` cells some of which are left to the exact evaluation (the double branch's with a target
  * open, well below 1 %; under the chunk-cell rule the tied ones too; cells beyond the record are evaluated in place) */
 long long ow_open_cap(long long cells);
-/* a group's requests (fm: the float branch's); open_pass: the recorded cells, after the tiles */
-int launch_ow_batch(bool fm, int tie, bool open_pass, const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees,
+/* a group's requests (fm: the float branch's); open_pass: the recorded cells, after the tiles; overlap: the launch before this one
+ * in the stream is a kernel of the same batch (overlap.cuh) */
+int launch_ow_batch(bool fm, int tie, bool open_pass, bool overlap, const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees,
                     const MgBatchReq *d_reqs, int nreq, long long ntiles, const MgLattice *d_pool, unsigned long long *d_counter,
                     MgOpenCell *d_open, unsigned long long *d_nopen, long long open_cap, uint8_t *d_out, cudaStream_t st);
 
@@ -54,9 +55,10 @@ extern const int kBatchTileWidths[BATCH_SHAPES];
 /* tiles of a request of group `group`: 16 x 16 cells (owtile.cu); in the rest, 128 quart cells of shape `shape`
  * (Overworld, Nether) or 8 x 8 chunks (End) */
 long long batch_tiles(int group, const MgWorldDesc &W, int qx0, int qz0, int nx, int nz, int shape);
-/* lattices of a list of entries of one dimension; Overworld needs the prefix sums of lattices per entry */
+/* lattices of a list of entries of one dimension; Overworld needs the prefix sums of lattices per entry; overlap: the launch before
+ * this one in the stream is another dimension's */
 int launch_setup_list(const MgWorldDesc *d_worlds, int dim, const MgSetupEntry *d_ent, int n, const int *d_first,
-                      long long total_lattices, MgLattice *d_pool, cudaStream_t st);
+                      long long total_lattices, MgLattice *d_pool, bool overlap, cudaStream_t st);
 /* kernel attributes and resident grid sizes; call before any stream capture */
 int batch_prepare(int *ctas_per_sm);
 /* d_reqs: the requests in group order, all under one tie rule.  ctas: upper bound on the rest's persistent grid, 0 = every

@@ -6,6 +6,7 @@
 #include "batch.h"
 #include "batchdev.cuh"
 #include "launch.h"
+#include "overlap.cuh"
 #include "owtile.cuh"
 #include "prof.h"
 #include "warpcell.cuh"
@@ -144,10 +145,11 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const __grid_constant__ OtWor
     const int col = ot_col(), row = ot_row();
     if (t == 0) sm.state = -1;
     sm.hint[t] = 0;
+    overlap_next();
     if (warp == 0) ot_next(sm.cur[0], K, -1);
     __syncthreads();
     for (int c = 0;; c ^= 1) {
-        if (sm.cur[c].req < 0) return;
+        if (sm.cur[c].req < 0) break;
         const int tile = sm.cur[c].tile;
         const MgBatchReq &R = sm.cur[c].r;
         const MgWorldDesc &W = K.worlds[R.world];
@@ -385,6 +387,7 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const __grid_constant__ OtWor
         }
         __syncthreads(); /* the tables are free for the next tile */
     }
+    overlap_wait();
 }
 
 /* ============================================================================ double branch */
@@ -420,10 +423,11 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const __grid_constant__ OtWor
     const int col = ot_col(), row = ot_row();
     if (t == 0) sm.state = -1;
     sm.hint[t] = 0;
+    overlap_next();
     if (warp == 0) ot_next(sm.cur[0], K, -1);
     __syncthreads();
     for (int c = 0;; c ^= 1) {
-        if (sm.cur[c].req < 0) return;
+        if (sm.cur[c].req < 0) break;
         const int tile = sm.cur[c].tile;
         const MgBatchReq &R = sm.cur[c].r;
         const MgWorldDesc &W = K.worlds[R.world];
@@ -732,6 +736,7 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const __grid_constant__ OtWor
         }
         __syncthreads(); /* the tables are free for the next tile */
     }
+    overlap_wait();
 }
 
 /* the open cells: up to 65,536 by a warp each (25 us for the first, then its throughput), more by a thread each (200 us for any
@@ -743,6 +748,9 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const __grid_constant__ OtWor
 template <bool FM, int MODE>
 __global__ void __launch_bounds__(OT_OPEN_NT, 6) k_ow_open(const __grid_constant__ OtWork K) {
     extern __shared__ uint4 smem_raw[];
+    WcStage &s = *reinterpret_cast<WcStage *>(smem_raw);
+    if (!K.reqs) wc_stage(s, K.worlds[0], K.pool, threadIdx.x, OT_OPEN_NT); /* while the tiles' last blocks run */
+    overlap_wait(); /* the cells are recorded */
     const long long n = min((long long)*K.nopen, K.open_cap);
     const bool by_warp = n <= 65536 || MODE == OT_CHUNK || MODE == OT_BLOCK;
     const int lane = threadIdx.x & 31;
@@ -758,11 +766,7 @@ __global__ void __launch_bounds__(OT_OPEN_NT, 6) k_ow_open(const __grid_constant
         return;
     }
     if ((long long)blockIdx.x * (MODE == OT_CHUNK || MODE == OT_BLOCK ? 1 : OT_OPEN_NT / 32) >= n) return;
-    WcStage &s = *reinterpret_cast<WcStage *>(smem_raw);
-    if (!K.reqs) {
-        wc_stage(s, K.worlds[0], K.pool, threadIdx.x, OT_OPEN_NT);
-        __syncthreads();
-    }
+    __syncthreads();
     __shared__ WcStep steps[MODE == OT_CHUNK || MODE == OT_BLOCK ? WC_STEPS : 1];
     constexpr bool chains = MODE == OT_CHUNK || MODE == OT_BLOCK; /* a block per cell, else a warp */
     for (long long i = chains ? (long long)blockIdx.x : id >> 5; i < n; i += chains ? (long long)gridDim.x : threads >> 5) {
@@ -851,21 +855,21 @@ int ow_prepare() {
 long long ow_open_cap(long long cells) { return cells > 0 ? cells / 32 + 4096 : 0; }
 
 template <int MODE>
-static void tiles_t(bool fm, const OtWork &K, int grid, cudaStream_t st) {
-    if (fm) k_ow_f<MODE><<<grid, OT_NT, sizeof(OtSmemF), st>>>(K);
-    else k_ow_d<MODE><<<grid, OT_NT, sizeof(OtSmemD), st>>>(K);
+static void tiles_t(bool fm, bool overlap, const OtWork &K, int grid, cudaStream_t st) {
+    if (fm) launch_on(overlap, k_ow_f<MODE>, grid, OT_NT, sizeof(OtSmemF), st, K);
+    else launch_on(overlap, k_ow_d<MODE>, grid, OT_NT, sizeof(OtSmemD), st, K);
 }
-static int launch_tiles(bool fm, int mode, const OtWork &K, cudaStream_t st) {
+static int launch_tiles(bool fm, int mode, bool overlap, const OtWork &K, cudaStream_t st) {
     const int resident = g_ow_resident[fm][mode];
     if (resident <= 0) return (int)cudaErrorInvalidValue;
     const int grid = (long long)resident < K.ntiles ? resident : (int)K.ntiles;
     {
         ProfScope ps_(fm ? K_OW_TILE_F : K_OW_TILE_D, st);
         switch (mode) {
-        case OT_CHUNK: tiles_t<OT_CHUNK>(fm, K, grid, st); break;
-        case OT_BLOCK: tiles_t<OT_BLOCK>(fm, K, grid, st); break;
-        case OT_CHAIN: tiles_t<OT_CHAIN>(fm, K, grid, st); break;
-        default: tiles_t<OT_ENGINE>(fm, K, grid, st); break;
+        case OT_CHUNK: tiles_t<OT_CHUNK>(fm, overlap, K, grid, st); break;
+        case OT_BLOCK: tiles_t<OT_BLOCK>(fm, overlap, K, grid, st); break;
+        case OT_CHAIN: tiles_t<OT_CHAIN>(fm, overlap, K, grid, st); break;
+        default: tiles_t<OT_ENGINE>(fm, overlap, K, grid, st); break;
         }
     }
     count_launch_external();
@@ -873,8 +877,8 @@ static int launch_tiles(bool fm, int mode, const OtWork &K, cudaStream_t st) {
 }
 template <int MODE>
 static void open_t(bool fm, const OtWork &K, int grid, cudaStream_t st) {
-    if (fm) k_ow_open<true, MODE><<<grid, OT_OPEN_NT, OT_OPEN_SMEM, st>>>(K);
-    else k_ow_open<false, MODE><<<grid, OT_OPEN_NT, OT_OPEN_SMEM, st>>>(K);
+    if (fm) launch_on(true, k_ow_open<true, MODE>, grid, OT_OPEN_NT, OT_OPEN_SMEM, st, K);
+    else launch_on(true, k_ow_open<false, MODE>, grid, OT_OPEN_NT, OT_OPEN_SMEM, st, K);
 }
 static int launch_open(bool fm, int mode, const OtWork &K, cudaStream_t st) {
     if (!K.open || K.open_cap <= 0) return 0;
@@ -884,15 +888,15 @@ static int launch_open(bool fm, int mode, const OtWork &K, cudaStream_t st) {
         switch (mode) {
         case OT_CHUNK: open_t<OT_CHUNK>(fm, K, grid, st); break;
         case OT_BLOCK: open_t<OT_BLOCK>(fm, K, grid, st); break;
-        case OT_CHAIN: if (!fm) k_ow_open<false, OT_CHAIN><<<grid, OT_OPEN_NT, OT_OPEN_SMEM, st>>>(K); break;
-        default: if (!fm) k_ow_open<false, OT_ENGINE><<<grid, OT_OPEN_NT, OT_OPEN_SMEM, st>>>(K); break;
+        case OT_CHAIN: if (!fm) launch_on(true, k_ow_open<false, OT_CHAIN>, grid, OT_OPEN_NT, OT_OPEN_SMEM, st, K); break;
+        default: if (!fm) launch_on(true, k_ow_open<false, OT_ENGINE>, grid, OT_OPEN_NT, OT_OPEN_SMEM, st, K); break;
         }
     }
     count_launch_external();
     return (int)cudaGetLastError();
 }
 
-int launch_ow_batch(bool fm, int tie, bool open_pass, const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees,
+int launch_ow_batch(bool fm, int tie, bool open_pass, bool overlap, const MgWorldDesc *d_worlds, const MgTreeNode *const *d_trees,
                     const MgBatchReq *d_reqs, int nreq, long long ntiles, const MgLattice *d_pool, unsigned long long *d_counter,
                     MgOpenCell *d_open, unsigned long long *d_nopen, long long open_cap, uint8_t *d_out, cudaStream_t st) {
     if (ntiles <= 0) return 0;
@@ -909,7 +913,7 @@ int launch_ow_batch(bool fm, int tie, bool open_pass, const MgWorldDesc *d_world
     K.open_cap = d_open ? open_cap : 0;
     K.out = d_out;
     const int mode = tie == MG_TIE_CHUNK_CELL ? OT_CHUNK : OT_ENGINE;
-    return open_pass ? (fm && mode == OT_ENGINE ? 0 : launch_open(fm, mode, K, st)) : launch_tiles(fm, mode, K, st);
+    return open_pass ? (fm && mode == OT_ENGINE ? 0 : launch_open(fm, mode, K, st)) : launch_tiles(fm, mode, overlap, K, st);
 }
 
 /* ---- one grid: scratch for the open cells' record (a counter, then the cells) */
@@ -933,7 +937,7 @@ static int grid_run(const MgWorldDesc &W, int mode, OtWork &K, void *scratch, cu
         const cudaError_t e = cudaMemsetAsync(K.nopen, 0, sizeof(unsigned long long), st);
         if (e) return (int)e;
     }
-    rc = launch_tiles(fm, mode, K, st);
+    rc = launch_tiles(fm, mode, false, K, st);
     return rc ? rc : launch_open(fm, mode, K, st);
 }
 int launch_ow_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const MgLattice *state, int qx0,

@@ -99,10 +99,12 @@ cudaError_t plan_pool(cudaMemPool_t *out) {
 }
 
 int enqueue(McGb300Plan *p, uint8_t *d_out, int shape, cudaStream_t st) {
+    bool setup = false;
     for (int d = 0; d < 3; d++) {
         if (!p->nent[d]) continue;
-        int rc = mg::launch_setup_list(p->d_worlds, d, p->d_ent[d], p->nent[d], p->d_first, p->ow_lattices, p->d_pool, st);
+        int rc = mg::launch_setup_list(p->d_worlds, d, p->d_ent[d], p->nent[d], p->d_first, p->ow_lattices, p->d_pool, setup, st);
         if (rc) return rc;
+        setup = true;
     }
     return mg::launch_batch(p->d_worlds, p->d_trees, p->d_reqs[shape], p->groups[shape], p->tie, p->d_pool, p->d_counter,
                             p->d_open, p->open_cap, d_out, p->ctas, shape, st);

@@ -314,10 +314,12 @@ int launch_batch(McGb300Server *s, Batch &b) {
     if (!e && !first.empty()) e = cudaMemcpyAsync(b.d_first, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice, st);
     if (e) return crc(e);
     eo = 0;
+    bool setup = false;
     for (int d = 0; d < 3; d++) {
         if (ent[d].empty()) continue;
-        int rc = mg::launch_setup_list(b.d_worlds, d, b.d_ent + eo, (int)ent[d].size(), b.d_first, ow, s->pool[0].base, st);
+        int rc = mg::launch_setup_list(b.d_worlds, d, b.d_ent + eo, (int)ent[d].size(), b.d_first, ow, s->pool[0].base, setup, st);
         if (rc) return MCGEN_E_INTERNAL;
+        setup = true;
         eo += ent[d].size();
     }
     if ((e = cudaEventRecord(b.setup_done, st))) return crc(e);
