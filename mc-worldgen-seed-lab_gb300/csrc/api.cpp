@@ -513,7 +513,7 @@ static int seed_points_on(const McWorld *w, const int64_t *d_seeds, int ns, cons
         DevBuf clim(st);
         cudaError_t e = clim.alloc(mg::fused_scratch_bytes(w->desc, (long long)ns * np));
         if (e) return cuda_code(e);
-        int rc = mg::launch_ow_seed_points(w->desc, w->d_tree, d_seeds, ns, d_pts, np, d_out, d_tg, clim.p, st);
+        int rc = mg::launch_ow_seed_points(w->desc, w->d_desc, w->d_tree, d_seeds, ns, d_pts, np, d_out, d_tg, clim.p, st);
         return rc ? cuda_code((cudaError_t)rc) : MCGEN_OK;
     }
     DevBuf states(st);

@@ -21,8 +21,10 @@
 
 #include <type_traits>
 
+#include "batch.h"
 #include "climate.cuh"
 #include "launch.h"
+#include "owtile.cuh"
 #include "search.cuh"
 #include "prof.h"
 
@@ -261,13 +263,286 @@ __global__ void __launch_bounds__(FNT) k_ow_seed_climate(const __grid_constant__
     }
 }
 
+/* a thread's octave at c = {x, z, and their second-stack multiples} */
+template <bool FM, typename V>
+__device__ __forceinline__ V search_octave(const MgWorldDesc &W, const FusedOwn &own, const OffHdr &h, const IlvPerm<FPS> &perm,
+                                           const double *c) {
+    const MgNoise &N = W.noise[own.noise];
+    const double x = c[own.st ? 2 : 0], z = c[own.st ? 3 : 1], f = N.freq[own.lev];
+    const int k = N.fexp[own.lev];
+    int ix, iz;
+    if constexpr (FM) {
+        float fx, fz;
+        split_fk(x, f, k, own.ox, ix, fx);
+        split_fk(z, f, k, own.oz, iz, fz);
+        return (V)octave_y0<float>(perm, h, ix, fx, iz, fz);
+    } else {
+        double fx, fz;
+        int64_t FX, FZ;
+        split_dk(x, f, k, own.ox, ix, fx, FX);
+        split_dk(z, f, k, own.oz, iz, fz, FZ);
+        return (V)octave_d_y0(perm, h, ix, fx, FX, iz, fz, FZ);
+    }
+}
+/* a noise's sum of its octaves, in the reference's order (engine/mc_noise.h:285-324); first: val index of its first lattice */
+template <bool FM, typename V>
+__device__ __forceinline__ V search_sum(const MgNoise &N, const V *val, int first, int spc, int s) {
+    if constexpr (FM) {
+        float acc = 0.0f;
+        for (int k = 0; k < N.nlev; k++) {
+            acc += N.amp_f[k] * val[(first + k) * spc + s];
+            acc += N.amp_f[k] * val[(first + N.nlev + k) * spc + s];
+        }
+        return acc;
+    } else {
+        double a1 = 0.0, a2 = 0.0;
+        for (int k = 0; k < N.nlev; k++) a1 += N.amp_d[k] * val[(first + k) * spc + s] * N.vf_d[k];
+        for (int k = 0; k < N.nlev; k++) a2 += N.amp_d[k] * val[(first + N.nlev + k) * spc + s] * N.vf_d[k];
+        return (a1 + a2) * N.vfac;
+    }
+}
+
+/* ---- the double branch's many seeds x points in the Overworld tiles' fixed point (owtile.cuh): the double evaluation's 72 FP64
+ * operations an octave kept the FP64 pipe 73 % busy (1,501 seeds x 33 points: 424 us; this form 232).  A sample whose targets the
+ * error bounds leave open (2 %) is kept in its seed's queue and evaluated in double at the end, one per seed at a time, from the
+ * lattices that are still there.  Writes the six targets of every sample. */
+#define TQ_CAP 64 /* points whose values are kept until their targets are formed, by all threads at once */
+struct TargetSmem {
+    uint32_t perm[64][FPS];
+    union {
+        int64_t val[FNT][FNPC]; /* octave value of lattice (owner thread) t at point p of the chunk, units of 2^-60 */
+        struct {                /* the exact evaluation's */
+            double val, valb;
+        } exact[FNT];
+    };
+    int64_t sh[2][FMAXOFF][FNPC]; /* ShiftA, ShiftB octaves */
+    union {
+        int64_t coord[FMAXS][FNPC][4]; /* per (seed, point): x, z and their second-stack multiples, units of 2^-32 */
+        double exact_at[FMAXS][4];
+    };
+    struct {
+        double ox, oy, oz;
+        OtFix fy, fz;
+        int iy, iz;
+    } hdr[FMAXOFF];
+    int32_t v[FMAXS][TQ_CAP][MG_OW_NOISES - 1]; /* units of 2^-29 */
+    int queue[FMAXS][TQ_CAP], queued[FMAXS];
+};
+__global__ void __launch_bounds__(FNT, 3) k_ow_seed_targets(const __grid_constant__ MgWorldDesc W, const MgSpline *__restrict__ spline,
+                                                            const int64_t *__restrict__ seeds, int ns, const int32_t *__restrict__ pts,
+                                                            int np, int32_t *__restrict__ targets) {
+    extern __shared__ uint4 smem_raw[];
+    TargetSmem &sm = *reinterpret_cast<TargetSmem *>(smem_raw);
+    const int t = threadIdx.x, nt = W.ntables, spc = FNT / nt, s0 = blockIdx.x * spc, j = t / spc, ls = t % spc;
+    const bool active = j < nt && s0 + ls < ns;
+    const MgNoise &O = W.noise[0];
+    const int noff = 2 * O.nlev, nown = noff * spc;
+    FusedOwn own;
+    if (active) fused_lattice(W, seeds[s0 + ls], j, &sm.perm[0][t], own);
+    OffHdr h;
+    h.ox = own.ox; h.oy = own.oy; h.oz = own.oz;
+    lattice_header(h, true);
+    const OtFix fix = ot_fix(h.fyd, h.uyd);
+    const int iy = h.iy, lev = -W.noise[own.noise].fexp[own.lev];
+    const int64_t oxq = __double2ll_rn(own.ox * 0x1.0p32), ozq = __double2ll_rn(own.oz * 0x1.0p32);
+    if (t < nown) {
+        sm.hdr[t].ox = own.ox; sm.hdr[t].oy = own.oy; sm.hdr[t].oz = own.oz;
+        sm.hdr[t].fy = fix;
+        sm.hdr[t].fz = ot_fix(h.fzd, h.uzd);
+        sm.hdr[t].iy = h.iy; sm.hdr[t].iz = h.iz;
+    }
+    if (t < FMAXS) sm.queued[t] = 0;
+    const uint8_t *pbase = reinterpret_cast<const uint8_t *>(&sm.perm[0][0]);
+    const IlvPerm<FPS> mine{pbase, t};
+
+    /* the samples in the queues, the r-th of every seed at once, in double (all threads call it) */
+    auto drain = [&]() {
+        for (int r = 0;; r++) {
+            __syncthreads();
+            int most = 0;
+            for (int s = 0; s < spc; s++) most = max(most, sm.queued[s]);
+            if (r >= most) break;
+            const bool go = active && r < sm.queued[ls];
+            const int32_t *pp = pts + 3 * (go ? sm.queue[ls][r] : 0);
+            OffHdr x;
+            x.ox = own.ox; x.oy = own.oy; x.oz = own.oz;
+            lattice_header(x, true);
+            if (go && own.noise == 0) {
+                double X = (double)pp[0], Z = (double)pp[2];
+                if (own.st) { X = X * MG_SECOND_STACK; Z = Z * MG_SECOND_STACK; }
+                const double f = O.freq[own.lev];
+                const int k = O.fexp[own.lev];
+                int ix, iz, iyy;
+                double fx, fz, fy;
+                int64_t FX, FZ, FY;
+                split_dk(X, f, k, own.ox, ix, fx, FX);
+                split_dk(Z, f, k, own.oz, iz, fz, FZ);
+                sm.exact[t].val = octave_d_y0(mine, x, ix, fx, FX, iz, fz, FZ);
+                split_dk(Z, f, k, own.ox, ix, fx, FX);
+                split_dk(X, f, k, own.oy, iyy, fy, FY);
+                sm.exact[t].valb = octave_d_z0(mine, x, ix, fx, FX, iyy, fy, FY);
+            }
+            __syncthreads();
+            const bool one = t < spc && r < sm.queued[t];
+            if (one) {
+                const int32_t *q = pts + 3 * sm.queue[t][r];
+                double a1 = 0.0, a2 = 0.0, b1 = 0.0, b2 = 0.0;
+                for (int k = 0; k < O.nlev; k++) {
+                    a1 += O.amp_d[k] * sm.exact[k * spc + t].val * O.vf_d[k];
+                    a2 += O.amp_d[k] * sm.exact[(O.nlev + k) * spc + t].val * O.vf_d[k];
+                    b1 += O.amp_d[k] * sm.exact[k * spc + t].valb * O.vf_d[k];
+                    b2 += O.amp_d[k] * sm.exact[(O.nlev + k) * spc + t].valb * O.vf_d[k];
+                }
+                const double x = (double)q[0] + ((a1 + a2) * O.vfac) * 4.0, z = (double)q[2] + ((b1 + b2) * O.vfac) * 4.0;
+                sm.exact_at[t][0] = x;
+                sm.exact_at[t][1] = z;
+                sm.exact_at[t][2] = x * MG_SECOND_STACK;
+                sm.exact_at[t][3] = z * MG_SECOND_STACK;
+            }
+            __syncthreads();
+            if (go && own.noise != 0) sm.exact[t].val = search_octave<false, double>(W, own, x, mine, sm.exact_at[ls]);
+            __syncthreads();
+            if (one) {
+                const int p = sm.queue[t][r];
+                double v[MG_OW_NOISES - 1];
+                for (int q = 1; q < MG_OW_NOISES; q++) {
+                    const MgNoise &N = W.noise[q];
+                    double a1 = 0.0, a2 = 0.0;
+                    for (int k = 0; k < N.nlev; k++) a1 += N.amp_d[k] * sm.exact[(N.base + k) * spc + t].val * N.vf_d[k];
+                    for (int k = 0; k < N.nlev; k++) a2 += N.amp_d[k] * sm.exact[(N.base + N.nlev + k) * spc + t].val * N.vf_d[k];
+                    v[q - 1] = (a1 + a2) * N.vfac;
+                }
+                climate_finish_d(W, *spline, v[0], v[1], v[2], v[3], v[4], pts[3 * p + 1] * 4, targets + ((size_t)(s0 + t) * np + p) * 6);
+            }
+        }
+        if (t < FMAXS) sm.queued[t] = 0;
+        __syncthreads();
+    };
+
+    auto within = [](const int32_t *q, int lim) { return q[0] > -lim && q[0] < lim && q[2] > -lim && q[2] < lim; };
+    for (int p0 = 0; p0 < np; p0 += FNPC) {
+        const int npc = min(FNPC, np - p0);
+        __syncthreads(); /* lattices and headers complete / previous chunk consumed */
+        /* ---- B: ShiftA (x, 0, z) and ShiftB (z, x, 0) octaves, item = (owner, point) */
+        for (int item = t; item < nown * npc; item += FNT) {
+            const int o = item % nown, p = item / nown, oj = o / spc;
+            if (s0 + o % spc >= ns) continue;
+            const auto &oh = sm.hdr[o];
+            const IlvPerm<FPS> perm{pbase, o};
+            const int32_t *pp = pts + 3 * (p0 + p);
+            if (!within(pp, OT_COORD_LIM)) continue;
+            const double f = O.freq[oj >= O.nlev ? oj - O.nlev : oj];
+            double X = (double)pp[0], Z = (double)pp[2];
+            if (oj >= O.nlev) { X = X * MG_SECOND_STACK; Z = Z * MG_SECOND_STACK; }
+            int ia, ib;
+            int32_t ta, ua, tb, ub;
+            ot_split_d(X, f, oh.ox, ia, ta, ua);
+            ot_split_d(Z, f, oh.oz, ib, tb, ub);
+            sm.sh[0][o][p] = ot_sample_d(perm, oh.iy, false, oh.fy, ia, ib, ta, ua, tb, ub);
+            ot_split_d(Z, f, oh.ox, ia, ta, ua);
+            ot_split_d(X, f, oh.oy, ib, tb, ub);
+            sm.sh[1][o][p] = ot_sample_d(perm, oh.iz, true, oh.fz, ia, ib, ta, ua, tb, ub);
+        }
+        __syncthreads();
+        /* ---- C: shifted coordinates of every (seed, point) */
+        const int cs = t / FNPC, cp = t % FNPC;
+        const bool item = t < spc * FNPC && cp < npc && s0 + cs < ns;
+        const int32_t *pp = pts + 3 * (p0 + (item ? cp : 0));
+        const bool skip = !within(pp, OT_COORD_LIM);
+        if (item) {
+            int64_t sa = 0, sb = 0; /* units of 2^-59 */
+            for (int k = 0; k < O.nlev; k++) {
+                const int64_t va = sm.sh[0][k * spc + cs][cp] + sm.sh[0][(O.nlev + k) * spc + cs][cp];
+                const int64_t vb = sm.sh[1][k * spc + cs][cp] + sm.sh[1][(O.nlev + k) * spc + cs][cp];
+                sa = ot_madw((int32_t)(va >> 31), O.c30[k], sa);
+                sb = ot_madw((int32_t)(vb >> 31), O.c30[k], sb);
+            }
+            const int64_t x = skip ? 0 : ((int64_t)pp[0] << 32) + (sa >> 25), z = skip ? 0 : ((int64_t)pp[2] << 32) + (sb >> 25);
+            sm.coord[cs][cp][0] = x;
+            sm.coord[cs][cp][1] = z;
+            sm.coord[cs][cp][2] = x + __mul64hi(x, OT_STACK_C);
+            sm.coord[cs][cp][3] = z + __mul64hi(z, OT_STACK_C);
+        }
+        __syncthreads();
+        /* ---- D: climate octaves, each thread on its own lattice */
+        if (active && own.noise != 0) {
+            for (int p = 0; p < npc; p++) {
+                const int64_t sx = (sm.coord[ls][p][own.st ? 2 : 0] >> lev) + oxq, sz = (sm.coord[ls][p][own.st ? 3 : 1] >> lev) + ozq;
+                sm.val[t][p] = ot_sample_d(mine, iy, false, fix, ot_hi(sx), ot_hi(sz), (int32_t)((uint32_t)sx >> 1), ot_fade31((uint32_t)sx),
+                                           (int32_t)((uint32_t)sz >> 1), ot_fade31((uint32_t)sz));
+            }
+        }
+        __syncthreads();
+        /* ---- E: the five noises */
+        if (item) {
+#pragma unroll
+            for (int q = 1; q < MG_OW_NOISES; q++) {
+                const MgNoise &N = W.noise[q];
+                int64_t acc = 0;
+                for (int k = 0; k < N.nlev; k++) {
+                    const int64_t l = sm.val[(N.base + k) * spc + cs][cp] + sm.val[(N.base + N.nlev + k) * spc + cs][cp];
+                    acc = ot_madw((int32_t)(l >> 31), N.c30[k], acc);
+                }
+                sm.v[cs][(p0 + cp) % TQ_CAP][q - 1] = (int32_t)(acc >> 30);
+            }
+        }
+        const int done = p0 + npc, from = (done - 1) / TQ_CAP * TQ_CAP; /* points [from, done) have values */
+        if (done != np && done % TQ_CAP) continue;
+        __syncthreads();
+        /* ---- F: the targets that they may have */
+        for (int i = t; i < spc * (done - from); i += FNT) {
+            const int s = i / (done - from), p = from + i % (done - from);
+            if (s0 + s >= ns) continue;
+            const int32_t *q = pts + 3 * p;
+            const bool out17 = !within(q, (1 << 17) - OT_W);
+            int32_t v[MG_OW_NOISES - 1], ta[6], tb[6], eq[MG_OW_NOISES];
+#pragma unroll
+            for (int k = 1; k < MG_OW_NOISES; k++) {
+                v[k - 1] = sm.v[s][p - from][k - 1];
+                eq[k] = out17 ? W.noise[k].tile_eq_far : W.noise[k].tile_eq;
+            }
+            float es;
+            ot_climate_targets(W, *spline, v, eq, (int32_t)__double2ll_rn((depth_grad_d(W, q[1] * 4) + W.off_d) * 0x1.0p28), ta, tb, es);
+            bool ok = es < 1.0f && within(q, OT_COORD_LIM);
+#pragma unroll
+            for (int k = 0; k < 6; k++) ok &= ta[k] == tb[k];
+            if (ok) {
+                int32_t *o = targets + ((size_t)(s0 + s) * np + p) * 6;
+#pragma unroll
+                for (int k = 0; k < 6; k++) o[k] = ta[k];
+            } else {
+                sm.queue[s][atomicAdd(&sm.queued[s], 1)] = p;
+            }
+        }
+        drain();
+    }
+}
+/* samples of a warp in the tree kernels, whose lanes' targets it takes one after another: fewer than 32 when there are too few
+ * samples to fill the chip with warps of 32 (49,533 samples: 106 -> 88 us) */
+static int tree_lanes(long long n) {
+    const long long k = (n + 152 * 40 - 1) / (152 * 40);
+    return k < 32 ? (int)k : 32;
+}
+/* the tree for samples whose targets are known */
+__global__ void __launch_bounds__(128) k_ow_targets_tree(const __grid_constant__ MgWorldDesc W, const MgTreeNode *__restrict__ tree,
+                                                         const int32_t *__restrict__ tg, long long n, int lanes,
+                                                         uint8_t *__restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const long long g = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * lanes + lane;
+    const bool in = lane < lanes && g < n;
+    int32_t t[6] = {0, 0, 0, 0, 0, 0};
+    if (in)
+        for (int k = 0; k < 6; k++) t[k] = tg[g * 6 + k];
+    const int leaf = tree_search_lanes(tree, W, t, in);
+    if (in) out[g] = tree[leaf].biome;
+}
 /* Finish the climate of every sample from its five noise values (ridges_folded, offset spline, depth,
  * quantisation; engine/mc_climate.h:126-170) and search the R-tree (ENGINE rule). One thread per sample. */
 template <bool FM>
 __global__ void __launch_bounds__(128) k_ow_finish_tree(const __grid_constant__ MgWorldDesc W,
                                                         const MgTreeNode *__restrict__ tree,
                                                         const typename std::conditional<FM, float, double>::type *__restrict__ clim,
-                                                        int ns, const int32_t *__restrict__ pts, int np,
+                                                        int ns, const int32_t *__restrict__ pts, int np, int lanes,
                                                         uint8_t *__restrict__ out, int32_t *__restrict__ targets) {
     __shared__ MgSpline S;
     {
@@ -276,8 +551,9 @@ __global__ void __launch_bounds__(128) k_ow_finish_tree(const __grid_constant__ 
         for (int i = threadIdx.x; i < (int)(sizeof(MgSpline) / 16); i += blockDim.x) d[i] = c[i];
     }
     __syncthreads();
-    const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool in = g < (long long)ns * np;
+    const int lane = threadIdx.x & 31;
+    const long long g = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * lanes + lane;
+    const bool in = lane < lanes && g < (long long)ns * np;
     int32_t tg[6] = {0, 0, 0, 0, 0, 0};
     if (in) {
         const int p = (int)(g % np);
@@ -356,44 +632,6 @@ struct SearchSmem {
     V val[FPS], valb[FPS]; /* octave values by owner */
     double coord[FPS / 2][4];
 };
-/* lattices [j0, j1) of each seed, spc seeds per CTA: thread t owns lattice j0 + t / spc of local seed t % spc */
-template <bool FM, typename V>
-__device__ __forceinline__ V search_octave(const MgWorldDesc &W, const FusedOwn &own, const OffHdr &h, const IlvPerm<FPS> &perm,
-                                           const double *c) {
-    const MgNoise &N = W.noise[own.noise];
-    const double x = c[own.st ? 2 : 0], z = c[own.st ? 3 : 1], f = N.freq[own.lev];
-    const int k = N.fexp[own.lev];
-    int ix, iz;
-    if constexpr (FM) {
-        float fx, fz;
-        split_fk(x, f, k, own.ox, ix, fx);
-        split_fk(z, f, k, own.oz, iz, fz);
-        return (V)octave_y0<float>(perm, h, ix, fx, iz, fz);
-    } else {
-        double fx, fz;
-        int64_t FX, FZ;
-        split_dk(x, f, k, own.ox, ix, fx, FX);
-        split_dk(z, f, k, own.oz, iz, fz, FZ);
-        return (V)octave_d_y0(perm, h, ix, fx, FX, iz, fz, FZ);
-    }
-}
-/* a noise's sum of its octaves, in the reference's order (engine/mc_noise.h:285-324); first: val index of its first lattice */
-template <bool FM, typename V>
-__device__ __forceinline__ V search_sum(const MgNoise &N, const V *val, int first, int spc, int s) {
-    if constexpr (FM) {
-        float acc = 0.0f;
-        for (int k = 0; k < N.nlev; k++) {
-            acc += N.amp_f[k] * val[(first + k) * spc + s];
-            acc += N.amp_f[k] * val[(first + N.nlev + k) * spc + s];
-        }
-        return acc;
-    } else {
-        double a1 = 0.0, a2 = 0.0;
-        for (int k = 0; k < N.nlev; k++) a1 += N.amp_d[k] * val[(first + k) * spc + s] * N.vf_d[k];
-        for (int k = 0; k < N.nlev; k++) a2 += N.amp_d[k] * val[(first + N.nlev + k) * spc + s] * N.vf_d[k];
-        return (a1 + a2) * N.vfac;
-    }
-}
 template <bool FM>
 __global__ void __launch_bounds__(FPS) k_ow_search_th(const __grid_constant__ MgWorldDesc W, const int64_t *__restrict__ seeds, int ns,
                                                       const int32_t *__restrict__ pts, const uint32_t *__restrict__ possible,
@@ -530,11 +768,12 @@ __global__ void __launch_bounds__(128) k_ow_search_first(const __grid_constant__
         for (int i = threadIdx.x; i < (int)(sizeof(MgSpline) / 16); i += blockDim.x) d[i] = c[i];
     }
     __syncthreads();
-    const int n = (int)*list.count;
+    const int n = (int)*list.count, lane = threadIdx.x & 31, warps = (int)(gridDim.x * blockDim.x) >> 5;
+    const int lanes = min((n + warps - 1) / warps, 32); /* (tree_lanes) */
     int nf = 0;
-    for (int b = (int)blockIdx.x * 128; b < n; b += (int)gridDim.x * 128) {
-        const int k = b + (int)threadIdx.x;
-        const bool in = k < n;
+    for (int b = (int)blockIdx.x * 4 * lanes; b < n; b += warps * lanes) {
+        const int k = b + (int)(threadIdx.x >> 5) * lanes + lane;
+        const bool in = lane < lanes && k < n;
         const int g = in ? list.index[k] : 0;
         int32_t tg[6] = {0, 0, 0, 0, 0, 0};
         if (in) {
@@ -634,15 +873,43 @@ static int fused_t(const MgWorldDesc &W, const MgTreeNode *tree, const int64_t *
     const long long n = (long long)ns * np;
     {
         ProfScope ps_(K_OW_FINISH_TREE, st);
-        k_ow_finish_tree<FM><<<(unsigned)((n + 127) / 128), 128, 0, st>>>(W, tree, clim, ns, pts, np, out, tg);
+        const int lanes = tree_lanes(n);
+        k_ow_finish_tree<FM><<<(unsigned)((n + 4 * lanes - 1) / (4 * lanes)), 128, 0, st>>>(W, tree, clim, ns, pts, np, lanes, out, tg);
     }
     count_launch_external();
     return 0;
 }
 
-int launch_ow_seed_points(const MgWorldDesc &W, const MgTreeNode *tree, const int64_t *seeds, int ns, const int32_t *pts,
-                          int np, uint8_t *out, int32_t *tg, void *scratch, cudaStream_t st) {
+/* the double branch in fixed point: targets into tg, or the scratch */
+static int targets_t(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const int64_t *seeds, int ns, const int32_t *pts,
+                     int np, uint8_t *out, int32_t *tg, cudaStream_t st) {
+    const int sm = (int)sizeof(TargetSmem);
+    cudaError_t e = cudaFuncSetAttribute(k_ow_seed_targets, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    if (!e) e = cudaFuncSetAttribute(k_ow_seed_targets, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    if (e) return (int)e;
+    const int spc = FNT / W.ntables;
+    {
+        ProfScope ps_(K_OW_SEED_CLIMATE, st);
+        k_ow_seed_targets<<<(unsigned)((ns + spc - 1) / spc), FNT, sm, st>>>(W, &d_world->spline, seeds, ns, pts, np, tg);
+    }
+    count_launch_external();
+    const long long n = (long long)ns * np;
+    {
+        ProfScope ps_(K_OW_FINISH_TREE, st);
+        const int lanes = tree_lanes(n);
+        k_ow_targets_tree<<<(unsigned)((n + 4 * lanes - 1) / (4 * lanes)), 128, 0, st>>>(W, tree, tg, n, lanes, out);
+    }
+    count_launch_external();
+    return 0;
+}
+
+int launch_ow_seed_points(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const int64_t *seeds, int ns,
+                          const int32_t *pts, int np, uint8_t *out, int32_t *tg, void *scratch, cudaStream_t st) {
     if ((long long)ns * np <= 0) return 0;
+    if (!W.fmode && ow_tile_supported(W)) {
+        const int r = targets_t(W, d_world, tree, seeds, ns, pts, np, out, tg ? tg : (int32_t *)scratch, st);
+        return r ? r : (int)cudaGetLastError();
+    }
     int rc = W.fmode ? fused_t<true>(W, tree, seeds, ns, pts, np, out, tg, scratch, st)
                      : fused_t<false>(W, tree, seeds, ns, pts, np, out, tg, scratch, st);
     return rc ? rc : (int)cudaGetLastError();

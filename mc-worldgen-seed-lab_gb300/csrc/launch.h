@@ -27,8 +27,8 @@ int launch_points(const MgWorldDesc &W, const MgTreeNode *tree, const MgLattice 
  * sample).  fused_supported() tells whether a world's lattice count fits the kernel. */
 bool fused_supported(const MgWorldDesc &W);
 size_t fused_scratch_bytes(const MgWorldDesc &W, long long samples);
-int launch_ow_seed_points(const MgWorldDesc &W, const MgTreeNode *tree, const int64_t *seeds, int ns, const int32_t *pts,
-                          int np, uint8_t *out, int32_t *targets, void *scratch, cudaStream_t st);
+int launch_ow_seed_points(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const int64_t *seeds, int ns,
+                          const int32_t *pts, int np, uint8_t *out, int32_t *targets, void *scratch, cudaStream_t st);
 
 /* seed search, Overworld, one observation (one quart cell per candidate at pts[3i..3i+2]): candidates
  * that pass go to surv (count *nsurv), failures are added to *fail.  Scratch: search_scratch_bytes(W, ns). */

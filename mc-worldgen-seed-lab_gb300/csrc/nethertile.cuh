@@ -132,15 +132,8 @@ __device__ __noinline__ void nether_tile(const MgWorldDesc &W, NetherTile &e, co
             v.node = zc ? cell * e.nx[l] : cell + e.off[l];
             e.sh.f[l][s] = v;
         } else {
-            uint64_t F;
-            if (!ot_split(c, f, off, cell, F)) { /* rare: the sum near zero or beyond 2^20 */
-                const double v = __fma_rn(c, f, off);
-                cell = ifloor(v);
-                F = (uint64_t)__double2ll_rn((v - (double)cell) * 0x1.0p63) << 1;
-            }
             OtShiftD v;
-            v.f = (int32_t)min((uint32_t)(((F >> 32) + 1) >> 1), 0x7FFFFFFFu);
-            v.u = (int32_t)min((uint32_t)((fadeq((int64_t)(F >> (64 - MG_Q))) + (1LL << 27)) >> 28), 0x7FFFFFFFu);
+            ot_split_d(c, f, off, cell, v.f, v.u);
             cell -= ifloor(__fma_rn(c0, f, off));
             v.edge = zc ? cell * e.nx[l] : cell + e.off[l];
             v.pad = 0;

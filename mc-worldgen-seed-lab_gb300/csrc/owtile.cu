@@ -392,7 +392,6 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const __grid_constant__ OtWor
 
 /* ============================================================================ double branch */
 #define OT_CAP_D 896 /* edges a tile's table holds */
-#define OT_STACK_C ((int64_t)((MG_SECOND_STACK - 1.0) * 0x1.0p64)) /* exact */
 
 struct OtSmemD {
     MgLattice lat[MG_MAX_TABLES];
@@ -489,15 +488,8 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const __grid_constant__ OtWor
             double c = fam < 2 ? (double)(qx0 + idx) : (double)(qz0 + idx), c0 = fam < 2 ? (double)qx0 : (double)qz0;
             if (j >= nlev) { c = c * MG_SECOND_STACK; c0 = c0 * MG_SECOND_STACK; }
             int i;
-            uint64_t F;
-            if (!ot_split(c, f, off, i, F)) { /* rare: the sum near zero or beyond 2^20 */
-                const double s = __fma_rn(c, f, off);
-                i = ifloor(s);
-                F = (uint64_t)__double2ll_rn((s - (double)i) * 0x1.0p63) << 1;
-            }
             OtShiftD s;
-            s.f = (int32_t)min((uint32_t)(((F >> 32) + 1) >> 1), 0x7FFFFFFFu);
-            s.u = (int32_t)min((uint32_t)((fadeq((int64_t)(F >> (64 - MG_Q))) + (1LL << 27)) >> 28), 0x7FFFFFFFu);
+            ot_split_d(c, f, off, i, s.f, s.u);
             const int tab = 2 * j + (fam & 1), rel = i - ifloor(__fma_rn(c0, f, off));
             s.edge = fam == 0 || fam == 3 ? rel + 32 * sm.sbuild.unit0[tab] : rel * sm.sbuild.nx[tab];
             s.pad = 0;
@@ -656,34 +648,12 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const __grid_constant__ OtWor
 #pragma unroll
                 for (int k = 0; k < MG_OW_NOISES - 1; k++) v[k] = n == k ? (int32_t)(acc >> 30) : v[k];
             }
-            const float s29 = 10000.0f * 0x1.0p-29f, s28 = 10000.0f * 0x1.0p-28f;
             const bool out17 = max(max(abs(qx0), abs(qz0)) + OT_W, 0) >= 1 << 17;
             int32_t eq[MG_OW_NOISES];
 #pragma unroll
             for (int n = 1; n < MG_OW_NOISES; n++) eq[n] = out17 ? W.noise[n].tile_eq_far : W.noise[n].tile_eq;
-            const int32_t ec = eq[3], ee = eq[4], ew = eq[5];
-            ot_target(v[0], eq[1], s29, ta[0], tb[0]);
-            ot_target(v[1], eq[2], s29, ta[1], tb[1]);
-            ot_target(v[2], ec, s29, ta[2], tb[2]);
-            ot_target(v[3], ee, s29, ta[3], tb[3]);
-            ot_target(v[4], ew, s29, ta[5], tb[5]);
-            /* spline coordinates: floats of the values, of ridges_folded (|(|r| + c0)| + c1) c2 (the sums in units of
-             * 2^-29); each within its noise's bound (times |c2|) and both sides' roundings to float */
-            const float u = 0x1.0p-29f;
-            const int32_t rs = abs(abs(v[4]) + (int32_t)((W.rf_q[0] + (1 << 29)) >> 30)) + (int32_t)((W.rf_q[1] + (1 << 29)) >> 30);
-            const float c2 = (float)W.rf_d[2] * u;
-            SplineIn si;
-            si.c = (float)v[2] * u;
-            si.e = (float)v[3] * u;
-            si.r = (float)v[4] * u;
-            si.f = (float)rs * c2;
-            si.dc = (float)ec * u + fabsf(si.c) * 1.2e-7f;
-            si.de = (float)ee * u + fabsf(si.e) * 1.2e-7f;
-            si.dr = (float)ew * u + fabsf(si.r) * 1.2e-7f;
-            si.df = fabsf(c2) * (float)(ew + 2) + fabsf(si.f) * 1.9e-7f;
             float es;
-            const float sp = spline_err<OT_SPL_DEPTH>(W.spline, W.spline.root, si, es);
-            ot_target(sm.depth[MODE == OT_BLOCK ? dy : 0] + __float2int_rn(sp * 0x1.0p28f), (int32_t)(es * (1.01f * 0x1.0p28f)) + 3, s28, ta[4], tb[4]);
+            ot_climate_targets(W, W.spline, v, eq, sm.depth[MODE == OT_BLOCK ? dy : 0], ta, tb, es);
             ok = es < 1.0f;
         }
         /* at most one target open, between two neighbouring values: both are looked up, and the cell is settled when they

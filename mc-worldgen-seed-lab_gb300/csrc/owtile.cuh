@@ -213,6 +213,7 @@ __device__ __forceinline__ int32_t ot_sub_sat(int32_t a, int32_t b) {
     asm("sub.sat.s32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
+#define OT_STACK_C ((int64_t)((MG_SECOND_STACK - 1.0) * 0x1.0p64)) /* exact */
 /* smoothstep of the fraction t (units of 2^-32) in units of 2^-31: t > 1/2 as 1 - smoothstep(1 - t), and with t' = 2 t <= 1,
  * t^3 (10 - 15 t + 6 t^2) = t'^3 / 8 (10 - t' (7.5 - 1.5 t')).  The 2 centres the truncations: within 1.43e-9 (all 2^32
  * fractions evaluated). */
@@ -242,22 +243,47 @@ __device__ __forceinline__ void ot_mix(int h0, int h1, bool z0, const OtFix &f, 
     B = z0 ? g.y * f.w + h.y * f.v : g.z * f.w + h.z * f.v;
     C = z0 ? g.z * f.c0 + h.z * f.c1 : g.y * f.c0 + h.y * f.c1;
 }
-/* edge (i, k) - (i + 1, k) */
-__device__ __forceinline__ void ot_edge(const MgLattice &L, bool z0, const OtFix &f, int i, int k, int4 &p, int2 &q) {
-    const PlainPerm P{L.p};
+/* edge (i, k) - (i + 1, k) of the plane at `fixed` (the cell of the fixed coordinate) */
+template <typename PERM>
+__device__ __forceinline__ void ot_edge(const PERM &P, int fixed, bool z0, const OtFix &f, int i, int k, int4 &p, int2 &q) {
     const int a = P(i), b = P(i + 1);
     int h0, h1, h2, h3;
     if (z0) {
-        const int aa = P(a + k) + L.iz, bb = P(b + k) + L.iz;
+        const int aa = P(a + k) + fixed, bb = P(b + k) + fixed;
         h0 = P(aa); h1 = P(aa + 1); h2 = P(bb); h3 = P(bb + 1);
     } else {
-        h0 = P(P(a + L.iy) + k); h1 = P(P(a + L.iy + 1) + k); h2 = P(P(b + L.iy) + k); h3 = P(P(b + L.iy + 1) + k);
+        h0 = P(P(a + fixed) + k); h1 = P(P(a + fixed + 1) + k); h2 = P(P(b + fixed) + k); h3 = P(P(b + fixed + 1) + k);
     }
     int32_t A0, B0, C0, A1, B1, C1;
     ot_mix(h0, h1, z0, f, A0, B0, C0);
     ot_mix(h2, h3, z0, f, A1, B1, C1);
     p = make_int4((A0 + 1) >> 1, (B0 + 1) >> 1, (C0 + 2) >> 2, ot_sub_sat(A1, A0));
     q = make_int2(ot_sub_sat(B1, B0), (int32_t)(((int64_t)C1 - A1 - C0 + 1) >> 1));
+}
+__device__ __forceinline__ void ot_edge(const MgLattice &L, bool z0, const OtFix &f, int i, int k, int4 &p, int2 &q) {
+    ot_edge(PlainPerm{L.p}, z0 ? L.iz : L.iy, z0, f, i, k, p, q);
+}
+/* ot_octave_d for one sample of a lattice, its two edges built on the way */
+template <typename PERM>
+__device__ __forceinline__ int64_t ot_sample_d(const PERM &P, int fixed, bool z0, const OtFix &f, int i, int k, int32_t X, int32_t U,
+                                               int32_t Z, int32_t W) {
+    OtEdge e0, e1;
+    ot_edge(P, fixed, z0, f, i, k, e0.p, e0.q);
+    ot_edge(P, fixed, z0, f, i, k + 1, e1.p, e1.q);
+    const int64_t l0 = ot_row_d(e0, X, Z, U), l1 = ot_row_d(e1, X, (int32_t)((uint32_t)Z - 0x80000000u), U);
+    return ot_madw(W, ot_hi((int64_t)((uint64_t)(l1 - l0) << 1)), l0);
+}
+/* cell, fraction and smoothstep (units of 2^-31, as the shift tables hold them) of a whole coordinate c (or its second-stack
+ * multiple) times f plus off */
+__device__ __forceinline__ void ot_split_d(double c, double f, double off, int &i, int32_t &t, int32_t &u) {
+    uint64_t F;
+    if (!ot_split(c, f, off, i, F)) { /* rare: the sum near zero or beyond 2^20 */
+        const double s = __fma_rn(c, f, off);
+        i = ifloor(s);
+        F = (uint64_t)__double2ll_rn((s - (double)i) * 0x1.0p63) << 1;
+    }
+    t = (int32_t)min((uint32_t)(((F >> 32) + 1) >> 1), 0x7FFFFFFFu);
+    u = (int32_t)min((uint32_t)((fadeq((int64_t)(F >> (64 - MG_Q))) + (1LL << 27)) >> 28), 0x7FFFFFFFu);
 }
 /* the targets a value within e of v may have (units of 2^-29, 2^-28 for the depth: `scale` is 10000 times the unit): the
  * rounding to float, the product by 10000 and the truncation are each monotone, so the ends' targets bound it */
@@ -316,6 +342,36 @@ __device__ __forceinline__ float spline_err(const MgSpline &S, int c, const Spli
         if (ad + ab + e1 + e2 == 0.0f) err = 2e-9f; /* a constant segment: its value is exact */
         return lerp<float>(t, y1, y2) + t * (1.0f - t) * lerp<float>(t, a, b);
     }
+}
+
+/* targets [ta, tb] of the five climate noises' values v (units of 2^-29, v[q - 1] within eq[q] of noise q's) and the depth
+ * gradient plus offset (units of 2^-28); es: the offset spline's error bound, 1 or more when the targets do not hold */
+__device__ __forceinline__ void ot_climate_targets(const MgWorldDesc &W, const MgSpline &S, const int32_t (&v)[MG_OW_NOISES - 1],
+                                                   const int32_t (&eq)[MG_OW_NOISES], int32_t depth, int32_t (&ta)[6], int32_t (&tb)[6],
+                                                   float &es) {
+    const float s29 = 10000.0f * 0x1.0p-29f, s28 = 10000.0f * 0x1.0p-28f;
+    const int32_t ec = eq[3], ee = eq[4], ew = eq[5];
+    ot_target(v[0], eq[1], s29, ta[0], tb[0]);
+    ot_target(v[1], eq[2], s29, ta[1], tb[1]);
+    ot_target(v[2], ec, s29, ta[2], tb[2]);
+    ot_target(v[3], ee, s29, ta[3], tb[3]);
+    ot_target(v[4], ew, s29, ta[5], tb[5]);
+    /* spline coordinates: floats of the values, of ridges_folded (|(|r| + c0)| + c1) c2 (the sums in units of
+     * 2^-29); each within its noise's bound (times |c2|) and both sides' roundings to float */
+    const float u = 0x1.0p-29f;
+    const int32_t rs = abs(abs(v[4]) + (int32_t)((W.rf_q[0] + (1 << 29)) >> 30)) + (int32_t)((W.rf_q[1] + (1 << 29)) >> 30);
+    const float c2 = (float)W.rf_d[2] * u;
+    SplineIn si;
+    si.c = (float)v[2] * u;
+    si.e = (float)v[3] * u;
+    si.r = (float)v[4] * u;
+    si.f = (float)rs * c2;
+    si.dc = (float)ec * u + fabsf(si.c) * 1.2e-7f;
+    si.de = (float)ee * u + fabsf(si.e) * 1.2e-7f;
+    si.dr = (float)ew * u + fabsf(si.r) * 1.2e-7f;
+    si.df = fabsf(c2) * (float)(ew + 2) + fabsf(si.f) * 1.9e-7f;
+    const float sp = spline_err<OT_SPL_DEPTH>(S, S.root, si, es);
+    ot_target(depth + __float2int_rn(sp * 0x1.0p28f), (int32_t)(es * (1.01f * 0x1.0p28f)) + 3, s28, ta[4], tb[4]);
 }
 
 }  // namespace mg

@@ -98,3 +98,27 @@ def test_nether_rejected_draws():
     _, tg = w.seed_points(seeds, pts, want_targets=True)
     _, et = ow.points(seeds, pts, want_targets=True)
     assert np.array_equal(np.asarray(tg).reshape(-1, 6), np.asarray(et).reshape(-1, 6))
+
+
+@pytest.mark.parametrize("version,preset", [("26.1", "normal"), ("26.2", "amplified"), ("26.1", "large_biomes")])
+def test_seed_targets_fixed_point(version, preset):
+    """The double branch's targets from fixed point: points around the flush of kept values, beyond the tables' coordinates (the
+    exact form), near and beyond 2^17, extreme heights; seeds around a block's number."""
+    mg = ge.package()
+    mg.load()
+    if mg.device_count() < 1:
+        pytest.fail("no CUDA device")
+    w = mg.Generator.open(ge.data_root(), version).world("minecraft:overworld", preset, 0)
+    ow = O.World(ge.data_root(), version, "overworld", preset)
+    rng = np.random.default_rng(4)
+    lims = (300, 131060, 131090, 7499990, 8388607, 500000000)
+    for ns, npt in ((5, 129), (1, 64), (3, 65), (41, 9), (4, 8)):
+        seeds = rng.integers(-2**63, 2**63 - 1, ns)
+        lim = np.array([lims[i % 6] for i in range(npt)])
+        pts = np.stack([rng.integers(-lim, lim), rng.integers(-90, 90, npt), rng.integers(-lim, lim)], 1).astype(np.int32)
+        if npt == 129: pts[:64, [0, 2]] = 8388600  # a full queue
+        got, tg = w.seed_points(seeds, pts, want_targets=True)
+        exp, et = ow.points(seeds, pts, want_targets=True)
+        assert np.array_equal(np.asarray(tg).reshape(-1, 6), np.asarray(et).reshape(-1, 6)), (ns, npt)
+        assert np.array_equal(np.asarray(got).reshape(-1), np.asarray(exp).reshape(-1)), (ns, npt)
+        assert np.array_equal(np.asarray(w.seed_points(seeds, pts)).reshape(-1), np.asarray(exp).reshape(-1)), (ns, npt)
