@@ -170,7 +170,7 @@ int block_biomes_dev(const McWorld *w, int x0, int z0, int nx, int nz, int step,
     int cx0 = 0, cz0 = 0, ncx = 0, ncz = 0;
     DevBuf cls(st); /* the End's chunk classes, or the Overworld's scratch */
     const long long n = (long long)nx * nz;
-    if (cudaError_t e = cls.alloc_optional(mg::block_scratch_bytes(w->desc, x0, z0, nx, nz, step, d_xyz != nullptr))) return cuda_code(e);
+    if (cudaError_t e = cls.alloc_optional(mg::block_scratch_bytes(w->desc, x0, z0, nx, nz, d_xyz != nullptr))) return cuda_code(e);
     if (w->desc.dim == MG_END) {
         end_chunk_range(xmin, xmax, zmin, zmax, &cx0, &cz0, &ncx, &ncz);
         /* a table is worth it when samples share chunks; sparse samples evaluate their chunk directly */

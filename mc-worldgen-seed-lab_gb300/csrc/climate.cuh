@@ -139,180 +139,6 @@ static __device__ __noinline__ void climate_ow_d(const MgWorldDesc &W, const MgS
     climate_ow_d_rest(W, S, T, X + sx, Z + sz, depth_grad_d(W, by), tg);
 }
 
-/* Shift noises of a tile, double branch.  Every input of ShiftA (x, 0, z) and ShiftB (z, x, 0) depends on
- * one coordinate: X f + o or Z f + o (first stack), X c f + o or Z c f + o (second stack).  So the cells of a
- * tile column share their X-side splits and smoothsteps, the cells of a row their Z-side ones, and the CTA
- * computes them once per tile into a table (entry (lattice, family, column or row); families: X with the
- * lattice's x offset (ShiftA's x input), X with its y offset (ShiftB's y input), Z with its z offset
- * (ShiftA's z input), Z with its x offset (ShiftB's x input)).  Each cell then runs only the octaves'
- * gradient sums and lerps: the splits and smoothsteps are the per-cell functions' values on the same
- * inputs, so the result is the same to the bit. */
-#define SHIFT_MAXLEV 3                        /* levels of the shift noise the table serves (26.x: 3) */
-struct ShiftSplit {
-    int64_t pk;                               /* fraction in units of 2^-52 | (cell & 255) << 52; -1: not a multiple */
-    double u;                                 /* smoothstep of the fraction */
-};
-template <int TW, int TH>
-struct ShiftTable {
-    ShiftSplit e[2 * SHIFT_MAXLEV][2 * TW + 2 * TH]; /* per lattice: X+ox, X+oy (TW each), Z+oz, Z+ox (TH each) */
-};
-/* true when the world's shift noise fits the table */
-__device__ __forceinline__ bool shift_table_ok(const MgWorldDesc &W) { return W.noise[0].nlev <= SHIFT_MAXLEV; }
-/* the table of the tile whose first cell is (qx0, qz0); all threads of the block take part */
-template <int TW, int TH, int NT>
-__device__ __forceinline__ void shift_table_fill(const MgNoise &N, const MgLattice *__restrict__ T, int qx0, int qz0,
-                                                 ShiftTable<TW, TH> &tab) {
-    const int per = 2 * TW + 2 * TH, nl = 2 * N.nlev;
-    const MgLattice *A = T + N.base;
-    for (int e = threadIdx.x; e < nl * per; e += NT) {
-        const int j = e / per, r = e % per; /* r: the entry's place in the lattice's row of the table */
-        const int fam = r < 2 * TW ? r / TW : 2 + (r - 2 * TW) / TH;
-        const int idx = r < 2 * TW ? r % TW : (r - 2 * TW) % TH;
-        const int st = j >= N.nlev, k = j - st * N.nlev;
-        const MgLattice *L = A + j;
-        double c = fam < 2 ? (double)(qx0 + idx) : (double)(qz0 + idx);
-        if (st) c = c * MG_SECOND_STACK;
-        const double off = fam == 0 ? L->ox : (fam == 1 ? L->oy : (fam == 2 ? L->oz : L->ox));
-        int i;
-        double fr;
-        int64_t F;
-        split_dk(c, N.freq[k], N.fexp[k], off, i, fr, F);
-        ShiftSplit &o = tab.e[j][r];
-        o.pk = F < 0 ? -1 : (F | ((int64_t)(i & 255) << 52));
-        o.u = F < 0 ? 0.0 : fade<double>(fr);
-    }
-}
-struct ShiftPair {
-    double a, b; /* ShiftA, ShiftB */
-    bool ok;
-};
-/* both shift noises of the cell in column col and row row from the table (same sums as nn_d); ok false when
- * an entry or a zero coordinate's split is not a multiple of 2^-52 (the per-cell form handles the cell) */
-template <int TW, int TH>
-static __device__ __noinline__ ShiftPair shift_from_table(const MgNoise &N, const MgLattice *__restrict__ T,
-                                                          const ShiftTable<TW, TH> &tab, int col, int row) {
-    const int64_t M52 = (1LL << 52) - 1;
-    double sa[2] = {0.0, 0.0}, sb[2] = {0.0, 0.0};
-    const MgLattice *A = T + N.base;
-    /* one octave per step (ShiftA and ShiftB of each level and stack in turn; each sum keeps its order): one
-     * copy of the octave code, where two per step measured slower, the hot code no longer fitting the
-     * instruction cache */
-#pragma unroll 1
-    for (int e = 0; e < 4 * N.nlev; e++) {
-        const int q = e >> 1, isb = e & 1, k = q >> 1, st = q & 1, j = st * N.nlev + k;
-        const MgLattice *L = A + j;
-        const ShiftSplit ex = tab.e[j][col], ey = tab.e[j][TW + col], ez = tab.e[j][2 * TW + row],
-                         ew = tab.e[j][2 * TW + TH + row];
-        if ((ex.pk | ey.pk | ez.pk | ew.pk | L->Fy | L->Fz) < 0) return ShiftPair{0.0, 0.0, false};
-        const PlainPerm p{L->p};
-        const ShiftSplit sx = isb ? ew : ex, sz = isb ? ey : ez;
-        const int ix = (int)(sx.pk >> 52), iy = isb ? (int)(sz.pk >> 52) : L->iy;
-        const int64_t FX = sx.pk & M52, FY = isb ? (sz.pk & M52) : L->Fy;
-        const double u = sx.u, v = isb ? sz.u : L->uyd;
-        const int iz = isb ? L->iz : (int)(sz.pk >> 52);
-        const int64_t FZ = isb ? L->Fz : (sz.pk & M52);
-        const double w = isb ? L->uzd : sz.u;
-        const double o = octave_dfix_u(p, ix, FX, u, iy, FY, v, iz, FZ, w);
-        const double t = N.amp_d[k] * o * N.vf_d[k];
-        if (isb) { if (st) sb[1] += t; else sb[0] += t; }
-        else { if (st) sa[1] += t; else sa[0] += t; }
-    }
-    return ShiftPair{(sa[0] + sa[1]) * N.vfac, (sb[0] + sb[1]) * N.vfac, true};
-}
-/* the double branch's Overworld climate of a tile cell, the shifts from the tile's table; g the tile's depth
- * gradient, depth_grad_d(W, 4 qy) */
-template <int TW, int TH>
-__device__ __forceinline__ void climate_ow_d_tab(const MgWorldDesc &W, const MgSpline &S, const MgLattice *__restrict__ T,
-                                                 const ShiftTable<TW, TH> &tab, int col, int row, int qx, int qy, int qz,
-                                                 double g, int32_t *tg) {
-    const ShiftPair sp = shift_from_table(W.noise[0], T, tab, col, row);
-    const double X = (double)qx, Z = (double)qz;
-    if (!sp.ok) {
-        climate_ow_d(W, S, T, X, Z, X * MG_SECOND_STACK, Z * MG_SECOND_STACK, qy * 4, tg);
-        return;
-    }
-    climate_ow_d_rest(W, S, T, X + sp.a * 4.0, Z + sp.b * 4.0, g, tg);
-}
-
-/* The float branch's shift noises of a tile from a table, as the double branch's: the entries are the float
- * splits (cell, fraction) and the fraction's smoothstep that oct_f computes per cell, on the same inputs (the
- * same families of X- and Z-side coordinates), so each cell's octaves run on the same values and give the same
- * bits; the sums keep nn_f's order. */
-struct ShiftSplitF {
-    int32_t i;  /* cell */
-    float f, u; /* fraction, its smoothstep */
-};
-template <int TW, int TH>
-struct ShiftTableF {
-    ShiftSplitF e[2 * SHIFT_MAXLEV][2 * TW + 2 * TH]; /* per lattice: X+ox, X+oy (TW each), Z+oz, Z+ox (TH each) */
-};
-template <int TW, int TH, int NT>
-__device__ __forceinline__ void shift_table_fill_f(const MgNoise &N, const MgLattice *__restrict__ T, int qx0, int qz0,
-                                                   ShiftTableF<TW, TH> &tab) {
-    const int per = 2 * TW + 2 * TH, nl = 2 * N.nlev;
-    const MgLattice *A = T + N.base;
-    for (int e = threadIdx.x; e < nl * per; e += NT) {
-        const int j = e / per, r = e % per;
-        const int fam = r < 2 * TW ? r / TW : 2 + (r - 2 * TW) / TH;
-        const int idx = r < 2 * TW ? r % TW : (r - 2 * TW) % TH;
-        const int st = j >= N.nlev, k = j - st * N.nlev;
-        const MgLattice *L = A + j;
-        double c = fam < 2 ? (double)(qx0 + idx) : (double)(qz0 + idx);
-        if (st) c = c * MG_SECOND_STACK;
-        const double off = fam == 0 ? L->ox : (fam == 1 ? L->oy : (fam == 2 ? L->oz : L->ox));
-        int i;
-        float fr;
-        split_fk(c, N.freq[k], N.fexp[k], off, i, fr);
-        ShiftSplitF &o = tab.e[j][r];
-        o.i = i;
-        o.f = fr;
-        o.u = fade<float>(fr);
-    }
-}
-/* ShiftA and ShiftB of the cell in column col and row row (nn_f's values: level by level, first stack then
- * second, each sum in its own order), one octave per loop step */
-template <int TW, int TH>
-static __device__ __noinline__ float2 shift_from_table_f(const MgNoise &N, const MgLattice *__restrict__ T,
-                                                         const ShiftTableF<TW, TH> &tab, int col, int row) {
-    float sa = 0.0f, sb = 0.0f;
-    const MgLattice *A = T + N.base;
-#pragma unroll 1
-    for (int e = 0; e < 4 * N.nlev; e++) {
-        const int q = e >> 1, isb = e & 1, k = q >> 1, st = q & 1, j = st * N.nlev + k;
-        const MgLattice *L = A + j;
-        /* ShiftA (x, 0, z): x input X + ox, z input Z + oz, y from the header; ShiftB (z, x, 0): x input Z + ox,
-         * y input X + oy, z from the header */
-        const ShiftSplitF ex = isb ? tab.e[j][2 * TW + TH + row] : tab.e[j][col];
-        const ShiftSplitF eo = isb ? tab.e[j][TW + col] : tab.e[j][2 * TW + row];
-        const int iy = isb ? eo.i : L->iy, iz = isb ? L->iz : eo.i;
-        const float fy = isb ? eo.f : L->z0.f.fy, fz = isb ? L->z0.f.fz : eo.f;
-        const float v = isb ? eo.u : L->z0.f.uy, w = isb ? L->z0.f.uz : eo.u;
-        const float o = octave_q<float>(PlainPerm{L->p}, ex.i, ex.f, iy, fy, fy - 1.0f, v, iz, fz, fz - 1.0f, w);
-        const float t = N.amp_f[k] * o;
-        if (isb) sb += t;
-        else sa += t;
-    }
-    return make_float2(sa, sb);
-}
-/* the float branch's Overworld climate of a tile cell, the shifts from the tile's table (climate_ow<true>'s
- * values) */
-template <int TW, int TH>
-__device__ __forceinline__ void climate_ow_f_tab(const MgWorldDesc &W, const MgSpline &S, const MgLattice *__restrict__ T,
-                                                 const ShiftTableF<TW, TH> &tab, int col, int row, int qx, int qy, int qz,
-                                                 int32_t tg[6]) {
-    const double X = (double)qx, Z = (double)qz;
-    const float2 sh = shift_from_table_f(W.noise[0], T, tab, col, row);
-    const float sx = sh.x * 4.0f, sz = sh.y * 4.0f;
-    const double x = X + (double)sx, z = Z + (double)sz;
-    const double xc = x * MG_SECOND_STACK, zc = z * MG_SECOND_STACK;
-    const float tv = nn_f_y0(W.noise[1], T, x, z, xc, zc);
-    const float hv = nn_f_y0(W.noise[2], T, x, z, xc, zc);
-    const float cv = nn_f_y0(W.noise[3], T, x, z, xc, zc);
-    const float ev = nn_f_y0(W.noise[4], T, x, z, xc, zc);
-    const float rv = nn_f_y0(W.noise[5], T, x, z, xc, zc);
-    climate_finish_f(W, S, tv, hv, cv, ev, rv, qy * 4, tg);
-}
-
 /* Overworld climate of quart cell (qx, qy, qz) -> 6 quantised targets (engine/mc_climate.h:113-170). */
 template <bool FM>
 __device__ __forceinline__ void climate_ow(const MgWorldDesc &W, const MgSpline &S, const MgLattice *__restrict__ T,
@@ -640,21 +466,6 @@ __device__ int cell_chunk_chain(const MgWorldDesc &W, const MgSpline &S, const M
     }
     if (node_dist(tree[leaf], tg0) != d0) leaf = leaf0; /* the cell's own step */
     return tree[leaf].biome;
-}
-/* cell_chunk for the 32 neighbouring cells of a warp (all lanes call it, inactive lanes get -1): the cell's
- * own search is the warp-shared walk; the chain (rare) runs per lane. */
-template <bool FM, int DIM>
-__device__ __forceinline__ int cell_chunk_warp(const MgWorldDesc &W, const MgSpline &S, const MgLattice *__restrict__ T,
-                                               const MgTreeNode *__restrict__ tree, int qx, int qy, int qz, bool active) {
-    const int qmin = W.min_y >> 2, qh = W.height >> 2;
-    const int cy = qy < qmin ? qmin : (qy > qmin + qh - 1 ? qmin + qh - 1 : qy);
-    int32_t tg[6] = {0, 0, 0, 0, 0, 0};
-    if (active) cell_target<FM, DIM>(W, S, T, qx, cy, qz, tg);
-    uint64_t d = 0;
-    bool tied = false;
-    const int leaf = tree_search_tie_warp(tree, W, tg, active, d, tied);
-    if (!active) return -1;
-    return cell_chunk_chain<FM, DIM>(W, S, T, tree, qx, qy, qz, tg, leaf, d, tied);
 }
 /* world_biome_cell (libmcgen/src/biome.c:87-114): y clamped into the dimension; a tied cell walks back along
  * LevelChunkSection.fillBiomesFromNoise order (sections bottom-up, then x, y, z) to an untied cell or the

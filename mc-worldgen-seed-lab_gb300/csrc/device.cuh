@@ -1361,13 +1361,15 @@ __device__ __forceinline__ bool rt_warp(const MgTreeNode *__restrict__ T, const 
     return true;
 }
 /* tree_search (no candidate) for 32 unrelated targets, called by all 32 lanes (inactive ones get -1): one after another, each
- * by the whole warp.  A lane alone visits 120 to 200 nodes, and lanes with unrelated targets diverge at most of them (2,000
+ * by the whole warp; tied: whether a second leaf is as near.  A lane alone visits 120 to 200 nodes, and lanes with unrelated targets diverge at most of them (2,000
  * instructions per target); the warp looks at 32 boxes at once (10 steps of 40). */
-__device__ __forceinline__ int tree_search_lanes(const MgTreeNode *__restrict__ T, const MgWorldDesc &W, const int32_t *t, bool active) {
+__device__ __forceinline__ int tree_search_lanes(const MgTreeNode *__restrict__ T, const MgWorldDesc &W, const int32_t *t, bool active,
+                                                 bool *tied = nullptr) {
     const unsigned FULL = 0xFFFFFFFFu;
     RtTarget q{};
     const bool ok = active && rt_packed(T) && rt_target(T, t, q);
     int leaf = -1;
+    bool tie = false;
     for (unsigned m = __ballot_sync(FULL, ok); m; m &= m - 1) {
         const int src = __ffs((int)m) - 1;
         RtTarget s;
@@ -1377,11 +1379,16 @@ __device__ __forceinline__ int tree_search_lanes(const MgTreeNode *__restrict__ 
             s.n[k] = __shfl_sync(FULL, q.n[k], src);
         }
         const RtWarp r = rt_point(T, W, s, 0xFFFFFFFEu);
-        if ((int)(threadIdx.x & 31) == src) leaf = r.leaf;
+        if ((int)(threadIdx.x & 31) == src) {
+            leaf = r.leaf;
+            tie = r.cnt >= 2;
+        }
     }
+    if (tied) *tied = tie;
     if (!active) return -1;
     uint64_t d;
-    return leaf >= 0 ? W.leaf_off + leaf : tree_search_stack(T, t, -1, d);
+    if (leaf >= 0) return W.leaf_off + leaf;
+    return tied ? tree_search_tie_stack(T, t, d, *tied) : tree_search_stack(T, t, -1, d);
 }
 /* tree_search (no candidate) for the 32 neighbouring cells of a warp, called by all 32 lanes; inactive lanes get -1.
  * NEAR: in the lanes that ask for it (sure), sure = every target one unit away in one dimension has this biome too. */

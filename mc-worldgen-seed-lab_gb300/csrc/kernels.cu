@@ -5,11 +5,13 @@
  *                   k_setup_legacy  Nether biome noises: java.util.Random, octaves from the zero octave down
  *                   k_setup_end     End island simplex: LCG(seed) jumped 17292 steps, one shuffle
  *  per-point        k_points        seeds x quart points (ENGINE tie rule), lattices read through L1
- *                   k_grid          one seed's quart grid, lattices staged in shared memory;
+ *                   k_grid          the Nether's quart grid, lattices staged in shared memory;
  *                                   ENGINE biomes or GRID_CHAIN records (leaf, fitness, tie flag, target)
+ *                   (the Overworld's grids and block maps: owtile.cu)
  *                   k_chain_resolve GRID_CHAIN replay for the (rare) tied cells
  *                   k_blockgrid     libmcgen mcgen_biome_grid: BiomeManager zoom + chunk-cell tie chain
- *                   k_end_chunks    End island class per chunk, 8 x 8-chunk tiles (endtile.cuh)
+ *                   k_end_chunks    End island class per chunk, tiles of chunks (endtile.cuh)
+ *                   k_end_samples, k_block_points  sparse End samples, block points: one per warp
  */
 #include <cuda_runtime.h>
 #include <stddef.h>
@@ -165,7 +167,8 @@ __global__ void __launch_bounds__(128) k_points(const __grid_constant__ MgWorldD
         for (int k = 0; k < 6; k++) targets[g * 6 + k] = tg[k];
 }
 
-/* One seed's quart grid.  ENGINE: biome ids.  GRID_CHAIN: first minimum leaf, its fitness, tie flag and
+/* One seed's quart grid, a thread per cell: the Nether's, and the Overworld's of worlds that the tile kernels do not take
+ * (ow_tile_supported).  ENGINE: biome ids.  GRID_CHAIN: first minimum leaf, its fitness, tie flag and
  * the target of every cell, for k_chain_resolve. */
 template <bool FM, int DIM, bool CHAIN>
 __global__ void __launch_bounds__(128) k_grid(const __grid_constant__ MgWorldDesc W, const MgTreeNode *__restrict__ tree,
@@ -175,44 +178,13 @@ __global__ void __launch_bounds__(128) k_grid(const __grid_constant__ MgWorldDes
     MgSpline *S = reinterpret_cast<MgSpline *>(smem_raw);
     MgLattice *T = reinterpret_cast<MgLattice *>(S + 1);
     stage(W, state, W.ntables, T, S, DIM == MG_OVERWORLD);
-    /* 8 x 16-cell tiles: an Overworld tile computes its shift noises' splits once per column and row
-     * (shift_table_fill, shift_table_fill_f) */
-    const int tw = (nx + 7) / 8;
-    const int col = threadIdx.x % 8, row = threadIdx.x / 8;
-    const int tx0 = (int)(blockIdx.x % (unsigned)tw) * 8, tz0 = (int)(blockIdx.x / (unsigned)tw) * 16;
-    ShiftTable<8, 16> *tab = nullptr;
-    ShiftTableF<8, 16> *tabf = nullptr;
-    __shared__ double depth_g; /* with a table: the depth gradient at qy (depth_grad_d), once per CTA */
-    if (DIM == MG_OVERWORLD && shift_table_ok(W)) {
-        __syncthreads(); /* the lattices are staged */
-        if (FM) {
-            tabf = reinterpret_cast<ShiftTableF<8, 16> *>(T + W.ntables);
-            shift_table_fill_f<8, 16, 128>(W.noise[0], T, qx0 + tx0, qz0 + tz0, *tabf);
-        } else {
-            tab = reinterpret_cast<ShiftTable<8, 16> *>(T + W.ntables);
-            shift_table_fill<8, 16, 128>(W.noise[0], T, qx0 + tx0, qz0 + tz0, *tab);
-            if (threadIdx.x == 127) depth_g = depth_grad_d(W, qy * 4);
-        }
-    }
     __syncthreads();
-    const int ix = tx0 + col, iz = tz0 + row;
-    const bool in = ix < nx && iz < nz;
+    const int tw = (nx + 7) / 8; /* 8 x 16-cell tiles */
+    const int ix = (int)(blockIdx.x % (unsigned)tw) * 8 + threadIdx.x % 8, iz = (int)(blockIdx.x / (unsigned)tw) * 16 + threadIdx.x / 8;
+    if (ix >= nx || iz >= nz) return;
     const long long g = (long long)iz * nx + ix;
-    if (FM && !CHAIN && DIM == MG_OVERWORLD) { /* one pruned search per warp */
-        int32_t tg[6] = {0, 0, 0, 0, 0, 0};
-        if (in) {
-            if (FM && tabf) climate_ow_f_tab(W, *S, T, *tabf, col, row, qx0 + ix, qy, qz0 + iz, tg);
-            else cell_target<FM, DIM>(W, *S, T, qx0 + ix, qy, qz0 + iz, tg);
-        }
-        const int leaf = tree_search_warp(tree, W, tg, in);
-        if (in) out[g] = tree[leaf].biome;
-        return;
-    }
-    if (!in) return;
     int32_t tg[6];
-    if (!FM && DIM == MG_OVERWORLD && tab) climate_ow_d_tab(W, *S, T, *tab, col, row, qx0 + ix, qy, qz0 + iz, depth_g, tg);
-    else if (FM && DIM == MG_OVERWORLD && tabf) climate_ow_f_tab(W, *S, T, *tabf, col, row, qx0 + ix, qy, qz0 + iz, tg);
-    else cell_target<FM, DIM>(W, *S, T, qx0 + ix, qy, qz0 + iz, tg);
+    cell_target<FM, DIM>(W, *S, T, qx0 + ix, qy, qz0 + iz, tg);
     uint64_t d;
     if (CHAIN) {
         bool tied;
@@ -273,7 +245,8 @@ __global__ void k_chain_resolve_ordered(const MgTreeNode *__restrict__ tree, con
     out[order[p]] = tree[leaf].biome;
 }
 
-/* mcgen_biome_grid: out[iz*nx+ix] = biome_at(x0 + ix*step, y, z0 + iz*step) (libmcgen/src/region.c:86-108) */
+/* (the Nether's, the End's by a table of classes, and the Overworld's of worlds that the tile kernels do not take)
+ * mcgen_biome_grid: out[iz*nx+ix] = biome_at(x0 + ix*step, y, z0 + iz*step) (libmcgen/src/region.c:86-108) */
 template <bool FM, int DIM>
 __global__ void __launch_bounds__(128, 6) k_blockgrid(const __grid_constant__ MgWorldDesc W, const MgTreeNode *__restrict__ tree,
                                                    const MgLattice *__restrict__ state, int64_t zseed, int x0, int z0,
@@ -286,20 +259,6 @@ __global__ void __launch_bounds__(128, 6) k_blockgrid(const __grid_constant__ Mg
     if (DIM != MG_END) {
         stage(W, state, W.ntables, T, S, DIM == MG_OVERWORLD);
         __syncthreads();
-    }
-    /* grids (the launcher sizes the grid in tiles for this form): the CTA takes a 16 x 8-cell tile and each warp an 8 x 4 block
-     * of it, neighbours whose targets are close, so the cells' own R-tree searches share one pruning (the chunk-cell chain,
-     * rare, stays per lane); not for scattered points or sparse grids, whose warps' targets are unrelated */
-    if (FM && DIM == MG_OVERWORLD && !xyz && step <= 16) {
-        const int tw = (nx + 15) / 16, w = threadIdx.x >> 5, l = threadIdx.x & 31;
-        const int ix = (int)(blockIdx.x % tw) * 16 + (w & 1) * 8 + (l & 7);
-        const int iz = (int)(blockIdx.x / tw) * 8 + (w >> 1) * 4 + (l >> 3);
-        const bool in = ix < nx && iz < nz;
-        int cx = 0, cy = 0, cz = 0;
-        if (in) zoom_cell(zseed, x0 + ix * step, y, z0 + iz * step, cx, cy, cz);
-        const int b = cell_chunk_warp<FM, DIM>(W, *S, T, tree, cx, cy, cz, in);
-        if (in) out[(long long)iz * nx + ix] = (uint8_t)b;
-        return;
     }
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = g < (long long)nx * nz;
@@ -380,11 +339,6 @@ static void end_chunks(const MgWorldDesc &W, const MgLattice *state, int cx0, in
     count_launch();
 }
 static size_t grid_smem(const MgWorldDesc &W) { return sizeof(MgSpline) + (size_t)W.ntables * sizeof(MgLattice); }
-/* k_grid's: the Overworld adds its tiles' shift table */
-static size_t grid_smem_k(const MgWorldDesc &W) {
-    return grid_smem(W) + (W.dim == MG_OVERWORLD ? (W.fmode ? sizeof(ShiftTableF<8, 16>) : sizeof(ShiftTable<8, 16>)) : 0);
-}
-
 int launch_setup(const MgWorldDesc &W, const int64_t *d_seeds, int ns, MgLattice *d_states, cudaStream_t st) {
     if (ns <= 0) return 0;
     if (W.dim == MG_OVERWORLD) {
@@ -477,7 +431,7 @@ int launch_density(const MgWorldDesc &W, const MgLattice *state, int n, const in
 template <bool FM, int DIM, bool CHAIN>
 static void grid_t(const MgWorldDesc &W, const MgTreeNode *tree, const MgLattice *state, int qx0, int qz0, int nx, int nz,
                    int qy, uint8_t *out, ChainRec *rec, cudaStream_t st) {
-    size_t sm = grid_smem_k(W);
+    size_t sm = grid_smem(W);
     cudaFuncSetAttribute(k_grid<FM, DIM, CHAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     const long long tiles = (long long)((nx + 7) / 8) * ((nz + 15) / 16);
     { ProfScope ps_(K_GRID, st); k_grid<FM, DIM, CHAIN><<<(unsigned)tiles, 128, sm, st>>>(W, tree, state, qx0, qz0, nx, nz, qy, out, rec); }
@@ -499,12 +453,10 @@ int launch_end_lookup(const MgWorldDesc &W, const uint8_t *cls, int cx0, int cz0
 /* chain records and their order, then (Overworld) the tile kernels' scratch */
 static size_t chain_bytes(long long n) { return ((size_t)n * (sizeof(ChainRec) + sizeof(int32_t)) + 15) & ~(size_t)15; }
 static bool chain_rule(int rule) { return rule == MG_TIE_GRID_CHAIN || rule == MG_TIE_CHUNK_ORDER; }
-/* cell indices of a tile grid are 32-bit */
-static bool quart_tiles(const MgWorldDesc &W, long long n) { return ow_tile_supported(W) && n < (1LL << 31); }
 size_t quart_scratch_bytes(const MgWorldDesc &W, int rule, int nx, int nz) {
     if (W.dim == MG_END) return (size_t)(nx / 4 + 3) * (size_t)(nz / 4 + 3);
     const long long n = (long long)nx * nz;
-    return (chain_rule(rule) ? chain_bytes(n) : 0) + (quart_tiles(W, n) ? ow_grid_scratch_bytes(W, false, n) : 0);
+    return (chain_rule(rule) ? chain_bytes(n) : 0) + (ow_tile_supported(W) ? ow_grid_scratch_bytes(W, false, n) : 0);
 }
 int launch_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const MgLattice *state, int qx0, int qz0,
                       int nx, int nz, int qy, int rule, uint8_t *out, void *scratch, cudaStream_t st) {
@@ -521,11 +473,16 @@ int launch_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const Mg
     }
     const bool chain = chain_rule(rule);
     ChainRec *rec = (ChainRec *)scratch;
-    if (quart_tiles(W, n)) {
+    if (ow_tile_supported(W)) {
         uint8_t *more = chain ? (uint8_t *)scratch + chain_bytes(n) : (uint8_t *)scratch;
-        const int rc = launch_ow_quart_grid(W, d_world, tree, state, qx0, qz0, nx, nz, qy, chain ? rec : nullptr, out,
-                                            ow_grid_scratch_bytes(W, false, n) ? more : nullptr, st);
-        if (rc) return rc;
+        const int rows = (int)(0x7FFFFFFF / nx); /* cell indices of a tile grid are 32-bit */
+        for (int z = 0; z < nz; z += rows) {
+            const size_t at = (size_t)z * (size_t)nx;
+            const int rc = launch_ow_quart_grid(W, d_world, tree, state, qx0, qz0 + z, nx, rows < nz - z ? rows : nz - z, qy,
+                                                chain ? rec + at : nullptr, out + at, ow_grid_scratch_bytes(W, false, n) ? more : nullptr, st);
+            if (rc) return rc;
+            if (rows >= nz - z) break;
+        }
     } else if (W.fmode) {
         if (W.dim == MG_OVERWORLD) {
             if (chain) grid_t<true, MG_OVERWORLD, true>(W, tree, state, qx0, qz0, nx, nz, qy, out, rec, st);
@@ -571,7 +528,8 @@ static void blockgrid_t(const MgWorldDesc &W, const MgTreeNode *tree, const MgLa
     if constexpr (DIM != MG_END) {
         /* the Nether's cells are cheap enough for a thread each once there are enough of them (26.1: 3,000 points 19.8 us by warps,
          * 22.0 by threads; 14,108 points 67.6 and 30.5) */
-        if (xyz && (DIM == MG_OVERWORLD || nx <= 3072)) {
+        const bool lanes = DIM == MG_OVERWORLD ? W.noise[0].nlev <= 8 : W.ntables <= 32; /* wc_target's lists */
+        if (xyz && lanes && (DIM == MG_OVERWORLD || nx <= 3072)) {
             const long long nb = ((long long)nx + 3) / 4;
             k_block_points<FM, DIM><<<(unsigned)(nb < 16 * 152 ? nb : 16 * 152), 128, sizeof(WcStage), st>>>(W, tree, state, zseed, xyz, nx,
                                                                                                           out);
@@ -579,16 +537,14 @@ static void blockgrid_t(const MgWorldDesc &W, const MgTreeNode *tree, const MgLa
         }
     }
     if (sm) cudaFuncSetAttribute(k_blockgrid<FM, DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    /* the kernel's warp-tile form (its own test of the same condition): one CTA per 16 x 8-cell tile */
-    const bool tiles = FM && DIM == MG_OVERWORLD && !xyz && step <= 16;
-    const unsigned nb = tiles ? (unsigned)(((long long)(nx + 15) / 16) * ((nz + 7) / 8)) : blocks_for((long long)nx * nz, 128);
+    const unsigned nb = blocks_for((long long)nx * nz, 128);
     k_blockgrid<FM, DIM><<<nb, 128, sm, st>>>(W, tree, state, zseed, x0, z0, nx, nz, step, y, xyz, out, cls, ecx0, ecz0,
                                               encx);
 }
 /* the scratch holds only the record of open cells, and without it (null) those are evaluated where they occur */
 bool quart_scratch_optional(const MgWorldDesc &W, int rule) { return W.dim == MG_OVERWORLD && !chain_rule(rule); }
-size_t block_scratch_bytes(const MgWorldDesc &W, int x0, int z0, int nx, int nz, int step, bool points) {
-    return W.dim == MG_OVERWORLD && !points && ow_block_grid_supported(W, x0, z0, step) ? ow_grid_scratch_bytes(W, true, (long long)nx * nz) : 0;
+size_t block_scratch_bytes(const MgWorldDesc &W, int x0, int z0, int nx, int nz, bool points) {
+    return W.dim == MG_OVERWORLD && !points && ow_block_grid_supported(W, x0, z0) ? ow_grid_scratch_bytes(W, true, (long long)nx * nz) : 0;
 }
 /* Block-coordinate biomes: a grid (xyz == nullptr) or n = nx points (nz == 1) at xyz. For the End,
  * `scratch` holds the chunk classes of [ecx0, ecx0+encx) x [ecz0, ecz0+encz). */
@@ -596,7 +552,7 @@ int launch_block_biomes(const MgWorldDesc &W, const MgWorldDesc *d_world, const 
                         int x0, int z0, int nx, int nz, int step, int y, const int32_t *xyz, uint8_t *out, void *scratch,
                         int ecx0, int ecz0, int encx, int encz, cudaStream_t st) {
     if ((long long)nx * nz <= 0) return 0;
-    if (W.dim == MG_OVERWORLD && !xyz && ow_block_grid_supported(W, x0, z0, step))
+    if (W.dim == MG_OVERWORLD && !xyz && ow_block_grid_supported(W, x0, z0))
         return launch_ow_block_grid(W, d_world, tree, state, zseed, x0, z0, nx, nz, step, y, out, scratch, st);
     uint8_t *cls = (uint8_t *)scratch; /* End chunk classes, or null: evaluate per sample */
     if (W.dim == MG_END && cls) {

@@ -46,14 +46,14 @@ int launch_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const Mg
 /* block-coordinate biomes (zoom + chunk-cell ties): a grid when xyz == nullptr, else nx points at xyz
  * (nz == 1).  d_world: the description's device copy.  Scratch: block_scratch_bytes; for the End the chunk classes of
  * [ecx0, ecx0+encx) x [ecz0, ecz0+encz), or null to evaluate the class per sample. */
-size_t block_scratch_bytes(const MgWorldDesc &W, int x0, int z0, int nx, int nz, int step, bool points);
+size_t block_scratch_bytes(const MgWorldDesc &W, int x0, int z0, int nx, int nz, bool points);
 int launch_block_biomes(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const MgLattice *state, int64_t zseed,
                         int x0, int z0, int nx, int nz, int step, int y, const int32_t *xyz, uint8_t *out, void *scratch,
                         int ecx0, int ecz0, int encx, int encz, cudaStream_t st);
 
-/* the same through the tile kernels (owtile.cu), for worlds ow_tile_supported takes and blocks at most 4 apart.  rec: the
+/* the same through the tile kernels (owtile.cu), for worlds ow_tile_supported takes.  rec: the
  * cells' chain records, or null.  Scratch: ow_grid_scratch_bytes. */
-bool ow_block_grid_supported(const MgWorldDesc &W, int x0, int z0, int step);
+bool ow_block_grid_supported(const MgWorldDesc &W, int x0, int z0);
 size_t ow_grid_scratch_bytes(const MgWorldDesc &W, bool chunk_rule, long long cells);
 int launch_ow_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const MgLattice *state, int qx0,
                          int qz0, int nx, int nz, int qy, ChainRec *rec, uint8_t *out, void *scratch, cudaStream_t st);

@@ -709,6 +709,134 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const __grid_constant__ OtWor
     overlap_wait();
 }
 
+/* ============================================================================ sparse block maps
+ * Blocks more than 4 apart: neighbouring cells share too few nodes for a tile's tables, so each is evaluated by its lane: the float
+ * branch by the per-cell form, the double branch in the tiles' fixed point with its octaves' edges built on the way (per cell in
+ * double, its shift noises took 864 FP64 operations).  Tied cells and open targets are left to k_ow_open like the tiles'.  The
+ * lattices, spline and fixed coordinates' parts are in shared memory; warps take 8 x 4 cells, whose tree search they share up to 16
+ * blocks apart (a box of 4 x 8 chunks of terrain) and do one by one beyond.  256 x 256 blocks, spacing 16: 26.1 531 -> 205 us, 26.3 379
+ * -> 237 us; spacing 37: 578 -> 313, 552 -> 229 (its search shared: 324 and 288). */
+struct OtSparse {
+    WcStage st;
+    OtFix fix[MG_MAX_TABLES], fz[2 * OT_MAXLEV]; /* of the y plane; the shift's z plane */
+    int64_t off[MG_MAX_TABLES][2];               /* offsets in units of 2^-32 */
+    int32_t depth[2];
+};
+template <bool FM>
+__global__ void __launch_bounds__(128, 4) k_ow_sparse(const __grid_constant__ OtWork K) {
+    extern __shared__ uint4 smem_raw[];
+    OtSparse &sm = *reinterpret_cast<OtSparse *>(smem_raw);
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const MgWorldDesc &W = K.worlds[0];
+    const MgSpline &S = sm.st.spline;
+    const MgTreeNode *tree = K.tree;
+    const MgNoise &O = W.noise[0];
+    const int nlev = O.nlev, nx = K.one.nx, nz = K.one.nz, tw = (nx + 15) / 16, qy0 = (K.y - 2) >> 2;
+    wc_stage(sm.st, W, K.pool, t, 128);
+    overlap_next();
+    __syncthreads();
+    if (!FM) {
+        for (int l = t; l < W.ntables; l += 128) {
+            const MgLattice &L = sm.st.lat[l];
+            sm.fix[l] = ot_fix(L.fyd, L.uyd);
+            if (l < 2 * nlev) sm.fz[l] = ot_fix(L.fzd, L.uzd);
+            sm.off[l][0] = __double2ll_rn(L.ox * 0x1.0p32);
+            sm.off[l][1] = __double2ll_rn(L.oz * 0x1.0p32);
+        }
+        if (t >= 126) sm.depth[127 - t] = (int32_t)__double2ll_rn((depth_grad_d(W, ot_clamp_y(W, qy0 + 127 - t) * 4) + W.off_d) * 0x1.0p28);
+        __syncthreads();
+    }
+    for (long long tile = blockIdx.x; tile < K.ntiles; tile += gridDim.x) {
+        const int ix = (int)(tile % tw) * 16 + (warp & 1) * 8 + (lane & 7), iz = (int)(tile / tw) * 8 + (warp >> 1) * 4 + (lane >> 3);
+        const bool in = ix < nx && iz < nz;
+        int cx = 0, cy = qy0, cz = 0;
+        if (in) zoom_cell(K.zseed, K.x0 + ix * K.step, K.y, K.z0 + iz * K.step, cx, cy, cz);
+        bool ok = in;
+        int32_t ta[6] = {0, 0, 0, 0, 0, 0}, amb = 0;
+        if (FM) {
+            if (in) climate_ow<true>(W, S, sm.st.lat, cx, ot_clamp_y(W, cy), cz, ta);
+        } else {
+            ok = in && cx > -OT_COORD_LIM && cx < OT_COORD_LIM && cz > -OT_COORD_LIM && cz < OT_COORD_LIM;
+            if (ok) {
+                int64_t sa = 0, sb = 0; /* units of 2^-59 */
+#pragma unroll 1
+                for (int k = 0; k < nlev; k++) {
+                    int64_t va = 0, vb = 0;
+#pragma unroll 1
+                    for (int st = 0; st < 2; st++) {
+                        const int l = st * nlev + k;
+                        const MgLattice &L = sm.st.lat[l];
+                        const PlainPerm P{L.p};
+                        double X = (double)cx, Z = (double)cz;
+                        if (st) { X = X * MG_SECOND_STACK; Z = Z * MG_SECOND_STACK; }
+                        int ia, ib;
+                        int32_t pa, ua, pb, ub;
+                        ot_split_d(X, O.freq[k], L.ox, ia, pa, ua);
+                        ot_split_d(Z, O.freq[k], L.oz, ib, pb, ub);
+                        va += ot_sample_d(P, L.iy, false, sm.fix[l], ia, ib, pa, ua, pb, ub);
+                        ot_split_d(Z, O.freq[k], L.ox, ia, pa, ua);
+                        ot_split_d(X, O.freq[k], L.oy, ib, pb, ub);
+                        vb += ot_sample_d(P, L.iz, true, sm.fz[l], ia, ib, pa, ua, pb, ub);
+                    }
+                    sa = ot_madw((int32_t)(va >> 31), O.c30[k], sa);
+                    sb = ot_madw((int32_t)(vb >> 31), O.c30[k], sb);
+                }
+                const int64_t x = ((int64_t)cx << 32) + (sa >> 25), z = ((int64_t)cz << 32) + (sb >> 25);
+                const int64_t xc = x + __mul64hi(x, OT_STACK_C), zc = z + __mul64hi(z, OT_STACK_C);
+                int32_t v[MG_OW_NOISES - 1], tb[6], eq[MG_OW_NOISES];
+                const bool out17 = max(abs(cx), abs(cz)) >= (1 << 17) - OT_W;
+#pragma unroll 1
+                for (int n = 1; n < MG_OW_NOISES; n++) {
+                    const MgNoise &N = W.noise[n];
+                    int64_t acc = 0;
+#pragma unroll 1
+                    for (int k = 0; k < N.nlev; k++) {
+                        int64_t lev = 0;
+#pragma unroll 1
+                        for (int st = 0; st < 2; st++) {
+                            const int l = N.base + st * N.nlev + k;
+                            const MgLattice &L = sm.st.lat[l];
+                            const int64_t sx = ((st ? xc : x) >> -N.fexp[k]) + sm.off[l][0], sz = ((st ? zc : z) >> -N.fexp[k]) + sm.off[l][1];
+                            lev += ot_sample_d(PlainPerm{L.p}, L.iy, false, sm.fix[l], ot_hi(sx), ot_hi(sz), (int32_t)((uint32_t)sx >> 1),
+                                               ot_fade31((uint32_t)sx), (int32_t)((uint32_t)sz >> 1), ot_fade31((uint32_t)sz));
+                        }
+                        acc = ot_madw((int32_t)(lev >> 31), N.c30[k], acc);
+                    }
+                    const int32_t e = out17 ? N.tile_eq_far : N.tile_eq;
+#pragma unroll
+                    for (int k = 1; k < MG_OW_NOISES; k++) {
+                        v[k - 1] = n == k ? (int32_t)(acc >> 30) : v[k - 1];
+                        eq[k] = n == k ? e : eq[k];
+                    }
+                }
+                float es;
+                ot_climate_targets(W, S, v, eq, sm.depth[cy - qy0], ta, tb, es);
+                ok = es < 1.0f;
+#pragma unroll
+                for (int k = 0; k < 6; k++) {
+                    amb += tb[k] - ta[k];
+                    ok &= (unsigned)(tb[k] - ta[k]) <= 1u;
+                }
+                ok &= amb <= 1;
+            }
+        }
+        uint64_t d;
+        bool tied = false, sure = amb != 0;
+        int leaf;
+        if (K.step <= 16) {
+            if (FM) leaf = tree_search_tie_warp(tree, W, ta, ok, d, tied);
+            else leaf = tree_search_tie_warp<true>(tree, W, ta, ok, d, tied, -1, &sure);
+        } else {
+            leaf = tree_search_lanes(tree, W, ta, ok, &tied);
+            sure = false;
+        }
+        if (!in) continue;
+        const int cell = iz * nx + ix;
+        if (ok && !tied && (!amb || sure)) put_id(K.out + cell, tree[leaf].biome);
+        else ot_leave_open<FM, OT_BLOCK>(K, W, sm.st.lat, tree, 0, cell, cx, cy, cz, cell);
+    }
+}
+
 /* the open cells: up to 65,536 by a warp each (25 us for the first, then its throughput), more by a thread each (200 us for any
  * number).  One grid's lattices and spline are copied to shared memory by each block; a batch's are read through L1.  24 warps
  * per SM: a cell by a warp is a chain of latencies, so its rate is the warps in flight.  Under the chunk-cell rule a block takes
@@ -894,19 +1022,19 @@ size_t ow_grid_scratch_bytes(const MgWorldDesc &W, bool chunk_rule, long long ce
     const long long cap = grid_open_cap(W.fmode != 0, chunk_rule ? OT_BLOCK : OT_CHAIN, cells);
     return cap > 0 ? 16 + (size_t)cap * sizeof(MgOpenCell) : 0;
 }
+static int open_scratch(bool fm, int mode, OtWork &K, void *scratch, cudaStream_t st) {
+    K.open_cap = scratch ? grid_open_cap(fm, mode, (long long)K.one.nx * K.one.nz) : 0;
+    if (K.open_cap <= 0) return 0;
+    K.nopen = (unsigned long long *)scratch;
+    K.open = (MgOpenCell *)((uint8_t *)scratch + 16);
+    return (int)cudaMemsetAsync(K.nopen, 0, sizeof(unsigned long long), st);
+}
 static int grid_run(const MgWorldDesc &W, int mode, OtWork &K, void *scratch, cudaStream_t st) {
     const bool fm = W.fmode != 0;
-    const long long cells = (long long)K.one.nx * K.one.nz;
     K.ntiles = ow_tiles(K.one.nx, K.one.nz);
-    K.open_cap = scratch ? grid_open_cap(fm, mode, cells) : 0;
     int rc = ow_prepare();
+    if (!rc) rc = open_scratch(fm, mode, K, scratch, st);
     if (rc) return rc;
-    if (K.open_cap > 0) {
-        K.nopen = (unsigned long long *)scratch;
-        K.open = (MgOpenCell *)((uint8_t *)scratch + 16);
-        const cudaError_t e = cudaMemsetAsync(K.nopen, 0, sizeof(unsigned long long), st);
-        if (e) return (int)e;
-    }
     rc = launch_tiles(fm, mode, false, K, st);
     return rc ? rc : launch_open(fm, mode, K, st);
 }
@@ -925,8 +1053,27 @@ int launch_ow_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const
     K.one.qy = qy;
     return grid_run(W, rec ? OT_CHAIN : OT_ENGINE, K, scratch, st);
 }
-bool ow_block_grid_supported(const MgWorldDesc &W, int x0, int z0, int step) {
-    return ow_tile_supported(W) && step <= 4 && x0 >= INT32_MIN + 16 && z0 >= INT32_MIN + 16;
+/* blocks more than 4 apart */
+static int sparse_run(const MgWorldDesc &W, OtWork &K, void *scratch, cudaStream_t st) {
+    const bool fm = W.fmode != 0;
+    K.ntiles = (long long)((K.one.nx + 15) / 16) * ((K.one.nz + 7) / 8);
+    int rc = open_scratch(fm, OT_BLOCK, K, scratch, st);
+    if (rc) return rc;
+    rc = (int)(fm ? cudaFuncSetAttribute(k_ow_sparse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(OtSparse))
+                  : cudaFuncSetAttribute(k_ow_sparse<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(OtSparse)));
+    if (rc) return rc;
+    const unsigned grid = (unsigned)(K.ntiles < 4 * 152 ? K.ntiles : 4 * 152);
+    {
+        ProfScope ps_(K_BLOCKGRID, st);
+        if (fm) k_ow_sparse<true><<<grid, 128, sizeof(OtSparse), st>>>(K);
+        else k_ow_sparse<false><<<grid, 128, sizeof(OtSparse), st>>>(K);
+    }
+    count_launch_external();
+    rc = (int)cudaGetLastError();
+    return rc ? rc : launch_open(fm, OT_BLOCK, K, st);
+}
+bool ow_block_grid_supported(const MgWorldDesc &W, int x0, int z0) {
+    return ow_tile_supported(W) && x0 >= INT32_MIN + 16 && z0 >= INT32_MIN + 16;
 }
 int launch_ow_block_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const MgLattice *state, int64_t zseed,
                          int x0, int z0, int nx, int nz, int step, int y, uint8_t *out, void *scratch, cudaStream_t st) {
@@ -942,7 +1089,7 @@ int launch_ow_block_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const
     K.z0 = z0;
     K.step = step;
     K.y = y;
-    return grid_run(W, OT_BLOCK, K, scratch, st);
+    return step <= 4 ? grid_run(W, OT_BLOCK, K, scratch, st) : sparse_run(W, K, scratch, st);
 }
 
 }  // namespace mg
