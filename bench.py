@@ -193,15 +193,13 @@ def gpu_peaks(mg) -> dict:
 # Lattice (octave) samples per biome sample: 52 in the Overworld (six NormalNoises, two stacks each, with
 # the shift noise sampled twice), 8 in the Nether; the oracle's work counter pins both numbers.
 OCTAVES_PER_SAMPLE = {"minecraft:overworld": 52, "minecraft:the_nether": 8, "minecraft:the_end": 0}
-# FP64 operations per sample as the kernels compute them.  Float branch (26.3+): the two rounded coordinate
-# adds of every octave sample (Overworld 52 x 2, Nether 8 x 2).  Double branch (26.1/26.2), Overworld: the
-# shift noise's 12 octave samples exactly in double, their splits and smoothsteps taken from the tile's
-# table (29 each: 8 conversions of the exact gradient sums and differences, 4 first-level lerp products and
-# sums, 3 lerps of 3, the product undoing the 2^52 scale, the amplitude products and sum), the table itself
-# (6 lattices x 48 entries of 8 per 128-cell tile: 18 per sample), and the 40 climate octave samples in
-# 59-bit fixed point with only their 2 coordinate adds on the FP64 pipe (the screens and ridges_folded run
-# on the integer and conversion pipes): 348 + 18 + 80 = 446.  Nether: 8 x 2 = 16.  The rare values the
-# screen leaves to the exact double path and the End's simplex are left out, so the model is a lower bound.
+# FP64 operations per sample of the per-cell forms (points and cells that the tile kernels leave to the exact evaluation).
+# Float branch (26.3+): the two rounded coordinate adds of every octave sample (Overworld 52 x 2, Nether 8 x 2).  Double
+# branch (26.1/26.2), Overworld: the shift noise's 12 octave samples exactly in double (29 each: 8 conversions of the exact
+# gradient sums and differences, 4 first-level lerp products and sums, 3 lerps of 3, the product undoing the 2^52 scale, the
+# amplitude products and sum), their splits and smoothsteps where a tile's cells share them (18 per sample), and the 40 climate
+# octave samples in 59-bit fixed point with only their 2 coordinate adds on the FP64 pipe: 348 + 18 + 80 = 446.  Nether: 16.
+# The tile kernels need less: none per cell in the double branch.
 FP64_PER_SAMPLE = {("double", "minecraft:overworld"): 446, ("double", "minecraft:the_nether"): 16,
                    ("float", "minecraft:overworld"): 104, ("float", "minecraft:the_nether"): 16,
                    ("double", "minecraft:the_end"): 0, ("float", "minecraft:the_end"): 0}
@@ -213,16 +211,28 @@ def batch_fp64_ops(reqs) -> float:
                      for v, d, s, qx0, qz0, n, qy in reqs))
 
 
+# k_ow_d, the double branch's Overworld tiles and the uneven batch's longest kernel: an octave sample in its fixed point is 11
+# 32 x 32 + 64-bit multiply-adds (two rows of 5, one between them), 52 octave samples a cell, each taking 2.5 issue slots of the
+# multiply-add pipe (microbenchmark: 23.8 lanes per SM and clock against 59.9).
+OW_D_MADW_PER_CELL = 52 * 11
+MADW_SLOTS = 2.5
+
+
+def ow_d_mad_ops(reqs) -> float:
+    """32-bit multiply-add slots of the batch's double-branch Overworld octave samples."""
+    cells = sum(n * n for v, d, s, qx0, qz0, n, qy in reqs if v in DOUBLE_BRANCH and d.endswith("overworld"))
+    return cells * OW_D_MADW_PER_CELL * MADW_SLOTS
+
+
 # Algorithmic work per launch of each kernel, counted from the reference algorithm:
 # (work units per launch, unit name, pipe peak key).
-# DRAM bytes (read + write) per work unit of a launch, from one ncu capture each: k_batch per sample
-# (the first 4,000 requests of the uneven batch), k_ow_seed_climate per seed (4,096 seeds x 8 points).
-DRAM_BYTES_PER_UNIT = {"k_batch": (72375552 + 1504797696) / 147087943, "k_ow_seed_climate": 83200 / 4096}
-K_BATCH_TRAFFIC_NOTE = ("DRAM bytes read + written per sample in an ncu capture of one k_batch<8, 8> launch over the "
-                        "first 4,000 requests (147 M samples, an output larger than L2) x this launch's samples; "
-                        "the writes are mostly local-memory write-back (register spills), the ids 1 B per sample")
-# pipe utilisation of k_batch<8, 8> from ncu (sm__inst_executed_pipe_*, issue active) on a 300-request launch
-K_BATCH_PIPES = {"fp64": 0.547, "integer_alu": 0.546, "issue_active": 0.682}
+# DRAM bytes (read + write) per work unit of a launch, from one ncu capture each: k_ow_d per cell (the uneven batch's 4,068
+# requests, an output larger than L2), k_ow_seed_climate per seed (4,096 seeds x 8 points).
+DRAM_BYTES_PER_UNIT = {"k_ow_d": (74819072 + 120869888) / 151592325, "k_ow_seed_climate": 83200 / 4096}
+OW_D_TRAFFIC_NOTE = ("DRAM bytes read + written per cell in an ncu capture of one k_ow_d launch over the batch's double-branch "
+                     "Overworld requests (151.6 M cells, an output larger than L2): the ids 1 B per cell, the lattices")
+# utilisation of k_ow_d from ncu (sm__inst_executed_pipe_*, pipe and issue active) on a 400-request launch
+OW_D_PIPES = {"issue_active": 0.635, "integer_alu": 0.559, "multiply_add_heavy": 0.527, "fp64": 0.162}
 
 
 def kernel_work(kernel: str, seeds8: bool, ns: int, np_: int, ntables: int) -> tuple[float, str, str] | None:
@@ -519,7 +529,7 @@ def run_batch(args, rank, world, local_rank, mg, ge):
            "config": {"workload": f"uneven mixed batch: {len(reqs)} SplitMix64(3) requests, versions 26.1/26.2/26.3, "
                                   "Overworld:Nether:End 6:2:2, square side log-uniform in [16,512) quart cells, origin "
                                   "uniform in [-30000,30000] blocks, y=64, ENGINE tie rule",
-                      "form": "one persistent launch (CUDA graph) vs one plain launch pair per request",
+                      "form": "one launch per code path (CUDA graph) vs one plain launch pair per request",
                       **({"class_only": args.batch_class} if args.batch_class else {}),
                       "requests": len(reqs), "samples_per_step": samples, "tile_shape": plan.shape,
                       "autotune_ms": round(tuned_ms, 3), "l2": f"output {samples/1e6:.0f} MB per step > L2",
@@ -544,17 +554,18 @@ def run_batch(args, rank, world, local_rank, mg, ge):
             out["clocks"] = clocks
         peaks = gpu_peaks(mg) if not args.skip_extras else {}
         out["pipe_peaks_gops"] = peaks
-        if "k_batch" in prof and peaks:
-            ops = batch_fp64_ops(reqs)
-            avg_s = prof["k_batch"][0] / prof["k_batch"][1] * 1e-3
+        if "k_ow_d" in prof and peaks:
+            ops = ow_d_mad_ops(reqs)
+            avg_s = prof["k_ow_d"][0] / prof["k_ow_d"][1] * 1e-3
             achieved = ops / avg_s / 1e9
-            out["roofline"] = {"kernel": "k_batch", "bound": "fp64", "achieved": round(achieved, 1),
-                               "peak": peaks["fp64_add"], "unit": "Gop/s", "frac": round(achieved / peaks["fp64_add"], 4),
-                               "traffic": round(DRAM_BYTES_PER_UNIT["k_batch"] * samples),
-                               "traffic_note": K_BATCH_TRAFFIC_NOTE,
-                               "work": f"{ops:.4g} FP64 ops per launch (per-sample model of the screened evaluation)",
-                               "peak_source": "measured in-run (FP64 add pipe microbenchmark)",
-                               "binding_pipes": K_BATCH_PIPES}
+            out["roofline"] = {"kernel": "k_ow_d", "bound": "issue", "achieved": round(achieved, 1),
+                               "peak": peaks["int32_mad"], "unit": "Gop/s", "frac": round(achieved / peaks["int32_mad"], 4),
+                               "traffic": round(DRAM_BYTES_PER_UNIT["k_ow_d"] * ops / (OW_D_MADW_PER_CELL * MADW_SLOTS)),
+                               "traffic_note": OW_D_TRAFFIC_NOTE,
+                               "work": f"{ops:.4g} multiply-add slots per launch (octave samples alone; tables, spline, quantisation "
+                                       "and R-tree not counted)",
+                               "peak_source": "measured in-run (int32 multiply-add pipe microbenchmark)",
+                               "binding_pipes": OW_D_PIPES}
         if args.split_classes:
             out["classes"] = batch_classes(reqs, worlds, mg, dev, stream)
         if not args.skip_extras:

@@ -86,9 +86,9 @@ __global__ void __launch_bounds__(LNT) k_setup_list_legacy(const MgWorldDesc *__
                                                            MgLattice *__restrict__ pool) {
     __shared__ uint32_t perm[64][LNT];
     const int t = threadIdx.x;
-    const long long g = ((long long)blockIdx.x * LNT + t) / LEGACY_GROUP;
+    const long long g = legacy_index((long long)blockIdx.x * LNT + t);
     overlap_next();
-    if (g >= 2LL * n) return;
+    if (g < 0 || g >= 2LL * n) return;
     const MgSetupEntry &E = ent[g >> 1];
     const MgWorldDesc &W = worlds[E.world];
     const MgNoise &N = W.nether[g & 1];
@@ -264,7 +264,7 @@ int launch_setup_list(const MgWorldDesc *d_worlds, int dim, const MgSetupEntry *
         launch_on(overlap, k_setup_list_xo, (unsigned)((total_lattices + LNT - 1) / LNT), LNT, 0, st, d_worlds, d_ent, n, d_first, total_lattices, d_pool);
     } else if (dim == MG_NETHER) {
         ProfScope ps_(K_SETUP_LEGACY, st);
-        launch_on(overlap, k_setup_list_legacy, (unsigned)((2LL * LEGACY_GROUP * n + LNT - 1) / LNT), LNT, 0, st, d_worlds, d_ent, n, d_pool);
+        launch_on(overlap, k_setup_list_legacy, (unsigned)((legacy_threads(2LL * n) + LNT - 1) / LNT), LNT, 0, st, d_worlds, d_ent, n, d_pool);
     } else {
         ProfScope ps_(K_SETUP_END, st);
         launch_on(overlap, k_setup_list_end, (unsigned)((n + LNT - 1) / LNT), LNT, 0, st, d_ent, n, d_pool);

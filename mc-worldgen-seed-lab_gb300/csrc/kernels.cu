@@ -97,8 +97,8 @@ __global__ void __launch_bounds__(SETUP_NT) k_setup_legacy(const __grid_constant
                                                            int ns, MgLattice *__restrict__ out) {
     __shared__ uint32_t perm[64][SETUP_NT];
     const int t = threadIdx.x;
-    const long long g = ((long long)blockIdx.x * SETUP_NT + t) / LEGACY_GROUP;
-    if (g >= 2LL * ns) return;
+    const long long g = legacy_index((long long)blockIdx.x * SETUP_NT + t);
+    if (g < 0 || g >= 2LL * ns) return;
     const MgNoise &N = W.nether[g & 1];
     MgLattice *T = out + (size_t)(g >> 1) * W.ntables + N.base;
     legacy_noise<SETUP_NT>(N, (int)(g & 1), seeds[g >> 1], &perm[0][t], [&](int i, MgLattice &h) {
@@ -345,7 +345,7 @@ int launch_setup(const MgWorldDesc &W, const int64_t *d_seeds, int ns, MgLattice
         long long n = (long long)ns * W.ntables;
         { ProfScope ps_(K_SETUP_XO, st); k_setup_xo<<<blocks_for(n, SETUP_NT), SETUP_NT, 0, st>>>(W, d_seeds, ns, d_states); }
     } else if (W.dim == MG_NETHER) {
-        { ProfScope ps_(K_SETUP_LEGACY, st); k_setup_legacy<<<blocks_for(2LL * LEGACY_GROUP * ns, SETUP_NT), SETUP_NT, 0, st>>>(W, d_seeds, ns, d_states); }
+        { ProfScope ps_(K_SETUP_LEGACY, st); k_setup_legacy<<<blocks_for(legacy_threads(2LL * ns), SETUP_NT), SETUP_NT, 0, st>>>(W, d_seeds, ns, d_states); }
     } else {
         { ProfScope ps_(K_SETUP_END, st); k_setup_end<<<blocks_for(ns, SETUP_NT), SETUP_NT, 0, st>>>(d_seeds, ns, d_states); }
     }

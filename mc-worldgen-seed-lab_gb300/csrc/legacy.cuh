@@ -23,11 +23,18 @@ __device__ __noinline__ int legacy_octave(uint64_t &s, uint32_t *col, MgLattice 
  * from the state that many draws on; those after a rejection once more, from the state moved on by it.  Six shuffles in a row, 31 us
  * each, were the latency of a small batch: 187 -> 45 us.  A noise with more octaves than lanes is built by the first lane.
  * store(i, h) writes lattice i of the noise from the calling thread's column.  All lanes of the group call it. */
-#define LEGACY_GROUP 8
+#define LEGACY_GROUP 6 /* the game's: three octaves in each of two stacks */
+#define LEGACY_PER_WARP (32 / LEGACY_GROUP)
+/* threads for n noises, in whole blocks' warps; the noise of this thread (its group's), or -1 */
+__host__ __device__ inline long long legacy_threads(long long n) { return (n + LEGACY_PER_WARP - 1) / LEGACY_PER_WARP * 32; }
+__device__ __forceinline__ long long legacy_index(long long thread) {
+    const int lane = (int)(thread & 31);
+    return lane < LEGACY_GROUP * LEGACY_PER_WARP ? (thread >> 5) * LEGACY_PER_WARP + lane / LEGACY_GROUP : -1;
+}
 template <int ROW, typename STORE>
 __device__ __forceinline__ void legacy_noise(const MgNoise &N, int n, int64_t seed, uint32_t *col, const STORE &store) {
-    const int gl = threadIdx.x & (LEGACY_GROUP - 1);
-    const unsigned group = ((1u << LEGACY_GROUP) - 1) << (threadIdx.x & 31 & ~(LEGACY_GROUP - 1));
+    const int gl = (threadIdx.x & 31) % LEGACY_GROUP, first = (threadIdx.x & 31) - gl;
+    const unsigned group = ((1u << LEGACY_GROUP) - 1) << first;
     const uint64_t st = lcg_init((int64_t)((uint64_t)seed + (uint64_t)n));
     const int zero = -N.first;
     auto level = [&](int q) { /* of octave q, or -1 */
@@ -57,7 +64,7 @@ __device__ __forceinline__ void legacy_noise(const MgNoise &N, int n, int64_t se
             }
             before = 0;
             for (int k = 0; k < LEGACY_GROUP - 1; k++) {
-                const int r = __shfl_sync(group, rejected, k, LEGACY_GROUP);
+                const int r = __shfl_sync(group, rejected, first + k);
                 if (k < gl) before += r;
             }
         }
