@@ -68,11 +68,11 @@ MCGEN_API int mcgen_gb300_quart_grid_dev(const McWorld *w, int qx0, int qz0, int
 MCGEN_API int mcgen_gb300_quart_grid_seed_dev(const McWorld *w, int64_t seed, int qx0, int qz0, int nx, int nz,
                                               int qy, int tie_rule, uint8_t *d_out, void *stream);
 
-/* ---- batched form: many biome-map requests of uneven size in one persistent launch ----
+/* ---- batched form: many biome-map requests of uneven size, one persistent launch per code path ----
  * A request is a quart-resolution region (qx0.., qz0.., nx x nz at quart y) of one world (version,
  * dimension, preset) and seed.  A plan freezes a request list: it builds every distinct (world, seed)'s
- * noise lattices into a pool, splits requests into tiles that one persistent kernel takes from a device
- * work queue, and lays outputs back to back (request i's nx*nz ids, row-major, at output offset i).
+ * noise lattices into a pool, splits requests into tiles that one persistent kernel per code path takes from a
+ * device work queue, and lays outputs back to back (request i's nx*nz ids, row-major, at output offset i).
  * Runs replay a CUDA graph of the setup and batch launches.  tie_rule: MCGEN_TIE_ENGINE or
  * MCGEN_TIE_CHUNK_CELL (each cell resolved as the chunk that holds it stores it). */
 typedef struct McGb300Request {
@@ -87,8 +87,8 @@ MCGEN_API int mcgen_gb300_plan_new(const McGb300Request *reqs, int n, int tie_ru
 MCGEN_API void mcgen_gb300_plan_free(McGb300Plan *p);
 MCGEN_API long long mcgen_gb300_plan_output_bytes(const McGb300Plan *p);
 MCGEN_API long long mcgen_gb300_plan_output_offset(const McGb300Plan *p, int i);
-/* the tile shape in use (cells x rows, resident CTAs per SM): 0 (8 x 16, 9), 1 (8 x 16, 7), 2 (8 x 16, 6),
- * 3 (8 x 16, 8) */
+/* the shape in use: the register budget (resident CTAs per SM) of the Nether's and End's kernel, 0 (9), 1 (7), 2 (6), 3 (8);
+ * the Overworld's tiles are 16 x 16 cells in all */
 MCGEN_API int mcgen_gb300_plan_shape(const McGb300Plan *p);
 MCGEN_API int mcgen_gb300_plan_set_shape(McGb300Plan *p, int shape);
 /* bytes plan_new copied to the device (worlds, request and setup lists) */
