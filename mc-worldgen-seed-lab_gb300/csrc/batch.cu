@@ -1,21 +1,16 @@
-/* batch.cu -- many biome-map requests of uneven size in a few persistent launches: Overworld requests under the ENGINE
- * rule go to the tile kernels of owtile.cu, one per branch, everything else to k_batch here.
+/* batch.cu -- many biome-map requests of uneven size in a few persistent launches: the Overworld's go to the tile kernels of
+ * owtile.cu, one per branch, everything else to k_batch here.
  *
  * A request is (world: version + dimension + preset, seed, quart region qx0..qx0+nx-1 x qz0..qz0+nz-1 at
- * quart y, tie rule).  The host splits every request into tiles -- 128 quart cells (8 x 16; the autotuner
- * picks the register budget) for Overworld and Nether, 8 x 8 chunks (32 x 32 quart cells) for the End --
- * and numbers them.  k_batch runs one CTA per SM slot for the whole batch; each CTA takes the next tile
+ * quart y, tie rule).  The host splits every request into tiles -- 32 x 32 cells for the Nether (nethertile.cuh), equal parts of
+ * up to 24 x 24 chunks for the End (endtile.cuh), 128 cells (8 x 16) for worlds without a tile form --
+ * and numbers them.  k_batch runs as many CTAs as fit for the whole batch; each CTA takes the next tile
  * from a device counter (the work queue), finds its request among the requests' first-tile numbers, stages
  * that request's seed lattices in shared memory when they differ from the previous tile's, and computes the
  * tile.  Uneven requests therefore cost no idle SMs and no per-request launches.
  *
  * The seed lattices of every (world, seed) of the batch are built beforehand by k_setup_list_* into a
- * state pool (the served form keeps that pool across batches as a device cache).
- *
- * End tiles: the class of chunk (cx, cz) needs the island noise over the 25 x 25 chunk cells around it
- * (engine/mc_end.h:66-93).  An 8 x 8-chunk tile evaluates the (8+24)^2 simplex cells of its window once
- * into shared memory (island flag and size) instead of 64 x 625 evaluations, then each chunk scans its
- * window there.
+ * state pool (the served form keeps that pool across batches as a device cache).  All these kernels overlap (overlap.cuh).
  */
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -32,7 +27,7 @@
 
 namespace mg {
 
-#define BNT 128        /* threads per CTA: one quart cell per thread in Overworld / Nether tiles */
+#define BNT 128        /* threads per CTA */
 
 /* ---------------------------------------------------------------- setup of a list of (world, seed) */
 #define LNT 128
@@ -109,7 +104,7 @@ __global__ void __launch_bounds__(LNT) k_setup_list_end(const MgSetupEntry *__re
 }
 
 /* ---------------------------------------------------------------- the persistent batch kernel */
-/* The lattices of an Overworld/Nether request and the End's scratch are never live in the same tile, so they share
+/* A request's lattices, the Nether's tables and the End's scratch are never live in the same tile, so they share
  * storage: 17 KB per CTA, which leaves the register budget as the occupancy limit (up to 9 CTAs per SM). */
 struct BatchEnd {
     uint8_t endp[256];

@@ -49,11 +49,11 @@ int launch_ow_batch(bool fm, int tie, bool open_pass, bool overlap, const MgWorl
                     const MgBatchReq *d_reqs, int nreq, long long ntiles, const MgLattice *d_pool, unsigned long long *d_counter,
                     MgOpenCell *d_open, unsigned long long *d_nopen, long long open_cap, uint8_t *d_out, cudaStream_t st);
 
-/* tile widths of the four Overworld/Nether tile shapes (128 cells each; the shapes also differ in the
- * register budget: 9, 7, 6 and 8 resident CTAs per SM) */
+/* tile widths of the rest's four shapes for cells without a tile form (128 cells; the shapes differ in the register budget: 9, 7,
+ * 6 and 8 resident CTAs per SM) */
 extern const int kBatchTileWidths[BATCH_SHAPES];
-/* tiles of a request of group `group`: 16 x 16 cells (owtile.cu); in the rest, 128 quart cells of shape `shape`
- * (Overworld, Nether) or 8 x 8 chunks (End) */
+/* tiles of a request of group `group`: 16 x 16 cells (owtile.cu); in the rest, 32 x 32 cells (nethertile.cuh), equal parts of up
+ * to 24 x 24 chunks (endtile.cuh), or 128 quart cells of shape `shape` */
 long long batch_tiles(int group, const MgWorldDesc &W, int qx0, int qz0, int nx, int nz, int shape);
 /* lattices of a list of entries of one dimension; Overworld needs the prefix sums of lattices per entry; overlap: the launch before
  * this one in the stream is another dimension's */

@@ -136,7 +136,7 @@ __device__ __forceinline__ void ot_leave_open(const OtWork &K, const MgWorldDesc
 
 /* Float branch (26.3 on), bit for bit the per-cell form's operations.  Bound by instruction issue (66 % of peak; the octaves'
  * separately rounded lerps, the splits' mantissa shifts, the tree scan).  64 registers and 55 KB of shared memory: 4 CTAs,
- * 32 warps per SM.  The uneven batch's 70.8 M float-branch cells: 47.6 ms in the per-cell form, 37.9 ms here. */
+ * 32 warps per SM.  The uneven batch's 70.8 M float-branch cells: 47.6 ms in the per-cell form, 34.2 ms here (8 of it the tree). */
 template <int MODE>
 __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const __grid_constant__ OtWork K) {
     extern __shared__ uint4 smem_raw[];
@@ -413,7 +413,7 @@ struct OtSmemD {
 /* Double branch (26.1, 26.2).  The per-cell form was bound by the FP64 pipe (12 exact shift octaves, 348 operations of 446 a
  * cell at two lanes per SM and clock) beside 40 octaves of 64 x 64-bit products; here nothing per cell uses FP64 and an octave
  * is 11 32 x 32-bit products.  Bound by instruction issue and the wide multiplies.  The uneven batch's 151.6 M double-branch
- * cells: 222.5 ms in the per-cell form, 79.2 ms here (k_ow_open 0.6 ms of it). */
+ * cells: 222.5 ms in the per-cell form, 66.1 ms here (22 of it the tree), and 0.5 ms in k_ow_open. */
 template <int MODE>
 __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const __grid_constant__ OtWork K) {
     extern __shared__ uint4 smem_raw[];

@@ -170,7 +170,8 @@ __device__ __forceinline__ void ot_node_f(const MgLattice &L, bool z0, int i, in
  * The double branch's five climate noises and ridges_folded reach the biome only through quantised targets (steps of 1e-4),
  * so the tile form evaluates them in 32-bit fixed point with 64-bit accumulators (no FP64 pipe, which the exact shift octaves
  * of the per-cell form kept 55 % busy) and takes a target when every value within the form's error bound has it
- * (MgNoise::tile_eq; about 2 % of the cells keep a target open and go to the exact evaluation of a later launch).
+ * (MgNoise::tile_eq).  About 2 % of the cells keep a target open between two values; nearly all of them have the same biome for
+ * both, and the rest (0.1 %) go to the exact evaluation of a later launch.
  *
  * Over a plane of the lattice an octave is V = (1 - W) L0 + W L1 with a row's value L = P + U Q, P = N0 and Q = N1 - N0
  * linear in the fractions (X, Z): N = A dx + B dz + C, whose A, B and C mix the two planes' gradients by the fixed

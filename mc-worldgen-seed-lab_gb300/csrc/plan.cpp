@@ -280,6 +280,11 @@ MCGEN_API int mcgen_gb300_plan_new(const McGb300Request *reqs, int n, int tie_ru
     cudaStream_t ast = mg::abi_stream();
     cudaError_t e = plan_pool(&mp);
     if (!e) e = cudaMallocFromPoolAsync(&p->d_arena, arena_bytes, mp, ast);
+    if (e == cudaErrorMemoryAllocation && open_off < arena_bytes) { /* without the records open cells are evaluated in place */
+        cudaGetLastError();
+        p->open_cap[0] = p->open_cap[1] = 0;
+        e = cudaMallocFromPoolAsync(&p->d_arena, open_off, mp, ast);
+    }
     if (!e && staged) e = cudaMemcpyAsync(p->d_arena, host.data(), staged, cudaMemcpyHostToDevice, ast);
     if (!e) e = cudaStreamSynchronize(ast); /* the arena is ready for any stream */
     if (!e) {
