@@ -31,6 +31,7 @@ int g_features = MCGEN_GPU_BIOMES;
 int g_device = 0;
 int g_dev_state = 0; /* 0 unknown, 1 ready, -1 unavailable */
 cudaStream_t g_stream = nullptr;
+uint8_t *g_few = nullptr; /* FEW_POINTS ids in pinned host memory, used under the lock */
 char g_dev_name[256] = "";
 int g_cc_major = 0, g_cc_minor = 0;
 size_t g_mem_mb = 0;
@@ -86,6 +87,11 @@ int device_ready_locked() {
     if (cudaDeviceGetDefaultMemPool(&pool, g_device) == cudaSuccess) {
         uint64_t keep = ~0ULL;
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    if (cudaHostAlloc((void **)&g_few, FEW_POINTS, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        /* without it few points go the general way */
+        cudaGetLastError();
+        g_few = nullptr;
     }
     g_dev_state = 1;
     return 1;
@@ -350,9 +356,17 @@ MCGEN_API int mcgen_gpu_biome_points(const McWorld *w, int n, const int *xyz, ui
     if (!device_ready_locked()) return MCGEN_E_UNSUPPORTED;
     int rc = world_device_locked(const_cast<McWorld *>(w));
     if (rc) return rc;
-    DevBuf d_xyz(g_stream), d_out(g_stream);
     cudaError_t e;
-    if ((e = d_xyz.alloc(sizeof(int32_t) * 3 * (size_t)n)) || (e = d_out.alloc((size_t)n))) return cuda_code(e);
+    if (g_few && mg::block_few_supported(w->desc, n)) { /* no copies: the ids straight into host memory */
+        rc = mg::launch_block_few(w->desc, w->d_tree, w->d_state, w->zoom_seed, xyz, n, g_few, g_stream);
+        if (rc) return cuda_code((cudaError_t)rc);
+        if ((e = cudaStreamSynchronize(g_stream))) return cuda_code(e);
+        memcpy(out, g_few, (size_t)n);
+        return MCGEN_OK;
+    }
+    DevBuf d_xyz(g_stream), d_out(g_stream);
+    if ((e = d_out.alloc((size_t)n))) return cuda_code(e);
+    if ((e = d_xyz.alloc(sizeof(int32_t) * 3 * (size_t)n))) return cuda_code(e);
     if ((e = cudaMemcpyAsync(d_xyz.p, xyz, sizeof(int32_t) * 3 * (size_t)n, cudaMemcpyHostToDevice, g_stream))) return cuda_code(e);
     rc = block_biomes_dev(w, 0, 0, n, 1, 1, 0, (const int32_t *)d_xyz.p, xmin, xmax, zmin, zmax, (uint8_t *)d_out.p, g_stream);
     if (rc) return rc;

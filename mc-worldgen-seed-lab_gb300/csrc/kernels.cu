@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "climate.cuh"
 #include "endtile.cuh"
@@ -278,9 +279,8 @@ __global__ void __launch_bounds__(128, 6) k_blockgrid(const __grid_constant__ Mg
 /* Block points, one per warp (wc_*): a point's octaves, zoom candidates and tree nodes over the lanes.  A thread per point ran
  * them in series: one point took 90 us, and a warp of unrelated points diverged in every search. */
 template <bool FM, int DIM>
-__global__ void __launch_bounds__(128) k_block_points(const __grid_constant__ MgWorldDesc W, const MgTreeNode *__restrict__ tree,
-                                                      const MgLattice *__restrict__ state, int64_t zseed,
-                                                      const int32_t *__restrict__ xyz, int n, uint8_t *__restrict__ out) {
+__device__ __forceinline__ void block_points(const MgWorldDesc &W, const MgTreeNode *__restrict__ tree, const MgLattice *__restrict__ state,
+                                             int64_t zseed, const int32_t *xyz, int n, uint8_t *__restrict__ out) {
     extern __shared__ uint4 smem_raw[];
     WcStage &st = *reinterpret_cast<WcStage *>(smem_raw);
     wc_stage(st, W, state, threadIdx.x, blockDim.x);
@@ -291,6 +291,23 @@ __global__ void __launch_bounds__(128) k_block_points(const __grid_constant__ Mg
         const int b = wc_cell_chunk<FM, DIM>(W, st.spline, st.lat, tree, cx, cy, cz);
         if ((threadIdx.x & 31) == 0) out[i] = (uint8_t)b;
     }
+}
+template <bool FM, int DIM>
+__global__ void __launch_bounds__(128) k_block_points(const __grid_constant__ MgWorldDesc W, const MgTreeNode *__restrict__ tree,
+                                                      const MgLattice *__restrict__ state, int64_t zseed,
+                                                      const int32_t *__restrict__ xyz, int n, uint8_t *__restrict__ out) {
+    block_points<FM, DIM>(W, tree, state, zseed, xyz, n, out);
+}
+/* a few points, their coordinates in the launch itself (no buffers, no copies, with the ids
+ * stored to pinned host memory: a one-point call 47 -> 36 us in 26.1, 38 -> 30 in 26.3, 34 -> 23 in the Nether) */
+struct FewPoints {
+    int32_t xyz[3 * FEW_POINTS];
+};
+template <bool FM, int DIM>
+__global__ void __launch_bounds__(128) k_block_few(const __grid_constant__ MgWorldDesc W, const MgTreeNode *__restrict__ tree,
+                                                   const MgLattice *__restrict__ state, int64_t zseed, const __grid_constant__ FewPoints p,
+                                                   int n, uint8_t *__restrict__ out) {
+    block_points<FM, DIM>(W, tree, state, zseed, p.xyz, n, out);
 }
 /* sparse End samples (a grid, or nx points at xyz), whose chunks are not worth a table of classes: one per warp */
 template <bool FM>
@@ -545,6 +562,29 @@ static void blockgrid_t(const MgWorldDesc &W, const MgTreeNode *tree, const MgLa
 bool quart_scratch_optional(const MgWorldDesc &W, int rule) { return W.dim == MG_OVERWORLD && !chain_rule(rule); }
 size_t block_scratch_bytes(const MgWorldDesc &W, int x0, int z0, int nx, int nz, bool points) {
     return W.dim == MG_OVERWORLD && !points && ow_block_grid_supported(W, x0, z0) ? ow_grid_scratch_bytes(W, true, (long long)nx * nz) : 0;
+}
+bool block_few_supported(const MgWorldDesc &W, int n) {
+    return n <= FEW_POINTS && (W.dim == MG_OVERWORLD ? W.noise[0].nlev <= 8 : W.dim == MG_NETHER && W.ntables <= 32);
+}
+template <bool FM, int DIM>
+static void few_t(const MgWorldDesc &W, const MgTreeNode *tree, const MgLattice *state, int64_t zseed, const FewPoints &p, int n,
+                  uint8_t *out, cudaStream_t st) {
+    ProfScope ps_(K_BLOCKGRID, st);
+    k_block_few<FM, DIM><<<(unsigned)((n + 3) / 4), 128, sizeof(WcStage), st>>>(W, tree, state, zseed, p, n, out);
+}
+int launch_block_few(const MgWorldDesc &W, const MgTreeNode *tree, const MgLattice *state, int64_t zseed, const int32_t *xyz, int n,
+                     uint8_t *out, cudaStream_t st) {
+    FewPoints p = {};
+    memcpy(p.xyz, xyz, sizeof(int32_t) * 3 * (size_t)n);
+    if (W.dim == MG_OVERWORLD) {
+        if (W.fmode) few_t<true, MG_OVERWORLD>(W, tree, state, zseed, p, n, out, st);
+        else few_t<false, MG_OVERWORLD>(W, tree, state, zseed, p, n, out, st);
+    } else {
+        if (W.fmode) few_t<true, MG_NETHER>(W, tree, state, zseed, p, n, out, st);
+        else few_t<false, MG_NETHER>(W, tree, state, zseed, p, n, out, st);
+    }
+    count_launch();
+    return (int)cudaGetLastError();
 }
 /* Block-coordinate biomes: a grid (xyz == nullptr) or n = nx points (nz == 1) at xyz. For the End,
  * `scratch` holds the chunk classes of [ecx0, ecx0+encx) x [ecz0, ecz0+encz). */

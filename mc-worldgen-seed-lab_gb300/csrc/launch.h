@@ -51,6 +51,12 @@ int launch_block_biomes(const MgWorldDesc &W, const MgWorldDesc *d_world, const 
                         int x0, int z0, int nx, int nz, int step, int y, const int32_t *xyz, uint8_t *out, void *scratch,
                         int ecx0, int ecz0, int encx, int encz, cudaStream_t st);
 
+/* a few block points (host coordinates) of the worlds that block_few_supported takes */
+#define FEW_POINTS 64
+bool block_few_supported(const MgWorldDesc &W, int n);
+int launch_block_few(const MgWorldDesc &W, const MgTreeNode *tree, const MgLattice *state, int64_t zseed, const int32_t *xyz, int n,
+                     uint8_t *out, cudaStream_t st);
+
 /* the same through the tile kernels (owtile.cu), for worlds ow_tile_supported takes.  rec: the
  * cells' chain records, or null.  Scratch: ow_grid_scratch_bytes. */
 bool ow_block_grid_supported(const MgWorldDesc &W, int x0, int z0);
