@@ -560,8 +560,13 @@ static void blockgrid_t(const MgWorldDesc &W, const MgTreeNode *tree, const MgLa
 }
 /* the scratch holds only the record of open cells, and without it (null) those are evaluated where they occur */
 bool quart_scratch_optional(const MgWorldDesc &W, int rule) { return W.dim == MG_OVERWORLD && !chain_rule(rule); }
+/* maps, and lists of so many points that a thread each (k_ow_sparse, 140 to 180 us for the first) is faster than a warp each: 26.1
+ * 6,000 points 153 against 138 us, 10,000 161 and 204, 400,000 2,070 and 5,694; 26.3 20,000 points 188 and 180, 100,000 327 and 637 */
+static bool block_tiles(const MgWorldDesc &W, int x0, int z0, int nx, bool points) {
+    return ow_block_grid_supported(W, x0, z0) && (!points || nx > (W.fmode ? 24576 : 8192));
+}
 size_t block_scratch_bytes(const MgWorldDesc &W, int x0, int z0, int nx, int nz, bool points) {
-    return W.dim == MG_OVERWORLD && !points && ow_block_grid_supported(W, x0, z0) ? ow_grid_scratch_bytes(W, true, (long long)nx * nz) : 0;
+    return W.dim == MG_OVERWORLD && block_tiles(W, x0, z0, nx, points) ? ow_grid_scratch_bytes(W, true, (long long)nx * nz) : 0;
 }
 bool block_few_supported(const MgWorldDesc &W, int n) {
     return n <= FEW_POINTS && (W.dim == MG_OVERWORLD ? W.noise[0].nlev <= 8 : W.dim == MG_NETHER && W.ntables <= 32);
@@ -592,8 +597,8 @@ int launch_block_biomes(const MgWorldDesc &W, const MgWorldDesc *d_world, const 
                         int x0, int z0, int nx, int nz, int step, int y, const int32_t *xyz, uint8_t *out, void *scratch,
                         int ecx0, int ecz0, int encx, int encz, cudaStream_t st) {
     if ((long long)nx * nz <= 0) return 0;
-    if (W.dim == MG_OVERWORLD && !xyz && ow_block_grid_supported(W, x0, z0))
-        return launch_ow_block_grid(W, d_world, tree, state, zseed, x0, z0, nx, nz, step, y, out, scratch, st);
+    if (W.dim == MG_OVERWORLD && block_tiles(W, x0, z0, nx, xyz != nullptr))
+        return launch_ow_block_grid(W, d_world, tree, state, zseed, x0, z0, nx, nz, step, y, xyz, out, scratch, st);
     uint8_t *cls = (uint8_t *)scratch; /* End chunk classes, or null: evaluate per sample */
     if (W.dim == MG_END && cls) {
         end_chunks(W, state, ecx0, ecz0, encx, encz, cls, st);

@@ -64,7 +64,8 @@ size_t ow_grid_scratch_bytes(const MgWorldDesc &W, bool chunk_rule, long long ce
 int launch_ow_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const MgLattice *state, int qx0,
                          int qz0, int nx, int nz, int qy, ChainRec *rec, uint8_t *out, void *scratch, cudaStream_t st);
 int launch_ow_block_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const MgLattice *state, int64_t zseed,
-                         int x0, int z0, int nx, int nz, int step, int y, uint8_t *out, void *scratch, cudaStream_t st);
+                         int x0, int z0, int nx, int nz, int step, int y, const int32_t *xyz, uint8_t *out, void *scratch,
+                         cudaStream_t st);
 
 /* Overworld density functions (continents, erosion, ridges, offset, depth) at n block points xyz[3i..3i+2] of
  * one seed's lattices: out[5i + k] (cudaErrorInvalidValue for other dimensions) */

@@ -63,6 +63,7 @@ struct OtWork {
     MgBatchReq one;             /* one grid */
     int64_t zseed;              /* OT_BLOCK: zoom seed, first block, spacing, block y */
     int32_t x0, z0, step, y;
+    const int32_t *xyz;         /* or the blocks themselves (k_ow_sparse) */
     ChainRec *rec;              /* OT_CHAIN */
 };
 /* next tile and its request (one whole warp calls it); prev: the CTA's last tile of one grid, -1 at first */
@@ -709,12 +710,12 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const __grid_constant__ OtWor
     overlap_wait();
 }
 
-/* ============================================================================ sparse block maps
- * Blocks more than 4 apart: neighbouring cells share too few nodes for a tile's tables, so each is evaluated by its lane: the float
+/* ============================================================================ sparse block maps, long point lists
+ * Blocks more than 4 apart or anywhere: neighbouring cells share too few nodes for a tile's tables, so each is evaluated by its lane: the float
  * branch by the per-cell form, the double branch in the tiles' fixed point with its octaves' edges built on the way (per cell in
  * double, its shift noises took 864 FP64 operations).  Tied cells and open targets are left to k_ow_open like the tiles'.  The
  * lattices, spline and fixed coordinates' parts are in shared memory; warps take 8 x 4 cells, whose tree search they share up to 16
- * blocks apart (a box of 4 x 8 chunks of terrain) and do one by one beyond.  256 x 256 blocks, spacing 16: 26.1 531 -> 205 us, 26.3 379
+ * blocks apart (a box of 4 x 8 chunks of terrain) and do one by one beyond and for points.  256 x 256 blocks, spacing 16: 26.1 531 -> 205 us, 26.3 379
  * -> 237 us; spacing 37: 578 -> 313, 552 -> 229 (its search shared: 324 and 288). */
 struct OtSparse {
     WcStage st;
@@ -747,10 +748,15 @@ __global__ void __launch_bounds__(128, 4) k_ow_sparse(const __grid_constant__ Ot
         __syncthreads();
     }
     for (long long tile = blockIdx.x; tile < K.ntiles; tile += gridDim.x) {
-        const int ix = (int)(tile % tw) * 16 + (warp & 1) * 8 + (lane & 7), iz = (int)(tile / tw) * 8 + (warp >> 1) * 4 + (lane >> 3);
+        const int ix = K.xyz ? (int)tile * 128 + t : (int)(tile % tw) * 16 + (warp & 1) * 8 + (lane & 7);
+        const int iz = K.xyz ? 0 : (int)(tile / tw) * 8 + (warp >> 1) * 4 + (lane >> 3);
         const bool in = ix < nx && iz < nz;
         int cx = 0, cy = qy0, cz = 0;
-        if (in) zoom_cell(K.zseed, K.x0 + ix * K.step, K.y, K.z0 + iz * K.step, cx, cy, cz);
+        if (in) {
+            const int32_t *p = K.xyz + 3 * (size_t)ix;
+            if (K.xyz) zoom_cell(K.zseed, p[0], p[1], p[2], cx, cy, cz);
+            else zoom_cell(K.zseed, K.x0 + ix * K.step, K.y, K.z0 + iz * K.step, cx, cy, cz);
+        }
         bool ok = in;
         int32_t ta[6] = {0, 0, 0, 0, 0, 0}, amb = 0;
         if (FM) {
@@ -810,7 +816,9 @@ __global__ void __launch_bounds__(128, 4) k_ow_sparse(const __grid_constant__ Ot
                     }
                 }
                 float es;
-                ot_climate_targets(W, S, v, eq, sm.depth[cy - qy0], ta, tb, es);
+                const int32_t depth = K.xyz ? (int32_t)__double2ll_rn((depth_grad_d(W, ot_clamp_y(W, cy) * 4) + W.off_d) * 0x1.0p28)
+                                            : sm.depth[cy - qy0];
+                ot_climate_targets(W, S, v, eq, depth, ta, tb, es);
                 ok = es < 1.0f;
 #pragma unroll
                 for (int k = 0; k < 6; k++) {
@@ -823,7 +831,7 @@ __global__ void __launch_bounds__(128, 4) k_ow_sparse(const __grid_constant__ Ot
         uint64_t d;
         bool tied = false, sure = amb != 0;
         int leaf;
-        if (K.step <= 16) {
+        if (!K.xyz && K.step <= 16) {
             if (FM) leaf = tree_search_tie_warp(tree, W, ta, ok, d, tied);
             else leaf = tree_search_tie_warp<true>(tree, W, ta, ok, d, tied, -1, &sure);
         } else {
@@ -877,7 +885,11 @@ __global__ void __launch_bounds__(OT_OPEN_NT, 6) k_ow_open(const __grid_constant
         const int iz = c.cell / R.nx, ix = c.cell - iz * R.nx;
         int qx = R.qx0 + ix, qy = R.qy, qz = R.qz0 + iz;
         const long long o = R.out_off + c.cell;
-        if (MODE == OT_BLOCK) wc_zoom(K.zseed, K.x0 + ix * K.step, K.y, K.z0 + iz * K.step, qx, qy, qz);
+        if (MODE == OT_BLOCK) {
+            const int32_t *p = K.xyz + 3 * (size_t)c.cell;
+            if (K.xyz) wc_zoom(K.zseed, p[0], p[1], p[2], qx, qy, qz);
+            else wc_zoom(K.zseed, K.x0 + ix * K.step, K.y, K.z0 + iz * K.step, qx, qy, qz);
+        }
         if (chains) {
             const int b = wc_block_chunk<FM, MG_OVERWORLD, OT_OPEN_NT / 32>(W, S, T, tree, qx, qy, qz, steps);
             if (threadIdx.x == 0) put_id(K.out + o, b);
@@ -1056,7 +1068,7 @@ int launch_ow_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const
 /* blocks more than 4 apart */
 static int sparse_run(const MgWorldDesc &W, OtWork &K, void *scratch, cudaStream_t st) {
     const bool fm = W.fmode != 0;
-    K.ntiles = (long long)((K.one.nx + 15) / 16) * ((K.one.nz + 7) / 8);
+    K.ntiles = K.xyz ? ((long long)K.one.nx + 127) / 128 : (long long)((K.one.nx + 15) / 16) * ((K.one.nz + 7) / 8);
     int rc = open_scratch(fm, OT_BLOCK, K, scratch, st);
     if (rc) return rc;
     rc = (int)(fm ? cudaFuncSetAttribute(k_ow_sparse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(OtSparse))
@@ -1076,7 +1088,8 @@ bool ow_block_grid_supported(const MgWorldDesc &W, int x0, int z0) {
     return ow_tile_supported(W) && x0 >= INT32_MIN + 16 && z0 >= INT32_MIN + 16;
 }
 int launch_ow_block_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const MgLattice *state, int64_t zseed,
-                         int x0, int z0, int nx, int nz, int step, int y, uint8_t *out, void *scratch, cudaStream_t st) {
+                         int x0, int z0, int nx, int nz, int step, int y, const int32_t *xyz, uint8_t *out, void *scratch,
+                         cudaStream_t st) {
     OtWork K{};
     K.worlds = d_world;
     K.tree = tree;
@@ -1089,7 +1102,8 @@ int launch_ow_block_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const
     K.z0 = z0;
     K.step = step;
     K.y = y;
-    return step <= 4 ? grid_run(W, OT_BLOCK, K, scratch, st) : sparse_run(W, K, scratch, st);
+    K.xyz = xyz;
+    return !xyz && step <= 4 ? grid_run(W, OT_BLOCK, K, scratch, st) : sparse_run(W, K, scratch, st);
 }
 
 }  // namespace mg

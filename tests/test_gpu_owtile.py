@@ -83,7 +83,8 @@ def test_quart_grids_and_chunk_plans(version, preset):
 @pytest.mark.parametrize("version,dim", [("26.1", "overworld"), ("26.3", "overworld"), ("26.2", "the_nether"), ("26.4-snapshot-2", "the_nether"),
                                          ("26.3", "the_end")])
 def test_few_points(version, dim):
-    """Point lists around the number whose coordinates travel in the launch, and around a Nether list's change of form."""
+    """Point lists around the number whose coordinates travel in the launch, and around the changes of form of the Nether's and the
+    Overworld's longer lists."""
     seed = -1
     mg = ge.package()
     mg.load()
@@ -92,7 +93,7 @@ def test_few_points(version, dim):
     w = mg.Generator.open(ge.data_root(), version).world("minecraft:" + dim, "normal", seed)
     ow = O.World(ge.data_root(), version, dim, "normal")
     rng = np.random.default_rng(1)
-    for n in (1, 2, 63, 64, 65, 3072, 3073):
+    for n in (1, 2, 63, 64, 65, 3072, 3073, 8193, 24577):
         xyz = rng.integers(-30000000, 30000000, (n, 3)).astype(np.int32)
         xyz[:, 1] = rng.integers(-100, 400, n)
         assert np.array_equal(w.biome_points(xyz), ow.block_points(seed, xyz)), n
