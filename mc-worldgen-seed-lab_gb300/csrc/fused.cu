@@ -415,6 +415,7 @@ __global__ void __launch_bounds__(FNT, 3) k_ow_seed_targets(const __grid_constan
                 climate_finish_d(W, *spline, v[0], v[1], v[2], v[3], v[4], pts[3 * p + 1] * 4, targets + ((size_t)(s0 + t) * np + p) * 6);
             }
         }
+        __syncthreads(); /* every thread has read the lengths (the loop's last round) */
         if (t < FMAXS) sm.queued[t] = 0;
         __syncthreads();
     };
