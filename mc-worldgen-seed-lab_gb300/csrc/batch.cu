@@ -148,11 +148,17 @@ __device__ __noinline__ void batch_end(const MgWorldDesc &W, BatchSmem &sm, cons
     const int c0 = R.qx0 >> 2, d0 = R.qz0 >> 2, ncx = ((R.qx0 + R.nx - 1) >> 2) - c0 + 1, ncz = ((R.qz0 + R.nz - 1) >> 2) - d0 + 1;
     const int w = end_tile_side(ncx, END_TC), h = end_tile_side(ncz, END_TC), tw = (ncx + w - 1) / w;
     const int cx0 = c0 + t % tw * w, cz0 = d0 + t / tw * h;
+    /* the request's columns and rows in the tile's chunks (in 64 bits: a tile may end beyond the last one) */
+    const long long bx = 4LL * cx0 - R.qx0, bz = 4LL * cz0 - R.qz0;
+    const int ix0 = (int)max(bx, 0LL), ix1 = (int)min(bx + 4 * w, (long long)R.nx);
+    const int iz0 = (int)max(bz, 0LL), iz1 = (int)min(bz + 4 * h, (long long)R.nz);
     end_tile_classes<FM>(sm.end.endp, W.end_f2, W.end_g2, cx0, cz0, w, h, sm.end.tile);
-    for (int iz = max(4 * cz0 - R.qz0, 0) + (int)(threadIdx.x >> 5); iz < min(4 * (cz0 + h) - R.qz0, R.nz); iz += BNT / 32)
-        for (int ix = max(4 * cx0 - R.qx0, 0) + (int)(threadIdx.x & 31); ix < min(4 * (cx0 + w) - R.qx0, R.nx); ix += 32)
+    for (int r = (int)(threadIdx.x >> 5); r < iz1 - iz0; r += BNT / 32)
+        for (int c = (int)(threadIdx.x & 31); c < ix1 - ix0; c += 32) {
+            const int ix = ix0 + c, iz = iz0 + r;
             put_id(out + R.out_off + (size_t)iz * R.nx + ix,
                    W.end_ids[sm.end.tile.cls[(((R.qz0 + iz) >> 2) - cz0) * w + ((R.qx0 + ix) >> 2) - cx0]]);
+        }
 }
 
 /* TILE_W: tile width in cells (tiles are 128 cells); MINB: resident CTAs per SM the register allocation
@@ -207,13 +213,13 @@ __global__ void __launch_bounds__(BNT, MINB) k_batch(const MgWorldDesc *__restri
             continue;
         }
         if (nether_tile_supported(W)) {
-            const int tw = (R.nx + NT_W - 1) / NT_W;
+            const int tw = mg_parts(R.nx, NT_W);
             if (W.fmode) nether_tile<true>(W, sm.nether, trees[R.world], R, tile % tw * NT_W, tile / tw * NT_W, out);
             else nether_tile<false>(W, sm.nether, trees[R.world], R, tile % tw * NT_W, tile / tw * NT_W, out);
             continue;
         }
         constexpr int TILE_H = BNT / TILE_W;
-        const int tw = (R.nx + TILE_W - 1) / TILE_W;
+        const int tw = mg_parts(R.nx, TILE_W);
         const int tx0 = (tile % tw) * TILE_W, tz0 = (tile / tw) * TILE_H;
         const MgTreeNode *tree = trees[R.world];
         if (W.fmode) {
@@ -246,9 +252,9 @@ long long batch_tiles(int group, const MgWorldDesc &W, int qx0, int qz0, int nx,
         const int w = end_tile_side((int)ncx, END_TC), h = end_tile_side((int)ncz, END_TC);
         return ((ncx + w - 1) / w) * ((ncz + h - 1) / h);
     }
-    if (nether_tile_supported(W)) return (long long)((nx + NT_W - 1) / NT_W) * ((nz + NT_W - 1) / NT_W);
+    if (nether_tile_supported(W)) return (long long)mg_parts(nx, NT_W) * mg_parts(nz, NT_W);
     const int tw = kBatchTileWidths[shape], th = BNT / tw;
-    return (long long)((nx + tw - 1) / tw) * ((nz + th - 1) / th);
+    return (long long)mg_parts(nx, tw) * mg_parts(nz, th);
 }
 
 int launch_setup_list(const MgWorldDesc *d_worlds, int dim, const MgSetupEntry *d_ent, int n, const int *d_first,

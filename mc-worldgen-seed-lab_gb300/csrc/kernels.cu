@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(128) k_grid(const __grid_constant__ MgWorldDes
     MgLattice *T = reinterpret_cast<MgLattice *>(S + 1);
     stage(W, state, W.ntables, T, S, DIM == MG_OVERWORLD);
     __syncthreads();
-    const int tw = (nx + 7) / 8; /* 8 x 16-cell tiles */
+    const int tw = mg_parts(nx, 8); /* 8 x 16-cell tiles */
     const int ix = (int)(blockIdx.x % (unsigned)tw) * 8 + threadIdx.x % 8, iz = (int)(blockIdx.x / (unsigned)tw) * 16 + threadIdx.x / 8;
     if (ix >= nx || iz >= nz) return;
     const long long g = (long long)iz * nx + ix;
@@ -450,7 +450,7 @@ static void grid_t(const MgWorldDesc &W, const MgTreeNode *tree, const MgLattice
                    int qy, uint8_t *out, ChainRec *rec, cudaStream_t st) {
     size_t sm = grid_smem(W);
     cudaFuncSetAttribute(k_grid<FM, DIM, CHAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    const long long tiles = (long long)((nx + 7) / 8) * ((nz + 15) / 16);
+    const long long tiles = (long long)mg_parts(nx, 8) * mg_parts(nz, 16);
     { ProfScope ps_(K_GRID, st); k_grid<FM, DIM, CHAIN><<<(unsigned)tiles, 128, sm, st>>>(W, tree, state, qx0, qz0, nx, nz, qy, out, rec); }
 }
 __global__ void k_end_lookup(const __grid_constant__ MgWorldDesc W, const uint8_t *__restrict__ cls, int cx0, int cz0,

@@ -88,6 +88,12 @@ typedef struct __attribute__((aligned(16))) {
 #define MG_MAX_CUTS 31
 #define MG_TREE_PACKED_BOUND 12767
 
+/* parts of `side` that n > 0 cells are cut into; n + side - 1 need not fit an int */
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+static inline int mg_parts(int n, int side) { return (int)(((unsigned)n + (unsigned)side - 1u) / (unsigned)side); }
+
 /* Seed-independent world description, copied once to the device. */
 typedef struct {
     int32_t version, dim, fmode;   /* fmode 1: float branch (26.3+), 0: double branch */

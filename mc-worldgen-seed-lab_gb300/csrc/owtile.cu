@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const __grid_constant__ OtWor
         const MgWorldDesc &W = K.worlds[R.world];
         const MgNoise &O = W.noise[0];
         const int nlev = O.nlev, nsh = 2 * nlev, nclim = W.ntables - nsh;
-        const int tw = (R.nx + OT_W - 1) / OT_W;
+        const int tw = mg_parts(R.nx, OT_W);
         const int tx0 = (tile % tw) * OT_W, tz0 = (tile / tw) * OT_W;
         /* first quart cell of the tile (of a block map: the lowest the zoom can give) */
         const int qx0 = MODE == OT_BLOCK ? (K.x0 + tx0 * K.step - 2) >> 2 : R.qx0 + tx0;
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const __grid_constant__ OtWor
         else leaf = tree_search_tie_warp(tree, W, tg, in, d, tied, sm.hint[t]);
         if (in) {
             sm.hint[t] = ot_hint(W, leaf);
-            const int cell = (tile / tw * OT_W + row) * R.nx + tile % tw * OT_W + col;
+            const int cell = (int)((unsigned)(tile / tw * OT_W + row) * (unsigned)R.nx) + tile % tw * OT_W + col; /* of a cell in the request: fits */
             const int64_t o = R.out_off + cell;
             if (MODE == OT_CHAIN) {
                 ChainRec &q = K.rec[o];
@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const __grid_constant__ OtWor
         const MgWorldDesc &W = K.worlds[R.world];
         const MgNoise &O = W.noise[0];
         const int nlev = O.nlev, nsh = 2 * nlev, nclim = W.ntables - nsh;
-        const int tw = (R.nx + OT_W - 1) / OT_W;
+        const int tw = mg_parts(R.nx, OT_W);
         const int tx0 = (tile % tw) * OT_W, tz0 = (tile / tw) * OT_W;
         /* first quart cell of the tile (of a block map: the lowest the zoom can give) */
         const int qx0 = MODE == OT_BLOCK ? (K.x0 + tx0 * K.step - 2) >> 2 : R.qx0 + tx0;
@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const __grid_constant__ OtWor
         }
         ok &= amb <= 1;
         const MgTreeNode *tree = K.trees ? K.trees[R.world] : K.tree;
-        const int cell = (tile / tw * OT_W + row) * R.nx + tile % tw * OT_W + col;
+        const int cell = (int)((unsigned)(tile / tw * OT_W + row) * (unsigned)R.nx) + tile % tw * OT_W + col; /* of a cell in the request: fits */
         const int64_t o = R.out_off + cell;
         int biome = -1; /* (OT_CHAIN: the leaf) */
 #pragma unroll 1
@@ -732,7 +732,7 @@ __global__ void __launch_bounds__(128, 4) k_ow_sparse(const __grid_constant__ Ot
     const MgSpline &S = sm.st.spline;
     const MgTreeNode *tree = K.tree;
     const MgNoise &O = W.noise[0];
-    const int nlev = O.nlev, nx = K.one.nx, nz = K.one.nz, tw = (nx + 15) / 16, qy0 = (K.y - 2) >> 2;
+    const int nlev = O.nlev, nx = K.one.nx, nz = K.one.nz, tw = mg_parts(nx, 16), qy0 = (K.y - 2) >> 2;
     wc_stage(sm.st, W, K.pool, t, 128);
     overlap_next();
     __syncthreads();
@@ -936,7 +936,7 @@ bool ow_tile_supported(const MgWorldDesc &W) {
     }
     return cap <= (W.fmode ? OT_CAP_F : OT_CAP_D);
 }
-long long ow_tiles(int nx, int nz) { return (long long)((nx + OT_W - 1) / OT_W) * ((nz + OT_W - 1) / OT_W); }
+long long ow_tiles(int nx, int nz) { return (long long)mg_parts(nx, OT_W) * mg_parts(nz, OT_W); }
 
 static int g_ow_resident[2][4]; /* CTAs per SM x SMs by branch and mode (ow_prepare; callers hold the ABI lock) */
 template <int MODE>
@@ -1068,7 +1068,7 @@ int launch_ow_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const
 /* blocks more than 4 apart */
 static int sparse_run(const MgWorldDesc &W, OtWork &K, void *scratch, cudaStream_t st) {
     const bool fm = W.fmode != 0;
-    K.ntiles = K.xyz ? ((long long)K.one.nx + 127) / 128 : (long long)((K.one.nx + 15) / 16) * ((K.one.nz + 7) / 8);
+    K.ntiles = K.xyz ? mg_parts(K.one.nx, 128) : (long long)mg_parts(K.one.nx, 16) * mg_parts(K.one.nz, 8);
     int rc = open_scratch(fm, OT_BLOCK, K, scratch, st);
     if (rc) return rc;
     rc = (int)(fm ? cudaFuncSetAttribute(k_ow_sparse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(OtSparse))
