@@ -1265,7 +1265,8 @@ __device__ __forceinline__ void rt_warp_group(const uint4 *__restrict__ L, const
     const RtNode n(L, first + lane);
     const uint32_t lb = rt_dist(n.a, n.b, lbq);
     auto within = [&](uint32_t d) { return NEXT && near ? rt_beyond(d) : d; };
-    if (ub) U = min(U, within(__reduce_min_sync(FULL, rt_ub_or_inf(n.a, n.b, ubq))));
+    /* (the last group's lanes without a leaf read the block's padding, which bounds nothing) */
+    if (ub) U = min(U, within(__reduce_min_sync(FULL, in ? rt_ub_or_inf(n.a, n.b, ubq) : 0xFFFFFFFFu)));
     unsigned m = __ballot_sync(FULL, in && lb <= U);
     if (!m) return;
     if (m & (m - 1)) { /* does any lane need it?  Where terrain breaks (amplified heights) the targets' box meets up to 95 groups
