@@ -227,6 +227,14 @@ MCGEN_API int mcgen_gb300_check_noise_quant(const McWorld *w, long long n, unsig
  * float-branch, Nether and End worlds. */
 MCGEN_API int mcgen_gb300_check_climate(const McWorld *w, long long n, unsigned long long seed, long long *bad,
                                         long long *fallback);
+/* Device self-check of the double branch's tile form (fixed point with an error bound per value; a cell whose bounds allow two
+ * targets is left open) against the double evaluation, on the world's own seed lattices: n random cells, up to the last coordinate
+ * that the form takes.  *bad counts cells with a target that the bounds rule out, *open the cells whose targets are not all
+ * settled; worst_ratio: the largest |noise - exact| over its bound within 2^17 quarts of the origin and beyond, and the largest
+ * error of the offset spline over its bound at n more sets of coordinates, many of them on its points (*spline_open: those that it
+ * leaves open).  MCGEN_E_ARG for float-branch and End worlds, MCGEN_E_UNSUPPORTED for worlds the form does not take. */
+MCGEN_API int mcgen_gb300_check_tile(const McWorld *w, long long n, unsigned long long seed, long long *bad, long long *open,
+                                     long long *spline_open, double worst_ratio[3]);
 /* Device self-check of the R-tree searches of a world's tree (Overworld or Nether): the level-unrolled and
  * single-loop searches with 32-bit box distances, and the tie search, against the 64-bit stack searches on
  * n random targets (half of them beyond the 32-bit distances' clamp); and the warp-shared search (one pruned

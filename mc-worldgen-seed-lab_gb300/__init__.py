@@ -100,6 +100,8 @@ _PROTOS = {
                                                 C.POINTER(C.c_longlong)]),
     "mcgen_gb300_check_climate": (C.c_int, [_P, C.c_longlong, C.c_ulonglong, C.POINTER(C.c_longlong),
                                             C.POINTER(C.c_longlong)]),
+    "mcgen_gb300_check_tile": (C.c_int, [_P, C.c_longlong, C.c_ulonglong, C.POINTER(C.c_longlong),
+                                         C.POINTER(C.c_longlong), C.POINTER(C.c_longlong), C.POINTER(C.c_double)]),
     "mcgen_gb300_check_tree": (C.c_int, [_P, C.c_longlong, C.c_ulonglong, C.POINTER(C.c_longlong),
                                          C.POINTER(C.c_longlong)]),
     "mcgen_gb300_search": (C.c_int, [_P, C.c_int, _P, C.c_uint64, C.c_uint64, _P, C.c_int, C.c_int, _P, C.c_uint32,
@@ -279,6 +281,16 @@ def check_climate(world: "World", n: int, seed: int = 1) -> tuple[int, int]:
     _check(load().mcgen_gb300_check_climate(world.handle, n, seed, C.byref(b), C.byref(c)),
            "mcgen_gb300_check_climate")
     return b.value, c.value
+
+
+def check_tile(world: "World", n: int, seed: int = 1) -> tuple[int, int, int, tuple[float, float, float]]:
+    """(cells with a target that the bounds rule out, cells with an open target, spline cases left open, worst error /
+    bound of the noises within 2^17 quarts and beyond and of the offset spline) of the double branch's tile form
+    against the double evaluation, on the world's own seed lattices."""
+    b, o, s, r = C.c_longlong(), C.c_longlong(), C.c_longlong(), (C.c_double * 3)()
+    _check(load().mcgen_gb300_check_tile(world.handle, n, seed, C.byref(b), C.byref(o), C.byref(s), r),
+           "mcgen_gb300_check_tile")
+    return b.value, o.value, s.value, tuple(r)
 
 
 def check_tree(world: "World", n: int, seed: int = 1) -> tuple[int, int]:

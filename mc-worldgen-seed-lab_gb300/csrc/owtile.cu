@@ -731,19 +731,12 @@ __global__ void __launch_bounds__(128, 4) k_ow_sparse(const __grid_constant__ Ot
     const MgWorldDesc &W = K.worlds[0];
     const MgSpline &S = sm.st.spline;
     const MgTreeNode *tree = K.tree;
-    const MgNoise &O = W.noise[0];
-    const int nlev = O.nlev, nx = K.one.nx, nz = K.one.nz, tw = mg_parts(nx, 16), qy0 = (K.y - 2) >> 2;
+    const int nx = K.one.nx, nz = K.one.nz, tw = mg_parts(nx, 16), qy0 = (K.y - 2) >> 2;
     wc_stage(sm.st, W, K.pool, t, 128);
     overlap_next();
     __syncthreads();
     if (!FM) {
-        for (int l = t; l < W.ntables; l += 128) {
-            const MgLattice &L = sm.st.lat[l];
-            sm.fix[l] = ot_fix(L.fyd, L.uyd);
-            if (l < 2 * nlev) sm.fz[l] = ot_fix(L.fzd, L.uzd);
-            sm.off[l][0] = __double2ll_rn(L.ox * 0x1.0p32);
-            sm.off[l][1] = __double2ll_rn(L.oz * 0x1.0p32);
-        }
+        ot_cell_fix(W, sm.st.lat, sm.fix, sm.fz, sm.off, t, 128);
         if (t >= 126) sm.depth[127 - t] = (int32_t)__double2ll_rn((depth_grad_d(W, ot_clamp_y(W, qy0 + 127 - t) * 4) + W.off_d) * 0x1.0p28);
         __syncthreads();
     }
@@ -764,57 +757,8 @@ __global__ void __launch_bounds__(128, 4) k_ow_sparse(const __grid_constant__ Ot
         } else {
             ok = in && cx > -OT_COORD_LIM && cx < OT_COORD_LIM && cz > -OT_COORD_LIM && cz < OT_COORD_LIM;
             if (ok) {
-                int64_t sa = 0, sb = 0; /* units of 2^-59 */
-#pragma unroll 1
-                for (int k = 0; k < nlev; k++) {
-                    int64_t va = 0, vb = 0;
-#pragma unroll 1
-                    for (int st = 0; st < 2; st++) {
-                        const int l = st * nlev + k;
-                        const MgLattice &L = sm.st.lat[l];
-                        const PlainPerm P{L.p};
-                        double X = (double)cx, Z = (double)cz;
-                        if (st) { X = X * MG_SECOND_STACK; Z = Z * MG_SECOND_STACK; }
-                        int ia, ib;
-                        int32_t pa, ua, pb, ub;
-                        ot_split_d(X, O.freq[k], L.ox, ia, pa, ua);
-                        ot_split_d(Z, O.freq[k], L.oz, ib, pb, ub);
-                        va += ot_sample_d(P, L.iy, false, sm.fix[l], ia, ib, pa, ua, pb, ub);
-                        ot_split_d(Z, O.freq[k], L.ox, ia, pa, ua);
-                        ot_split_d(X, O.freq[k], L.oy, ib, pb, ub);
-                        vb += ot_sample_d(P, L.iz, true, sm.fz[l], ia, ib, pa, ua, pb, ub);
-                    }
-                    sa = ot_madw((int32_t)(va >> 31), O.c30[k], sa);
-                    sb = ot_madw((int32_t)(vb >> 31), O.c30[k], sb);
-                }
-                const int64_t x = ((int64_t)cx << 32) + (sa >> 25), z = ((int64_t)cz << 32) + (sb >> 25);
-                const int64_t xc = x + __mul64hi(x, OT_STACK_C), zc = z + __mul64hi(z, OT_STACK_C);
                 int32_t v[MG_OW_NOISES - 1], tb[6], eq[MG_OW_NOISES];
-                const bool out17 = max(abs(cx), abs(cz)) >= (1 << 17) - OT_W;
-#pragma unroll 1
-                for (int n = 1; n < MG_OW_NOISES; n++) {
-                    const MgNoise &N = W.noise[n];
-                    int64_t acc = 0;
-#pragma unroll 1
-                    for (int k = 0; k < N.nlev; k++) {
-                        int64_t lev = 0;
-#pragma unroll 1
-                        for (int st = 0; st < 2; st++) {
-                            const int l = N.base + st * N.nlev + k;
-                            const MgLattice &L = sm.st.lat[l];
-                            const int64_t sx = ((st ? xc : x) >> -N.fexp[k]) + sm.off[l][0], sz = ((st ? zc : z) >> -N.fexp[k]) + sm.off[l][1];
-                            lev += ot_sample_d(PlainPerm{L.p}, L.iy, false, sm.fix[l], ot_hi(sx), ot_hi(sz), (int32_t)((uint32_t)sx >> 1),
-                                               ot_fade31((uint32_t)sx), (int32_t)((uint32_t)sz >> 1), ot_fade31((uint32_t)sz));
-                        }
-                        acc = ot_madw((int32_t)(lev >> 31), N.c30[k], acc);
-                    }
-                    const int32_t e = out17 ? N.tile_eq_far : N.tile_eq;
-#pragma unroll
-                    for (int k = 1; k < MG_OW_NOISES; k++) {
-                        v[k - 1] = n == k ? (int32_t)(acc >> 30) : v[k - 1];
-                        eq[k] = n == k ? e : eq[k];
-                    }
-                }
+                ot_cell_d(W, sm.st.lat, sm.fix, sm.fz, sm.off, cx, cz, v, eq);
                 float es;
                 const int32_t depth = K.xyz ? (int32_t)__double2ll_rn((depth_grad_d(W, ot_clamp_y(W, cy) * 4) + W.off_d) * 0x1.0p28)
                                             : sm.depth[cy - qy0];

@@ -293,13 +293,15 @@ __device__ __forceinline__ void ot_target(int32_t v, int32_t e, float scale, int
     b = __float2int_rz(__int2float_rn(v + e) * scale);
 }
 
-/* The offset spline with a bound: at coordinates within ce of the reference's, the value is within `err` of the reference's.
- * A Hermite segment's value is a convex combination of its two points' values (so their errors pass through at most) plus
- * a cubic in t, whose slope in the input is at most (|y2 - y1| + 1.25 (|a| + |b|)) / (x2 - x1); the spline is C1, and a
- * neighbouring segment's slope differs near the joint by its curvature (below 1e5) times ce (below 1e-6), covered by 0.01 and
- * 0.1 (and 2e-9 where a segment is constant); the roundings of one evaluation are within 2^-24 times 2 u_t = 2 (|y2 - y1| +
+/* The offset spline with a bound: at coordinates within de of the reference's, the value is within `err` of the reference's.
+ * A coordinate within de of an end of its segment may lie in the neighbouring one for the reference, whose roundings and curvature
+ * are others: the cell is left open (coordinates are within 4e-7, so that this is a few cells in 10^5).  Else both evaluate the
+ * same segment: its value is a convex combination of its two points' values (so their errors pass through at most) plus a cubic in
+ * t, whose slope in the input is at most (|y2 - y1| + 1.25 (|a| + |b|)) / (x2 - x1), 3.5 (e1 + e2) / (x2 - x1) more where the
+ * points' values are within e1 and e2; the roundings of one evaluation are within 2^-24 times 2 u_t = 2 (|y2 - y1| +
  * 1.25 (|a| + |b|)) for t's two, 2 |y2 - y1| + max |y| for the first lerp, a quarter of |y2 - y1| and 1.75 (|a| + |b|) for the
- * cubic, max |y| + 0.25 (|a| + |b|) for the sum: 4.25 |y2 - y1| + 2 max |y| + 4.5 (|a| + |b|), and both sides round. */
+ * cubic, max |y| + 0.25 (|a| + |b|) for the sum: 4.25 |y2 - y1| + 2 max |y| + 4.5 (|a| + |b|), and both sides round.  A constant
+ * segment has no roundings. */
 #define OT_SPL_DEPTH 4 /* nesting levels unrolled (every 26.x table: 4) */
 struct SplineIn {
     float c, e, r, f;     /* continents, erosion, ridges, ridges_folded */
@@ -329,18 +331,20 @@ __device__ __forceinline__ float spline_err(const MgSpline &S, int c, const Spli
             e1 = e2;
             y2 = spline_err<D - 1>(S, S.child[p + q], x, e2);
         }
-        const float x1 = S.loc[p], d1 = S.der[p];
+        const float x1 = S.loc[p], d1 = S.der[p], dx = in - x1;
         if (ext) { /* linear extension */
-            const float v = d1 * (in - x1);
-            err = d1 == 0.0f ? e2 + 2e-9f : e2 + (fabsf(d1) + 0.1f) * de + 1.2e-7f * (4.0f * fabsf(v) + fabsf(y2));
+            const float v = d1 * dx;
+            err = d1 == 0.0f ? e2 : e2 + fabsf(d1) * 1.001f * de + 1.2e-7f * (4.0f * fabsf(v) + fabsf(y2));
+            if (fabsf(dx) <= 1.001f * de) err = 1e30f;
             return d1 == 0.0f ? y2 : y2 + v;
         }
-        const float w = S.loc[p + 1] - x1, t = (in - x1) / w, d2 = S.der[p + 1], dy = y2 - y1;
+        const float x2 = S.loc[p + 1], w = x2 - x1, t = dx / w, d2 = S.der[p + 1], dy = y2 - y1;
         const float a = d1 * w - dy, b = -d2 * w + dy;
         const float ab = fabsf(a) + fabsf(b), ad = fabsf(dy);
-        err = fmaxf(e1, e2) + (__fdividef(ad + 1.25f * ab, w) * 1.001f + 0.1f) * de +
+        err = fmaxf(e1, e2) + __fdividef(ad + 1.25f * ab + 3.5f * (e1 + e2), w) * 1.001f * de +
               1.2e-7f * (4.3f * ad + 2.0f * fmaxf(fabsf(y1), fabsf(y2)) + 4.6f * ab);
-        if (ad + ab + e1 + e2 == 0.0f) err = 2e-9f; /* a constant segment: its value is exact */
+        if (ad + ab + e1 + e2 == 0.0f) err = 0.0f;
+        if (fminf(dx, x2 - in) <= 1.001f * de) err = 1e30f;
         return lerp<float>(t, y1, y2) + t * (1.0f - t) * lerp<float>(t, a, b);
     }
 }
@@ -373,6 +377,76 @@ __device__ __forceinline__ void ot_climate_targets(const MgWorldDesc &W, const M
     si.df = fabsf(c2) * (float)(ew + 2) + fabsf(si.f) * 1.9e-7f;
     const float sp = spline_err<OT_SPL_DEPTH>(S, S.root, si, es);
     ot_target(depth + __float2int_rn(sp * 0x1.0p28f), (int32_t)(es * (1.01f * 0x1.0p28f)) + 3, s28, ta[4], tb[4]);
+}
+
+/* ---- one cell of its own (neighbours that share no tables): its octaves' edges are built on the way */
+/* the lattices' fixed coordinates' parts (fz: of the shift's z planes) and offsets in units of 2^-32, by threads t of nt */
+__device__ __forceinline__ void ot_cell_fix(const MgWorldDesc &W, const MgLattice *lat, OtFix *fix, OtFix *fz, int64_t (*off)[2], int t,
+                                            int nt) {
+    for (int l = t; l < W.ntables; l += nt) {
+        const MgLattice &L = lat[l];
+        fix[l] = ot_fix(L.fyd, L.uyd);
+        if (l < 2 * W.noise[0].nlev) fz[l] = ot_fix(L.fzd, L.uzd);
+        off[l][0] = __double2ll_rn(L.ox * 0x1.0p32);
+        off[l][1] = __double2ll_rn(L.oz * 0x1.0p32);
+    }
+}
+/* the five climate noises of quart cell (cx, cz), |cx|, |cz| < OT_COORD_LIM: values v in units of 2^-29, v[n - 1] within eq[n] of
+ * noise n's */
+__device__ __forceinline__ void ot_cell_d(const MgWorldDesc &W, const MgLattice *lat, const OtFix *fix, const OtFix *fz,
+                                          const int64_t (*off)[2], int cx, int cz, int32_t (&v)[MG_OW_NOISES - 1],
+                                          int32_t (&eq)[MG_OW_NOISES]) {
+    const MgNoise &O = W.noise[0];
+    int64_t sa = 0, sb = 0; /* units of 2^-59 */
+#pragma unroll 1
+    for (int k = 0; k < O.nlev; k++) {
+        int64_t va = 0, vb = 0;
+#pragma unroll 1
+        for (int st = 0; st < 2; st++) {
+            const int l = st * O.nlev + k;
+            const MgLattice &L = lat[l];
+            const PlainPerm P{L.p};
+            double X = (double)cx, Z = (double)cz;
+            if (st) { X = X * MG_SECOND_STACK; Z = Z * MG_SECOND_STACK; }
+            int ia, ib;
+            int32_t pa, ua, pb, ub;
+            ot_split_d(X, O.freq[k], L.ox, ia, pa, ua);
+            ot_split_d(Z, O.freq[k], L.oz, ib, pb, ub);
+            va += ot_sample_d(P, L.iy, false, fix[l], ia, ib, pa, ua, pb, ub);
+            ot_split_d(Z, O.freq[k], L.ox, ia, pa, ua);
+            ot_split_d(X, O.freq[k], L.oy, ib, pb, ub);
+            vb += ot_sample_d(P, L.iz, true, fz[l], ia, ib, pa, ua, pb, ub);
+        }
+        sa = ot_madw((int32_t)(va >> 31), O.c30[k], sa);
+        sb = ot_madw((int32_t)(vb >> 31), O.c30[k], sb);
+    }
+    const int64_t x = ((int64_t)cx << 32) + (sa >> 25), z = ((int64_t)cz << 32) + (sb >> 25);
+    const int64_t xc = x + __mul64hi(x, OT_STACK_C), zc = z + __mul64hi(z, OT_STACK_C);
+    const bool out17 = max(abs(cx), abs(cz)) >= (1 << 17) - OT_W;
+#pragma unroll 1
+    for (int n = 1; n < MG_OW_NOISES; n++) {
+        const MgNoise &N = W.noise[n];
+        int64_t acc = 0;
+#pragma unroll 1
+        for (int k = 0; k < N.nlev; k++) {
+            int64_t lev = 0;
+#pragma unroll 1
+            for (int st = 0; st < 2; st++) {
+                const int l = N.base + st * N.nlev + k;
+                const MgLattice &L = lat[l];
+                const int64_t sx = ((st ? xc : x) >> -N.fexp[k]) + off[l][0], sz = ((st ? zc : z) >> -N.fexp[k]) + off[l][1];
+                lev += ot_sample_d(PlainPerm{L.p}, L.iy, false, fix[l], ot_hi(sx), ot_hi(sz), (int32_t)((uint32_t)sx >> 1),
+                                   ot_fade31((uint32_t)sx), (int32_t)((uint32_t)sz >> 1), ot_fade31((uint32_t)sz));
+            }
+            acc = ot_madw((int32_t)(lev >> 31), N.c30[k], acc);
+        }
+        const int32_t e = out17 ? N.tile_eq_far : N.tile_eq;
+#pragma unroll
+        for (int k = 1; k < MG_OW_NOISES; k++) {
+            v[k - 1] = n == k ? (int32_t)(acc >> 30) : v[k - 1];
+            eq[k] = n == k ? e : eq[k];
+        }
+    }
 }
 
 }  // namespace mg

@@ -9,7 +9,8 @@
  * fixed-point screen of the double branch's climate noises (nn_q + cast_settled_q) against the exact double
  * evaluation on a world's own seed lattices, and the double branch's whole Overworld climate as the kernels
  * compute it (climate_ow_d) against the plain double evaluation, and the 32-bit R-tree searches against
- * the 64-bit stack searches. */
+ * the 64-bit stack searches; and the tile kernels' fixed point (ot_cell_d, spline_err, the Nether tiles' noises) against the
+ * bounds it is used with. */
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
@@ -17,8 +18,12 @@
 #include "../../include/mcgen.h"
 #include "abi_internal.h"
 #include "climate.cuh"
+#include "batch.h"
+#include "batchdev.cuh"
+#include "nethertile.cuh"
 
 using namespace mgd;
+using namespace mg;
 
 namespace {
 
@@ -270,6 +275,132 @@ __global__ void k_check_climate(const __grid_constant__ MgWorldDesc W, const MgL
     atomicAdd(&out[1], left);
 }
 
+/* The tile kernels' fixed point (owtile.cuh) against the double evaluation of the same cell, on a world's own seed lattices.
+ * Coordinates of magnitude up to 2^10, 2^14, 2^17, 2^20 and the limit, a quarter of them at the ends of those ranges, on both
+ * sides of the change of bound and up to the last one that the fixed point takes; heights inside and around the build range.
+ * out: cells with a target outside the two that the bounds allow; cells left open; the largest |noise - exact| / bound below and
+ * beyond 2^17 quarts; spline cases (below) left open; the largest |spline_err - spline_eval| / its bound. */
+struct TileCheck {
+    unsigned long long bad, open, near, far, spline_open, spline;
+};
+__device__ __forceinline__ int tile_coord(uint64_t r) {
+    const int lims[5] = {1 << 10, 1 << 14, 1 << 17, 1 << 20, OT_COORD_LIM};
+    const int lim = lims[(r & 0xFF) % 5], end = (int)((r >> 8) % 40);
+    int q = (int)((r >> 16) % (uint64_t)lim);
+    if (((r >> 56) & 3) == 0) q = lim == OT_COORD_LIM ? lim - 1 - end : lim + 4 - end;
+    return (r >> 63) ? -q : q;
+}
+__device__ __forceinline__ double worse(double w, double err, double bound) { return fmax(w, err / bound); }
+__device__ __forceinline__ void tile_report(TileCheck *out, unsigned long long bad, unsigned long long open, double near, double far,
+                                            unsigned long long sopen, double spline) {
+    atomicAdd(&out->bad, bad);
+    atomicAdd(&out->open, open);
+    atomicMax(&out->near, (unsigned long long)__double_as_longlong(near));
+    atomicMax(&out->far, (unsigned long long)__double_as_longlong(far));
+    atomicAdd(&out->spline_open, sopen);
+    atomicMax(&out->spline, (unsigned long long)__double_as_longlong(spline));
+}
+__global__ void __launch_bounds__(128) k_check_tile_ow(const __grid_constant__ MgWorldDesc W, const MgLattice *__restrict__ T, long long n,
+                                                       uint64_t seed, TileCheck *out) {
+    __shared__ OtFix fix[MG_MAX_TABLES], fz[2 * OT_MAXLEV];
+    __shared__ int64_t off[MG_MAX_TABLES][2];
+    ot_cell_fix(W, T, fix, fz, off, threadIdx.x, blockDim.x);
+    __syncthreads();
+    unsigned long long bad = 0, open = 0, sopen = 0;
+    double near = 0.0, far = 0.0, spline = 0.0;
+    const float s29 = 0x1.0p-29f;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        uint64_t r = mix64(seed ^ mix64((uint64_t)i)), r2 = mix64(r);
+        const int cx = tile_coord(r), cz = tile_coord(r2), qy = (int)(mix64(r2) % 120) - 30;
+        int32_t v[MG_OW_NOISES - 1], eq[MG_OW_NOISES], ta[6], tb[6], want[6];
+        ot_cell_d(W, T, fix, fz, off, cx, cz, v, eq);
+        const double X = (double)cx, Z = (double)cz, Xc = X * MG_SECOND_STACK, Zc = Z * MG_SECOND_STACK;
+        const double x = X + nn_d_y0(W.noise[0], T, X, Z, Xc, Zc) * 4.0, z = Z + nn_d_z0(W.noise[0], T, Z, X, Zc, Xc) * 4.0;
+        const double xc = x * MG_SECOND_STACK, zc = z * MG_SECOND_STACK;
+        const bool out17 = max(abs(cx), abs(cz)) >= (1 << 17) - OT_W;
+        double e[MG_OW_NOISES - 1];
+        for (int k = 0; k < MG_OW_NOISES - 1; k++) {
+            e[k] = nn_d_y0(W.noise[1 + k], T, x, z, xc, zc);
+            const double err = fabs((double)v[k] * 0x1.0p-29 - e[k]), b = (double)eq[k + 1] * 0x1.0p-29;
+            (out17 ? far : near) = worse(out17 ? far : near, err, b);
+        }
+        float es;
+        ot_climate_targets(W, W.spline, v, eq, (int32_t)__double2ll_rn((depth_grad_d(W, qy * 4) + W.off_d) * 0x1.0p28), ta, tb, es);
+        climate_finish_d(W, W.spline, e[0], e[1], e[2], e[3], e[4], qy * 4, want);
+        bool settled = es < 1.0f, wrong = false;
+        for (int k = 0; k < 6; k++) {
+            wrong |= es < 1.0f && (want[k] < ta[k] || want[k] > tb[k]);
+            settled &= ta[k] == tb[k];
+        }
+        bad += wrong;
+        open += !settled;
+        /* the spline alone, at coordinates on or around its points: any of the reference's coordinates, and the tile's anywhere
+         * within their bounds of them */
+        if (W.spline.nmp <= 0) continue;
+        float co[4], d[4], in[4];
+        const int32_t q[4] = {eq[3], eq[4], eq[5], eq[5] + 2};
+        for (int k = 0; k < 4; k++) {
+            r = mix64(r);
+            co[k] = (float)((double)(int64_t)r * 0x1.0p-63 * 1.5);
+            const int m = (int)((r >> 8) % (uint64_t)W.spline.nmp);
+            d[k] = (float)q[k] * s29 * (k == 3 ? fabsf((float)W.rf_d[2]) : 1.0f) + fabsf(co[k]) * (k == 3 ? 1.9e-7f : 1.2e-7f);
+            if (W.spline.coord[m] == k && (r & 1)) {
+                const float at = W.spline.loc[W.spline.first[m] + (int)((r >> 24) % W.spline.npts[m])];
+                co[k] = at + d[k] * (float)((int)((r >> 40) % 33) - 16) * 0.125f; /* within twice the bound */
+                d[k] = (float)q[k] * s29 * (k == 3 ? fabsf((float)W.rf_d[2]) : 1.0f) + fabsf(co[k]) * (k == 3 ? 1.9e-7f : 1.2e-7f);
+            }
+            r = mix64(r);
+            in[k] = co[k] + d[k] * (float)((int)(r % 17) - 8) * 0.125f;
+            if (fabs((double)in[k] - (double)co[k]) > (double)d[k]) in[k] = co[k];
+        }
+        SplineIn si{in[0], in[1], in[2], in[3], d[0], d[1], d[2], d[3]};
+        float err;
+        const float got = spline_err<OT_SPL_DEPTH>(W.spline, W.spline.root, si, err), ref = spline_eval(W.spline, co);
+        if (!(err < 1.0f)) sopen++;
+        else if (got != ref) spline = worse(spline, fabs((double)got - (double)ref), (double)err);
+    }
+    tile_report(out, bad, open, near, far, sopen, spline);
+}
+/* the Nether's two noises as nether_tile forms them: splits of whole coordinates, edges, levels */
+__global__ void __launch_bounds__(128) k_check_tile_nether(const __grid_constant__ MgWorldDesc W, const MgLattice *__restrict__ T,
+                                                           long long n, uint64_t seed, TileCheck *out) {
+    unsigned long long bad = 0, open = 0;
+    double near = 0.0, far = 0.0;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const uint64_t r = mix64(seed ^ mix64((uint64_t)i));
+        const int cx = tile_coord(r), cz = tile_coord(mix64(r));
+        const double X = (double)cx, Z = (double)cz, Xc = X * MG_SECOND_STACK, Zc = Z * MG_SECOND_STACK;
+        bool wrong = false, settled = true;
+        for (int j = 0; j < 2; j++) {
+            const MgNoise &N = W.nether[j];
+            int64_t acc = 0;
+            for (int k = 0; k < N.nlev; k++) {
+                int64_t lev = 0;
+                for (int st = 0; st < 2; st++) {
+                    const MgLattice &L = T[N.base + st * N.nlev + k];
+                    int ia, ib;
+                    int32_t pa, ua, pb, ub;
+                    ot_split_d(st ? Xc : X, N.freq[k], L.ox, ia, pa, ua);
+                    ot_split_d(st ? Zc : Z, N.freq[k], L.oz, ib, pb, ub);
+                    lev += ot_sample_d(PlainPerm{L.p}, L.iy, false, ot_fix(L.fyd, L.uyd), ia, ib, pa, ua, pb, ub);
+                }
+                acc = ot_madw((int32_t)(lev >> 31), N.c30[k], acc);
+            }
+            const double e = nn_d_y0(N, T, X, Z, Xc, Zc);
+            const bool out17 = max(abs(cx), abs(cz)) >= 1 << 17;
+            (out17 ? far : near) = worse(out17 ? far : near, fabs((double)(acc >> 30) * 0x1.0p-29 - e), (double)N.tile_eq * 0x1.0p-29);
+            int32_t a, b;
+            ot_target((int32_t)(acc >> 30), N.tile_eq, 10000.0f * 0x1.0p-29f, a, b);
+            const int32_t want = quantize((float)e);
+            wrong |= want < a || want > b;
+            settled &= a == b;
+        }
+        bad += wrong;
+        open += !settled;
+    }
+    tile_report(out, bad, open, near, far, 0, 0.0);
+}
+
 /* R-tree searches: the level-unrolled and single-loop 32-bit searches (ENGINE rule) and the unrolled tie
  * search against the 64-bit stack searches, on random targets: quantised climate values in [-12000, 12000]
  * (the tables' range) for half of the cases, in [-40000, 40000] (beyond the 32-bit clamp, where the exact
@@ -474,6 +605,33 @@ extern "C" MCGEN_API int mcgen_gb300_check_climate(const McWorld *w, long long n
     if (e != cudaSuccess) return MCGEN_E_INTERNAL;
     *bad = (long long)h[0];
     *fallback = (long long)h[1];
+    return MCGEN_OK;
+}
+
+extern "C" MCGEN_API int mcgen_gb300_check_tile(const McWorld *w, long long n, unsigned long long seed, long long *bad, long long *open,
+                                               long long *spline_open, double worst_ratio[3]) {
+    if (!w || n < 0 || !bad || !open || !spline_open || !worst_ratio) return MCGEN_E_ARG;
+    if (w->desc.dim == MG_END || w->desc.fmode) return MCGEN_E_ARG; /* the double branch's fixed point */
+    const bool ow = w->desc.dim == MG_OVERWORLD;
+    if (ow ? !mg::ow_tile_supported(w->desc) : !mg::nether_tile_supported(w->desc)) return MCGEN_E_UNSUPPORTED;
+    std::lock_guard<std::mutex> lk(mg::abi_lock());
+    if (!mg::abi_device_ready()) return MCGEN_E_UNSUPPORTED;
+    int rc = mg::abi_world_device(const_cast<McWorld *>(w));
+    if (rc) return rc;
+    TileCheck *d = nullptr, h{};
+    if (cudaMalloc(&d, sizeof h) != cudaSuccess) return MCGEN_E_NOMEM;
+    cudaMemset(d, 0, sizeof h);
+    if (ow) k_check_tile_ow<<<152 * 4, 128>>>(w->desc, w->d_state, n, seed, d);
+    else k_check_tile_nether<<<152 * 4, 128>>>(w->desc, w->d_state, n, seed, d);
+    cudaError_t e = cudaMemcpy(&h, d, sizeof h, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    if (e != cudaSuccess) return MCGEN_E_INTERNAL;
+    *bad = (long long)h.bad;
+    *open = (long long)h.open;
+    *spline_open = (long long)h.spline_open;
+    memcpy(worst_ratio, &h.near, sizeof(double));
+    memcpy(worst_ratio + 1, &h.far, sizeof(double));
+    memcpy(worst_ratio + 2, &h.spline, sizeof(double));
     return MCGEN_OK;
 }
 
