@@ -109,6 +109,7 @@ typedef struct {
      * < 0: a constant is not a multiple of 2^-59 below 8, and the ridge noise is not screened) */
     int64_t rf_q[3];
     int64_t rf_eq;
+    int32_t rf_tile; /* the sums of ridges_folded stay below 4 (the tile kernels' units) */
     float grad_from_f, grad_to_f, off_f, grad_fac_f;
     float rf_f[3];
     int32_t end_ids[5];            /* the_end, end_highlands, end_midlands, small_end_islands, end_barrens */

@@ -862,8 +862,12 @@ __global__ void __launch_bounds__(OT_OPEN_NT, 6) k_ow_open(const __grid_constant
  * the identity up to the world border, and the tables' sizes hold), shift levels and nodes within the tables */
 bool ow_tile_supported(const MgWorldDesc &W) {
     if (W.dim != MG_OVERWORLD) return false;
-    for (int n = 0; n < MG_OW_NOISES && !W.fmode; n++)
-        if (W.noise[n].tile_eq < 0 || W.rf_eq < 0) return false;
+    if (!W.fmode) { /* the fixed point's ranges */
+        for (int n = 0; n < MG_OW_NOISES; n++)
+            if (W.noise[n].tile_eq < 0) return false;
+        if (W.rf_eq < 0 || !W.rf_tile) return false;
+        if (!(fmax(fabs(W.grad_from_d), fabs(W.grad_to_d)) + fabs(W.off_d) < OT_DEPTH_LIM) || W.grad_from_y == W.grad_to_y) return false;
+    }
     if (W.noise[0].base != 0 || W.noise[0].nlev > OT_MAXLEV) return false;
     int base = 0, cap = 0;
     for (int n = 0; n < MG_OW_NOISES; n++) {

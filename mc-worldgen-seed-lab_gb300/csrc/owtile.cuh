@@ -25,6 +25,7 @@ namespace mg {
 #define OT_NT (OT_W * OT_W)       /* threads per CTA */
 #define OT_MAXLEV 3               /* levels of the shift noise (26.x: 3) */
 #define OT_SHIFT_TABS (4 * OT_MAXLEV)
+#define OT_DEPTH_LIM 3.0          /* |depth gradient + offset constant|, for the depth in units of 2^-28 */
 #define OT_COORD_LIM ((1 << 23) - 4096) /* |quart| below which every wrap of the path is the identity */
 
 /* column and row of this thread's cell: warps take 8 x 4 blocks, so the R-tree walk of a warp has a compact box */
@@ -375,7 +376,11 @@ __device__ __forceinline__ void ot_climate_targets(const MgWorldDesc &W, const M
     si.de = (float)ee * u + fabsf(si.e) * 1.2e-7f;
     si.dr = (float)ew * u + fabsf(si.r) * 1.2e-7f;
     si.df = fabsf(c2) * (float)(ew + 2) + fabsf(si.f) * 1.9e-7f;
-    const float sp = spline_err<OT_SPL_DEPTH>(S, S.root, si, es);
+    float sp = spline_err<OT_SPL_DEPTH>(S, S.root, si, es);
+    if (fabsf(sp) > 3.9f) { /* the depth (|gradient + offset| < 3: ow_tile_supported) must fit its units: left open */
+        sp = 0.0f;
+        es = 1e30f;
+    }
     ot_target(depth + __float2int_rn(sp * 0x1.0p28f), (int32_t)(es * (1.01f * 0x1.0p28f)) + 3, s28, ta[4], tb[4]);
 }
 

@@ -883,6 +883,10 @@ int build_world(const char *root, int version, int dim, const char *preset, MgWo
             exact = exact && fabs(c) < 8.0 && ldexp(floor(ldexp(c, 59)), -59) == c;
             D->rf_q[i] = exact ? (int64_t)ldexp(c, 59) : 0;
         }
+        /* the tile form's units hold values below 4: |r| <= 2.12 csum (tile_bounds), |r| + c0 in [c0, 2.12 csum + c0], its magnitude
+         * plus c1 */
+        const double a1 = std::max(fabs(D->rf_d[0]), fabs(2.12 * csum + D->rf_d[0]));
+        D->rf_tile = exact && a1 < 3.95 && fabs(D->rf_d[1]) < 3.95 && fabs(a1 + D->rf_d[1]) < 3.95;
         if (exact) D->rf_eq = (int64_t)ceil((fabs(D->rf_d[2]) * (D->noise[5].fix_err + 1e-14) + 1e-13) * 0x1.0p59) + 1;
     }
     int nleaf = 0;
