@@ -24,6 +24,7 @@
 #include "launch.h"
 #include "legacy.cuh"
 #include "batch.h"
+#include "owtile.cuh"
 #include "prof.h"
 #include "warpcell.cuh"
 
@@ -467,6 +468,13 @@ int launch_end_lookup(const MgWorldDesc &W, const uint8_t *cls, int cx0, int cz0
     count_launch();
     return (int)cudaGetLastError();
 }
+/* a double-branch grid of more cells than its tiles leave open (OT_FEW), all of it beyond the tile form's coordinates: a thread per
+ * cell here (26.1, 256 x 256 cells 272 us, 1,024 x 1,024 1,844; the tiles' per-cell form 279 and 2,199) */
+static bool ow_plain_grid(const MgWorldDesc &W, int qx0, int qz0, int nx, int nz) {
+    const long long lim = OT_COORD_LIM;
+    return !W.fmode && (long long)nx * nz > 4096 &&
+           (qx0 >= lim || qz0 >= lim || (long long)qx0 + nx <= -lim || (long long)qz0 + nz <= -lim);
+}
 /* chain records and their order, then (Overworld) the tile kernels' scratch */
 static size_t chain_bytes(long long n) { return ((size_t)n * (sizeof(ChainRec) + sizeof(int32_t)) + 15) & ~(size_t)15; }
 static bool chain_rule(int rule) { return rule == MG_TIE_GRID_CHAIN || rule == MG_TIE_CHUNK_ORDER; }
@@ -490,7 +498,7 @@ int launch_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const Mg
     }
     const bool chain = chain_rule(rule);
     ChainRec *rec = (ChainRec *)scratch;
-    if (ow_tile_supported(W)) {
+    if (ow_tile_supported(W) && !ow_plain_grid(W, qx0, qz0, nx, nz)) {
         uint8_t *more = chain ? (uint8_t *)scratch + chain_bytes(n) : (uint8_t *)scratch;
         const int rows = (int)(0x7FFFFFFF / nx); /* cell indices of a tile grid are 32-bit */
         for (int z = 0; z < nz; z += rows) {

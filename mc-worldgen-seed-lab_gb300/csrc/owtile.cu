@@ -35,10 +35,16 @@ struct OtSmemF {
     uint16_t hint[OT_NT]; /* each thread's last leaf: where its next R-tree search starts */
 };
 
-/* the old per-cell form, for a tile whose nodes do not fit (out of line: rare) */
-static __device__ __noinline__ void ot_cell_f(const MgWorldDesc &W, const MgLattice *T, int qx, int qy, int qz, int32_t *tg) {
+/* the per-cell form, for a tile whose nodes do not fit or beyond the tables' coordinates (out of line: rare) */
+/* cells of a request up to which such tiles leave all of theirs open in the double branch: k_ow_open has them sooner, by a warp (a
+ * block under the chunk-cell rule) each, than a tile by a thread each (FP64: two lanes per SM and clock).  26.1 beyond 2^23 quarts:
+ * 16 x 16 cells 40 against 161 us, 64 x 64 81 against 165; of a map of 16 x 16 blocks 72 against 183, of 64 x 64 275 against 187.
+ * Beyond it, cells left open filled the record and were done one by one in its place: 256 x 256 450 us, in the tile 279. */
+#define OT_FEW(MODE) ((MODE) == OT_CHUNK || (MODE) == OT_BLOCK ? 1024 : 4096)
+template <bool FM>
+static __device__ __noinline__ void ot_cell_plain(const MgWorldDesc &W, const MgLattice *T, int qx, int qy, int qz, int32_t *tg) {
     int32_t t[6];
-    climate_ow<true>(W, W.spline, T, qx, qy, qz, t);
+    climate_ow<FM>(W, W.spline, T, qx, qy, qz, t);
     for (int k = 0; k < 6; k++) tg[k] = t[k];
 }
 
@@ -361,7 +367,7 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_f(const __grid_constant__ OtWor
                 climate_finish_f(W, W.spline, v[0], v[1], v[2], v[3], v[4],
                                  (MODE == OT_CHUNK || MODE == OT_BLOCK ? ot_clamp_y(W, qy0 + dy) : qy0) * 4, tg);
             } else {
-                ot_cell_f(W, sm.lat, qx0 + dx, MODE == OT_CHUNK || MODE == OT_BLOCK ? ot_clamp_y(W, qy0 + dy) : qy0, qz0 + dz, tg);
+                ot_cell_plain<true>(W, sm.lat, qx0 + dx, MODE == OT_CHUNK || MODE == OT_BLOCK ? ot_clamp_y(W, qy0 + dy) : qy0, qz0 + dz, tg);
             }
         }
         const MgTreeNode *tree = K.trees ? K.trees[R.world] : K.tree;
@@ -656,6 +662,11 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const __grid_constant__ OtWor
             float es;
             ot_climate_targets(W, W.spline, v, eq, sm.depth[MODE == OT_BLOCK ? dy : 0], ta, tb, es);
             ok = es < 1.0f;
+        } else if (in && (long long)R.nx * R.nz > OT_FEW(MODE)) {
+            ot_cell_plain<false>(W, sm.lat, qx0 + dx, MODE == OT_CHUNK || MODE == OT_BLOCK ? ot_clamp_y(W, qy0 + dy) : qy0, qz0 + dz, ta);
+#pragma unroll
+            for (int k = 0; k < 6; k++) tb[k] = ta[k];
+            ok = true;
         }
         /* at most one target open, between two neighbouring values: both are looked up, and the cell is settled when they
          * give the same biome (nearly always: a step is 1e-4 of the range) */
@@ -770,6 +781,9 @@ __global__ void __launch_bounds__(128, 4) k_ow_sparse(const __grid_constant__ Ot
                     ok &= (unsigned)(tb[k] - ta[k]) <= 1u;
                 }
                 ok &= amb <= 1;
+            } else if (in && (long long)nx * nz > OT_FEW(OT_BLOCK)) {
+                ot_cell_plain<false>(W, sm.st.lat, cx, ot_clamp_y(W, cy), cz, ta);
+                ok = true;
             }
         }
         uint64_t d;
