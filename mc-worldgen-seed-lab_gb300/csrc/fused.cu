@@ -304,21 +304,23 @@ __device__ __forceinline__ V search_sum(const MgNoise &N, const V *val, int firs
 
 /* ---- the double branch's many seeds x points in the Overworld tiles' fixed point (owtile.cuh): the double evaluation's 72 FP64
  * operations an octave kept the FP64 pipe 73 % busy (1,501 seeds x 33 points: 424 us; this form 232).  A sample whose targets the
- * error bounds leave open (2 %) is kept in its seed's queue and evaluated in double at the end, one per seed at a time, from the
+ * error bounds leave open (2 %) is kept in its seed's queue and evaluated in double at the end, eight per seed at a time, from the
  * lattices that are still there.  Writes the six targets of every sample. */
 #define TQ_CAP 64 /* points whose values are kept until their targets are formed, by all threads at once */
 struct TargetSmem {
     uint32_t perm[64][FPS];
+    /* of the fixed point, and of the exact evaluation of the samples in the queues (FNPC of every seed at a time) */
     union {
         int64_t val[FNT][FNPC]; /* octave value of lattice (owner thread) t at point p of the chunk, units of 2^-60 */
-        struct {                /* the exact evaluation's */
-            double val, valb;
-        } exact[FNT];
+        double val_d[FNT][FNPC];
     };
-    int64_t sh[2][FMAXOFF][FNPC]; /* ShiftA, ShiftB octaves */
+    union {
+        int64_t sh[2][FMAXOFF][FNPC]; /* ShiftA, ShiftB octaves */
+        double sh_d[2][FMAXOFF][FNPC];
+    };
     union {
         int64_t coord[FMAXS][FNPC][4]; /* per (seed, point): x, z and their second-stack multiples, units of 2^-32 */
-        double exact_at[FMAXS][4];
+        double coord_d[FMAXS][FNPC][4];
     };
     struct {
         double ox, oy, oz;
@@ -355,64 +357,73 @@ __global__ void __launch_bounds__(FNT, 3) k_ow_seed_targets(const __grid_constan
     const uint8_t *pbase = reinterpret_cast<const uint8_t *>(&sm.perm[0][0]);
     const IlvPerm<FPS> mine{pbase, t};
 
-    /* the samples in the queues, the r-th of every seed at once, in double (all threads call it) */
+    /* the samples in the queues, FNPC of every seed at once, in double: k_ow_seed_climate's phases (all threads call it) */
     auto drain = [&]() {
-        for (int r = 0;; r++) {
+        for (int r0 = 0;; r0 += FNPC) {
             __syncthreads();
             int most = 0;
             for (int s = 0; s < spc; s++) most = max(most, sm.queued[s]);
-            if (r >= most) break;
-            const bool go = active && r < sm.queued[ls];
-            const int32_t *pp = pts + 3 * (go ? sm.queue[ls][r] : 0);
-            OffHdr x;
-            x.ox = own.ox; x.oy = own.oy; x.oz = own.oz;
-            lattice_header(x, true);
-            if (go && own.noise == 0) {
+            if (r0 >= most) break;
+            for (int item = t; item < nown * FNPC; item += FNT) {
+                const int o = item % nown, r = item / nown, oj = o / spc, s = o % spc;
+                if (r0 + r >= sm.queued[s]) continue;
+                const IlvPerm<FPS> perm{pbase, o};
+                const int32_t *pp = pts + 3 * sm.queue[s][r0 + r];
+                OffHdr x;
+                x.ox = sm.hdr[o].ox; x.oy = sm.hdr[o].oy; x.oz = sm.hdr[o].oz;
+                lattice_header(x, true);
+                const int lv = oj >= O.nlev ? oj - O.nlev : oj, k = O.fexp[lv];
                 double X = (double)pp[0], Z = (double)pp[2];
-                if (own.st) { X = X * MG_SECOND_STACK; Z = Z * MG_SECOND_STACK; }
-                const double f = O.freq[own.lev];
-                const int k = O.fexp[own.lev];
+                if (oj >= O.nlev) { X = X * MG_SECOND_STACK; Z = Z * MG_SECOND_STACK; }
+                const double f = O.freq[lv];
                 int ix, iz, iyy;
                 double fx, fz, fy;
                 int64_t FX, FZ, FY;
-                split_dk(X, f, k, own.ox, ix, fx, FX);
-                split_dk(Z, f, k, own.oz, iz, fz, FZ);
-                sm.exact[t].val = octave_d_y0(mine, x, ix, fx, FX, iz, fz, FZ);
-                split_dk(Z, f, k, own.ox, ix, fx, FX);
-                split_dk(X, f, k, own.oy, iyy, fy, FY);
-                sm.exact[t].valb = octave_d_z0(mine, x, ix, fx, FX, iyy, fy, FY);
+                split_dk(X, f, k, x.ox, ix, fx, FX);
+                split_dk(Z, f, k, x.oz, iz, fz, FZ);
+                sm.sh_d[0][o][r] = octave_d_y0(perm, x, ix, fx, FX, iz, fz, FZ);
+                split_dk(Z, f, k, x.ox, ix, fx, FX);
+                split_dk(X, f, k, x.oy, iyy, fy, FY);
+                sm.sh_d[1][o][r] = octave_d_z0(perm, x, ix, fx, FX, iyy, fy, FY);
             }
             __syncthreads();
-            const bool one = t < spc && r < sm.queued[t];
+            const int qs = t / FNPC, qr = t % FNPC;
+            const bool one = t < spc * FNPC && r0 + qr < sm.queued[qs];
             if (one) {
-                const int32_t *q = pts + 3 * sm.queue[t][r];
+                const int32_t *q = pts + 3 * sm.queue[qs][r0 + qr];
                 double a1 = 0.0, a2 = 0.0, b1 = 0.0, b2 = 0.0;
                 for (int k = 0; k < O.nlev; k++) {
-                    a1 += O.amp_d[k] * sm.exact[k * spc + t].val * O.vf_d[k];
-                    a2 += O.amp_d[k] * sm.exact[(O.nlev + k) * spc + t].val * O.vf_d[k];
-                    b1 += O.amp_d[k] * sm.exact[k * spc + t].valb * O.vf_d[k];
-                    b2 += O.amp_d[k] * sm.exact[(O.nlev + k) * spc + t].valb * O.vf_d[k];
+                    a1 += O.amp_d[k] * sm.sh_d[0][k * spc + qs][qr] * O.vf_d[k];
+                    a2 += O.amp_d[k] * sm.sh_d[0][(O.nlev + k) * spc + qs][qr] * O.vf_d[k];
+                    b1 += O.amp_d[k] * sm.sh_d[1][k * spc + qs][qr] * O.vf_d[k];
+                    b2 += O.amp_d[k] * sm.sh_d[1][(O.nlev + k) * spc + qs][qr] * O.vf_d[k];
                 }
                 const double x = (double)q[0] + ((a1 + a2) * O.vfac) * 4.0, z = (double)q[2] + ((b1 + b2) * O.vfac) * 4.0;
-                sm.exact_at[t][0] = x;
-                sm.exact_at[t][1] = z;
-                sm.exact_at[t][2] = x * MG_SECOND_STACK;
-                sm.exact_at[t][3] = z * MG_SECOND_STACK;
+                sm.coord_d[qs][qr][0] = x;
+                sm.coord_d[qs][qr][1] = z;
+                sm.coord_d[qs][qr][2] = x * MG_SECOND_STACK;
+                sm.coord_d[qs][qr][3] = z * MG_SECOND_STACK;
             }
             __syncthreads();
-            if (go && own.noise != 0) sm.exact[t].val = search_octave<false, double>(W, own, x, mine, sm.exact_at[ls]);
+            if (active && own.noise != 0) {
+                OffHdr x;
+                x.ox = own.ox; x.oy = own.oy; x.oz = own.oz;
+                lattice_header(x, true);
+                const int n = min(sm.queued[ls] - r0, FNPC);
+                for (int r = 0; r < n; r++) sm.val_d[t][r] = search_octave<false, double>(W, own, x, mine, sm.coord_d[ls][r]);
+            }
             __syncthreads();
             if (one) {
-                const int p = sm.queue[t][r];
+                const int p = sm.queue[qs][r0 + qr];
                 double v[MG_OW_NOISES - 1];
                 for (int q = 1; q < MG_OW_NOISES; q++) {
                     const MgNoise &N = W.noise[q];
                     double a1 = 0.0, a2 = 0.0;
-                    for (int k = 0; k < N.nlev; k++) a1 += N.amp_d[k] * sm.exact[(N.base + k) * spc + t].val * N.vf_d[k];
-                    for (int k = 0; k < N.nlev; k++) a2 += N.amp_d[k] * sm.exact[(N.base + N.nlev + k) * spc + t].val * N.vf_d[k];
+                    for (int k = 0; k < N.nlev; k++) a1 += N.amp_d[k] * sm.val_d[(N.base + k) * spc + qs][qr] * N.vf_d[k];
+                    for (int k = 0; k < N.nlev; k++) a2 += N.amp_d[k] * sm.val_d[(N.base + N.nlev + k) * spc + qs][qr] * N.vf_d[k];
                     v[q - 1] = (a1 + a2) * N.vfac;
                 }
-                climate_finish_d(W, *spline, v[0], v[1], v[2], v[3], v[4], pts[3 * p + 1] * 4, targets + ((size_t)(s0 + t) * np + p) * 6);
+                climate_finish_d(W, *spline, v[0], v[1], v[2], v[3], v[4], pts[3 * p + 1] * 4, targets + ((size_t)(s0 + qs) * np + p) * 6);
             }
         }
         __syncthreads(); /* every thread has read the lengths (the loop's last round) */
@@ -464,9 +475,9 @@ __global__ void __launch_bounds__(FNT, 3) k_ow_seed_targets(const __grid_constan
             sm.coord[cs][cp][2] = x + __mul64hi(x, OT_STACK_C);
             sm.coord[cs][cp][3] = z + __mul64hi(z, OT_STACK_C);
         }
-        __syncthreads();
+        const bool any = __syncthreads_or(item && !skip); /* else every point of the chunk is for the queues */
         /* ---- D: climate octaves, each thread on its own lattice */
-        if (active && own.noise != 0) {
+        if (any && active && own.noise != 0) {
             for (int p = 0; p < npc; p++) {
                 const int64_t sx = (sm.coord[ls][p][own.st ? 2 : 0] >> lev) + oxq, sz = (sm.coord[ls][p][own.st ? 3 : 1] >> lev) + ozq;
                 sm.val[t][p] = ot_sample_d(mine, iy, false, fix, ot_hi(sx), ot_hi(sz), (int32_t)((uint32_t)sx >> 1), ot_fade31((uint32_t)sx),
