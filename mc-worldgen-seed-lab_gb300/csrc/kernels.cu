@@ -453,6 +453,7 @@ static void grid_t(const MgWorldDesc &W, const MgTreeNode *tree, const MgLattice
     cudaFuncSetAttribute(k_grid<FM, DIM, CHAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     const long long tiles = (long long)mg_parts(nx, 8) * mg_parts(nz, 16);
     { ProfScope ps_(K_GRID, st); k_grid<FM, DIM, CHAIN><<<(unsigned)tiles, 128, sm, st>>>(W, tree, state, qx0, qz0, nx, nz, qy, out, rec); }
+    count_launch();
 }
 __global__ void k_end_lookup(const __grid_constant__ MgWorldDesc W, const uint8_t *__restrict__ cls, int cx0, int cz0,
                              int ncx, int qx0, int qz0, int nx, int nz, uint8_t *__restrict__ out) {
@@ -525,7 +526,6 @@ int launch_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const Mg
             else grid_t<false, MG_NETHER, false>(W, tree, state, qx0, qz0, nx, nz, qy, out, rec, st);
         }
     }
-    count_launch();
     if (rule == MG_TIE_GRID_CHAIN) {
         { ProfScope ps_(K_CHAIN_RESOLVE, st); k_chain_resolve<<<blocks_for(n, 256), 256, 0, st>>>(tree, rec, n, out); }
         count_launch();
