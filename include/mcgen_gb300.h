@@ -136,7 +136,9 @@ MCGEN_API int mcgen_gb300_server_stats(McGb300Server *s, McGb300ServerStats *out
 MCGEN_API int mcgen_gb300_server_replay(McGb300Server *s, const McGb300Request *reqs, const double *arrival_s, int n,
                                         uint8_t *out, const long long *out_off, double *latency_ms, double *elapsed_s);
 /* Testing aid: the next batch the server forms fails at its device-allocation step with `code` (> 0), as if
- * that allocation had failed; host-side only, no device fault. */
+ * that allocation had failed; host-side only, no device fault.  MCGEN_GB300_FAIL_RECORD: the next batch that records open cells
+ * for a later launch forms as if the memory for the record alone were missing (it evaluates them in place and succeeds). */
+#define MCGEN_GB300_FAIL_RECORD 0x10000
 MCGEN_API int mcgen_gb300_server_fail_next(McGb300Server *s, int code);
 
 /* ---- biome seed search: which candidate seeds produce the observed biomes ----

@@ -292,10 +292,19 @@ int launch_batch(McGb300Server *s, Batch &b) {
     for (const auto &r : reqs)
         if (wgroup[(size_t)r.world] != BATCH_REST) ow_cells[wgroup[(size_t)r.world]] += (long long)r.nx * r.nz;
     mg::batch_open_cap(ow_cells, MG_TIE_ENGINE, open_cap);
-    const long long nopen = open_cap[0] + open_cap[1];
-    if (!e && nopen > 0) e = grow_dev(&b.d_open, &b.cap_open, (size_t)nopen);
+    long long nopen = open_cap[0] + open_cap[1];
+    if (!e && nopen > 0) { /* without the record open cells are evaluated in place */
+        const bool none = s->fail_next == MCGEN_GB300_FAIL_RECORD;
+        if (none) s->fail_next = 0;
+        e = none ? cudaErrorMemoryAllocation : grow_dev(&b.d_open, &b.cap_open, (size_t)nopen);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            nopen = open_cap[0] = open_cap[1] = 0;
+            e = cudaSuccess;
+        }
+    }
     if (e) return crc(e);
-    if (s->fail_next) { /* injected failure of this step (tests of the failure path) */
+    if (s->fail_next && s->fail_next != MCGEN_GB300_FAIL_RECORD) { /* injected failure of this step (tests of the failure path) */
         const int f = s->fail_next;
         s->fail_next = 0;
         return f;

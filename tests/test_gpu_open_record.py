@@ -62,3 +62,19 @@ def test_grids_beyond_the_record(tmp_path):
     _, tg = w.seed_points(seeds, pts, want_targets=True)
     _, et = ow.points(seeds, pts, want_targets=True)
     assert np.array_equal(np.asarray(tg).reshape(-1), np.asarray(et).reshape(-1))
+
+
+@pytest.mark.parametrize("version", ["26.1", "26.3"])
+def test_server_without_room_for_the_record(version):
+    """A batch whose record cannot be allocated (injected on the host) is served all the same."""
+    mg, w, ow = pair(version)
+    srv = mg.Server(hbm_budget_bytes=64 << 20, max_inflight=1)
+    try:
+        for q in ((8388600, 4, 90, 70, 16), (-300, 77, 90, 70, 16), (8388600, 4, 33, 20, 16)):
+            srv.fail_next(mg.FAIL_RECORD)
+            ids, _ = srv.wait(srv.submit(w, SEED, *q))
+            assert np.array_equal(ids, ow.quart_grid(SEED, *q, O.TIE_ENGINE)), q
+        ids, _ = srv.wait(srv.submit(w, SEED, -300, 77, 90, 70, 16))  # and with the record again
+        assert np.array_equal(ids, ow.quart_grid(SEED, -300, 77, 90, 70, 16, O.TIE_ENGINE))
+    finally:
+        srv.close()
