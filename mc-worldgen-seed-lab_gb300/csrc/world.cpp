@@ -591,6 +591,7 @@ static int load_tree(const char *root, int version, int dim, std::vector<MgTreeN
     if (leaves.empty()) { *err = "no biome parameters in " + path; return MCGEN_E_DATA; }
     *nleaf = (int)leaves.size();
     int root_id = tb.build(leaves);
+    if (leaves.size() == 1) root_id = tb.subtree(leaves); /* the searches start at the root's children */
     /* the device search keeps a stack of 10 subtrees */
     std::vector<std::pair<int, int>> todo{{root_id, 0}};
     int depth = 0;
