@@ -476,13 +476,16 @@ static bool ow_plain_grid(const MgWorldDesc &W, int qx0, int qz0, int nx, int nz
     return !W.fmode && (long long)nx * nz > 4096 &&
            (qx0 >= lim || qz0 >= lim || (long long)qx0 + nx <= -lim || (long long)qz0 + nz <= -lim);
 }
-/* chain records and their order, then (Overworld) the tile kernels' scratch */
-static size_t chain_bytes(long long n) { return ((size_t)n * (sizeof(ChainRec) + sizeof(int32_t)) + 15) & ~(size_t)15; }
+/* chain records, then their order; (Overworld) the tile kernels' scratch takes the order's place, which is written later, or where
+ * the grid is too small for that follows it */
+static size_t order_bytes(long long n) { return (size_t)n * sizeof(int32_t); }
+static size_t chain_bytes(long long n) { return ((size_t)n * sizeof(ChainRec) + order_bytes(n) + 15) & ~(size_t)15; }
 static bool chain_rule(int rule) { return rule == MG_TIE_GRID_CHAIN || rule == MG_TIE_CHUNK_ORDER; }
 size_t quart_scratch_bytes(const MgWorldDesc &W, int rule, int nx, int nz) {
     if (W.dim == MG_END) return (size_t)(nx / 4 + 3) * (size_t)(nz / 4 + 3);
     const long long n = (long long)nx * nz;
-    return (chain_rule(rule) ? chain_bytes(n) : 0) + (ow_tile_supported(W) ? ow_grid_scratch_bytes(W, false, n) : 0);
+    const size_t tiles = ow_tile_supported(W) ? ow_grid_scratch_bytes(W, false, n) : 0;
+    return chain_rule(rule) ? chain_bytes(n) + (tiles > order_bytes(n) ? tiles : 0) : tiles;
 }
 int launch_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const MgTreeNode *tree, const MgLattice *state, int qx0, int qz0,
                       int nx, int nz, int qy, int rule, uint8_t *out, void *scratch, cudaStream_t st) {
@@ -500,12 +503,13 @@ int launch_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const Mg
     const bool chain = chain_rule(rule);
     ChainRec *rec = (ChainRec *)scratch;
     if (ow_tile_supported(W) && !ow_plain_grid(W, qx0, qz0, nx, nz)) {
-        uint8_t *more = chain ? (uint8_t *)scratch + chain_bytes(n) : (uint8_t *)scratch;
+        const size_t tiles = ow_grid_scratch_bytes(W, false, n);
+        uint8_t *more = !tiles ? nullptr : !chain ? (uint8_t *)scratch : (uint8_t *)scratch + (tiles > order_bytes(n) ? chain_bytes(n) : sizeof(ChainRec) * (size_t)n);
         const int rows = (int)(0x7FFFFFFF / nx); /* cell indices of a tile grid are 32-bit */
         for (int z = 0; z < nz; z += rows) {
             const size_t at = (size_t)z * (size_t)nx;
             const int rc = launch_ow_quart_grid(W, d_world, tree, state, qx0, qz0 + z, nx, rows < nz - z ? rows : nz - z, qy,
-                                                chain ? rec + at : nullptr, out + at, ow_grid_scratch_bytes(W, false, n) ? more : nullptr, st);
+                                                chain ? rec + at : nullptr, out + at, more, st);
             if (rc) return rc;
             if (rows >= nz - z) break;
         }
