@@ -240,9 +240,13 @@ __global__ void __launch_bounds__(BNT, MINB) k_batch(const MgWorldDesc *__restri
 const int kBatchTileWidths[BATCH_SHAPES] = {8, 8, 8, 8};
 static int g_resident[BATCH_SHAPES] = {0, 0, 0, 0}; /* CTAs per SM x SMs, per shape (batch_prepare) */
 
-int batch_group(const MgWorldDesc &W, int tie) {
+int batch_world_group(const MgWorldDesc &W, int tie) {
     if ((tie != MG_TIE_ENGINE && tie != MG_TIE_CHUNK_CELL) || !ow_tile_supported(W)) return BATCH_REST;
     return W.fmode ? BATCH_OW_F : BATCH_OW_D;
+}
+int batch_group(int world_group, int qx0, int qz0, int nx, int nz) {
+    if (world_group != BATCH_OW_D) return world_group;
+    return ow_beyond(false, 0, qx0, qz0, (long long)qx0 + nx - 1, (long long)qz0 + nz - 1, (long long)nx * nz) ? BATCH_REST : world_group;
 }
 
 long long batch_tiles(int group, const MgWorldDesc &W, int qx0, int qz0, int nx, int nz, int shape) {

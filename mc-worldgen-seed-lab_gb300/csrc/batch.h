@@ -34,11 +34,18 @@ struct BatchGroups {
 };
 /* device counters of a batch: tiles taken per group, cells recorded as open per Overworld group */
 #define BATCH_COUNTERS (BATCH_GROUPS + 2)
-int batch_group(const MgWorldDesc &W, int tie);
+/* the group of a world's requests, and of one of them */
+int batch_world_group(const MgWorldDesc &W, int tie);
+int batch_group(int world_group, int qx0, int qz0, int nx, int nz);
 
 /* ---- owtile.cu: worlds the tile kernels take, a request's tiles, attributes (call before any capture) */
 bool ow_tile_supported(const MgWorldDesc &W);
 long long ow_tiles(int nx, int nz);
+/* whether the tiles do not take an area of more than `few` cells all the same: quart cells (qx0, qz0) to (qx1, qz1), `cells` of them
+ * (or blocks in them) */
+bool ow_beyond(bool fm, long long few, long long qx0, long long qz0, long long qx1, long long qz1, long long cells);
+#define OT_FEW_CELLS 4096 /* for single grids and block maps */
+#define OT_FEW_BLOCKS 1024
 int ow_prepare();
 /* records to provide for `cells` cells some of which are left to the exact evaluation (the double branch's with a target
  * open, well below 1 %; under the chunk-cell rule the tied ones too; cells beyond the record are evaluated in place) */

@@ -24,7 +24,6 @@
 #include "launch.h"
 #include "legacy.cuh"
 #include "batch.h"
-#include "owtile.cuh"
 #include "prof.h"
 #include "warpcell.cuh"
 
@@ -469,13 +468,6 @@ int launch_end_lookup(const MgWorldDesc &W, const uint8_t *cls, int cx0, int cz0
     count_launch();
     return (int)cudaGetLastError();
 }
-/* a double-branch grid of more cells than its tiles leave open (OT_FEW), all of it beyond the tile form's coordinates: a thread per
- * cell here (26.1, 256 x 256 cells 272 us, 1,024 x 1,024 1,844; the tiles' per-cell form 279 and 2,199) */
-static bool ow_plain_grid(const MgWorldDesc &W, int qx0, int qz0, int nx, int nz) {
-    const long long lim = OT_COORD_LIM;
-    return !W.fmode && (long long)nx * nz > 4096 &&
-           (qx0 >= lim || qz0 >= lim || (long long)qx0 + nx <= -lim || (long long)qz0 + nz <= -lim);
-}
 /* chain records, then their order; (Overworld) the tile kernels' scratch takes the order's place, which is written later, or where
  * the grid is too small for that follows it */
 static size_t order_bytes(long long n) { return (size_t)n * sizeof(int32_t); }
@@ -502,7 +494,7 @@ int launch_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const Mg
     }
     const bool chain = chain_rule(rule);
     ChainRec *rec = (ChainRec *)scratch;
-    if (ow_tile_supported(W) && !ow_plain_grid(W, qx0, qz0, nx, nz)) {
+    if (ow_tile_supported(W) && !ow_beyond(W.fmode != 0, OT_FEW_CELLS, qx0, qz0, (long long)qx0 + nx - 1, (long long)qz0 + nz - 1, n)) {
         const size_t tiles = ow_grid_scratch_bytes(W, false, n);
         uint8_t *more = !tiles ? nullptr : !chain ? (uint8_t *)scratch : (uint8_t *)scratch + (tiles > order_bytes(n) ? chain_bytes(n) : sizeof(ChainRec) * (size_t)n);
         const int rows = (int)(0x7FFFFFFF / nx); /* cell indices of a tile grid are 32-bit */

@@ -36,11 +36,6 @@ struct OtSmemF {
 };
 
 /* the per-cell form, for a tile whose nodes do not fit or beyond the tables' coordinates (out of line: rare) */
-/* cells of a request up to which such tiles leave all of theirs open in the double branch: k_ow_open has them sooner, by a warp (a
- * block under the chunk-cell rule) each, than a tile by a thread each (FP64: two lanes per SM and clock).  26.1 beyond 2^23 quarts:
- * 16 x 16 cells 40 against 161 us, 64 x 64 81 against 165; of a map of 16 x 16 blocks 72 against 183, of 64 x 64 275 against 187.
- * Beyond it, cells left open filled the record and were done one by one in its place: 256 x 256 450 us, in the tile 279. */
-#define OT_FEW(MODE) ((MODE) == OT_CHUNK || (MODE) == OT_BLOCK ? 1024 : 4096)
 template <bool FM>
 static __device__ __noinline__ void ot_cell_plain(const MgWorldDesc &W, const MgLattice *T, int qx, int qy, int qz, int32_t *tg) {
     int32_t t[6];
@@ -662,11 +657,6 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const __grid_constant__ OtWor
             float es;
             ot_climate_targets(W, W.spline, v, eq, sm.depth[MODE == OT_BLOCK ? dy : 0], ta, tb, es);
             ok = es < 1.0f;
-        } else if (in && (long long)R.nx * R.nz > OT_FEW(MODE)) {
-            ot_cell_plain<false>(W, sm.lat, qx0 + dx, MODE == OT_CHUNK || MODE == OT_BLOCK ? ot_clamp_y(W, qy0 + dy) : qy0, qz0 + dz, ta);
-#pragma unroll
-            for (int k = 0; k < 6; k++) tb[k] = ta[k];
-            ok = true;
         }
         /* at most one target open, between two neighbouring values: both are looked up, and the cell is settled when they
          * give the same biome (nearly always: a step is 1e-4 of the range) */
@@ -781,7 +771,7 @@ __global__ void __launch_bounds__(128, 4) k_ow_sparse(const __grid_constant__ Ot
                     ok &= (unsigned)(tb[k] - ta[k]) <= 1u;
                 }
                 ok &= amb <= 1;
-            } else if (in && (long long)nx * nz > OT_FEW(OT_BLOCK)) {
+            } else if (in && (long long)nx * nz > OT_FEW_BLOCKS) {
                 ot_cell_plain<false>(W, sm.st.lat, cx, ot_clamp_y(W, cy), cz, ta);
                 ok = true;
             }
@@ -897,6 +887,15 @@ bool ow_tile_supported(const MgWorldDesc &W) {
         cap += 4 * ((m * m + 31) / 32) * 32;
     }
     return cap <= (W.fmode ? OT_CAP_F : OT_CAP_D);
+}
+/* In the double branch the tiles leave every cell beyond the tables' coordinates open.  Up to `few` k_ow_open has sooner, by a warp
+ * (a block under the chunk-cell rule) each, than a thread each (FP64: two lanes per SM and clock): 26.1 beyond 2^23 quarts, grids of
+ * 16 x 16 cells 40 against 161 us, 64 x 64 81 against 165, maps of 16 x 16 blocks 72 against 183, of 64 x 64 275 against 187.  More
+ * would fill the record and be done one by one, so an area of more cells that reaches there takes the forms with a thread per cell
+ * (a grid of 256 x 256 cells 450 us in the tiles, 272 so), and a batch's requests that do all of them. */
+bool ow_beyond(bool fm, long long few, long long qx0, long long qz0, long long qx1, long long qz1, long long cells) {
+    const long long lim = OT_COORD_LIM - 2 * OT_W;
+    return !fm && cells > few && (qx0 <= -lim || qz0 <= -lim || qx1 >= lim || qz1 >= lim);
 }
 long long ow_tiles(int nx, int nz) { return (long long)mg_parts(nx, OT_W) * mg_parts(nz, OT_W); }
 
@@ -1065,7 +1064,9 @@ int launch_ow_block_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const
     K.step = step;
     K.y = y;
     K.xyz = xyz;
-    return !xyz && step <= 4 ? grid_run(W, OT_BLOCK, K, scratch, st) : sparse_run(W, K, scratch, st);
+    const bool far = ow_beyond(W.fmode != 0, OT_FEW_BLOCKS, x0 >> 2, z0 >> 2, (x0 + (long long)(nx - 1) * step) >> 2,
+                               (z0 + (long long)(nz - 1) * step) >> 2, (long long)nx * nz);
+    return !xyz && step <= 4 && !far ? grid_run(W, OT_BLOCK, K, scratch, st) : sparse_run(W, K, scratch, st);
 }
 
 }  // namespace mg

@@ -214,11 +214,12 @@ MCGEN_API int mcgen_gb300_plan_new(const McGb300Request *reqs, int n, int tie_ru
      * dimension and branch; mixing them thrashes the instruction cache) and the light tiles come last */
     std::vector<int> order((size_t)n);
     for (int i = 0; i < n; i++) order[(size_t)i] = i;
-    std::vector<int> wgroup(worlds.size());
-    for (size_t w = 0; w < worlds.size(); w++) wgroup[w] = mg::batch_group(worlds[w]->desc, tie_rule);
+    std::vector<int> wgroup(worlds.size()), group((size_t)n);
+    for (size_t w = 0; w < worlds.size(); w++) wgroup[w] = mg::batch_world_group(worlds[w]->desc, tie_rule);
     long long ow_cells[2] = {0, 0}; /* of the Overworld groups: the cells the tile kernels may leave open */
     for (int i = 0; i < n; i++) {
-        const int g = wgroup[(size_t)wof[(size_t)i]];
+        const McGb300Request &r = reqs[i];
+        const int g = group[(size_t)i] = mg::batch_group(wgroup[(size_t)wof[(size_t)i]], r.qx0, r.qz0, r.nx, r.nz);
         if (g != BATCH_REST) ow_cells[g] += p->cells[(size_t)i];
     }
     p->tie = tie_rule;
@@ -227,7 +228,7 @@ MCGEN_API int mcgen_gb300_plan_new(const McGb300Request *reqs, int n, int tie_ru
     for (int i = 0; i < n; i++) {
         const int wi = wof[(size_t)i];
         const MgWorldDesc &W = worlds[(size_t)wi]->desc;
-        key[(size_t)i] = ((wgroup[(size_t)wi] * 3 + W.dim) * 2 + (W.fmode ? 1 : 0)) * (int)(worlds.size() + 1) + wi;
+        key[(size_t)i] = ((group[(size_t)i] * 3 + W.dim) * 2 + (W.fmode ? 1 : 0)) * (int)(worlds.size() + 1) + wi;
     }
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return key[(size_t)a] < key[(size_t)b]; });
     for (int s = 0; s < BATCH_SHAPES; s++) {
@@ -239,7 +240,7 @@ MCGEN_API int mcgen_gb300_plan_new(const McGb300Request *reqs, int n, int tie_ru
             b.state = slot[(size_t)i];
             b.qx0 = r.qx0; b.qz0 = r.qz0; b.nx = r.nx; b.nz = r.nz; b.qy = r.qy;
             b.tie = worlds[(size_t)wi]->desc.dim == MG_END ? MG_TIE_ENGINE : tie_rule;
-            const int g = wgroup[(size_t)wi];
+            const int g = group[(size_t)i];
             b.tile0 = p->groups[s].tiles[g];
             b.out_off = p->out_off[(size_t)i];
             p->groups[s].tiles[g] += mg::batch_tiles(g, worlds[(size_t)wi]->desc, r.qx0, r.qz0, r.nx, r.nz, s);

@@ -248,10 +248,13 @@ int launch_batch(McGb300Server *s, Batch &b) {
     if (b.tickets.empty()) return 0;
     /* processing order: the batch's groups, then by code path, heaviest first (as in a plan), then the tile numbering */
     std::vector<int> wgroup;
-    for (auto *w : worlds) wgroup.push_back(mg::batch_group(w->desc, MG_TIE_ENGINE));
+    for (auto *w : worlds) wgroup.push_back(mg::batch_world_group(w->desc, MG_TIE_ENGINE));
+    auto group = [&](const MgBatchReq &r) {
+        return mg::batch_group(wgroup[(size_t)r.world], r.qx0, r.qz0, r.nx, r.nz);
+    };
     auto path = [&](const MgBatchReq &r) {
         const MgWorldDesc &d = worlds[(size_t)r.world]->desc;
-        return (wgroup[(size_t)r.world] * 3 + d.dim) * 2 + (d.fmode ? 1 : 0);
+        return (group(r) * 3 + d.dim) * 2 + (d.fmode ? 1 : 0);
     };
     std::stable_sort(reqs.begin(), reqs.end(), [&](const MgBatchReq &x, const MgBatchReq &y) {
         const int px = path(x), py = path(y);
@@ -259,7 +262,7 @@ int launch_batch(McGb300Server *s, Batch &b) {
     });
     mg::BatchGroups groups = {};
     for (auto &r : reqs) {
-        const int g = wgroup[(size_t)r.world];
+        const int g = group(r);
         r.tile0 = groups.tiles[g];
         groups.tiles[g] += mg::batch_tiles(g, worlds[(size_t)r.world]->desc, r.qx0, r.qz0, r.nx, r.nz, kServeShape);
         groups.n[g]++;
@@ -290,7 +293,7 @@ int launch_batch(McGb300Server *s, Batch &b) {
     if (!e && !b.d_counter) e = cudaMalloc(&b.d_counter, BATCH_COUNTERS * sizeof(unsigned long long));
     long long ow_cells[2] = {0, 0}, open_cap[2]; /* of the Overworld groups: the cells the tile kernels may leave open */
     for (const auto &r : reqs)
-        if (wgroup[(size_t)r.world] != BATCH_REST) ow_cells[wgroup[(size_t)r.world]] += (long long)r.nx * r.nz;
+        if (const int g = group(r); g != BATCH_REST) ow_cells[g] += (long long)r.nx * r.nz;
     mg::batch_open_cap(ow_cells, MG_TIE_ENGINE, open_cap);
     long long nopen = open_cap[0] + open_cap[1];
     if (!e && nopen > 0) { /* without the record open cells are evaluated in place */
