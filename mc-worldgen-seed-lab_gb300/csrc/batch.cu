@@ -3,7 +3,8 @@
  *
  * A request is (world: version + dimension + preset, seed, quart region qx0..qx0+nx-1 x qz0..qz0+nz-1 at
  * quart y, tie rule).  The host splits every request into tiles -- 32 x 32 cells for the Nether (nethertile.cuh), equal parts of
- * up to 24 x 24 chunks for the End (endtile.cuh), 128 cells (8 x 16) for worlds without a tile form --
+ * up to 24 x 24 chunks for the End (endtile.cuh), 128 cells (8 x 16) for what has no tile form (worlds with other noises than the
+ * game's; the double branch's Overworld beyond the tables' coordinates) --
  * and numbers them.  k_batch runs as many CTAs as fit for the whole batch; each CTA takes the next tile
  * from a device counter (the work queue), finds its request among the requests' first-tile numbers, stages
  * that request's seed lattices in shared memory when they differ from the previous tile's, and computes the

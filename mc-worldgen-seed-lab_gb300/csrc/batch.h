@@ -25,7 +25,7 @@ typedef struct {
 
 #define BATCH_SHAPES 4
 /* The requests of a batch come in three groups, each contiguous and with a tile numbering of its own: Overworld
- * requests by branch (owtile.cu: 16 x 16-cell tiles), then everything else (batch.cu). */
+ * requests that the tile kernels take by branch (owtile.cu: 16 x 16-cell tiles), then everything else (batch.cu). */
 enum { BATCH_OW_D = 0, BATCH_OW_F = 1, BATCH_REST = 2, BATCH_GROUPS = 3 };
 namespace mg {
 struct BatchGroups {

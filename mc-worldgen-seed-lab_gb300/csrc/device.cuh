@@ -1362,8 +1362,8 @@ __device__ __forceinline__ bool rt_warp(const MgTreeNode *__restrict__ T, const 
     return true;
 }
 /* tree_search (no candidate) for 32 unrelated targets, called by all 32 lanes (inactive ones get -1): one after another, each
- * by the whole warp; tied: whether a second leaf is as near.  A lane alone visits 120 to 200 nodes, and lanes with unrelated targets diverge at most of them (2,000
- * instructions per target); the warp looks at 32 boxes at once (10 steps of 40). */
+ * by the whole warp; tied: whether a second leaf is as near.  A lane alone visits 120 to 200 nodes, and lanes with unrelated
+ * targets diverge at most of them (2,000 instructions per target); the warp looks at 32 boxes at once (10 steps of 40). */
 __device__ __forceinline__ int tree_search_lanes(const MgTreeNode *__restrict__ T, const MgWorldDesc &W, const int32_t *t, bool active,
                                                  bool *tied = nullptr) {
     const unsigned FULL = 0xFFFFFFFFu;

@@ -303,9 +303,9 @@ __device__ __forceinline__ V search_sum(const MgNoise &N, const V *val, int firs
 }
 
 /* ---- the double branch's many seeds x points in the Overworld tiles' fixed point (owtile.cuh): the double evaluation's 72 FP64
- * operations an octave kept the FP64 pipe 73 % busy (1,501 seeds x 33 points: 424 us; this form 232).  A sample whose targets the
- * error bounds leave open (2 %) is kept in its seed's queue and evaluated in double at the end, eight per seed at a time, from the
- * lattices that are still there.  Writes the six targets of every sample. */
+ * operations an octave kept the FP64 pipe 73 % busy (1,501 seeds x 33 points: 383 us; this form 158, 221 with the queued samples
+ * evaluated one at a time).  A sample whose targets the error bounds leave open (2 %) is kept in its seed's queue and evaluated in
+ * double at the end, eight per seed at a time, from the lattices that are still there.  Writes the six targets of every sample. */
 #define TQ_CAP 64 /* points whose values are kept until their targets are formed, by all threads at once */
 struct TargetSmem {
     uint32_t perm[64][FPS];

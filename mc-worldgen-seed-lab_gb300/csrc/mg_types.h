@@ -151,8 +151,9 @@ typedef struct __attribute__((aligned(16))) {
     uint8_t p[256];
 } MgLattice;
 
-/* A double-branch Overworld cell of the tile kernel with a quantised target its bounds left open: finished by the exact
- * evaluation of a later launch. */
+/* An Overworld cell that the tile kernels leave to the exact evaluation of a later launch: in the double branch one with a
+ * quantised target that its bounds leave open, or beyond the tables' coordinates; under the chunk-cell rule, in either branch, a
+ * tied one. */
 typedef struct {
     int32_t req;  /* request, counted from the batch's first */
     int32_t cell; /* row-major cell of the request */

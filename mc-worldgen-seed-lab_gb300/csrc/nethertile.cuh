@@ -2,7 +2,7 @@
  *
  * The two noises' octaves (8; inputs of at most 1/16 per quart) see the integer quart grid, so, as in the Overworld tiles' shift
  * noises (owtile.cuh), their splits are functions of a column or a row alone and a tile touches a few nodes of each octave's
- * plane: the tables are 64 splits and 4 to 25 nodes per octave for 1,024 cells.  A cell then has 8 octaves from 4 nodes each (the
+ * plane: the tables are 64 splits and 9 or 16 nodes per octave for 1,024 cells.  A cell then has 8 octaves from 4 nodes each (the
  * nodes are kept in registers while a warp's rows stay within them) and 5 leaves, the nearest of which it finds directly.
  * The double branch evaluates in the Overworld tiles' fixed point (MgNoise::tile_eq); a cell whose value may have either of two
  * targets is settled when both give the same biome, the rest are evaluated exactly.  4,096 requests of 64 x 64 cells: the per-cell
@@ -17,7 +17,7 @@ namespace mg {
 #define NT_W 32     /* tile width and height in cells */
 #define NT_OCT 8    /* octaves (lattices) */
 #define NT_LEAVES 8
-#define NT_NODES 200 /* NT_OCT x 25: 5 per axis at 1/16 per quart */
+#define NT_NODES 200 /* NT_OCT x 25; at most 16 an octave are used (nether_nodes: 4 per axis at 1/16 per quart) */
 #define NT_ROWS 4   /* rows of a thread evaluated together */
 
 /* a leaf: temperature and humidity bounds, squared distance in the other dimensions (their targets are 0) */

@@ -136,7 +136,7 @@ __device__ __forceinline__ void ot_leave_open(const OtWork &K, const MgWorldDesc
     else ot_exact<FM, MODE>(K, W, T, tree, qx, qy, qz, o);
 }
 
-/* Float branch (26.3 on), bit for bit the per-cell form's operations.  Bound by instruction issue (66 % of peak; the octaves'
+/* Float branch (26.3 on), bit for bit the per-cell form's operations.  Bound by instruction issue (69 % of peak; the octaves'
  * separately rounded lerps, the splits' mantissa shifts, the tree scan).  64 registers and 55 KB of shared memory: 4 CTAs,
  * 32 warps per SM.  The uneven batch's 70.8 M float-branch cells: 47.6 ms in the per-cell form, 34.2 ms here (8 of it the tree). */
 template <int MODE>
@@ -712,12 +712,13 @@ __global__ void __launch_bounds__(OT_NT, 4) k_ow_d(const __grid_constant__ OtWor
 }
 
 /* ============================================================================ sparse block maps, long point lists
- * Blocks more than 4 apart or anywhere: neighbouring cells share too few nodes for a tile's tables, so each is evaluated by its lane: the float
- * branch by the per-cell form, the double branch in the tiles' fixed point with its octaves' edges built on the way (per cell in
- * double, its shift noises took 864 FP64 operations).  Tied cells and open targets are left to k_ow_open like the tiles'.  The
- * lattices, spline and fixed coordinates' parts are in shared memory; warps take 8 x 4 cells, whose tree search they share up to 16
- * blocks apart (a box of 4 x 8 chunks of terrain) and do one by one beyond and for points.  256 x 256 blocks, spacing 16: 26.1 531 -> 205 us, 26.3 379
- * -> 237 us; spacing 37: 578 -> 313, 552 -> 229 (its search shared: 324 and 288). */
+ * Blocks more than 4 apart or anywhere: neighbouring cells share too few nodes for a tile's tables, so each is evaluated by its
+ * lane: the float branch by the per-cell form, the double branch in the tiles' fixed point with its octaves' edges built on the way
+ * (ot_cell_d; per cell in double, its shift noises took 864 FP64 operations), beyond the tables' coordinates by the per-cell form
+ * too.  Tied cells and open targets are left to k_ow_open like the tiles'.  The lattices, spline and fixed coordinates' parts are in
+ * shared memory; warps take 8 x 4 cells, whose tree search they share up to 16 blocks apart (a box of 4 x 8 chunks of terrain) and
+ * do one by one beyond and for points.  256 x 256 blocks, spacing 16: 26.1 531 -> 205 us, 26.3 379 -> 237 us; spacing 37: 578 ->
+ * 313, 552 -> 229 (its search shared: 324 and 288). */
 struct OtSparse {
     WcStage st;
     OtFix fix[MG_MAX_TABLES], fz[2 * OT_MAXLEV]; /* of the y plane; the shift's z plane */
@@ -1026,7 +1027,7 @@ int launch_ow_quart_grid(const MgWorldDesc &W, const MgWorldDesc *d_world, const
     K.one.qy = qy;
     return grid_run(W, rec ? OT_CHAIN : OT_ENGINE, K, scratch, st);
 }
-/* blocks more than 4 apart */
+/* blocks more than 4 apart, points, double-branch maps beyond the tables' coordinates */
 static int sparse_run(const MgWorldDesc &W, OtWork &K, void *scratch, cudaStream_t st) {
     const bool fm = W.fmode != 0;
     K.ntiles = K.xyz ? mg_parts(K.one.nx, 128) : (long long)mg_parts(K.one.nx, 16) * mg_parts(K.one.nz, 8);

@@ -2,10 +2,11 @@
  *
  * A plan freezes a list of requests: it uploads the distinct worlds (descriptions and R-tree pointers),
  * assigns every distinct (world, seed) a slot in a lattice pool, numbers the tiles of every request
- * (batch.cu), and lays the outputs out back to back.  Running it enqueues the per-seed setup launches (one
- * per dimension present) and the persistent k_batch launch.  The first run on a stream captures those
- * launches into a CUDA graph on a private stream and later runs replay it; the tile shape is chosen by
- * timing the four shapes on the plan itself (mcgen_gb300_plan_autotune).
+ * (batch.cu, owtile.cu), and lays the outputs out back to back.  Running it enqueues the per-seed setup launches (one
+ * per dimension present), a persistent launch per group of requests that is present (batch.h: the Overworld's tile kernels by
+ * branch, then k_batch) and the launches of the cells that the tiles left open.  The first run on a stream captures those
+ * launches into a CUDA graph on a private stream and later runs replay it; the shape, k_batch's register budget, is chosen by
+ * timing the four on the plan itself (mcgen_gb300_plan_autotune).
  */
 #include <cuda_runtime.h>
 #include <string.h>
@@ -209,8 +210,8 @@ MCGEN_API int mcgen_gb300_plan_new(const McGb300Request *reqs, int n, int tie_ru
         off += p->cells[(size_t)i];
     }
     p->out_bytes = off;
-    /* processing order: the batch's groups (batch.h), within the rest grouped by world, heaviest code path first (Overworld double branch, then
-     * float, Nether, End), so that the CTAs resident at any time run the same code (the kernel holds every
+    /* processing order: the batch's groups (batch.h), within the rest grouped by world, heaviest code path first (Overworld
+     * double branch, then float, Nether, End), so that the CTAs resident at any time run the same code (k_batch holds every
      * dimension and branch; mixing them thrashes the instruction cache) and the light tiles come last */
     std::vector<int> order((size_t)n);
     for (int i = 0; i < n; i++) order[(size_t)i] = i;

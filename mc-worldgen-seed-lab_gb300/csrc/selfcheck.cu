@@ -435,7 +435,8 @@ __global__ void k_check_tree(const MgTreeNode *__restrict__ T, long long n, uint
 /* The warp-shared search (tree_search_warp) against the 64-bit stack search on targets of the kind a warp of
  * neighbouring cells has: per warp a centre in the tables' range and per lane a spread of 50, 400, 2,000 or
  * 6,000 around it; about one lane in eight inactive; in one warp in sixteen one lane far outside the packed
- * range (the warp's fallback); with what NEAR says of the neighbouring targets, and rt_point.  Case i is lane i % 32 of warp case i / 32.  out[0]: differing leaves. */
+ * range (the warp's fallback); with what NEAR says of the neighbouring targets, and rt_point.  Case i is lane i % 32 of
+ * warp case i / 32.  out[0]: differing leaves. */
 __global__ void __launch_bounds__(128) k_check_tree_warp(const __grid_constant__ MgWorldDesc W, const MgTreeNode *__restrict__ T,
                                                          long long n, uint64_t seed, unsigned long long *out) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;

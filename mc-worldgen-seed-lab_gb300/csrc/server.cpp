@@ -4,9 +4,9 @@
  * worker thread admits every pending request into the next batch as soon as one of the server's streams
  * is free (up to `max_inflight` batches run at once, so a batch that forms while another is on the GPU
  * starts right away and the two overlap on the device), makes sure each request's seed lattices are
- * resident in the device noise-state cache, enqueues the setup launches for the cache misses and one
- * persistent k_batch launch, and copies the ids back.  When a batch's event completes the worker hands
- * every request its ids and wakes its waiters.
+ * resident in the device noise-state cache, enqueues the setup launches for the cache misses and the batch's
+ * launches (one per group of requests, then the cells left open), and copies the ids back.  When a batch's event
+ * completes the worker hands every request its ids and wakes its waiters.
  *
  * Noise-state cache: per dimension a pool of fixed-size slots (46 lattices of 352 B for the Overworld, 8 for
  * the Nether, 1 for the End) carved from one HBM budget, keyed by (world identity, seed) -- the world's
@@ -16,7 +16,8 @@
  * Failures: a batch that fails before its work is queued (an allocation, a copy or a launch) takes back the
  * cache entries it had created, so no later request can hit lattices that were never built, and fails its
  * own requests; an allocation failure leaves the server usable, any other error stops it: every pending
- * and later request then fails with that error.  A pending request holds its world, so mcgen_world_free
+ * and later request then fails with that error.  (Without memory for its record of open cells alone, a batch
+ * evaluates them in place.)  A pending request holds its world, so mcgen_world_free
  * during serving defers the free until the request completes.
  */
 #include <cuda_runtime.h>
@@ -79,7 +80,7 @@ struct Batch {
     const MgTreeNode **d_trees = nullptr;
     uint8_t *d_out = nullptr; size_t cap_out = 0;
     uint8_t *h_out = nullptr; size_t cap_hout = 0;
-    unsigned long long *d_counter = nullptr; /* tiles taken, cells recorded for the exact pass */
+    unsigned long long *d_counter = nullptr; /* BATCH_COUNTERS */
     MgOpenCell *d_open = nullptr; size_t cap_open = 0;
     std::vector<long long> out_off;
 };
@@ -104,8 +105,7 @@ struct McGb300Server {
 
 namespace {
 
-/* tile shape of the served batches: 8 x 16 cells at 6 resident CTAs per SM, the shape the autotuner picks
- * for the uneven mixed batch */
+/* shape of the served batches: k_batch at 6 resident CTAs per SM */
 const int kServeShape = 2;
 
 int crc(cudaError_t e) { return e == cudaSuccess ? 0 : e == cudaErrorMemoryAllocation ? MCGEN_E_NOMEM : MCGEN_E_INTERNAL; }
